@@ -116,6 +116,7 @@ class Arena {
     used_ += bytes;
     return p;
   }
+  bool fixed() const { return fixed_; }
   size_t used() const { return used_; }
   size_t capacity() const { return cap_; }
   static size_t bytes_for(size_t count, size_t elem) { return (count * elem + 255) & ~size_t(255); }
@@ -145,6 +146,8 @@ struct Tree {
   double2 *coef = nullptr;    // ncell * nterms, FP64 Laurent coefficients
   double2 *mac = nullptr;     // plain: per cell, the squared distances below / above which
                               // the opening test surely descends / accepts (k_mac_bounds)
+  long long *fix = nullptr;   // plain: the coefficients in fixed point (fix64.cuh), 2 per entry, strided as coef
+                              // (coef's own memory in arenas of a fixed size)
   float4 *cf32 = nullptr;     // plain: per cell, the centre as FP32 pairs (cx hi, cx lo, cy hi, cy lo)
   float2 *macf = nullptr;     // plain: mac rounded outwards to FP32 (-1 / +inf where that is unsafe)
   RootBox *root = nullptr;    // device
@@ -211,8 +214,9 @@ int build_tree(Workspace &ws, int n, const double *d_xy, const double *d_cir, co
 size_t build_blob_bytes(int n, int nsets);
 size_t build_tmp_bytes(int n, int nsets);
 // Bytes build_tree reserves in ws.cell_arena for a tree of ncell cells and
-// nleaf leaves with nterms coefficients per cell.
-size_t build_cell_bytes(long long ncell, long long nleaf, int nterms);
+// nleaf leaves with nterms coefficients per cell (in an arena of a fixed
+// size the plain form's fixed-point coefficients replace the FP64 ones).
+size_t build_cell_bytes(long long ncell, long long nleaf, int nterms, bool fixed_arena);
 
 // Keys of arbitrary points against an existing root box, then sorted:
 // order[i] = index of the i-th target in key order.

@@ -7,30 +7,30 @@
 //  k_m2m       one warp per internal cell of one level, deepest level first;
 //              children in quadrant order 3,2,1,0 (fmm.c:41-56); the
 //              level-1 -> root shift is skipped as in the reference.
-//  k_eval      one warp per 32 consecutive targets (tree order, so the warp's
-//              targets are neighbours).  The warp walks the UNION of its
-//              lanes' traversals with a shared LIFO of (cell, lane mask):
-//              restricted to one lane, the visit order is that lane's own
-//              LIFO order in fmm.c:90-112, so every lane accumulates M2S and
-//              direct terms in the reference's order.  The opening test uses
-//              round-to-nearest FP64 operations without contraction
-//              (r = sqrt(dx*dx + dy*dy); region > theta*r), so each lane
-//              takes exactly the reference's branch.  M2S (fmm.c:60-67) is
-//              evaluated by Horner in w = 1/(z - zc), from a per-lane queue
-//              of accepted cells that the warp empties in rounds (all lanes
-//              busy); P2P is fmm.c:121-142.
+//  k_eval      one warp per 8 consecutive targets (tree order, so the warp's
+//              targets are neighbours), four lanes per target.  The warp walks
+//              the UNION of its targets' traversals with a shared LIFO of
+//              (cell, lane mask): restricted to one target, the visit order
+//              is that target's own LIFO order in fmm.c:90-112.  The opening
+//              test uses round-to-nearest FP64 operations without contraction
+//              (r = sqrt(dx*dx + dy*dy); region > theta*r), so each target
+//              takes exactly the reference's branch.  The four lanes of a
+//              target share its accepted cells (M2S, fmm.c:60-67, by Horner in
+//              w = 1/(z - zc)) and its direct pairs (fmm.c:121-142); their
+//              four partial sums are added in a fixed order at the end.  Both
+//              in 64-bit fixed point (fix64.cuh): FP64 runs at 1/64 of the
+//              FP32 rate here.
+#include <mutex>
+
 #include "dev_common.cuh"
+#include "fix64.cuh"
 
 namespace t2d {
 namespace {
 
 // 1/x for a positive normal x: the SFU's approximate reciprocal refined by
 // two Newton-Raphson steps for f(y) = 1/y - x, y <- y + y (1 - x y), each
-// with the residual 1 - x y formed by one FMA.  Every step squares the
-// relative error, so the ~2^-20 seed ends within an ulp or so of the
-// correctly rounded 1/x, which is all the 1e-12 bar needs; it replaces the
-// IEEE division of the pair and M2S terms (the FP64 pipe is this kernel's
-// bound).
+// with the residual 1 - x y formed by one FMA.
 __device__ __forceinline__ double rcp_nr(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
@@ -48,9 +48,11 @@ __device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 c) {
 }
 
 __constant__ double c_binom[kMaxTerms][kMaxTerms];
+// e^-n and e^-(j / 2048) in units of 2^-62 (fix64.cuh)
+__device__ uint64_t g_exp_int[fix::kExpInts];
+__device__ uint64_t g_exp_frac[fix::kExpFracs];
 
 constexpr double kPi = 3.14159265358979323846;
-constexpr double kInv2Pi = 0.15915494309189533577;  // 1 / (2 pi), rounded
 
 __global__ void __launch_bounds__(256) k_s2m(Tree t, int nt) {
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -108,9 +110,12 @@ __global__ void __launch_bounds__(256) k_m2m(Tree t, int nt, int lev) {
 
 constexpr int kEvalWarps = 4;
 constexpr int kStackCap = 160;
-constexpr int kQueue = 32;  // deferred M2S cells per lane
+constexpr int kShare = 4;                // lanes per target (one per child of a cell)
+constexpr int kEvalTargets = 32 / kShare;  // targets per warp
+constexpr unsigned kEachTarget = 0x11111111u;  // the first lane of each target
+constexpr int kQueue = 64;  // deferred M2S cells per target
+static_assert(kShare == 4 && kEvalTargets * kShare == 32, "the masks below are for four lanes per target");
 static_assert((kQueue & (kQueue - 1)) == 0, "the M2S queues are rings indexed by a mask");
-constexpr int kLeafQueue = 16;  // deferred direct (P2P) leaves per lane
 
 struct EvalArgs {
   Tree t;
@@ -121,15 +126,37 @@ struct EvalArgs {
   const int *out_idx;
   double *uv;
   DevStatus *st;
+  int k0;        // first term of the sums in FP32 pairs (fix::first_pair_term)
+  bool keep64;   // t.coef still holds the FP64 coefficients (not converted in place)
+  fix::One one;
 };
 
-__global__ void __launch_bounds__(kEvalWarps * 32) k_eval(EvalArgs a) {
+// The multipole sums: in FP64 (theta above kFixTheta), or in fixed point with |w| 2^es < 1 or < 1/2.
+enum EvalForm { kFormFp64, kFormFull, kFormHalf };
+
+// Bound: instruction dispatch.  Integer instructions take two dispatch cycles
+// each (ALU and multiplier pipes alike; FP32 one), and on GB300 the kernel
+// spends, at 1M Lamb-Oseen blobs, 2.4 ms in the traversal, 8.0 ms in the 250
+// M2S and 8.8 ms (some of it overlapped) in the 500 pairs per target: 18.2 ms
+// against 67.5 with both in FP64, whose pipe was 89% busy; 0.30 against
+// 0.90 ms at 20,000 uniform blobs.  Four lanes per target, not one: 8
+// targets' traversals overlap more than 32 targets', the four children of a
+// cell are tested at once, a leaf's pairs need no queue, and a small set
+// fills four times the warps (20,000 blobs: 1.43 -> 1.07 ms per solve).
+// 80 registers, 24 warps per SM: 64 registers spill (24.0 against 21.4 ms
+// per solve), 2 or 8 warps per block are slower (23.6, 22.2).
+template <int kForm>
+__global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
   __shared__ int s_cell[kEvalWarps][kStackCap];
   __shared__ unsigned s_mask[kEvalWarps][kStackCap];
-  __shared__ int s_queue[kEvalWarps][kQueue][32];
-  __shared__ int s_leaves[kEvalWarps][kLeafQueue][32];
+  __shared__ int s_queue[kEvalWarps][kEvalTargets][kQueue];
+  __shared__ uint64_t s_exp_int[fix::kExpInts], s_exp_frac[fix::kExpFracs];
+  for (int j = threadIdx.x; j < fix::kExpFracs; j += kEvalWarps * 32) s_exp_frac[j] = g_exp_frac[j];
+  for (int j = threadIdx.x; j < fix::kExpInts; j += kEvalWarps * 32) s_exp_int[j] = g_exp_int[j];
+  __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long i = ((long)blockIdx.x * kEvalWarps + warp) * 32 + lane;
+  const int sub = lane & (kShare - 1), tgt = lane / kShare;
+  const long i = ((long)blockIdx.x * kEvalWarps + warp) * kEvalTargets + tgt;
   const bool valid = i < a.ntgt;
   const unsigned vmask = __ballot_sync(0xffffffffu, valid);
   if (vmask == 0) return;
@@ -141,116 +168,71 @@ __global__ void __launch_bounds__(kEvalWarps * 32) k_eval(EvalArgs a) {
   const float xh = __double2float_rn(x), yh = __double2float_rn(y);
   const float xl = __double2float_rn(x - (double)xh), yl = __double2float_rn(y - (double)yh);
   const float sxy = __fadd_rn(fabsf(xh), fabsf(yh));
-  double2 phi = make_double2(0.0, 0.0);
-  double ud0 = 0.0, ud1 = 0.0;
-  unsigned long long n_m2s = 0, n_pairs = 0;
+  fix::Sum2 far, near;                          // this lane's share of the target's sums
+  double2 far64 = make_double2(0.0, 0.0);       // kFormFp64, and targets far outside the blobs
+  unsigned n_m2s = 0;
+  unsigned long long n_pairs = 0;
   bool overflow = false;
 
-  // The lanes accept cells at different depths, so an M2S evaluated where
-  // it is accepted runs with the warp's other lanes idle.  Each lane
-  // instead queues its accepted cells (s_queue[warp][k][lane], in the order
-  // it accepts them) and the warp evaluates the queues together, one entry
-  // per lane per round, when a lane's queue could overflow and at the end.
-  // A lane's M2S terms still reach phi in its own acceptance order, each
-  // with the same operations (dx, dy, d2 formed again from the cell's
-  // centre, bit for bit); the direct terms are deferred too (below).
-  // The queues are rings (head qh, count nq).  A flush when some lane's
-  // queue could overflow evaluates only as many rounds as every lane can
-  // fill, or as the fullest lane needs to make room for four entries, if
+  // The targets accept cells at different depths, so an M2S evaluated where
+  // it is accepted runs with the warp's other lanes idle.  Each target
+  // instead queues its accepted cells (a ring: head qh, count nq, the same in
+  // its four lanes) and the warp evaluates the queues together, four entries
+  // per target and round.  Entry k of a target (counted over the whole
+  // traversal) is lane k mod 4's, so the partial sums do not depend on when
+  // the queues are emptied, nor on the warp's other targets.  A flush when
+  // some queue could overflow evaluates only as many rounds as every target
+  // can fill, or as the fullest one needs to make room for four entries, if
   // that is more; the end of the traversal empties them all.
-  int qh = 0, nq = 0;
+  unsigned qh = 0;
+  int nq = 0;
   auto flush = [&](bool all) {
     int hi = nq, lo = nq;
-    for (int o = 16; o; o >>= 1) {
+    for (int o = 16; o >= kShare; o >>= 1) {
       hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
       lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
     }
-    const int rounds = all ? hi : max(lo, hi - (kQueue - 4));
+    const int rounds = (all ? hi + kShare - 1 : max(lo, hi - (kQueue - kShare) + kShare - 1)) / kShare;
+    const int first = (int)((unsigned)(sub - (int)qh) & (kShare - 1));
+    fix::settle(far);  // at most kQueue / kShare terms follow
     for (int r = 0; r < rounds; r++) {
-      if (r < nq) {
+      const int k = first + r * kShare;
+      if (k < nq) {
         // M2S, fmm.c:60-67: sum_{k<nt-1} a_k w^{k+1}, w = 1/(z - zc)
-        const int cc = s_queue[warp][(qh + r) & (kQueue - 1)][lane];
+        const int cc = s_queue[warp][tgt][(qh + k) & (kQueue - 1)];
         const double dx = __dsub_rn(x, t.cx[cc]);
         const double dy = __dsub_rn(y, t.cy[cc]);
-        const double d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
-        const double inv = rcp_nr(d2);
-        const double2 w = make_double2(__dmul_rn(dx, inv), -__dmul_rn(dy, inv));
-        const double2 *cf = t.coef + (size_t)cc * nt;
-        // Horner, each step acc <- acc w + a_k as two FMAs per component
-        // (four per term against six for a product and a sum), and the
-        // last product added into phi the same way
-        double2 acc = cf[nt - 2];
-        for (int k = nt - 3; k >= 0; k--) acc = cfma(acc, w, cf[k]);
-        phi = cfma(acc, w, phi);
-      }
-    }
-    const int done = min(rounds, nq);
-    qh = (qh + done) & (kQueue - 1);
-    nq -= done;
-  };
-
-  // The direct sums are deferred the same way: a leaf reached by some of
-  // the warp's lanes would keep the others idle for its whole pair loop,
-  // and on this GPU an FP64 warp instruction takes the pipe for its full
-  // width whatever the lanes.  Each lane queues its leaves
-  // (s_leaves[warp][k][lane]) and the warp walks the queues together, one
-  // pair per lane per step, each lane through its own leaves in its own
-  // order.  A lane's pairs reach ax/ay and its leaf sums reach ud0/ud1 in
-  // the order and with the operations of an immediate evaluation, so the
-  // results are the same bit for bit.
-  int nl = 0;
-  auto flush_leaves = [&]() {
-    int q = 0, j = 0, e = 0;
-    double ax = 0.0, ay = 0.0;
-    if (nl > 0) {
-      const int c0 = s_leaves[warp][0][lane];
-      j = t.begin[c0];
-      e = t.end[c0];
-    }
-    // closes the leaves whose pairs are done (empty ones too) and opens the
-    // next: the reference adds 0.5 ax / pi per leaf (fmm.c:140-141); a
-    // product by 1/(2 pi) instead of the FP64 division (an ulp apart)
-    auto settle = [&]() {
-      while (q < nl && j >= e) {
-        ud0 = __dadd_rn(ud0, __dmul_rn(ax, kInv2Pi));
-        ud1 = __dadd_rn(ud1, __dmul_rn(ay, kInv2Pi));
-        ax = 0.0;
-        ay = 0.0;
-        if (++q < nl) {
-          const int cq = s_leaves[warp][q][lane];
-          j = t.begin[cq];
-          e = t.end[cq];
+        bool done = false;
+        if constexpr (kForm != kFormFp64) {
+          const longlong2 *cf = reinterpret_cast<const longlong2 *>(t.fix) + (size_t)cc * nt;
+          const longlong2 sc = __ldg(cf + (nt - 1));
+          done = fix::add_multipole<kForm == kFormHalf>(
+              far, dx, dy, fix::CellScale{(int)sc.x, (int)sc.y}, nt - 1, a.k0,
+              [&](int k) {
+                const longlong2 v = __ldg(cf + k);
+                return fix::Coef{v.x, v.y};
+              },
+              [&](int k) {
+                const float4 v = __ldg(reinterpret_cast<const float4 *>(cf + k));
+                return fix::PairCoef{v.x, v.y, v.z, v.w};
+              },
+              a.keep64, a.one);
+        }
+        if (!done) {
+          const double d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
+          const double inv = rcp_nr(d2);
+          const double2 w = make_double2(__dmul_rn(dx, inv), -__dmul_rn(dy, inv));
+          const double2 *cf = t.coef + (size_t)cc * nt;
+          // Horner, each step acc <- acc w + a_k as two FMAs per component
+          double2 acc = cf[nt - 2];
+          for (int k = nt - 3; k >= 0; k--) acc = cfma(acc, w, cf[k]);
+          far64 = cfma(acc, w, far64);
         }
       }
-    };
-    settle();
-    while (__any_sync(0xffffffffu, q < nl)) {
-      if (q < nl) {
-        // direct_evaluate, fmm.c:121-142
-        const double rx = __dsub_rn(x, t.x[j]);
-        const double ry = __dsub_rn(y, t.y[j]);
-        // The reference forms r = sqrt(r2), (r/sigma)^2 and 1/(r*r); here
-        // r2 and r2/sigma^2 (with 1/sigma^2 precomputed per blob) give the
-        // same quantities within an ulp or two and save the square root
-        // and a division per pair.  r > 1e-10 <=> r2 > 1e-20.
-        const double r2 = __dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry));
-        if (r2 > 1.0e-20) {
-          const double rv2 = rcp_nr(r2);
-          const double x2 = __dmul_rn(r2, t.icor2[j]);
-          // 1 - exp(-x2) rounds to exactly 1.0 once exp(-x2) < 2^-54
-          // (x2 > 37.4); the shortcut keeps the result bit-identical.
-          const double e1 = x2 > 40.0 ? 1.0 : 1.0 - exp(-x2);
-          // G (1 - e) / r^2 once, then one FMA per component
-          const double f = __dmul_rn(__dmul_rn(t.cir[j], e1), rv2);
-          ax = __fma_rn(-f, ry, ax);
-          ay = __fma_rn(f, rx, ay);
-        }
-        n_pairs++;
-        j++;
-        settle();
-      }
     }
-    nl = 0;
+    const int out = min(rounds * kShare, nq);
+    qh += (unsigned)out;
+    nq -= out;
   };
 
   int top = 0;
@@ -266,102 +248,146 @@ __global__ void __launch_bounds__(kEvalWarps * 32) k_eval(EvalArgs a) {
     top--;
     const bool act = (m >> lane) & 1u;
     if (t.leaf[c]) {
-      if (__any_sync(0xffffffffu, nl == kLeafQueue)) flush_leaves();
-      if (act) s_leaves[warp][nl++][lane] = c;
-    } else {
-      // a cell's four children can add four entries to a lane's queue
-      if (__any_sync(0xffffffffu, nq > kQueue - 4)) flush(false);
-      const int4 ch = reinterpret_cast<const int4 *>(t.child)[c];
-#pragma unroll 1
-      for (int q = 0; q < 4; q++) {
-        const int cc = (&ch.x)[q];
-        if (cc < 0) continue;
-        bool desc = false;
-        if (act) {
-          // The reference's test is region > theta * sqrt(d2), each step
-          // rounded.  Squared, region^2 > theta^2 d2, it needs no square
-          // root: below the cell's bound mb.x (region^2 / (theta^2 (1 +
-          // 2e-13))) it surely descends, above mb.y (the same with 1 -
-          // 2e-13) it surely accepts (the roundings of either side and of
-          // the bounds are below 1e-15 relative); only a d2 between the two
-          // takes the exact rounded path.
-          //
-          // An FP64 instruction costs this GPU's SM sub-partition about 64
-          // issue cycles, an FP32 one 1, so d2 is first formed in FP32 from
-          // the hi/lo pairs: dxf = (xh - cxh) + (xl - cxl).  Its error is at
-          // most 2^-23 |dx| + 2^-46 (|x| + |cx|), and so
-          //   |d2f - d2| <= 3 2^-23 d2 + 2^-45 S (|dxf| + |dyf|) + (...)^2,
-          // S = |x| + |y| + |cx| + |cy|.  err below takes 2^-20 d2f and
-          // 2^-44 S, over twice that, so d2f + err < the FP32 lower bound
-          // (rounded down from mb.x) means d2 < mb.x, and d2f - err > the
-          // upper one (rounded up from mb.y) d2 > mb.y: the FP64 test would
-          // decide the same.  Anything else (and any infinity or NaN on the
-          // way, where a comparison fails) takes the FP64 test as before.
-          const float4 cf = t.cf32[cc];
-          const float2 mf = t.macf[cc];
-          const float dxf = __fadd_rn(__fsub_rn(xh, cf.x), __fsub_rn(xl, cf.y));
-          const float dyf = __fadd_rn(__fsub_rn(yh, cf.z), __fsub_rn(yl, cf.w));
-          const float d2f = __fmaf_rn(dxf, dxf, __fmul_rn(dyf, dyf));
-          const float ef = __fmul_rn(0x1p-44f, __fadd_rn(sxy, __fadd_rn(fabsf(cf.x), fabsf(cf.z))));
-          const float err = __fmaf_rn(0x1p-20f, d2f, __fmul_rn(ef, __fadd_rn(__fadd_rn(fabsf(dxf), fabsf(dyf)), ef)));
-          if (__fadd_ru(d2f, err) < mf.x) {
-            desc = true;
-          } else if (__fsub_rd(d2f, err) > mf.y && d2f <= 3.0e38f) {
-            desc = false;
-          } else {
-            const double2 mb = t.mac[cc];
-            const double dx = __dsub_rn(x, t.cx[cc]);
-            const double dy = __dsub_rn(y, t.cy[cc]);
-            const double d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
-            if (d2 < mb.x) {
-              desc = true;
-            } else if (d2 > mb.y) {
-              desc = false;
-            } else {
-              desc = t.region[cc] > __dmul_rn(theta, __dsqrt_rn(d2));
+      // direct_evaluate, fmm.c:121-142: the leaf's blobs dealt to the four
+      // lanes of each target that opened it
+      const int b = t.begin[c], e = t.end[c];
+      if (act) {
+        for (int j0 = b; j0 < e; j0 += 32 * kShare) {
+          fix::settle(near);
+          const int j1 = min(e, j0 + 32 * kShare);
+          for (int j = j0 + sub; j < j1; j += kShare) {
+            const double rx = __dsub_rn(x, t.x[j]);
+            const double ry = __dsub_rn(y, t.y[j]);
+            // The reference forms r = sqrt(r2), (r/sigma)^2 and 1/(r*r); r2 and
+            // r2/sigma^2 (1/sigma^2 precomputed per blob) give the same
+            // quantities.  r > 1e-10 is sure from a component of 2^-32 on
+            // (exponent field 991), ruled out below 2^-34, and otherwise
+            // decided on r2 > 1e-20 in FP64.
+            const fix::Vec v = fix::vec(rx, ry);
+            bool apart = v.e >= 991;
+            if (!apart && v.e >= 989) apart = __dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry)) > 1.0e-20;
+            if (apart) {
+              int ge, ce;
+              const double g = t.cir[j];
+              const uint64_t gm = fix::mantissa(g, ge), cm = fix::mantissa(t.icor2[j], ce);
+              fix::add_pair(near, v, fix::hi32(fix::bits(rx)), fix::hi32(fix::bits(ry)), gm, ge,
+                            fix::hi32(fix::bits(g)), cm, ce, s_exp_int, s_exp_frac, a.one);
             }
           }
         }
-        const unsigned dmask = __ballot_sync(0xffffffffu, desc);
-        if (act && !desc && nt >= 2) s_queue[warp][(qh + nq++) & (kQueue - 1)][lane] = cc;
-        if (act && !desc) n_m2s++;
-        if (dmask) {
-          if (top + 1 >= kStackCap) {
-            overflow = true;
-            break;
-          }
-          top++;
-          if (lane == 0) {
-            s_cell[warp][top] = cc;
-            s_mask[warp][top] = dmask;
+        if (sub == 0) n_pairs += (unsigned)(e - b);
+      }
+      __syncwarp();
+    } else {
+      // a cell's four children can add four entries to a target's queue
+      if (__any_sync(0xffffffffu, nq > kQueue - kShare)) flush(false);
+      // each of a target's lanes tests one child
+      const int cc = t.child[4 * (long)c + sub];
+      bool desc = false;
+      if (act && cc >= 0) {
+        // The reference's test is region > theta * sqrt(d2), each step
+        // rounded.  Squared, region^2 > theta^2 d2, it needs no square
+        // root: below the cell's bound mb.x (region^2 / (theta^2 (1 +
+        // 2e-13))) it surely descends, above mb.y (the same with 1 -
+        // 2e-13) it surely accepts (the roundings of either side and of
+        // the bounds are below 1e-15 relative); only a d2 between the two
+        // takes the exact rounded path.
+        //
+        // An FP64 instruction costs this GPU's SM sub-partition about 64
+        // issue cycles, an FP32 one 1, so d2 is first formed in FP32 from
+        // the hi/lo pairs: dxf = (xh - cxh) + (xl - cxl).  Its error is at
+        // most 2^-23 |dx| + 2^-46 (|x| + |cx|), and so
+        //   |d2f - d2| <= 3 2^-23 d2 + 2^-45 S (|dxf| + |dyf|) + (...)^2,
+        // S = |x| + |y| + |cx| + |cy|.  err below takes 2^-20 d2f and
+        // 2^-44 S, over twice that, so d2f + err < the FP32 lower bound
+        // (rounded down from mb.x) means d2 < mb.x, and d2f - err > the
+        // upper one (rounded up from mb.y) d2 > mb.y: the FP64 test would
+        // decide the same.  Anything else (and any infinity or NaN on the
+        // way, where a comparison fails) takes the FP64 test as before.
+        const float4 cf = t.cf32[cc];
+        const float2 mf = t.macf[cc];
+        const float dxf = __fadd_rn(__fsub_rn(xh, cf.x), __fsub_rn(xl, cf.y));
+        const float dyf = __fadd_rn(__fsub_rn(yh, cf.z), __fsub_rn(yl, cf.w));
+        const float d2f = __fmaf_rn(dxf, dxf, __fmul_rn(dyf, dyf));
+        const float ef = __fmul_rn(0x1p-44f, __fadd_rn(sxy, __fadd_rn(fabsf(cf.x), fabsf(cf.z))));
+        const float err = __fmaf_rn(0x1p-20f, d2f, __fmul_rn(ef, __fadd_rn(__fadd_rn(fabsf(dxf), fabsf(dyf)), ef)));
+        if (__fadd_ru(d2f, err) < mf.x) {
+          desc = true;
+        } else if (__fsub_rd(d2f, err) > mf.y && d2f <= 3.0e38f) {
+          desc = false;
+        } else {
+          const double2 mb = t.mac[cc];
+          const double dx = __dsub_rn(x, t.cx[cc]);
+          const double dy = __dsub_rn(y, t.cy[cc]);
+          const double d2 = __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy));
+          if (d2 < mb.x) {
+            desc = true;
+          } else if (d2 > mb.y) {
+            desc = false;
+          } else {
+            desc = t.region[cc] > __dmul_rn(theta, __dsqrt_rn(d2));
           }
         }
-        __syncwarp();
       }
-      if (__any_sync(0xffffffffu, overflow)) break;
+      const unsigned dmask = __ballot_sync(0xffffffffu, desc);
+      const unsigned amask = __ballot_sync(0xffffffffu, act && cc >= 0 && !desc);
+      const unsigned mine = (amask >> (lane & ~(kShare - 1))) & 0xfu;  // children this target accepts
+      if (nt >= 2) {
+        if ((mine >> sub) & 1u)
+          s_queue[warp][tgt][(qh + (unsigned)(nq + __popc(mine & ((1u << sub) - 1u)))) & (kQueue - 1)] = cc;
+        nq += __popc(mine);
+      }
+      n_m2s += __popc(mine);
+      // lane q < 4 pushes child q with the lanes of the targets that open it
+      const unsigned open = (dmask >> sub) & kEachTarget;
+      const unsigned some = __ballot_sync(0xffffffffu, open != 0) & 0xfu;
+      const int cnt = __popc(some);
+      if (top + cnt >= kStackCap) {
+        overflow = true;
+        break;
+      }
+      if (lane < kShare && open) {
+        const int at = top + 1 + __popc(some & ((1u << lane) - 1u));
+        s_cell[warp][at] = cc;
+        s_mask[warp][at] = open * 0xfu;
+      }
+      top += cnt;
+      __syncwarp();
     }
   }
   flush(true);
-  flush_leaves();
-  if (__any_sync(0xffffffffu, overflow)) {
-    if (lane == 0) set_err(a.st, TREE2D_ERR_TIMEOUT);
+  if (overflow && lane == 0) set_err(a.st, TREE2D_ERR_TIMEOUT);
+  // the four lanes' sums
+  double2 phi = kForm != kFormFp64 ? make_double2(fix::to_double(far.x, far.xl, far.e), fix::to_double(far.y, far.yl, far.e))
+                                   : make_double2(0.0, 0.0);
+  phi.x = __dadd_rn(phi.x, far64.x);
+  phi.y = __dadd_rn(phi.y, far64.y);
+  double2 dir = make_double2(fix::to_double(near.x, near.xl, near.e), fix::to_double(near.y, near.yl, near.e));
+  for (int o = 1; o < kShare; o <<= 1) {
+    phi.x = __dadd_rn(phi.x, __shfl_xor_sync(0xffffffffu, phi.x, o));
+    phi.y = __dadd_rn(phi.y, __shfl_xor_sync(0xffffffffu, phi.y, o));
+    dir.x = __dadd_rn(dir.x, __shfl_xor_sync(0xffffffffu, dir.x, o));
+    dir.y = __dadd_rn(dir.y, __shfl_xor_sync(0xffffffffu, dir.y, o));
   }
-  if (valid) {
-    // fmm.c:115-117
-    const double pre = (0.5 * -phi.y) / kPi;
-    const double pim = (0.5 * phi.x) / kPi;
-    const double u = -pre + ud0;
-    const double v = pim + ud1;
+  if (valid && sub == 0) {
+    // fmm.c:115-117 with its direct part 0.5 a / pi
+    double u = (0.5 * (phi.y + dir.x)) / kPi;
+    double v = (0.5 * (phi.x + dir.y)) / kPi;
+    // the fixed-point terms do not carry an infinity or a NaN of the target
+    if (!isfinite(x) || !isfinite(y)) {
+      if ((nt >= 2 && n_m2s > 0) || (n_pairs > 0 && !isnan(x) && !isnan(y))) u = v = NAN;
+    }
     const long o = a.out_idx ? a.out_idx[i] : i;
     a.uv[2 * o] = overflow ? NAN : u;
     a.uv[2 * o + 1] = overflow ? NAN : v;
   }
+  unsigned long long m2s = valid && sub == 0 ? n_m2s : 0;
   for (int o = 16; o; o >>= 1) {
-    n_m2s += __shfl_xor_sync(0xffffffffu, n_m2s, o);
+    m2s += __shfl_xor_sync(0xffffffffu, m2s, o);
     n_pairs += __shfl_xor_sync(0xffffffffu, n_pairs, o);
   }
   if (lane == 0) {
-    atomicAdd(&a.st->n_m2s, n_m2s);
+    atomicAdd(&a.st->n_m2s, m2s);
     atomicAdd(&a.st->n_pairs, n_pairs);
   }
 }
@@ -377,7 +403,7 @@ __global__ void __launch_bounds__(kEvalWarps * 32) k_eval(EvalArgs a) {
 // nearest float, lo = the rest, rounded) and the bounds rounded outwards to
 // FP32; a lower bound below 1e-30 becomes -1 and an upper one below 1e-30
 // +inf (no sure answer: the FP32 error bound does not cover subnormals).
-__global__ void k_mac_bounds(Tree t, double theta) {
+__global__ void k_mac_bounds(Tree t, double theta, int nt, int fixed) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= t.ncell) return;
   const double r2 = t.region[c] * t.region[c], th2 = theta * theta;
@@ -389,26 +415,78 @@ __global__ void k_mac_bounds(Tree t, double theta) {
   t.cf32[c] = make_float4(cxh, __double2float_rn(cx - (double)cxh), cyh, __double2float_rn(cy - (double)cyh));
   t.macf[c] = make_float2(mb.x >= 1e-30 ? __double2float_rd(mb.x) : -1.0f,
                           mb.y >= 1e-30 ? __double2float_ru(mb.y) : INFINITY);
+  if (fixed && nt >= 2) {
+    // The coefficients in fixed point, the cell's scale in the last entry
+    // (whose a_k the sums do not use).  t.fix may be t.coef: a thread has
+    // read what it needs of its cell before it writes entry k.
+    const double2 *src = t.coef + (size_t)c * nt;
+    longlong2 *dst = reinterpret_cast<longlong2 *>(t.fix) + (size_t)c * nt;
+    const fix::CellScale sc = fix::cell_scale(nt - 1, t.region[c], theta, [&](int k, double &re, double &im) {
+      const double2 a = src[k];
+      re = a.x;
+      im = a.y;
+    });
+    const int k0 = fix::first_pair_term(theta);
+    for (int k = 0; k < nt - 1; k++) {
+      const double2 a = src[k];
+      if (nt - 1 > k0 && k >= k0) {
+        float4 v;
+        fix::pair_coef(a.x, k, sc, v.x, v.y);
+        fix::pair_coef(a.y, k, sc, v.z, v.w);
+        reinterpret_cast<float4 *>(dst)[k] = v;
+      } else {
+        dst[k] = make_longlong2(fix::fix_coef(a.x, k, sc), fix::fix_coef(a.y, k, sc));
+      }
+    }
+    dst[nt - 1] = make_longlong2(sc.es, sc.eb);
+  }
 }
 
-cudaError_t mac_bounds(Workspace &ws, const Tree &t, double theta, cudaStream_t s) {
+// Opening angle up to which the multipole sums run in fixed point: es can
+// reach log2(0.71 R), the farthest blob's, so that the coefficients do not
+// grow with k (fix::cell_scale).  Above it FP64, as before.
+constexpr double kFixTheta = 2.0 * fix::kHalfTheta;
+
+cudaError_t mac_bounds(Workspace &ws, const Tree &t, double theta, int nt, cudaStream_t s) {
   if (ws.mac_theta == theta || t.ncell <= 0) return cudaSuccess;
-  k_mac_bounds<<<(t.ncell + 255) / 256, 256, 0, s>>>(t, theta);
+  k_mac_bounds<<<(t.ncell + 63) / 64, 64, 0, s>>>(t, theta, nt, theta <= kFixTheta);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   const cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) ws.mac_theta = theta;
   return e;
 }
 
-// Binomial table, uploaded once per device (the table lives in each
-// device's copy of the module).
-bool g_binom_ready[64] = {};
+// High 128 bits of a product of 128-bit numbers.
+unsigned __int128 mul128(unsigned __int128 a, unsigned __int128 b) {
+  const uint64_t ah = (uint64_t)(a >> 64), al = (uint64_t)a, bh = (uint64_t)(b >> 64), bl = (uint64_t)b;
+  const unsigned __int128 m1 = (unsigned __int128)ah * bl, m2 = (unsigned __int128)al * bh,
+                          l = (unsigned __int128)al * bl;
+  const unsigned __int128 mid = (l >> 64) + (uint64_t)m1 + (uint64_t)m2;
+  return (unsigned __int128)ah * bh + (m1 >> 64) + (m2 >> 64) + (mid >> 64);
+}
 
-cudaError_t upload_binom() {
+// e^-(j / 2048) in units of 2^-100 by its Taylor series in integers.
+unsigned __int128 exp_series(int j) {
+  const unsigned __int128 one = (unsigned __int128)1 << 100;
+  unsigned __int128 t = one, pos = one, neg = 0;
+  for (int k = 1; t; k++) {
+    t = (t * (unsigned)j >> 11) / (unsigned)k;
+    (k & 1 ? neg : pos) += t;
+  }
+  return pos - neg;
+}
+
+// The constant tables, uploaded once per device (they live in each device's
+// copy of the module).
+std::mutex g_tables_mu;
+bool g_tables_ready[64] = {};
+
+cudaError_t upload_tables() {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (dev >= 0 && dev < 64 && g_binom_ready[dev]) return cudaSuccess;
+  std::lock_guard<std::mutex> lk(g_tables_mu);
+  if (dev >= 0 && dev < 64 && g_tables_ready[dev]) return cudaSuccess;
   static double h[kMaxTerms][kMaxTerms];
   for (int n = 0; n < kMaxTerms; n++) {
     h[n][0] = 1.0;
@@ -417,14 +495,24 @@ cudaError_t upload_binom() {
   // exact: every C(n,k), n < 32, is an integer below 2^53 and the running
   // product above stays integral (C(n,k-1)*(n-k+1) is divisible by k).
   e = cudaMemcpyToSymbol(c_binom, h, sizeof(h));
-  if (e == cudaSuccess && dev >= 0 && dev < 64) g_binom_ready[dev] = true;
+  static uint64_t ints[fix::kExpInts], fracs[fix::kExpFracs];
+  for (int j = 0; j < fix::kExpFracs; j++) fracs[j] = (uint64_t)((exp_series(j) + ((unsigned __int128)1 << 37)) >> 38);
+  const unsigned __int128 e1 = exp_series(fix::kExpFracs) << 27;  // e^-1, units of 2^-127
+  unsigned __int128 v = (unsigned __int128)1 << 127;
+  for (int n = 0; n < fix::kExpInts; n++) {
+    ints[n] = (uint64_t)((v + ((unsigned __int128)1 << 64)) >> 65);
+    v = mul128(v, e1) << 1;
+  }
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_exp_int, ints, sizeof(ints));
+  if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_exp_frac, fracs, sizeof(fracs));
+  if (e == cudaSuccess && dev >= 0 && dev < 64) g_tables_ready[dev] = true;
   return e;
 }
 
 }  // namespace
 
 int plain_upward(Workspace &ws, const Tree &t, const Params &p, cudaStream_t s) {
-  T2D_CUDA_TRY(upload_binom());
+  T2D_CUDA_TRY(upload_tables());
   const int nt = p.nterms;
   long tot = (long)t.ncell * nt;
   if (tot == 0) return TREE2D_OK;
@@ -442,10 +530,15 @@ int plain_upward(Workspace &ws, const Tree &t, const Params &p, cudaStream_t s) 
 int plain_evaluate(Workspace &ws, const Tree &t, const Params &p, int ntgt, const double *tx, const double *ty,
                    const int *out_idx, double *uv, cudaStream_t s) {
   if (ntgt <= 0) return TREE2D_OK;
-  T2D_CUDA_TRY(mac_bounds(ws, t, p.theta, s));
-  EvalArgs a{t, p.nterms, p.theta, ntgt, tx, ty, out_idx, uv, ws.status};
-  const int warps = (ntgt + 31) / 32;
-  k_eval<<<(warps + kEvalWarps - 1) / kEvalWarps, kEvalWarps * 32, 0, s>>>(a);
+  T2D_CUDA_TRY(mac_bounds(ws, t, p.theta, p.nterms, s));
+  EvalArgs a{t, p.nterms, p.theta, ntgt, tx, ty, out_idx, uv, ws.status, fix::first_pair_term(p.theta),
+             reinterpret_cast<const void *>(t.fix) != reinterpret_cast<const void *>(t.coef), fix::One()};
+  const int warps = (ntgt + kEvalTargets - 1) / kEvalTargets;
+  const int blocks = (warps + kEvalWarps - 1) / kEvalWarps;
+  auto kernel = p.theta > kFixTheta           ? k_eval<kFormFp64>
+                : p.theta > fix::kHalfTheta ? k_eval<kFormFull>
+                                            : k_eval<kFormHalf>;
+  kernel<<<blocks, kEvalWarps * 32, 0, s>>>(a);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;
