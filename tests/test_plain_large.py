@@ -226,3 +226,34 @@ def test_keys_on_cell_edges_match_oracle(gpu_lib):
     assert np.array_equal(d["perm"], od["perm"])
     assert np.array_equal(d["level"], od["level"]) and np.array_equal(d["begin"], od["begin"])
     assert np.array_equal(d["cx"].view(np.uint64), od["cx"].view(np.uint64))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nterms", [1, 2, 15, 16, 17, 32])
+@pytest.mark.parametrize("n,num_p", [(1, 33), (700, 2), (3000, 33), (2000, 500)])
+def test_coefficients_are_the_cells_moments(gpu_lib, nterms, n, num_p):
+    """Every cell's coefficients below the root are its blobs' moments sum G
+    (z - c)^k, for leaves of one blob, leaves longer than a warp, and both
+    widths of the shift.  Bound: a moment of order k is formed by at most k
+    products per blob and a shift of k sweeps per level, each a few roundings
+    of terms no larger than sum |G| (1.5 R)^k."""
+    P = gpu_lib
+    b = workloads().uniform(n, seed=n + nterms)
+    P.set_params(nterms, num_p, 0.5)
+    P.set_mode(P.MODE_PLAIN)
+    try:
+        P.make_tree(b.xy, b.cir, b.cor)
+        t = P.export_tree(n, nterms)
+    finally:
+        P.clear_params()
+    z = (b.xy[:, 0].astype(np.longdouble) + 1j * b.xy[:, 1].astype(np.longdouble))[t["perm"]]
+    g = b.cir[t["perm"]]
+    pick = np.unique(np.linspace(0, len(t["level"]) - 1, min(len(t["level"]), 400)).astype(int))
+    for c in pick:
+        s = slice(t["begin"][c], t["end"][c])
+        d = z[s] - (np.longdouble(t["cx"][c]) + 1j * np.longdouble(t["cy"][c]))
+        k = np.arange(nterms)
+        exact = (g[s][:, None] * d[:, None] ** k).sum(axis=0)
+        scale = np.abs(g[s]).sum() * (1.5 * t["region"][c]) ** k
+        err = np.abs(t["coef"][c] - exact).astype(float)
+        assert (err <= 8 * (k + 1) * (t["level"].max() + 1) * 2.0**-53 * scale).all(), (c, err / scale)
