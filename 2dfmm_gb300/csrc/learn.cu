@@ -13,9 +13,10 @@
 //
 // Labels come from the FMM itself against the FP64 exact contribution of
 // the interaction (the direct sum restricted to it): `k_labels`.  Training
-// runs on the GPU: tiled FP32 GEMMs over BF16-rounded operands, GELU,
-// softmax cross-entropy and Adam, one kernel each; gradients are checked
-// against the CPU oracle (oracle/mlp_oracle.py).
+// runs on the GPU in FP32 over BF16-rounded operands: per step one kernel for
+// the forward pass, the softmax cross-entropy and the layers' gradients, and
+// one for the weight gradients and Adam; gradients are checked against the
+// CPU oracle (oracle/mlp_oracle.py).
 #include <cuda_bf16.h>
 
 #include <cmath>
@@ -168,48 +169,6 @@ __device__ __forceinline__ float gelu_grad_f(float z) {
   return 0.5f * (1.f + t) + 0.5f * z * (1.f - t * t) * c * (1.f + 3.f * 0.044715f * z * z);
 }
 
-// C(i,j) = beta*C(i,j) + sum_k A(i,k) B(k,j) (+ bias[j]); A(i,k) =
-// A[i*sa0 + k*sa1], B(k,j) = B[k*sb0 + j*sb1], C row-major ldc.  32x32 tiles.
-__global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, const float *A, long sa0, long sa1, const float *Bm,
-                                              long sb0, long sb1, float *C, int ldc, const float *bias, int beta) {
-  __shared__ float As[32][33], Bs[32][33];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-  const int i0 = blockIdx.y * 32, j0 = blockIdx.x * 32;
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int k0 = 0; k0 < K; k0 += 32) {
-    for (int r = ty; r < 32; r += 8) {
-      const int i = i0 + r, k = k0 + tx;
-      As[r][tx] = (i < M && k < K) ? A[(long)i * sa0 + (long)k * sa1] : 0.f;
-      const int kk = k0 + r, j = j0 + tx;
-      Bs[r][tx] = (kk < K && j < N) ? Bm[(long)kk * sb0 + (long)j * sb1] : 0.f;
-    }
-    __syncthreads();
-    for (int k = 0; k < 32; k++) {
-      const float b = Bs[k][tx];
-      for (int q = 0; q < 4; q++) acc[q] = fmaf(As[ty + 8 * q][k], b, acc[q]);
-    }
-    __syncthreads();
-  }
-  const int j = j0 + tx;
-  if (j >= N) return;
-  for (int q = 0; q < 4; q++) {
-    const int i = i0 + ty + 8 * q;
-    if (i >= M) continue;
-    float v = acc[q] + (bias ? bias[j] : 0.f);
-    C[(long)i * ldc + j] = beta ? C[(long)i * ldc + j] + v : v;
-  }
-}
-
-// mode 0: A = bf16(gelu(Z)); mode 1: D = D * gelu'(Z)
-__global__ void k_act(int n, const float *Z, float *out, int mode) {
-  long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  if (mode == 0)
-    out[i] = bf16r(gelu_f(Z[i]));
-  else
-    out[i] *= gelu_grad_f(Z[i]);
-}
-
 __device__ __forceinline__ uint32_t hash32(uint32_t x) {
   x ^= x >> 16;
   x *= 0x7feb352du;
@@ -219,131 +178,339 @@ __device__ __forceinline__ uint32_t hash32(uint32_t x) {
   return x;
 }
 
-// Mini-batch rows: X rows (BF16-rounded) and labels, drawn uniformly.
-__global__ void k_gather_batch(int n, const float *X, const int *y, int bt, unsigned seed, float *A0, int *yb) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= bt) return;
-  const int r = seed == 0xffffffffu ? i : (int)(hash32(seed * 2654435761u + (unsigned)i) % (unsigned)n);
-  for (int k = 0; k < kMlpIn; k++) A0[(long)i * kMlpIn + k] = bf16r(X[(long)r * kMlpIn + k]);
-  yb[i] = y[r];
-}
-
-// D4 = (softmax(Z4[:, :14]) - onehot) / bt, loss summed into *loss.
-__global__ void k_softmax_ce(int bt, const float *Z4, const int *yb, float *D4, float *loss) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= bt) return;
-  const float *z = Z4 + (long)i * kMlpOut;
-  float mx = z[0];
-  for (int c = 1; c < kMlpClasses; c++) mx = fmaxf(mx, z[c]);
-  float p[kMlpClasses], s = 0.f;
-  for (int c = 0; c < kMlpClasses; c++) {
-    p[c] = expf(z[c] - mx);
-    s += p[c];
-  }
-  const int y = yb[i];
-  for (int c = 0; c < kMlpOut; c++) {
-    float d = c < kMlpClasses ? p[c] / s : 0.f;
-    if (c == y) d -= 1.f;
-    D4[(long)i * kMlpOut + c] = d / (float)bt;
-  }
-  atomicAdd(loss, -logf(fmaxf(p[y] / s, 1e-30f)) / (float)bt);
-}
-
-__global__ void k_colsum(int rows, int cols, const float *D, float *out) {
-  int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= cols) return;
-  float s = 0.f;
-  for (int i = 0; i < rows; i++) s += D[(long)i * cols + j];
-  out[j] = s;
-}
-
-__global__ void k_round_weights(int n, const float *theta, float *wb) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) wb[i] = bf16r(theta[i]);
-}
-
-__global__ void k_adam(int n, float *theta, float *m1, float *v1, const float *g, float lr, float b1c, float b2c) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float b1 = 0.9f, b2 = 0.999f;
-  const float mi = b1 * m1[i] + (1.f - b1) * g[i];
-  const float vi = b2 * v1[i] + (1.f - b2) * g[i] * g[i];
-  m1[i] = mi;
-  v1[i] = vi;
-  theta[i] -= lr * (mi / b1c) / (sqrtf(vi / b2c) + 1e-8f);
-}
-
+constexpr int kH = kMlpHidden;
 struct Offs {
   int W1, b1, W2, b2, W3, b3, W4, b4;
 };
 constexpr Offs kOff{0, 1024, 1088, 5184, 5248, 9344, 9408, 10432};
+static_assert(kMlpIn == 16 && kMlpHidden == 64 && kMlpOut == 16, "the tiles below are for 16 -> 64 -> 64 -> 64 -> 16");
 
-// Scratch of one mini-batch pass.
+// A mini-batch's layer inputs A (BF16-rounded) and the loss's gradients D by
+// the layers' sums, row-major, for the weight gradients.
 struct Pass {
-  float *A0, *Z1, *A1, *Z2, *A2, *Z3, *A3, *Z4, *D4, *D3, *D2, *D1;
-  int *yb;
+  float *A0, *A1, *A2, *A3, *D1, *D2, *D3, *D4;
 };
 
-void gemm(cudaStream_t s, int M, int N, int K, const float *A, long sa0, long sa1, const float *B, long sb0, long sb1,
-          float *C, int ldc, const float *bias, int beta) {
-  dim3 g((N + 31) / 32, (M + 31) / 32);
-  k_gemm<<<g, 256, 0, s>>>(M, N, K, A, sa0, sa1, B, sb0, sb1, C, ldc, bias, beta);
+// Rows of the batch and how they are drawn: row i is X's row i, or with
+// `draw` one drawn by `seed` and i.
+struct Rows {
+  const float *X;
+  const int *y;  // null: forward only
+  int n, bt, draw;
+  unsigned seed;
+};
+__device__ __forceinline__ int row_of(const Rows &r, int i) {
+  return r.draw ? (int)(hash32(r.seed * 2654435761u + (unsigned)i) % (unsigned)r.n) : i;
+}
+
+constexpr int kRowsPerBlock = 32;
+constexpr int kPadH = kH + 4, kPadIn = kMlpIn + 4;  // row strides in shared memory (16-byte loads of 8 rows: 32 banks)
+struct RowsShared {
+  float W1[kH][kPadIn], W2[kH][kPadH], W3[kH][kPadH], W4[kMlpOut][kPadH];
+  float A0[kRowsPerBlock][kPadIn];
+  float A[kRowsPerBlock][kPadH], Z1[kRowsPerBlock][kPadH], Z2[kRowsPerBlock][kPadH], Z3[kRowsPerBlock][kPadH];
+  float Z4[kRowsPerBlock][kPadIn], D4[kRowsPerBlock][kPadIn], Da[kRowsPerBlock][kPadH], Db[kRowsPerBlock][kPadH];
+};
+
+// Z[r][o] = sum_k A[r][k] W[o][k] + bias[o] (k ascending, one FMA per term),
+// for 16 O outputs; a thread forms 2 rows x O outputs.
+template <int K, int O, int SA, int SW, int SZ>
+__device__ __forceinline__ void layer(const float (*A)[SA], const float (*W)[SW], const float *bias, float (*Z)[SZ]) {
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  float acc[2][O];
+#pragma unroll
+  for (int r = 0; r < 2; r++)
+#pragma unroll
+    for (int o = 0; o < O; o++) acc[r][o] = 0.f;
+#pragma unroll 4
+  for (int k = 0; k < K; k += 4) {
+    float4 a[2], w[O];
+#pragma unroll
+    for (int r = 0; r < 2; r++) a[r] = *reinterpret_cast<const float4 *>(&A[ty + 16 * r][k]);
+#pragma unroll
+    for (int o = 0; o < O; o++) w[o] = *reinterpret_cast<const float4 *>(&W[tx + 16 * o][k]);
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+      for (int o = 0; o < O; o++) {
+        acc[r][o] = fmaf(a[r].x, w[o].x, acc[r][o]);
+        acc[r][o] = fmaf(a[r].y, w[o].y, acc[r][o]);
+        acc[r][o] = fmaf(a[r].z, w[o].z, acc[r][o]);
+        acc[r][o] = fmaf(a[r].w, w[o].w, acc[r][o]);
+      }
+  }
+#pragma unroll
+  for (int r = 0; r < 2; r++)
+#pragma unroll
+    for (int o = 0; o < O; o++) Z[ty + 16 * r][tx + 16 * o] = acc[r][o] + bias[tx + 16 * o];
+}
+
+// out[r][h] = (sum_o D[r][o] W[o][h]) gelu'(Z[r][h]), o ascending; also to the
+// row-major global array g (rows below `rows`).
+template <int O, int SD>
+__device__ __forceinline__ void back(const float (*D)[SD], const float (*W)[kPadH], const float (*Z)[kPadH],
+                                     float (*out)[kPadH], float *g, int rows) {
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  float acc[2][4] = {};
+#pragma unroll 2
+  for (int o = 0; o < O; o += 4) {
+    float4 d[2];
+#pragma unroll
+    for (int r = 0; r < 2; r++) d[r] = *reinterpret_cast<const float4 *>(&D[ty + 16 * r][o]);
+#pragma unroll
+    for (int q = 0; q < 4; q++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        const float w = W[o + q][tx + 16 * j];
+        acc[0][j] = fmaf((&d[0].x)[q], w, acc[0][j]);
+        acc[1][j] = fmaf((&d[1].x)[q], w, acc[1][j]);
+      }
+  }
+#pragma unroll
+  for (int r = 0; r < 2; r++)
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int i = ty + 16 * r, h = tx + 16 * j;
+      float v = acc[r][j] + 0.f;
+      v *= gelu_grad_f(Z[i][h]);
+      out[i][h] = v;
+      if (i < rows) g[(size_t)i * kH + h] = v;
+    }
+}
+
+// A = bf16(gelu(Z)), also to the row-major global array g (if any).
+__device__ __forceinline__ void activate(const float (*Z)[kPadH], float (*A)[kPadH], float *g, int rows) {
+  for (int e = threadIdx.x; e < kRowsPerBlock * kH; e += blockDim.x) {
+    const int i = e / kH, h = e & (kH - 1);
+    const float v = bf16r(gelu_f(Z[i][h]));
+    A[i][h] = v;
+    if (g && i < rows) g[(size_t)i * kH + h] = v;
+  }
+}
+
+template <int K, int O, int S>
+__device__ __forceinline__ void load_weights(const float *theta, float (*W)[S]) {
+#pragma unroll
+  for (int e = 4 * threadIdx.x; e < K * O; e += 4 * 256) {
+    const float4 v = *reinterpret_cast<const float4 *>(theta + e);
+    *reinterpret_cast<float4 *>(&W[e / K][e % K]) = make_float4(bf16r(v.x), bf16r(v.y), bf16r(v.z), bf16r(v.w));
+  }
+}
+
+// Forward pass, loss and the gradients by the layers' sums for 32 rows per
+// block, everything between the layers in shared memory.  Each sum runs in
+// the order of a plain loop, so the values do not depend on the tiling.
+__global__ void __launch_bounds__(256) k_rows(Rows rows, const float *__restrict__ theta, Pass p, float *logits,
+                                              float *loss) {
+  extern __shared__ float4 shared_rows[];
+  RowsShared &s = *reinterpret_cast<RowsShared *>(shared_rows);
+  const int i0 = blockIdx.x * kRowsPerBlock, left = min(kRowsPerBlock, rows.bt - i0);
+  const bool train = rows.y != nullptr;
+  load_weights<kMlpIn, kH>(theta + kOff.W1, s.W1);
+  load_weights<kH, kH>(theta + kOff.W2, s.W2);
+  load_weights<kH, kH>(theta + kOff.W3, s.W3);
+  load_weights<kH, kMlpOut>(theta + kOff.W4, s.W4);
+  for (int e = threadIdx.x; e < kRowsPerBlock * kMlpIn; e += blockDim.x) {
+    const int i = e / kMlpIn, k = e & (kMlpIn - 1);
+    float v = 0.f;
+    if (i < left) v = bf16r(rows.X[(size_t)row_of(rows, i0 + i) * kMlpIn + k]);
+    s.A0[i][k] = v;
+    if (train && i < left) p.A0[(size_t)(i0 + i) * kMlpIn + k] = v;
+  }
+  const size_t at = (size_t)i0 * kH;
+  __syncthreads();
+  layer<kMlpIn, 4>(s.A0, s.W1, theta + kOff.b1, s.Z1);
+  __syncthreads();
+  activate(s.Z1, s.A, train ? p.A1 + at : nullptr, left);
+  __syncthreads();
+  layer<kH, 4>(s.A, s.W2, theta + kOff.b2, s.Z2);
+  __syncthreads();
+  activate(s.Z2, s.A, train ? p.A2 + at : nullptr, left);
+  __syncthreads();
+  layer<kH, 4>(s.A, s.W3, theta + kOff.b3, s.Z3);
+  __syncthreads();
+  activate(s.Z3, s.A, train ? p.A3 + at : nullptr, left);
+  __syncthreads();
+  layer<kH, 1>(s.A, s.W4, theta + kOff.b4, s.Z4);
+  __syncthreads();
+  if (!train) {
+    for (int e = threadIdx.x; e < left * kMlpOut; e += blockDim.x)
+      logits[(size_t)i0 * kMlpOut + e] = s.Z4[e / kMlpOut][e & (kMlpOut - 1)];
+    return;
+  }
+  // D4 = (softmax(Z4[:14]) - onehot) / bt, loss summed into *loss
+  if (threadIdx.x < kRowsPerBlock) {
+    const int i = threadIdx.x;
+    const float *z = s.Z4[i];
+    float mx = z[0];
+    for (int c = 1; c < kMlpClasses; c++) mx = fmaxf(mx, z[c]);
+    float q[kMlpClasses], sum = 0.f;
+    for (int c = 0; c < kMlpClasses; c++) {
+      q[c] = expf(z[c] - mx);
+      sum += q[c];
+    }
+    const int y = i < left ? rows.y[row_of(rows, i0 + i)] : 0;
+    float py = 1.f;
+    for (int c = 0; c < kMlpOut; c++) {
+      float d = c < kMlpClasses ? q[c < kMlpClasses ? c : 0] / sum : 0.f;
+      if (c == y) {
+        if (c < kMlpClasses) py = d;
+        d -= 1.f;
+      }
+      d /= (float)rows.bt;
+      s.D4[i][c] = i < left ? d : 0.f;
+      if (i < left) p.D4[(size_t)(i0 + i) * kMlpOut + c] = d;
+    }
+    float l = i < left ? -logf(fmaxf(py, 1e-30f)) / (float)rows.bt : 0.f;
+    for (int o = 16; o; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    if (i == 0) atomicAdd(loss, l);
+  }
+  __syncthreads();
+  back<kMlpOut>(s.D4, s.W4, s.Z3, s.Da, p.D3 + at, left);
+  __syncthreads();
+  back<kH>(s.Da, s.W3, s.Z2, s.Db, p.D2 + at, left);
+  __syncthreads();
+  back<kH>(s.Db, s.W2, s.Z1, s.Da, p.D1 + at, left);
+}
+
+// Weight gradients g[o][h] = sum_i D[i][o] A[i][h], i ascending: 16 x 16 of
+// them per block, 2 x 2 per thread of the first two warps; the other two copy
+// the rows' columns asynchronously, three stages of 64 rows ahead (more change
+// nothing).  The last blocks sum the columns of D (biases).  Bound by the one
+// chain of multiply-adds per weight that the sums' order leaves: 33 us for
+// 4,096 rows.  A step takes 54 us with k_rows, where one tiled product per
+// layer and direction (4 blocks walking the rows for each weight gradient)
+// and one block per bias took 1,440.
+constexpr int kStage = 64, kStages = 4;
+constexpr int kWTiles2 = (kH / 16) * (kH / 16), kWTiles1 = kH / 16;
+constexpr int kWeightBlocks = 2 * kWTiles2 + 2 * kWTiles1 + 7;
+struct Adam {
+  float *theta, *m1, *v1;  // null theta: gradients only
+  float lr, b1c, b2c;
+};
+__device__ __forceinline__ void adam(const Adam &a, int i, float g) {
+  const float b1 = 0.9f, b2 = 0.999f;
+  const float mi = b1 * a.m1[i] + (1.f - b1) * g;
+  const float vi = b2 * a.v1[i] + (1.f - b2) * g * g;
+  a.m1[i] = mi;
+  a.v1[i] = vi;
+  a.theta[i] -= a.lr * (mi / a.b1c) / (sqrtf(vi / a.b2c) + 1e-8f);
+}
+
+__global__ void __launch_bounds__(128) k_weights(int bt, Pass p, float *grad, Adam a) {
+  __shared__ __align__(16) float cols[kStages][kStage][32];  // [buffer][row][16 columns of D, 16 of A, or 32 of D]
+  const bool copier = threadIdx.x >= 64;
+  const int t = threadIdx.x & 63;
+  auto put = [&](int i, float g) {
+    if (grad) grad[i] = g;
+    if (a.theta) adam(a, i, g);
+  };
+  // nd columns of D from dc and, for a weight tile, 16 of A from ac
+  const float *D, *A = nullptr;
+  int ld, la = 0, dc = 0, ac = 0, nd = 16, out, so = 0;
+  int b = blockIdx.x;
+  if (b < 2 * kWTiles2) {
+    const bool second = b >= kWTiles2;
+    b -= second ? kWTiles2 : 0;
+    D = second ? p.D3 : p.D2, A = second ? p.A2 : p.A1;
+    ld = la = kH, dc = 16 * (b / 4), ac = 16 * (b & 3), out = second ? kOff.W3 : kOff.W2, so = kH;
+  } else if ((b -= 2 * kWTiles2) < kWTiles1) {
+    D = p.D4, A = p.A3, ld = kMlpOut, la = kH, ac = 16 * b, out = kOff.W4, so = kH;
+  } else if ((b -= kWTiles1) < kWTiles1) {
+    D = p.D1, A = p.A0, ld = kH, la = kMlpIn, dc = 16 * b, out = kOff.W1, so = kMlpIn;
+  } else {
+    b -= kWTiles1;  // 32 columns of D1, D1, D2, D2, D3, D3, D4
+    const int l = b >> 1;
+    D = l == 0 ? p.D1 : l == 1 ? p.D2 : l == 2 ? p.D3 : p.D4;
+    ld = l == 3 ? kMlpOut : kH;
+    nd = min(ld, 32);
+    dc = 32 * (b & 1);
+    out = (l == 0 ? kOff.b1 : l == 1 ? kOff.b2 : l == 2 ? kOff.b3 : kOff.b4) + dc;
+  }
+  // a copying thread takes 4 columns (of 32, or 16 of D4) of every 8th row
+  const int col = 4 * (t & 7);
+  const float *from = col < nd ? D + dc + col : A ? A + ac + (col - nd) : nullptr;
+  const int stride = col < nd ? ld : la;
+  auto stage = [&](int k) {
+    const int r0 = k * kStage;
+    if (r0 < bt && from) {
+      unsigned dst = (unsigned)__cvta_generic_to_shared(&cols[k % kStages][t >> 3][col]);
+      const float *src = from + (size_t)(r0 + (t >> 3)) * stride;
+#pragma unroll
+      for (int r = t >> 3; r < kStage; r += 8, dst += 8 * 32 * 4, src += (size_t)8 * stride) {
+        const bool in = r0 + r < bt;  // rows past the batch: zeros
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(in ? src : from), "r"(in ? 16 : 0));
+      }
+    }
+    asm volatile("cp.async.commit_group;");
+  };
+  const int h = 2 * (t & 7), o = 2 * (t >> 3);
+  float g00 = 0.f, g01 = 0.f, g10 = 0.f, g11 = 0.f;  // [o][h]
+  const int nk = (bt + kStage - 1) / kStage;
+  if (copier) {
+    for (int k = 0; k < kStages - 1; k++) stage(k);
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2));
+  }
+  for (int k = 0; k < nk; k++) {
+    __syncthreads();  // stage k is in, and stage k - 1 done with
+    if (copier) {
+      stage(k + kStages - 1);
+      asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2));  // stage k + 1
+      continue;
+    }
+    const int buf = k % kStages;
+    if (A) {
+#pragma unroll 16
+      for (int r = 0; r < kStage; r++) {
+        const float2 x = *reinterpret_cast<const float2 *>(&cols[buf][r][16 + h]);
+        const float2 d = *reinterpret_cast<const float2 *>(&cols[buf][r][o]);
+        g00 = fmaf(d.x, x.x, g00);
+        g01 = fmaf(d.x, x.y, g01);
+        g10 = fmaf(d.y, x.x, g10);
+        g11 = fmaf(d.y, x.y, g11);
+      }
+    } else if (t < nd) {
+#pragma unroll 16
+      for (int r = 0; r < kStage; r++) g00 += cols[buf][r][t];
+    }
+  }
+  if (copier) {
+    asm volatile("cp.async.wait_all;");
+    return;
+  }
+  if (A) {
+    const int i = out + (dc + o) * so + ac + h;
+    put(i, g00 + 0.f);
+    put(i + 1, g01 + 0.f);
+    put(i + so, g10 + 0.f);
+    put(i + so + 1, g11 + 0.f);
+  } else if (t < nd) {
+    put(out + t, g00);
+  }
+}
+
+cudaError_t run_weights(int bt, const Pass &p, float *grad, const Adam &a, cudaStream_t s) {
+  k_weights<<<kWeightBlocks, 128, 0, s>>>(bt, p, grad, a);
   g_launches.fetch_add(1, std::memory_order_relaxed);
+  return cudaGetLastError();
 }
 
-void forward_pass(cudaStream_t s, int bt, const float *wb, const float *theta, Pass &p) {
-  const int H = kMlpHidden;
-  gemm(s, bt, H, kMlpIn, p.A0, kMlpIn, 1, wb + kOff.W1, 1, kMlpIn, p.Z1, H, theta + kOff.b1, 0);
-  k_act<<<(bt * H + 255) / 256, 256, 0, s>>>(bt * H, p.Z1, p.A1, 0);
-  gemm(s, bt, H, H, p.A1, H, 1, wb + kOff.W2, 1, H, p.Z2, H, theta + kOff.b2, 0);
-  k_act<<<(bt * H + 255) / 256, 256, 0, s>>>(bt * H, p.Z2, p.A2, 0);
-  gemm(s, bt, H, H, p.A2, H, 1, wb + kOff.W3, 1, H, p.Z3, H, theta + kOff.b3, 0);
-  k_act<<<(bt * H + 255) / 256, 256, 0, s>>>(bt * H, p.Z3, p.A3, 0);
-  gemm(s, bt, kMlpOut, H, p.A3, H, 1, wb + kOff.W4, 1, H, p.Z4, kMlpOut, theta + kOff.b4, 0);
-  g_launches.fetch_add(3, std::memory_order_relaxed);
-}
-
-void backward_pass(cudaStream_t s, int bt, const float *wb, Pass &p, float *g) {
-  const int H = kMlpHidden;
-  // layer 4
-  gemm(s, kMlpOut, H, bt, p.D4, 1, kMlpOut, p.A3, H, 1, g + kOff.W4, H, nullptr, 0);
-  k_colsum<<<1, 64, 0, s>>>(bt, kMlpOut, p.D4, g + kOff.b4);
-  gemm(s, bt, H, kMlpOut, p.D4, kMlpOut, 1, wb + kOff.W4, H, 1, p.D3, H, nullptr, 0);
-  k_act<<<(bt * H + 255) / 256, 256, 0, s>>>(bt * H, p.Z3, p.D3, 1);
-  // layer 3
-  gemm(s, H, H, bt, p.D3, 1, H, p.A2, H, 1, g + kOff.W3, H, nullptr, 0);
-  k_colsum<<<1, 64, 0, s>>>(bt, H, p.D3, g + kOff.b3);
-  gemm(s, bt, H, H, p.D3, H, 1, wb + kOff.W3, H, 1, p.D2, H, nullptr, 0);
-  k_act<<<(bt * H + 255) / 256, 256, 0, s>>>(bt * H, p.Z2, p.D2, 1);
-  // layer 2
-  gemm(s, H, H, bt, p.D2, 1, H, p.A1, H, 1, g + kOff.W2, H, nullptr, 0);
-  k_colsum<<<1, 64, 0, s>>>(bt, H, p.D2, g + kOff.b2);
-  gemm(s, bt, H, H, p.D2, H, 1, wb + kOff.W2, H, 1, p.D1, H, nullptr, 0);
-  k_act<<<(bt * H + 255) / 256, 256, 0, s>>>(bt * H, p.Z1, p.D1, 1);
-  // layer 1
-  gemm(s, H, kMlpIn, bt, p.D1, 1, H, p.A0, kMlpIn, 1, g + kOff.W1, kMlpIn, nullptr, 0);
-  k_colsum<<<1, 64, 0, s>>>(bt, H, p.D1, g + kOff.b1);
-  g_launches.fetch_add(7, std::memory_order_relaxed);
-}
-
-size_t pass_floats(int bt) { return (size_t)bt * (kMlpIn + 11 * kMlpHidden + 3 * kMlpOut) + 4 * 256; }
+size_t pass_floats(int bt) { return (size_t)bt * (2 * kMlpIn + 6 * kH); }
 
 void carve(float *base, int bt, Pass &p) {
-  const size_t H = (size_t)bt * kMlpHidden;
+  const size_t H = (size_t)bt * kH, I = (size_t)bt * kMlpIn;
   float *q = base;
-  p.A0 = q, q += (size_t)bt * kMlpIn;
-  p.Z1 = q, q += H;
-  p.A1 = q, q += H;
-  p.Z2 = q, q += H;
-  p.A2 = q, q += H;
-  p.Z3 = q, q += H;
-  p.A3 = q, q += H;
-  p.Z4 = q, q += (size_t)bt * kMlpOut;
-  p.D4 = q, q += (size_t)bt * kMlpOut;
-  p.D3 = q, q += H;
-  p.D2 = q, q += H;
-  p.D1 = q, q += H;
-  p.yb = reinterpret_cast<int *>(q);
+  for (float **a : {&p.A1, &p.A2, &p.A3, &p.D1, &p.D2, &p.D3}) *a = q, q += H;
+  for (float **a : {&p.A0, &p.D4}) *a = q, q += I;
+}
+
+cudaError_t run_rows(const Rows &rows, const float *theta, const Pass &p, float *logits, float *loss, cudaStream_t s) {
+  const int bytes = (int)sizeof(RowsShared);
+  cudaError_t e = cudaFuncSetAttribute(k_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return e;
+  k_rows<<<(rows.bt + kRowsPerBlock - 1) / kRowsPerBlock, 256, bytes, s>>>(rows, theta, p, logits, loss);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -434,76 +601,47 @@ int mlp_train(int n, const float *X, const int *y, float *theta, float *m1, floa
               float lr, unsigned seed, float *loss_out, cudaStream_t s) {
   if (n <= 0 || steps <= 0 || batch <= 0) return TREE2D_ERR_BAD_INPUT;
   float *buf = nullptr;
-  const size_t nf = pass_floats(batch) + 2 * kMlpParams + 1;
-  T2D_CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&buf), nf * sizeof(float)));
+  T2D_CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&buf), (pass_floats(batch) + 1) * sizeof(float)));
   Pass p;
   carve(buf, batch, p);
-  float *wb = buf + pass_floats(batch);
-  float *g = wb + kMlpParams;
-  float *loss = g + kMlpParams;
-  T2D_CUDA_TRY(cudaMemsetAsync(loss, 0, sizeof(float), s));
-  const int pb = (kMlpParams + 255) / 256;
-  for (int it = 0; it < steps; it++) {
-    k_round_weights<<<pb, 256, 0, s>>>(kMlpParams, theta, wb);
-    k_gather_batch<<<(batch + 255) / 256, 256, 0, s>>>(n, X, y, batch, seed + (unsigned)it * 7919u, p.A0, p.yb);
-    forward_pass(s, batch, wb, theta, p);
-    if (it == steps - 1) T2D_CUDA_TRY(cudaMemsetAsync(loss, 0, sizeof(float), s));
-    k_softmax_ce<<<(batch + 255) / 256, 256, 0, s>>>(batch, p.Z4, p.yb, p.D4, loss);
-    backward_pass(s, batch, wb, p, g);
+  float *loss = buf + pass_floats(batch);
+  cudaError_t e = cudaSuccess;
+  for (int it = 0; it < steps && e == cudaSuccess; it++) {
+    if (it == steps - 1) e = cudaMemsetAsync(loss, 0, sizeof(float), s);  // only the last step's is reported
+    if (e == cudaSuccess) e = run_rows(Rows{X, y, n, batch, 1, seed + (unsigned)it * 7919u}, theta, p, nullptr, loss, s);
     const float b1c = 1.f - powf(0.9f, (float)(it + 1)), b2c = 1.f - powf(0.999f, (float)(it + 1));
-    k_adam<<<pb, 256, 0, s>>>(kMlpParams, theta, m1, v1, g, lr, b1c, b2c);
-    g_launches.fetch_add(4, std::memory_order_relaxed);
+    if (e == cudaSuccess) e = run_weights(batch, p, nullptr, Adam{theta, m1, v1, lr, b1c, b2c}, s);
   }
-  T2D_CUDA_TRY(cudaGetLastError());
-  if (loss_out) T2D_CUDA_TRY(cudaMemcpyAsync(loss_out, loss, sizeof(float), cudaMemcpyDeviceToHost, s));
-  cudaError_t e = cudaStreamSynchronize(s);
+  if (e == cudaSuccess && loss_out) e = cudaMemcpyAsync(loss_out, loss, sizeof(float), cudaMemcpyDeviceToHost, s);
+  const cudaError_t es = cudaStreamSynchronize(s);
   cudaFree(buf);
   T2D_CUDA_TRY(e);
+  T2D_CUDA_TRY(es);
   return TREE2D_OK;
 }
 
 int mlp_grad(int n, const float *X, const int *y, const float *theta, float *grad, float *loss_out, cudaStream_t s) {
   if (n <= 0) return TREE2D_ERR_BAD_INPUT;
   float *buf = nullptr;
-  const size_t nf = pass_floats(n) + kMlpParams + 1;
-  T2D_CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&buf), nf * sizeof(float)));
+  T2D_CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&buf), (pass_floats(n) + 1) * sizeof(float)));
   Pass p;
   carve(buf, n, p);
-  float *wb = buf + pass_floats(n);
-  float *loss = wb + kMlpParams;
-  T2D_CUDA_TRY(cudaMemsetAsync(loss, 0, sizeof(float), s));
-  k_round_weights<<<(kMlpParams + 255) / 256, 256, 0, s>>>(kMlpParams, theta, wb);
-  k_gather_batch<<<(n + 255) / 256, 256, 0, s>>>(n, X, y, n, 0xffffffffu, p.A0, p.yb);
-  forward_pass(s, n, wb, theta, p);
-  k_softmax_ce<<<(n + 255) / 256, 256, 0, s>>>(n, p.Z4, p.yb, p.D4, loss);
-  backward_pass(s, n, wb, p, grad);
-  g_launches.fetch_add(3, std::memory_order_relaxed);
-  T2D_CUDA_TRY(cudaMemcpyAsync(loss_out, loss, sizeof(float), cudaMemcpyDeviceToHost, s));
-  cudaError_t e = cudaStreamSynchronize(s);
+  float *loss = buf + pass_floats(n);
+  cudaError_t e = cudaMemsetAsync(loss, 0, sizeof(float), s);
+  if (e == cudaSuccess) e = run_rows(Rows{X, y, n, n, 0, 0u}, theta, p, nullptr, loss, s);
+  if (e == cudaSuccess) e = run_weights(n, p, grad, Adam{}, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(loss_out, loss, sizeof(float), cudaMemcpyDeviceToHost, s);
+  const cudaError_t es = cudaStreamSynchronize(s);
   cudaFree(buf);
   T2D_CUDA_TRY(e);
+  T2D_CUDA_TRY(es);
   return TREE2D_OK;
 }
 
 int mlp_forward_cc(int n, const float *X, const float *theta, float *logits, cudaStream_t s) {
   if (n <= 0) return TREE2D_OK;
-  float *buf = nullptr;
-  const size_t nf = pass_floats(n) + kMlpParams;
-  T2D_CUDA_TRY(cudaMalloc(reinterpret_cast<void **>(&buf), nf * sizeof(float)));
-  Pass p;
-  carve(buf, n, p);
-  float *wb = buf + pass_floats(n);
-  int *yz = p.yb;
-  T2D_CUDA_TRY(cudaMemsetAsync(yz, 0, sizeof(int) * (size_t)n, s));
-  k_round_weights<<<(kMlpParams + 255) / 256, 256, 0, s>>>(kMlpParams, theta, wb);
-  // rows in order, labels unused
-  k_gather_batch<<<(n + 255) / 256, 256, 0, s>>>(n, X, yz, n, 0xffffffffu, p.A0, p.yb);
-  forward_pass(s, n, wb, theta, p);
-  T2D_CUDA_TRY(cudaMemcpyAsync(logits, p.Z4, sizeof(float) * (size_t)n * kMlpOut, cudaMemcpyDeviceToDevice, s));
-  g_launches.fetch_add(2, std::memory_order_relaxed);
-  cudaError_t e = cudaStreamSynchronize(s);
-  cudaFree(buf);
-  T2D_CUDA_TRY(e);
+  T2D_CUDA_TRY(run_rows(Rows{X, nullptr, n, n, 0, 0u}, theta, Pass{}, logits, nullptr, s));
+  T2D_CUDA_TRY(cudaStreamSynchronize(s));
   return TREE2D_OK;
 }
 

@@ -235,3 +235,29 @@ def test_far_orders_keep_accuracy(gpu_lib):
         P.learn_set_options()
         P.learn_set_envelope(0.0)
         P.set_mode(P.MODE_PLAIN)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 63, 64, 65, 193, 4097])
+def test_gradient_around_the_tiles(gpu_lib, n):
+    """The training kernels' gradient and logits for row counts around their
+    32-row and 64-row tiles, against the oracle (the tolerances of
+    test_training_gradient_matches_oracle: BF16 roundings that fall the other
+    way), and the labels' last class."""
+    from mlp_oracle import forward, init, loss_and_grad
+    P = gpu_lib
+    rng = np.random.default_rng(n)
+    X = rng.standard_normal((n, 16)).astype(np.float32)
+    y = rng.integers(0, 14, n).astype(np.int32)
+    y[-1] = 13
+    theta = init(n)
+    theta[[1024, 5184, 9344, 10432]] = 0.25  # biases, too
+    loss, g = P.mlp_grad(X, y, theta)
+    lref, gref = loss_and_grad(theta.astype(np.float64), X.astype(np.float64), y)
+    assert abs(loss - lref) <= 5e-5 * abs(lref)
+    # one activation rounded the other way moves a single row's gradient by
+    # about 2^-8 of it: 5e-4 of the mean over many rows
+    assert np.linalg.norm(g - gref) <= (5e-4 if n > 32 else 4e-3) * np.linalg.norm(gref)
+    z = P.mlp_forward(X, theta)
+    zref = forward(theta.astype(np.float64), X.astype(np.float64))[0]
+    assert np.quantile(np.abs(z - zref), 0.99) <= 2e-2 * np.abs(zref).max()
