@@ -1,9 +1,10 @@
 // FP64 direct O(N*M) sum of the regularised Biot-Savart kernel: the yardstick
 // of the approximate modes.  The pair kernel is direct_evaluate's
-// (ver-c/src/fmm.c:121-142, r > 1e-10) applied to every source.  Sources are
-// staged through shared memory in tiles (with 1/sigma^2 per source); one
-// thread per target.
+// (ver-c/src/fmm.c:121-142, r > 1e-10) applied to every source, in 64-bit
+// fixed point (fix64.cuh).  Sources are staged through shared memory in tiles,
+// decoded once; one thread per target.
 #include "dev_common.cuh"
+#include "fix64.cuh"
 #include "tc_ptx.cuh"
 
 namespace t2d {
@@ -23,47 +24,93 @@ __device__ __forceinline__ double rcp_nr(double x) {
   return y;
 }
 
+__device__ const fix::ExpTables g_exp = fix::make_exp_tables();
+
+// A source as the pairs need it: |G| and 1/sigma^2 as mantissas and exponent
+// fields (fix::mantissa), the upper word of G for its sign.  `odd`: a NaN or
+// an infinity among its numbers (not a core radius of 0 or infinity), whose
+// pairs run in FP64 so that they come out as they always did.
+struct Source {
+  double x, y;
+  uint64_t gm, cm;
+  int ge, ce;
+  uint32_t gh;
+  int odd;
+};
+
+// The pair in FP64: (r/sigma)^2 as r2 / sigma^2 and 1/r2 by a Newton-refined
+// reciprocal; r > 1e-10 <=> r2 > 1e-20.
+__device__ __noinline__ void pair64(double rx, double ry, double g, double rc, double &ax, double &ay) {
+  const double ic = 1.0 / (rc * rc);
+  const double r2 = rx * rx + ry * ry;
+  if (r2 > 1.0e-20) {
+    const double x2 = r2 * ic;
+    const double e1 = x2 > 40.0 ? 1.0 : 1.0 - exp(-x2);
+    const double rv = g * e1 * rcp_nr(r2);
+    ax -= rv * ry;
+    ay += rv * rx;
+  }
+}
+
 // grid.y splits the sources into chunks; each block adds its partial sums
-// into uv (zeroed by the caller) with FP64 atomics.
+// into uv (zeroed by the caller) with FP64 atomics.  Bound by the dispatch of
+// integer instructions (two cycles each): 16,384 targets x 262,144 two-patch
+// sources take 32 ms, 125 ms with the pairs in FP64.
 __global__ void __launch_bounds__(kThreads) k_direct(int ntgt, const double *__restrict__ txy, int nsrc,
                                                      const double *__restrict__ sxy, const double *__restrict__ cir,
-                                                     const double *__restrict__ cor, double *__restrict__ uv,
-                                                     int chunk) {
-  __shared__ double sx[kThreads], sy[kThreads], sg[kThreads], sr2[kThreads];
+                                                     const double *__restrict__ cor, double *__restrict__ uv, int chunk,
+                                                     fix::One one) {
+  __shared__ Source src[kThreads];
+  __shared__ uint64_t s_exp_int[fix::kExpInts], s_exp_frac[fix::kExpFracs];
+  for (int j = threadIdx.x; j < fix::kExpFracs; j += kThreads) s_exp_frac[j] = g_exp.fracs[j];
+  for (int j = threadIdx.x; j < fix::kExpInts; j += kThreads) s_exp_int[j] = g_exp.ints[j];
   const long i = blockIdx.x * (long)kThreads + threadIdx.x;
   const bool valid = i < ntgt;
   const double x = valid ? txy[2 * i] : 0.0, y = valid ? txy[2 * i + 1] : 0.0;
-  double ax = 0.0, ay = 0.0;
+  int odd_target = !isfinite(x) || !isfinite(y);
+  asm volatile("" : "+r"(odd_target));  // once: not as two FP64 comparisons per pair
+  fix::Sum2 sum;
+  double ax = 0.0, ay = 0.0;  // the FP64 pairs
   const int s0 = blockIdx.y * chunk;
   const int s1 = min(nsrc, s0 + chunk);
   for (int base = s0; base < s1; base += kThreads) {
     const int j = base + threadIdx.x;
+    __syncthreads();
     if (j < s1) {
-      sx[threadIdx.x] = sxy[2 * (long)j];
-      sy[threadIdx.x] = sxy[2 * (long)j + 1];
-      sg[threadIdx.x] = cir[j];
-      sr2[threadIdx.x] = 1.0 / (cor[j] * cor[j]);
+      const double sx = sxy[2 * (long)j], sy = sxy[2 * (long)j + 1], g = cir[j], rc = cor[j];
+      const double ic = 1.0 / (rc * rc);
+      Source q;
+      q.x = sx;
+      q.y = sy;
+      q.gm = fix::mantissa(g, q.ge);
+      q.cm = fix::mantissa(ic, q.ce);
+      q.gh = fix::hi32(fix::bits(g));
+      q.odd = !isfinite(sx) || !isfinite(sy) || !isfinite(g) || isnan(rc);
+      src[threadIdx.x] = q;
     }
     __syncthreads();
     const int cnt = min(kThreads, s1 - base);
-    // (r/sigma)^2 as r2 / sigma^2 and 1/r2 by a Newton-refined reciprocal:
-    // the same quantities within an ulp or two, without a square root or
-    // an IEEE division per pair; r > 1e-10 <=> r2 > 1e-20
-    for (int k = 0; k < cnt; k++) {
-      const double rx = x - sx[k];
-      const double ry = y - sy[k];
-      const double r2 = rx * rx + ry * ry;
-      if (r2 > 1.0e-20) {
-        const double x2 = r2 * sr2[k];
-        const double e1 = x2 > 40.0 ? 1.0 : 1.0 - exp(-x2);
-        const double rv = sg[k] * e1 * rcp_nr(r2);
-        ax -= rv * ry;
-        ay += rv * rx;
+    for (int k0 = 0; k0 < cnt; k0 += 32) {
+      fix::settle(sum);
+      const int k1 = min(cnt, k0 + 32);
+      for (int k = k0; k < k1; k++) {
+        const Source &q = src[k];
+        const double rx = fix::minus(x, q.x);
+        const double ry = fix::minus(y, q.y);
+        const fix::Vec v = fix::vec(rx, ry);
+        if (q.odd || odd_target || v.e == 0x7ff) {
+          pair64(rx, ry, cir[base + k], cor[base + k], ax, ay);
+          continue;
+        }
+        if (fix::apart(v, rx, ry))
+          fix::add_pair(sum, v, fix::hi32(fix::bits(rx)), fix::hi32(fix::bits(ry)), q.gm, q.ge, q.gh, q.cm, q.ce,
+                        s_exp_int, s_exp_frac, one);
       }
     }
-    __syncthreads();
   }
   if (valid) {
+    ax += fix::to_double(sum.x, sum.xl, sum.e);
+    ay += fix::to_double(sum.y, sum.yl, sum.e);
     atomicAdd(&uv[2 * i], 0.5 * ax / kPi);
     atomicAdd(&uv[2 * i + 1], 0.5 * ay / kPi);
   }
@@ -227,7 +274,7 @@ cudaError_t direct_sum(int ntgt, const double *txy, int nsrc, const double *sxy,
   if (chunk < kThreads) chunk = kThreads;
   chunks = (nsrc + chunk - 1) / chunk;
   if (chunks < 1) chunks = 1;
-  k_direct<<<dim3(tblocks, chunks), kThreads, 0, s>>>(ntgt, txy, nsrc, sxy, cir, cor, uv, chunk);
+  k_direct<<<dim3(tblocks, chunks), kThreads, 0, s>>>(ntgt, txy, nsrc, sxy, cir, cor, uv, chunk, fix::One());
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   return cudaGetLastError();
 }

@@ -285,11 +285,65 @@ T2D_HD double to_double(int64_t v, uint32_t l, int e) {
 }
 
 // ------------------------------------------------------ regularised pair
+// r > 1e-10 (fmm.c:131), decided on r^2 > 1e-20 in FP64 where the exponent
+// leaves it open: a component of 2^-33 or more decides it (field 990), none of
+// 2^-34 or more rules it out.  The call keeps the FP64 products out of the
+// pairs that do not need them (the compiler would predicate them into all).
+#ifdef __CUDACC__
+static __device__ __noinline__ bool apart64(double dx, double dy) {
+  return __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)) > 1.0e-20;
+}
+// a - b, once: opaque to the compiler, which would otherwise subtract again
+// where it needs the sign (it takes FP64 additions to be cheap)
+static __device__ __forceinline__ double minus(double a, double b) {
+  double d = __dsub_rn(a, b);
+  asm volatile("" : "+d"(d));
+  return d;
+}
+static __device__ __forceinline__ bool apart(const Vec &v, double dx, double dy) {
+  return v.e >= 990 || (v.e == 989 && apart64(dx, dy));
+}
+#endif
+
 // e^-x = kExpInt[floor(x)] kExpFrac[next 11 bits] e^-r, r < 2^-11: a
 // table-driven exponential (P. T. P. Tang, ACM TOMS 15, 1989) with both
 // tables in units of 2^-62.
 constexpr int kExpInts = 40;  // e^-40 < 2^-57: 1 - e^-x is 1 from there on
 constexpr int kExpFracs = 2048;
+struct ExpTables {
+  uint64_t ints[kExpInts], fracs[kExpFracs];
+};
+typedef unsigned __int128 u128;
+// e^-(j / 2048) in units of 2^-100 by its Taylor series in integers
+constexpr u128 exp_series(int j) {
+  u128 t = (u128)1 << 100, pos = t, neg = 0;
+  for (int k = 1; t; k++) {
+    t = (t * (unsigned)j >> 11) / (unsigned)k;
+    if (k & 1)
+      neg += t;
+    else
+      pos += t;
+  }
+  return pos - neg;
+}
+// high 128 bits of a product
+constexpr u128 mul128(u128 a, u128 b) {
+  const uint64_t ah = (uint64_t)(a >> 64), al = (uint64_t)a, bh = (uint64_t)(b >> 64), bl = (uint64_t)b;
+  const u128 m1 = (u128)ah * bl, m2 = (u128)al * bh, l = (u128)al * bl;
+  const u128 mid = (l >> 64) + (uint64_t)m1 + (uint64_t)m2;
+  return (u128)ah * bh + (m1 >> 64) + (m2 >> 64) + (mid >> 64);
+}
+constexpr ExpTables make_exp_tables() {
+  ExpTables r{};
+  for (int j = 0; j < kExpFracs; j++) r.fracs[j] = (uint64_t)((exp_series(j) + ((u128)1 << 37)) >> 38);
+  const u128 e1 = exp_series(kExpFracs) << 27;  // e^-1, units of 2^-127
+  u128 v = (u128)1 << 127;
+  for (int n = 0; n < kExpInts; n++) {
+    r.ints[n] = (uint64_t)((v + ((u128)1 << 64)) >> 65);
+    v = mul128(v, e1) << 1;
+  }
+  return r;
+}
 
 // Adds G (1 - exp(-r^2 / sigma^2)) / r^2 times (-dy, dx) to `sum`, for the
 // offset (dx, dy) = v whose upper words are hx, hy: |G| = gm 2^(ge - 1085),
@@ -298,32 +352,36 @@ constexpr int kExpFracs = 2048;
 // an absolute 2^-55 in the bracket.
 T2D_HD void add_pair(Sum2 &sum, const Vec &v, uint32_t hx, uint32_t hy, uint64_t gm, int ge, uint32_t hg, uint64_t cm,
                      int ce, const uint64_t *exp_int, const uint64_t *exp_frac, One one) {
+  if (gm == 0) return;
   const uint64_t m2 = norm2(v, one);
-  const uint64_t y = recip(m2, one);
+  // f 2^z = (1 - e^-x) / r^2; where e^-x is nothing, the reciprocal
+  uint64_t f = recip(m2, one);
+  int z = 4;
   // x = r^2 / sigma^2 in units of 2^-55, below 64; a product of 2^60 or more
   // with a left shift would be x >= 64
   const int s = 3074 - 2 * v.e - ce;
-  const uint64_t x = shr(mulhi(m2, cm, one) << 2, s);
-  const uint32_t n = hi32(x) >> 23;
-  uint64_t d = 1ull << 60;  // 1 - e^-x in units of 2^-60
-  if (s >= 0 && n < kExpInts) {
-    if (x == 0) return;  // below 2^-55
-    const uint64_t t = mulhi(exp_int[n], exp_frac[(hi32(x) >> 12) & (kExpFracs - 1)], one);
-    // u = 1 - e^-r = r - r^2/2 + r^2/2 r/3 (1 - r/4) in units of 2^-64, from
-    // r = a 2^-43 + b 2^-55
-    const uint64_t r = x & ((1ull << 44) - 1);
-    const uint32_t a = (uint32_t)(r >> 12), b = (uint32_t)r & 4095u;
-    const uint32_t p = hi32(wide(hi32(wide(a, 0x55555555u)), ~(a >> 13)));  // r/3 (1 - r/4), 2^-43
-    const uint64_t rr = wide(a, a, wide(a, b) >> 11);                       // r^2, 2^-86
-    // x was truncated: half a unit on average
-    const uint64_t u = wide(hi32(wide(hi32(rr), p)) >> 2, (uint32_t)one.v, ((r << 9) | 256) - (rr >> 23));
-    d = d - t + mulhi(t, u, one);
+  if (s >= 0) {
+    const uint64_t x = shr(mulhi(m2, cm, one) << 2, s);
+    const uint32_t n = hi32(x) >> 23;
+    if (n < kExpInts) {
+      if (x == 0) return;  // below 2^-55
+      const uint64_t t = mulhi(exp_int[n], exp_frac[(hi32(x) >> 12) & (kExpFracs - 1)], one);
+      // u = 1 - e^-r = r - r^2/2 + r^2/2 r/3 (1 - r/4) in units of 2^-64, from
+      // r = a 2^-43 + b 2^-55
+      const uint64_t r = x & ((1ull << 44) - 1);
+      const uint32_t a = (uint32_t)(r >> 12), b = (uint32_t)r & 4095u;
+      const uint32_t p = hi32(wide(hi32(wide(a, 0x55555555u)), ~(a >> 13)));  // r/3 (1 - r/4), 2^-43
+      const uint64_t rr = wide(a, a, wide(a, b) >> 11);                       // r^2, 2^-86
+      // x was truncated: half a unit on average
+      const uint64_t u = wide(hi32(wide(hi32(rr), p)) >> 2, (uint32_t)one.v, ((r << 9) | 256) - (rr >> 23));
+      const uint64_t d = (1ull << 60) - t + mulhi(t, u, one);  // 1 - e^-x in units of 2^-60
+      // leading one to bit 62 (to bit 31 or above where 1 - e^-x < 2^-28 has
+      // fewer than 30 significant bits anyway)
+      z = clz32(hi32(d) | 1u) - 1;
+      f = mulhi(d << z, f, one);
+    }
   }
-  if (gm == 0) return;
-  // leading one to bit 62 (to bit 31 or above where 1 - e^-x < 2^-28 has
-  // fewer than 30 significant bits anyway)
-  const int z = clz32(hi32(d) | 1u) - 1;
-  const uint64_t f = mulhi(mulhi(d << z, y, one), gm, one);
+  f = mulhi(f, gm, one);
   const uint64_t px = mulhi(f, v.mx, one), py = mulhi(f, v.my, one);
   const int64_t sx = (int32_t)(hg ^ hx) >> 31, sy = ~((int32_t)(hg ^ hy) >> 31);
   add(sum, ((int64_t)py ^ sy) - sy, ((int64_t)px ^ sx) - sx, ge - v.e - z - 55);

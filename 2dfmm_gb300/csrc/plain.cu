@@ -19,8 +19,6 @@
 //              four partial sums are added in a fixed order at the end.  Both
 //              in 64-bit fixed point (fix64.cuh): FP64 runs at 1/64 of the
 //              FP32 rate here.
-#include <mutex>
-
 #include "dev_common.cuh"
 #include "fix64.cuh"
 
@@ -46,9 +44,7 @@ __device__ __forceinline__ double2 cfma(double2 a, double2 b, double2 c) {
   return make_double2(__fma_rn(a.x, b.x, __fma_rn(-a.y, b.y, c.x)), __fma_rn(a.x, b.y, __fma_rn(a.y, b.x, c.y)));
 }
 
-// e^-n and e^-(j / 2048) in units of 2^-62 (fix64.cuh)
-__device__ uint64_t g_exp_int[fix::kExpInts];
-__device__ uint64_t g_exp_frac[fix::kExpFracs];
+__device__ const fix::ExpTables g_exp = fix::make_exp_tables();
 
 constexpr double kPi = 3.14159265358979323846;
 
@@ -224,8 +220,8 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
   __shared__ unsigned s_mask[kEvalWarps][kStackCap];
   __shared__ int s_queue[kEvalWarps][kEvalTargets][kQueue];
   __shared__ uint64_t s_exp_int[fix::kExpInts], s_exp_frac[fix::kExpFracs];
-  for (int j = threadIdx.x; j < fix::kExpFracs; j += kEvalWarps * 32) s_exp_frac[j] = g_exp_frac[j];
-  for (int j = threadIdx.x; j < fix::kExpInts; j += kEvalWarps * 32) s_exp_int[j] = g_exp_int[j];
+  for (int j = threadIdx.x; j < fix::kExpFracs; j += kEvalWarps * 32) s_exp_frac[j] = g_exp.fracs[j];
+  for (int j = threadIdx.x; j < fix::kExpInts; j += kEvalWarps * 32) s_exp_int[j] = g_exp.ints[j];
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane & (kShare - 1), tgt = lane / kShare;
@@ -273,8 +269,8 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
       if (k < nq) {
         // M2S, fmm.c:60-67: sum_{k<nt-1} a_k w^{k+1}, w = 1/(z - zc)
         const int cc = s_queue[warp][tgt][(qh + k) & (kQueue - 1)];
-        const double dx = __dsub_rn(x, t.cx[cc]);
-        const double dy = __dsub_rn(y, t.cy[cc]);
+        const double dx = fix::minus(x, t.cx[cc]);
+        const double dy = fix::minus(y, t.cy[cc]);
         bool done = false;
         if constexpr (kForm != kFormFp64) {
           const longlong2 *cf = reinterpret_cast<const longlong2 *>(t.fix) + (size_t)cc * nt;
@@ -329,20 +325,19 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
           fix::settle(near);
           const int j1 = min(e, j0 + 32 * kShare);
           for (int j = j0 + sub; j < j1; j += kShare) {
-            const double rx = __dsub_rn(x, t.x[j]);
-            const double ry = __dsub_rn(y, t.y[j]);
+            const double rx = fix::minus(x, t.x[j]);
+            const double ry = fix::minus(y, t.y[j]);
             // The reference forms r = sqrt(r2), (r/sigma)^2 and 1/(r*r); r2 and
             // r2/sigma^2 (1/sigma^2 precomputed per blob) give the same
-            // quantities.  r > 1e-10 is sure from a component of 2^-32 on
-            // (exponent field 991), ruled out below 2^-34, and otherwise
-            // decided on r2 > 1e-20 in FP64.
+            // quantities.
             const fix::Vec v = fix::vec(rx, ry);
-            bool apart = v.e >= 991;
-            if (!apart && v.e >= 989) apart = __dadd_rn(__dmul_rn(rx, rx), __dmul_rn(ry, ry)) > 1.0e-20;
-            if (apart) {
-              int ge, ce;
-              const double g = t.cir[j];
-              const uint64_t gm = fix::mantissa(g, ge), cm = fix::mantissa(t.icor2[j], ce);
+            if (fix::apart(v, rx, ry)) {
+              int ge;
+              const double g = t.cir[j], ic = t.icor2[j];
+              const uint64_t gm = fix::mantissa(g, ge);
+              // 1/sigma^2 of zero or below the normal range makes x = 0 with any mantissa
+              const int ce = (int)(fix::bits(ic) >> 52);
+              const uint64_t cm = ((fix::bits(ic) << 10) & 0x3fffffffffffffffull) | 0x4000000000000000ull;
               fix::add_pair(near, v, fix::hi32(fix::bits(rx)), fix::hi32(fix::bits(ry)), gm, ge,
                             fix::hi32(fix::bits(g)), cm, ce, s_exp_int, s_exp_frac, a.one);
             }
@@ -529,55 +524,9 @@ cudaError_t mac_bounds(Workspace &ws, const Tree &t, double theta, int nt, cudaS
   return e;
 }
 
-// High 128 bits of a product of 128-bit numbers.
-unsigned __int128 mul128(unsigned __int128 a, unsigned __int128 b) {
-  const uint64_t ah = (uint64_t)(a >> 64), al = (uint64_t)a, bh = (uint64_t)(b >> 64), bl = (uint64_t)b;
-  const unsigned __int128 m1 = (unsigned __int128)ah * bl, m2 = (unsigned __int128)al * bh,
-                          l = (unsigned __int128)al * bl;
-  const unsigned __int128 mid = (l >> 64) + (uint64_t)m1 + (uint64_t)m2;
-  return (unsigned __int128)ah * bh + (m1 >> 64) + (m2 >> 64) + (mid >> 64);
-}
-
-// e^-(j / 2048) in units of 2^-100 by its Taylor series in integers.
-unsigned __int128 exp_series(int j) {
-  const unsigned __int128 one = (unsigned __int128)1 << 100;
-  unsigned __int128 t = one, pos = one, neg = 0;
-  for (int k = 1; t; k++) {
-    t = (t * (unsigned)j >> 11) / (unsigned)k;
-    (k & 1 ? neg : pos) += t;
-  }
-  return pos - neg;
-}
-
-// The exponential's tables, uploaded once per device (they live in each
-// device's copy of the module).
-std::mutex g_tables_mu;
-bool g_tables_ready[64] = {};
-
-cudaError_t upload_tables() {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return e;
-  std::lock_guard<std::mutex> lk(g_tables_mu);
-  if (dev >= 0 && dev < 64 && g_tables_ready[dev]) return cudaSuccess;
-  static uint64_t ints[fix::kExpInts], fracs[fix::kExpFracs];
-  for (int j = 0; j < fix::kExpFracs; j++) fracs[j] = (uint64_t)((exp_series(j) + ((unsigned __int128)1 << 37)) >> 38);
-  const unsigned __int128 e1 = exp_series(fix::kExpFracs) << 27;  // e^-1, units of 2^-127
-  unsigned __int128 v = (unsigned __int128)1 << 127;
-  for (int n = 0; n < fix::kExpInts; n++) {
-    ints[n] = (uint64_t)((v + ((unsigned __int128)1 << 64)) >> 65);
-    v = mul128(v, e1) << 1;
-  }
-  e = cudaMemcpyToSymbol(g_exp_int, ints, sizeof(ints));
-  if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_exp_frac, fracs, sizeof(fracs));
-  if (e == cudaSuccess && dev >= 0 && dev < 64) g_tables_ready[dev] = true;
-  return e;
-}
-
 }  // namespace
 
 int plain_upward(Workspace &ws, const Tree &t, const Params &p, cudaStream_t s) {
-  T2D_CUDA_TRY(upload_tables());
   const int nt = p.nterms;
   if (nt <= 0 || t.ncell <= 0) return TREE2D_OK;
   ws.mac_theta = -1.0;  // the climb uses the bounds' memory
