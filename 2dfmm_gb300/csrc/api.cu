@@ -138,6 +138,8 @@ struct Solver {
   Arena io;       // device copies of host inputs and outputs
   Arena targets;  // evaluation-order targets
   Arena lookup;   // query points and answers of a batch lookup
+  Arena resolve;  // its misses
+  Arena table;    // the blobs by position
   Arena keyed;    // the blobs as targets in key order (plain evaluation)
 };
 
@@ -171,6 +173,9 @@ struct Lib {
   // position -> blob index, built on first need
   std::mutex hash_mu;
   std::atomic<bool> hash_ready{false};
+  bool table_ready = false;  // the same on the device (Solver::table), for batch queries
+  const int *d_slot = nullptr;
+  unsigned slot_mask = 0;
   std::vector<int> hash_slot;
   size_t hash_mask = 0;
   tree2d_stats_t stats{};
@@ -446,24 +451,18 @@ long find_blob(Lib &L, double x, double y) {
   return find_blob_from(L, x, y, hint);
 }
 
-// GPU evaluation of m arbitrary points (host xy) into host uv; L.mu held.
-int eval_points(Lib &L, int m, const double *xy, double *uv) {
+// Evaluation of m arbitrary device points into device uv on the library's
+// stream; L.mu held.  Returns the status after the stream is done.
+int eval_device_points(Lib &L, int m, const double *d_xy, double *d_uv) {
   Solver &S = L.main;
-  if (L.n == 0) {
-    for (int i = 0; i < 2 * m; i++) uv[i] = 0.0;
-    return TREE2D_OK;
-  }
   cudaStream_t s = L.stream;
-  size_t need = Arena::bytes_for(2 * (size_t)m, 8) * 2 + Arena::bytes_for(m, 8) * 2 + Arena::bytes_for(m, 4) * 2;
+  size_t need = Arena::bytes_for(m, 8) * 2 + Arena::bytes_for(m, 4) * 2;
   T2D_CUDA_TRY(S.targets.reserve(need));
   S.targets.reset();
-  double *d_xy = S.targets.take<double>(2 * (size_t)m);
-  double *d_uv = S.targets.take<double>(2 * (size_t)m);
   double *tx = S.targets.take<double>(m);
   double *ty = S.targets.take<double>(m);
   int *order = S.targets.take<int>(m);
   int *out = S.targets.take<int>(m);
-  T2D_CUDA_TRY(cudaMemcpyAsync(d_xy, xy, sizeof(double) * 2 * (size_t)m, cudaMemcpyHostToDevice, s));
   int rc;
   // Points off the blobs: after a plain make_tree the plain FP64 treecode
   // (the reference's method); after a mixed or learned one a traversal of
@@ -474,6 +473,7 @@ int eval_points(Lib &L, int m, const double *xy, double *uv) {
     if (rc) return rc;
     S.plain_coef = true;
   }
+  T2D_CUDA_TRY(cudaMemsetAsync(S.ws.status, 0, sizeof(DevStatus), s));
   if (m > 1024) {
     rc = sort_targets(S.ws, m, d_xy, S.tree.root, order, s);
     if (rc) return rc;
@@ -482,37 +482,55 @@ int eval_points(Lib &L, int m, const double *xy, double *uv) {
     rc = gather_targets(m, d_xy, nullptr, tx, ty, out, s);
   }
   if (rc) return rc;
-  T2D_CUDA_TRY(cudaMemsetAsync(S.ws.status, 0, sizeof(DevStatus), s));
   rc = mixed ? mixed_eval_points(S.ws, m, tx, ty, out, d_uv, s)
              : plain_evaluate(S.ws, S.tree, L.params, m, tx, ty, out, d_uv, s);
   if (rc) return rc;
-  T2D_CUDA_TRY(cudaMemcpyAsync(uv, d_uv, sizeof(double) * 2 * (size_t)m, cudaMemcpyDeviceToHost, s));
   T2D_CUDA_TRY(cudaMemcpyAsync(S.ws.h_status, S.ws.status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
   T2D_CUDA_TRY(cudaStreamSynchronize(s));
   return S.ws.h_status->err;
 }
 
+// The same for one point in host memory.
+int eval_point(Lib &L, const double *xy, double *uv) {
+  if (L.n == 0) {
+    uv[0] = uv[1] = 0.0;
+    return TREE2D_OK;
+  }
+  Solver &S = L.main;
+  T2D_CUDA_TRY(S.resolve.reserve(2 * Arena::bytes_for(2, 8)));
+  S.resolve.reset();
+  double *d_xy = S.resolve.take<double>(2);
+  double *d_uv = S.resolve.take<double>(2);
+  T2D_CUDA_TRY(cudaMemcpyAsync(d_xy, xy, 2 * sizeof(double), cudaMemcpyHostToDevice, L.stream));
+  int rc = eval_device_points(L, 1, d_xy, d_uv);
+  if (rc) return rc;
+  T2D_CUDA_TRY(cudaMemcpyAsync(uv, d_uv, 2 * sizeof(double), cudaMemcpyDeviceToHost, L.stream));
+  T2D_CUDA_TRY(cudaStreamSynchronize(L.stream));
+  return TREE2D_OK;
+}
+
 }  // namespace
+
+// A batch lookup's buffers on the device.
+struct Lookup {
+  double *q = nullptr, *out = nullptr;
+  int *miss = nullptr;
+  int nmiss = 0;
+};
 
 // Batch lookup on the device: the queries go up in chunks on two streams
 // (one chunk's upload overlaps the previous chunk's download), query i is
 // matched against blob i, and the answers come back into uv.  Queries that
-// do not sit bitwise on their blob are returned in `miss` (ascending), with
-// NaN in uv.  L.mu held.
-int lookup_on_device(Lib &L, int n, const double *xy, double *uv, std::vector<int> &miss) {
-  miss.clear();
-  if (L.n == 0) {
-    miss.resize(n);
-    for (int i = 0; i < n; i++) miss[i] = i;
-    return TREE2D_OK;
-  }
+// do not sit bitwise on their blob are listed in lk.miss (in no order), with
+// NaN in uv.  L.mu held, L.n > 0.
+int lookup_on_device(Lib &L, int n, const double *xy, double *uv, Lookup &lk) {
   Solver &S = L.main;
   T2D_CUDA_TRY(S.lookup.reserve(Arena::bytes_for(2 * (size_t)n, 8) * 2 + Arena::bytes_for(n, 4) +
                                 Arena::bytes_for(1, 4)));
   S.lookup.reset();
-  double *q = S.lookup.take<double>(2 * (size_t)n);
-  double *out = S.lookup.take<double>(2 * (size_t)n);
-  int *midx = S.lookup.take<int>(n);
+  lk.q = S.lookup.take<double>(2 * (size_t)n);
+  lk.out = S.lookup.take<double>(2 * (size_t)n);
+  lk.miss = S.lookup.take<int>(n);
   int *cnt = S.lookup.take<int>(1);
   cudaStream_t st[2] = {L.stream, L.copy_stream};
   T2D_CUDA_TRY(cudaMemsetAsync(cnt, 0, sizeof(int), st[0]));
@@ -523,22 +541,68 @@ int lookup_on_device(Lib &L, int n, const double *xy, double *uv, std::vector<in
   for (long b = 0; b < n; b += chunk, k ^= 1) {
     const long e = std::min((long)n, b + chunk);
     const size_t bytes = sizeof(double) * 2 * (size_t)(e - b);
-    T2D_CUDA_TRY(cudaMemcpyAsync(q + 2 * b, xy + 2 * b, bytes, cudaMemcpyHostToDevice, st[k]));
-    T2D_CUDA_TRY(lookup_blobs(b, e, q, L.n, L.d_xy, L.d_uv, out, midx, cnt, st[k]));
-    T2D_CUDA_TRY(cudaMemcpyAsync(uv + 2 * b, out + 2 * b, bytes, cudaMemcpyDeviceToHost, st[k]));
+    T2D_CUDA_TRY(cudaMemcpyAsync(lk.q + 2 * b, xy + 2 * b, bytes, cudaMemcpyHostToDevice, st[k]));
+    T2D_CUDA_TRY(lookup_blobs(b, e, lk.q, L.n, L.d_xy, L.d_uv, lk.out, lk.miss, cnt, st[k]));
+    T2D_CUDA_TRY(cudaMemcpyAsync(uv + 2 * b, lk.out + 2 * b, bytes, cudaMemcpyDeviceToHost, st[k]));
   }
   T2D_CUDA_TRY(cudaEventRecord(L.ev_join, st[1]));
   T2D_CUDA_TRY(cudaStreamWaitEvent(st[0], L.ev_join, 0));
   T2D_CUDA_TRY(cudaMemcpyAsync(L.h_count, cnt, sizeof(int), cudaMemcpyDeviceToHost, st[0]));
   T2D_CUDA_TRY(cudaStreamSynchronize(st[0]));
-  const int nm = *L.h_count;
-  if (nm > 0) {
-    miss.resize(nm);
-    T2D_CUDA_TRY(cudaMemcpyAsync(miss.data(), midx, sizeof(int) * (size_t)nm, cudaMemcpyDeviceToHost, st[0]));
-    T2D_CUDA_TRY(cudaStreamSynchronize(st[0]));
-    std::sort(miss.begin(), miss.end());
-  }
+  lk.nmiss = *L.h_count;
   return TREE2D_OK;
+}
+
+// The missed queries: those at some blob's position take its velocity (a
+// table of the blobs by position, made on the first batch that needs it), the
+// rest are evaluated; everything stays on the device until the answers come
+// down to be put in their places.  `filled`: uv holds every answer that could
+// be formed (NaN for the others), whatever the status.  L.mu held.
+int resolve_misses(Lib &L, const Lookup &lk, double *uv, bool &filled) {
+  Solver &S = L.main;
+  cudaStream_t s = L.stream;
+  const size_t nm = (size_t)lk.nmiss;
+  if (!L.table_ready) {
+    size_t cap = 16;
+    while (cap < 2 * (size_t)L.n) cap <<= 1;
+    T2D_CUDA_TRY(S.table.reserve(Arena::bytes_for(cap, 4)));
+    S.table.reset();
+    int *slot = S.table.take<int>(cap);
+    T2D_CUDA_TRY(position_table(L.n, L.d_xy, slot, (unsigned)(cap - 1), s));
+    L.d_slot = slot;
+    L.slot_mask = (unsigned)(cap - 1);
+    L.table_ready = true;
+  }
+  T2D_CUDA_TRY(S.resolve.reserve(Arena::bytes_for(2 * nm, 8) * 3 + Arena::bytes_for(nm, 4) + Arena::bytes_for(1, 4)));
+  S.resolve.reset();
+  double *res = S.resolve.take<double>(2 * nm);
+  double *pts = S.resolve.take<double>(2 * nm);
+  double *puv = S.resolve.take<double>(2 * nm);
+  int *off = S.resolve.take<int>(nm);
+  int *noff = S.resolve.take<int>(1);
+  T2D_CUDA_TRY(position_find((int)nm, lk.miss, lk.q, L.d_xy, L.d_uv, L.d_slot, L.slot_mask, res, off, noff, s));
+  T2D_CUDA_TRY(cudaMemcpyAsync(L.h_count, noff, sizeof(int), cudaMemcpyDeviceToHost, s));
+  std::vector<int> miss(nm);
+  T2D_CUDA_TRY(cudaMemcpyAsync(miss.data(), lk.miss, sizeof(int) * nm, cudaMemcpyDeviceToHost, s));
+  T2D_CUDA_TRY(cudaStreamSynchronize(s));
+  const int no = *L.h_count;
+  int rc = TREE2D_OK;
+  if (no > 0) {
+    T2D_CUDA_TRY(off_points(no, off, lk.miss, lk.q, pts, s));
+    rc = eval_device_points(L, no, pts, puv);
+    if (rc == TREE2D_OK) T2D_CUDA_TRY(off_results(no, off, puv, res, s));
+  }
+  std::vector<double> ans(2 * nm);
+  T2D_CUDA_TRY(cudaMemcpyAsync(ans.data(), res, sizeof(double) * 2 * nm, cudaMemcpyDeviceToHost, s));
+  T2D_CUDA_TRY(cudaStreamSynchronize(s));
+  parallel_chunks((long)nm, 1 << 18, [&](long b, long e) {
+    for (long j = b; j < e; j++) {
+      uv[2 * (size_t)miss[j]] = ans[2 * j];
+      uv[2 * (size_t)miss[j] + 1] = ans[2 * j + 1];
+    }
+  });
+  filled = true;
+  return rc;
 }
 
 // Parameters in force for a device solve (as tree2d_solve_device resolves
@@ -574,6 +638,7 @@ void make_tree(int nvor_b, const double *vor_b, const double *cir_b, const doubl
   L.valid.store(false);
   L.host_ready.store(false);
   L.hash_ready.store(false);
+  L.table_ready = false;
   L.generation.fetch_add(1);
   L.last_error.store(TREE2D_OK);
   int rc = resolve_params(L);
@@ -669,7 +734,7 @@ void biot_tree(double x, double y, double *u, double *v) {
   }
   std::lock_guard<std::mutex> lk(L.mu);
   double xy[2] = {x, y}, uv[2];
-  int rc = eval_points(L, 1, xy, uv);
+  int rc = eval_point(L, xy, uv);
   if (rc) {
     fail(rc);
     *u = NAN;
@@ -689,54 +754,22 @@ int biot_tree_batch(int n, const double *xy, double *uv) {
   }
   if (n == 0) return TREE2D_OK;
   std::lock_guard<std::mutex> lk(L.mu);
-  std::vector<int> miss;
-  int rc = lookup_on_device(L, n, xy, uv, miss);
-  if (rc) {
+  if (L.n == 0) {
+    for (long i = 0; i < 2 * (long)n; i++) uv[i] = 0.0;
+    return TREE2D_OK;
+  }
+  Lookup found;
+  bool filled = false;
+  int rc = lookup_on_device(L, n, xy, uv, found);
+  if (rc == TREE2D_OK) {
+    if (found.nmiss == 0) return TREE2D_OK;
+    rc = resolve_misses(L, found, uv, filled);
+  }
+  if (rc && !filled) {
     // no copy into uv may still be in flight
     cudaStreamSynchronize(L.stream);
     cudaStreamSynchronize(L.copy_stream);
     for (long i = 0; i < 2 * (long)n; i++) uv[i] = NAN;
-    return fail(rc);
-  }
-  if (miss.empty()) return TREE2D_OK;
-  // Queries the device could not place: the host table (hash over the
-  // positions), then the treecode for points off the blobs.
-  rc = ensure_host_tables(L);
-  if (rc) {
-    for (int i : miss) uv[2 * (size_t)i] = uv[2 * (size_t)i + 1] = NAN;
-    return fail(rc);
-  }
-  const long nm = (long)miss.size();
-  const long grain = 1 << 14;
-  const long nparts = (nm + grain - 1) / grain;
-  std::vector<std::vector<int>> off_part(nparts);
-  parallel_chunks(nparts, 1, [&](long pb, long pe) {
-    for (long c = pb; c < pe; c++) {
-      long hint = -1;
-      for (long j = c * grain; j < std::min(nm, (c + 1) * grain); j++) {
-        const size_t i = (size_t)miss[j];
-        long k = find_blob_from(L, xy[2 * i], xy[2 * i + 1], hint);
-        if (k >= 0) {
-          uv[2 * i] = L.h_uv[2 * k];
-          uv[2 * i + 1] = L.h_uv[2 * k + 1];
-        } else {
-          off_part[c].push_back((int)i);
-        }
-      }
-    }
-  });
-  std::vector<int> off;
-  for (auto &m : off_part) off.insert(off.end(), m.begin(), m.end());
-  if (off.empty()) return TREE2D_OK;
-  std::vector<double> mxy(2 * off.size()), muv(2 * off.size());
-  for (size_t j = 0; j < off.size(); j++) {
-    mxy[2 * j] = xy[2 * (size_t)off[j]];
-    mxy[2 * j + 1] = xy[2 * (size_t)off[j] + 1];
-  }
-  rc = eval_points(L, (int)off.size(), mxy.data(), muv.data());
-  for (size_t j = 0; j < off.size(); j++) {
-    uv[2 * (size_t)off[j]] = rc ? NAN : muv[2 * j];
-    uv[2 * (size_t)off[j] + 1] = rc ? NAN : muv[2 * j + 1];
   }
   return rc ? fail(rc) : TREE2D_OK;
 }

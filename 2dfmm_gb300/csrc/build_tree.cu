@@ -383,6 +383,21 @@ __global__ void __launch_bounds__(256) k_keys(const double *__restrict__ xy, int
   vals[i] = (uint32_t)i;
 }
 
+// Points in Morton order, for warps of neighbours only: `levels` digits of the
+// position's fraction of the root box, packed over the point's index.
+__global__ void __launch_bounds__(256) k_point_keys(const double *__restrict__ xy, int n, const RootBox *__restrict__ root,
+                                                    int levels, uint64_t *__restrict__ words) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float rinv = __frcp_rn((float)root->region), span = (float)(1 << levels);
+  const float u = fmaf((float)(xy[2 * (long)i] - root->cx), rinv, 0.5f) * span;
+  const float v = fmaf((float)(root->cy - xy[2 * (long)i + 1]), rinv, 0.5f) * span;
+  const unsigned ix = (unsigned)fminf(fmaxf(u, 0.f), span - 1.f), iy = (unsigned)fminf(fmaxf(v, 0.f), span - 1.f);
+  uint64_t key = 0;
+  for (int l = levels - 1; l >= 0; l--) key = (key << 2) | ((ix >> l) & 1u) | (((iy >> l) & 1u) << 1);
+  words[i] = (key << (64 - 2 * levels)) | (uint64_t)(uint32_t)i;
+}
+
 __global__ void __launch_bounds__(256) k_cpl(const uint64_t *__restrict__ keys, int n, int num_p,
                                              uint8_t *__restrict__ cpl, uint8_t *__restrict__ w) {
   long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -1006,19 +1021,25 @@ retry:
 
 int sort_targets(Workspace &ws, int n, const double *d_xy, const RootBox *d_root, int *d_order, cudaStream_t s) {
   if (n <= 0) return TREE2D_OK;
-  size_t need = Arena::bytes_for(n, 8) * 2 + Arena::bytes_for(n, 4) + radix_sort_temp_bytes(n) + 512;
+  size_t need = Arena::bytes_for(n, 8) * 2 + radix_sort_temp_bytes(n) + 512;
   T2D_CUDA_TRY(ws.tmp_arena.reserve(need));
   ws.tmp_arena.reset();
-  uint64_t *k = ws.tmp_arena.take<uint64_t>(n);
-  uint64_t *k2 = ws.tmp_arena.take<uint64_t>(n);
-  uint32_t *v2 = ws.tmp_arena.take<uint32_t>(n);
+  uint64_t *a = ws.tmp_arena.take<uint64_t>(n);
+  uint64_t *b = ws.tmp_arena.take<uint64_t>(n);
   void *tmp = ws.tmp_arena.take<char>(radix_sort_temp_bytes(n));
-  // order only (for coherent warps): the short key depth is enough
-  k_keys<<<(n + 255) / 256, 256, 0, s>>>(d_xy, n, d_root, nullptr, 0, k, reinterpret_cast<uint32_t *>(d_order),
-                                          kShortKeyLevels, nullptr, 0, 0);
+  // only for warps of neighbours: digits down to about one point per cell
+  int levels = 4;
+  while (levels < 16 && (1l << (2 * levels)) < 4l * n) levels++;
+  const bool odd = ((2 * levels + 7) / 8) & 1;
+  k_point_keys<<<(n + 255) / 256, 256, 0, s>>>(d_xy, n, d_root, levels, a);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
-  T2D_CUDA_TRY(radix_sort_pairs(k, reinterpret_cast<uint32_t *>(d_order), k2, v2, n, 64 - 2 * kShortKeyLevels, 64,
-                                tmp, s));
+  if (n < 2) {
+    T2D_CUDA_TRY(cudaMemsetAsync(d_order, 0, sizeof(int), s));
+    return TREE2D_OK;
+  }
+  // the last pass reads `a` after an odd number of passes, `b` after an even one
+  T2D_CUDA_TRY(radix_sort_packed(a, b, n, 64 - 2 * levels, odd ? b : a, reinterpret_cast<uint32_t *>(d_order), tmp,
+                                 ws.status, s));
   return TREE2D_OK;
 }
 

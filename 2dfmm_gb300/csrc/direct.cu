@@ -241,6 +241,110 @@ cudaError_t lookup_blobs(long b, long e, const double *q, long nb, const double 
   return cudaGetLastError();
 }
 
+// ------------------------------------------------ blobs by their position
+
+namespace {
+
+__device__ __forceinline__ uint64_t mix64(uint64_t x) {
+  x += 0x9e3779b97f4a7c15ull;
+  x = (x ^ (x >> 30)) * 0xbf58476d1ce4e5b9ull;
+  x = (x ^ (x >> 27)) * 0x94d049bb133111ebull;
+  return x ^ (x >> 31);
+}
+__device__ __forceinline__ unsigned position_slot(double2 p, unsigned mask) {
+  return (unsigned)mix64((uint64_t)__double_as_longlong(p.x) ^ mix64((uint64_t)__double_as_longlong(p.y))) & mask;
+}
+__device__ __forceinline__ bool same_position(double2 a, double2 b) {
+  return __double_as_longlong(a.x) == __double_as_longlong(b.x) && __double_as_longlong(a.y) == __double_as_longlong(b.y);
+}
+
+// Open addressing, at most half full: slot = blob index + 1, the smallest of
+// the blobs that share a position bit for bit.
+__global__ void __launch_bounds__(256) k_position_insert(long n, const double2 *__restrict__ bxy, int *slot, unsigned mask) {
+  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double2 p = bxy[i];
+  unsigned h = position_slot(p, mask);
+  for (unsigned probe = 0; probe <= mask; probe++, h = (h + 1) & mask) {
+    const int cur = atomicCAS(&slot[h], 0, (int)i + 1);
+    if (cur == 0) return;
+    if (same_position(bxy[cur - 1], p)) {
+      atomicMin(&slot[h], (int)i + 1);
+      return;
+    }
+  }
+}
+
+// The missed queries miss[0..n): res[j] = the velocity of the blob at query
+// miss[j]'s position, else NaN and j appended to `off` (count in *noff).
+__global__ void __launch_bounds__(256) k_position_find(int n, const int *__restrict__ miss, const double2 *__restrict__ q,
+                                                       const double2 *__restrict__ bxy, const double2 *__restrict__ buv,
+                                                       const int *__restrict__ slot, unsigned mask, double2 *res,
+                                                       int *off, int *noff) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n) return;
+  const double2 p = q[miss[j]];
+  unsigned h = position_slot(p, mask);
+  for (unsigned probe = 0; probe <= mask; probe++, h = (h + 1) & mask) {
+    const int cur = slot[h];
+    if (cur == 0) break;
+    if (same_position(bxy[cur - 1], p)) {
+      res[j] = buv[cur - 1];
+      return;
+    }
+  }
+  res[j] = make_double2(NAN, NAN);
+  off[atomicAdd(noff, 1)] = j;
+}
+
+__global__ void __launch_bounds__(256) k_off_points(int n, const int *__restrict__ off, const int *__restrict__ miss,
+                                                    const double2 *__restrict__ q, double2 *pts) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < n) pts[k] = q[miss[off[k]]];
+}
+__global__ void __launch_bounds__(256) k_off_results(int n, const int *__restrict__ off, const double2 *__restrict__ uv,
+                                                     double2 *res) {
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k < n) res[off[k]] = uv[k];
+}
+
+cudaError_t launched() {
+  ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
+  return cudaGetLastError();
+}
+
+}  // namespace
+
+cudaError_t position_table(long n, const double *bxy, int *slot, unsigned mask, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(slot, 0, sizeof(int) * ((size_t)mask + 1), s);
+  if (e != cudaSuccess || n <= 0) return e;
+  k_position_insert<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(n, reinterpret_cast<const double2 *>(bxy), slot, mask);
+  return launched();
+}
+
+cudaError_t position_find(int n, const int *miss, const double *q, const double *bxy, const double *buv, const int *slot,
+                          unsigned mask, double *res, int *off, int *noff, cudaStream_t s) {
+  cudaError_t e = cudaMemsetAsync(noff, 0, sizeof(int), s);
+  if (e != cudaSuccess || n <= 0) return e;
+  k_position_find<<<(n + 255) / 256, 256, 0, s>>>(n, miss, reinterpret_cast<const double2 *>(q),
+                                                  reinterpret_cast<const double2 *>(bxy),
+                                                  reinterpret_cast<const double2 *>(buv), slot, mask,
+                                                  reinterpret_cast<double2 *>(res), off, noff);
+  return launched();
+}
+
+cudaError_t off_points(int n, const int *off, const int *miss, const double *q, double *pts, cudaStream_t s) {
+  k_off_points<<<(n + 255) / 256, 256, 0, s>>>(n, off, miss, reinterpret_cast<const double2 *>(q),
+                                               reinterpret_cast<double2 *>(pts));
+  return launched();
+}
+
+cudaError_t off_results(int n, const int *off, const double *uv, double *res, cudaStream_t s) {
+  k_off_results<<<(n + 255) / 256, 256, 0, s>>>(n, off, reinterpret_cast<const double2 *>(uv),
+                                                reinterpret_cast<double2 *>(res));
+  return launched();
+}
+
 cudaError_t advect(long n, double *xy, const double *uv, double dt, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
   k_advect<<<(int)((2 * n + 255) / 256), 256, 0, s>>>(n, xy, uv, dt);

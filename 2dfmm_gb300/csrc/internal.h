@@ -218,8 +218,8 @@ size_t build_tmp_bytes(int n, int nsets);
 // size the plain form's fixed-point coefficients replace the FP64 ones).
 size_t build_cell_bytes(long long ncell, long long nleaf, int nterms, bool fixed_arena);
 
-// Keys of arbitrary points against an existing root box, then sorted:
-// order[i] = index of the i-th target in key order.
+// Arbitrary points in Morton order of the root box (to about one point per
+// cell; points outside it at its edge): order[i] = index of the i-th.
 int sort_targets(Workspace &ws, int n, const double *d_xy, const RootBox *d_root, int *d_order,
                  cudaStream_t s);
 
@@ -267,6 +267,15 @@ cudaError_t advect(long n, double *xy, const double *uv, double dt, cudaStream_t
 // is bitwise at blob i, else NaN and i appended to miss (count in *nmiss).
 cudaError_t lookup_blobs(long b, long e, const double *q, long nb, const double *bxy, const double *buv, double *out,
                          int *miss, int *nmiss, cudaStream_t s);
+// Blobs by position: a table of mask + 1 slots (a power of two, over twice the
+// blobs), the queries miss[0..n) looked up in it (res[j] the velocity there,
+// else NaN and j appended to `off`), and the positions and results of those
+// left over.
+cudaError_t position_table(long n, const double *bxy, int *slot, unsigned mask, cudaStream_t s);
+cudaError_t position_find(int n, const int *miss, const double *q, const double *bxy, const double *buv, const int *slot,
+                          unsigned mask, double *res, int *off, int *noff, cudaStream_t s);
+cudaError_t off_points(int n, const int *off, const int *miss, const double *q, double *pts, cudaStream_t s);
+cudaError_t off_results(int n, const int *off, const double *uv, double *res, cudaStream_t s);
 // Blobs followed by their images in a wall at y = d (2n entries out).
 cudaError_t mirror_images(long n, const double *xy, const double *cir, const double *cor, double d, double *oxy,
                           double *ocir, double *ocor, cudaStream_t s);

@@ -1916,40 +1916,190 @@ __global__ void __launch_bounds__(32 * kWarps, (kWide ? 24 : 32) / kWarps) k_eva
 // ------------------------------------------------------------ off-blob points
 
 // Velocity at arbitrary points (not blob positions) on a mixed tree: one
-// warp per 32 points (in key order), each lane one point, the warp walking
-// the union of its lanes' traversals (a LIFO of cells with the lanes still
-// inside each).  A lane accepts a cell's multipole when the point is at
-// least kPtMac cell sides from the cell's centre (the scaled FP32 multipole
-// of order P then truncates at (sqrt(2)/2 / kPtMac)^P = 0.283^16 = 2e-9 of
-// the cell's field) and farther than the correction radius rc from the
-// cell's box (so the point-vortex form leaves out only exp(-rc^2/s^2)
-// terms, as the near field's correction list does).  Other cells are
-// descended; leaves are summed pair by pair with the regularised kernel
-// (fmm.c:121-142, the near field's FP32 pair), each leaf in FP32 and added
-// in FP64.  Cells without a multipole (the root and the level-1 cells above
-// the upward pass) are always descended.  The FP64 point is offset from
-// each cell's FP64 centre before rounding to FP32, as the near field's
-// centre offsets are.
+// warp per 8 points (in key order), four lanes per point, the warp walking
+// the union of its points' traversals (a LIFO of opened cells with the lanes
+// of the points that opened them).  A point accepts a cell's multipole when
+// it is at least kPtMac cell sides from the cell's centre (the scaled FP32
+// multipole of order P then truncates at (sqrt(2)/2 / kPtMac)^P = 0.283^16 =
+// 2e-9 of the cell's field) and farther than the correction radius rc from
+// the cell's box (so the point-vortex form leaves out only exp(-rc^2/s^2)
+// terms, as the near field's correction list does).  Other cells are opened;
+// leaves are summed pair by pair with the regularised kernel
+// (fmm.c:121-142, the near field's FP32 pair), each leaf in FP32.  Cells
+// without a multipole (the root and the level-1 cells above the upward pass)
+// are always opened.  The FP64 point is offset from each cell's FP64 centre
+// before rounding to FP32, as the near field's centre offsets are.
+//
+// FP64 runs at 1/64 of the FP32 rate, and the acceptance test took some 15
+// FP64 instructions per cell.  It is decided in FP32 with error bounds first
+// (far_from below), each of a point's lanes testing one child; accepted cells
+// and leaves wait in queues per point until every lane has one; the terms are
+// added in three-word FP32 sums, exact to 2^-72.  65,537 points around 262,144
+// two-patch blobs: 2.54 ms with one lane per point and all that in FP64,
+// 0.34 ms so.
 constexpr int kPtWarps = 4;
 constexpr int kPtStack = 160;
+constexpr int kPtShare = 4, kPtTargets = 32 / kPtShare;
+constexpr int kPtQueue = 64, kPtLeaves = 32;  // entries per point (rings)
 constexpr double kPtMac = 2.5;
+
+// A sum of FP32 terms in three words: each step's rounding error goes, exactly
+// (two-sum), to the next word.
+struct Sum3 {
+  float h = 0.f, m = 0.f, l = 0.f;
+  static __device__ __forceinline__ float two_sum(float &a, float b) {
+    const float s = __fadd_rn(a, b), t = __fsub_rn(s, a);
+    const float e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, t)), __fsub_rn(b, t));
+    a = s;
+    return e;
+  }
+  __device__ __forceinline__ void add(float v) { l = __fadd_rn(l, two_sum(m, two_sum(h, v))); }
+  __device__ __forceinline__ double value() const {
+    return isfinite(h) ? (double)h + ((double)m + (double)l) : (double)h;  // no inf - inf from the lower words
+  }
+};
+
+// The acceptance test of a cell with offset (dx, dy) and side `side`:
+// dx^2 + dy^2 >= mac2 side^2 and the point farther than rc from the box.
+__device__ __noinline__ bool far_from64(double x, double y, double cx, double cy, double side, double rc2) {
+  const double dx = x - cx, dy = y - cy;
+  const double gx = fmax(fabs(dx) - 0.5 * side, 0.0), gy = fmax(fabs(dy) - 0.5 * side, 0.0);
+  return dx * dx + dy * dy >= kPtMac * kPtMac * side * side && gx * gx + gy * gy > rc2;
+}
+
+// The same, decided in FP32 where that is sure.  (xh, xl) and (cxf, cxl) are
+// FP32 pairs, so |dxf - dx| <= ex below (2^-23 |dx| + 2^-46 (|x| + |cx|), over
+// twice that), and with q = 2^-20 the products' roundings (a few 2^-24) and
+// the FP32 side and rc^2 are covered: d2lo <= d2 <= d2hi and so on.  Values
+// below 1e-30 or overflowing comparisons decide nothing.
+__device__ __forceinline__ bool far_from(const MixedView &m, int c, double x, double y, float xh, float xl, float yh,
+                                         float yl, float sxy, double rc2, float rc2f) {
+  const float q = 0x1p-20f, side = m.h[c];
+  const float dx = fabsf(__fadd_rn(__fsub_rn(xh, m.cxf[c]), __fsub_rn(xl, m.cxl[c])));
+  const float dy = fabsf(__fadd_rn(__fsub_rn(yh, m.cyf[c]), __fsub_rn(yl, m.cyl[c])));
+  const float es = __fmul_rn(0x1p-44f, __fadd_rn(sxy, __fadd_rn(fabsf(m.cxf[c]), fabsf(m.cyf[c]))));
+  const float ex = fmaf(0x1p-22f, dx, es), ey = fmaf(0x1p-22f, dy, es);
+  const float xlo = fmaxf(dx - ex, 0.f), ylo = fmaxf(dy - ey, 0.f), xhi = dx + ex, yhi = dy + ey;
+  const float mac = (float)(kPtMac * kPtMac) * side * side;
+  const float hs = 0.5f * side, slack = q * side;
+  const float gxlo = fmaxf(xlo - hs - slack, 0.f), gylo = fmaxf(ylo - hs - slack, 0.f);
+  const float gxhi = fmaxf(xhi - hs + slack, 0.f), gyhi = fmaxf(yhi - hs + slack, 0.f);
+  const float d2lo = (1.f - q) * fmaf(xlo, xlo, ylo * ylo), d2hi = (1.f + q) * fmaf(xhi, xhi, yhi * yhi);
+  const float g2lo = (1.f - q) * fmaf(gxlo, gxlo, gylo * gylo), g2hi = (1.f + q) * fmaf(gxhi, gxhi, gyhi * gyhi);
+  const float mlo = (1.f - q) * mac, mhi = (1.f + q) * mac, rlo = (1.f - q) * rc2f, rhi = (1.f + q) * rc2f;
+  if (mlo > 1e-30f && d2hi < 3e38f) {
+    if (d2lo > mhi && g2lo > rhi && g2lo > 1e-30f) return true;
+    if (d2hi < mlo || (g2hi < rlo && rlo > 1e-30f)) return false;
+  }
+  return far_from64(x, y, m.cx[c], m.cy[c], m.region[c], rc2);
+}
 
 __global__ void __launch_bounds__(kPtWarps * 32) k_eval_points(MixedView m, int ntgt, const double *tx,
                                                                const double *ty, const int *out_idx, double *uv) {
   __shared__ int s_cell[kPtWarps][kPtStack];
   __shared__ unsigned s_mask[kPtWarps][kPtStack];
+  __shared__ int s_queue[kPtWarps][kPtTargets][kPtQueue];
+  __shared__ int s_leaves[kPtWarps][kPtTargets][kPtLeaves];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long i = ((long)blockIdx.x * kPtWarps + warp) * 32 + lane;
+  const int sub = lane & (kPtShare - 1), tgt = lane / kPtShare;
+  const long i = ((long)blockIdx.x * kPtWarps + warp) * kPtTargets + tgt;
   const bool valid = i < ntgt;
   const unsigned vmask = __ballot_sync(0xffffffffu, valid);
   if (vmask == 0) return;
   const double x = valid ? tx[i] : 0.0, y = valid ? ty[i] : 0.0;
+  const float xh = __double2float_rn(x), yh = __double2float_rn(y);
+  const float xl = __double2float_rn(x - (double)xh), yl = __double2float_rn(y - (double)yh);
+  const float sxy = __fadd_rn(fabsf(xh), fabsf(yh));
   const double rc = (double)*m.rc_ptr, rc2 = rc * rc;
-  const double mac2 = kPtMac * kPtMac;
+  const float rc2f = (float)rc2;
   const int P = m.P;
-  double phx = 0.0, phy = 0.0, ax = 0.0, ay = 0.0;
-  unsigned long long n_m2p = 0, n_pairs = 0;
+  Sum3 phx, phy, ax, ay;  // this lane's share
+  unsigned n_m2p = 0;
+  unsigned long long n_pairs = 0;
   bool overflow = false;
+
+  // Rounds of one entry per lane from a ring (head, count: the same in a
+  // point's four lanes); entry k of a point is lane k mod 4's whenever it is
+  // taken, so the sums do not depend on the warp's other points.
+  auto rounds_of = [&](int cnt, int keep, bool all) {
+    int hi = cnt, lo = cnt;
+    for (int o = 16; o >= kPtShare; o >>= 1) {
+      hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+      lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    }
+    return (all ? hi + kPtShare - 1 : max(lo, hi - keep + kPtShare - 1)) / kPtShare;
+  };
+  unsigned qh = 0, lh = 0;
+  int nq = 0, nl = 0;
+  auto flush_cells = [&](bool all) {
+    const int rounds = rounds_of(nq, kPtQueue - kPtShare, all);
+    const int first = (int)((unsigned)(sub - (int)qh) & (kPtShare - 1));
+    for (int r = 0; r < rounds; r++) {
+      const int k = first + r * kPtShare;
+      if (k < nq) {
+        // M2P: phi = (1/h) sum_k M_k w^(k+1), w = h / (z - zc)
+        const int c = s_queue[warp][tgt][(qh + k) & (kPtQueue - 1)];
+        const double dx = x - m.cx[c], dy = y - m.cy[c];
+        const float ih = m.inv_h[c];
+        const float zx = __fmul_rn((float)dx, ih), zy = __fmul_rn((float)dy, ih);
+        const float ir2 = __fdiv_rn(1.f, fmaf(zx, zx, __fmul_rn(zy, zy)));
+        const float2 w = make_float2(__fmul_rn(zx, ir2), -__fmul_rn(zy, ir2));
+        const float *MA = m.M + (size_t)c * 2 * P;
+        float2 a;
+        if (P == 16) {
+          float re[16], im[16];
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            *reinterpret_cast<float4 *>(re + 4 * q) = __ldg(reinterpret_cast<const float4 *>(MA) + q);
+            *reinterpret_cast<float4 *>(im + 4 * q) = __ldg(reinterpret_cast<const float4 *>(MA) + 4 + q);
+          }
+          a = make_float2(re[15], im[15]);
+#pragma unroll
+          for (int q = 14; q >= 0; q--) {
+            a = fmul(a, w);
+            a.x = __fadd_rn(a.x, re[q]);
+            a.y = __fadd_rn(a.y, im[q]);
+          }
+        } else {
+          a = make_float2(MA[P - 1], MA[2 * P - 1]);
+          for (int q = P - 2; q >= 0; q--) {
+            a = fmul(a, w);
+            a.x = __fadd_rn(a.x, MA[q]);
+            a.y = __fadd_rn(a.y, MA[P + q]);
+          }
+        }
+        a = fmul(a, w);
+        phx.add(__fmul_rn(a.x, ih));
+        phy.add(__fmul_rn(a.y, ih));
+      }
+    }
+    const int out = min(rounds * kPtShare, nq);
+    qh += (unsigned)out;
+    nq -= out;
+  };
+  auto flush_leaves = [&](bool all) {
+    const int rounds = rounds_of(nl, kPtLeaves - kPtShare, all);
+    const int first = (int)((unsigned)(sub - (int)lh) & (kPtShare - 1));
+    for (int r = 0; r < rounds; r++) {
+      const int k = first + r * kPtShare;
+      if (k < nl) {
+        const int c = s_leaves[warp][tgt][(lh + k) & (kPtLeaves - 1)];
+        const double dx = x - m.cx[c], dy = y - m.cy[c];
+        const float nfx = -(float)dx, nfy = -(float)dy;
+        float sa = 0.f, sb = 0.f;  // velocity (sa, -sb), see pair
+        const int e = m.end[c];
+        for (int j = m.begin[c]; j < e; j++) pair<false>(m.src4[j], nfx, nfy, sa, sb);
+        ax.add(sa);
+        ay.add(-sb);
+        n_pairs += (unsigned)(e - m.begin[c]);
+      }
+      __syncwarp();
+    }
+    const int out = min(rounds * kPtShare, nl);
+    lh += (unsigned)out;
+    nl -= out;
+  };
+
   int top = 0;
   if (lane == 0) {
     s_cell[warp][0] = 0;
@@ -1961,80 +2111,65 @@ __global__ void __launch_bounds__(kPtWarps * 32) k_eval_points(MixedView m, int 
     const unsigned msk = s_mask[warp][top];
     __syncwarp();
     top--;
+    if (__any_sync(0xffffffffu, nq > kPtQueue - kPtShare)) flush_cells(false);
+    if (__any_sync(0xffffffffu, nl > kPtLeaves - kPtShare)) flush_leaves(false);
     const bool act = (msk >> lane) & 1u;
-    const bool is_leaf = m.leaf[c] != 0;
-    const bool has_mp = is_leaf || m.level[c] >= 2 + m.lev0;
-    bool far = false;
-    double dx = 0.0, dy = 0.0;
-    if (act && c != 0) {
-      dx = x - m.cx[c];
-      dy = y - m.cy[c];
-      const double side = m.region[c];
-      const double gx = fmax(fabs(dx) - 0.5 * side, 0.0), gy = fmax(fabs(dy) - 0.5 * side, 0.0);
-      far = has_mp && dx * dx + dy * dy >= mac2 * side * side && gx * gx + gy * gy > rc2;
+    const int cc = m.child[4 * (long)c + sub];
+    bool far = false, leaf = false;
+    const bool test = act && cc >= 0;
+    if (test) {
+      leaf = m.leaf[cc] != 0;
+      if (leaf || m.level[cc] >= 2 + m.lev0) far = far_from(m, cc, x, y, xh, xl, yh, yl, sxy, rc2, rc2f);
     }
-    if (far) {
-      // M2P: phi = (1/h) sum_k M_k w^(k+1), w = h / (z - zc)
-      const float ih = m.inv_h[c];
-      const float zx = __fmul_rn((float)dx, ih), zy = __fmul_rn((float)dy, ih);
-      const float ir2 = __fdiv_rn(1.f, fmaf(zx, zx, __fmul_rn(zy, zy)));
-      const float2 w = make_float2(__fmul_rn(zx, ir2), -__fmul_rn(zy, ir2));
-      const float *MA = m.M + (size_t)c * 2 * P;
-      float2 a = make_float2(MA[P - 1], MA[2 * P - 1]);
-      for (int k = P - 2; k >= 0; k--) {
-        a = fmul(a, w);
-        a.x = __fadd_rn(a.x, MA[k]);
-        a.y = __fadd_rn(a.y, MA[P + k]);
-      }
-      a = fmul(a, w);
-      phx += (double)__fmul_rn(a.x, ih);
-      phy += (double)__fmul_rn(a.y, ih);
-      n_m2p++;
+    const unsigned fmask = __ballot_sync(0xffffffffu, far);
+    const unsigned lmask = __ballot_sync(0xffffffffu, test && !far && leaf);
+    const unsigned omask = __ballot_sync(0xffffffffu, test && !far && !leaf);
+    const int sh = lane & ~(kPtShare - 1);
+    const unsigned below = (1u << sub) - 1u;
+    const unsigned myf = (fmask >> sh) & 0xfu, myl = (lmask >> sh) & 0xfu;
+    if (far) s_queue[warp][tgt][(qh + (unsigned)(nq + __popc(myf & below))) & (kPtQueue - 1)] = cc;
+    if (test && !far && leaf) s_leaves[warp][tgt][(lh + (unsigned)(nl + __popc(myl & below))) & (kPtLeaves - 1)] = cc;
+    nq += __popc(myf);
+    n_m2p += __popc(myf);
+    nl += __popc(myl);
+    // lane q < 4 pushes child q with the lanes of the points that open it
+    const unsigned open = (omask >> sub) & 0x11111111u;
+    const unsigned some = __ballot_sync(0xffffffffu, open != 0) & 0xfu;
+    const int cnt = __popc(some);
+    if (top + cnt >= kPtStack) {
+      overflow = true;
+      break;  // warp-uniform
     }
-    if (is_leaf) {
-      if (act && !far) {
-        const float nfx = -(float)dx, nfy = -(float)dy;
-        float sa = 0.f, sb = 0.f;  // velocity (sa, -sb), see pair
-        for (int j = m.begin[c]; j < m.end[c]; j++) pair<false>(m.src4[j], nfx, nfy, sa, sb);
-        ax += (double)sa;
-        ay -= (double)sb;
-        n_pairs += (unsigned long long)(m.end[c] - m.begin[c]);
-      }
-    } else {
-      const unsigned dmask = __ballot_sync(0xffffffffu, act && !far);
-      if (dmask) {
-        const int4 ch = reinterpret_cast<const int4 *>(m.child)[c];
-        for (int q = 3; q >= 0; q--) {
-          const int cc = (&ch.x)[q];
-          if (cc < 0) continue;
-          if (top + 1 >= kPtStack) {
-            overflow = true;
-            break;
-          }
-          top++;
-          if (lane == 0) {
-            s_cell[warp][top] = cc;
-            s_mask[warp][top] = dmask;
-          }
-        }
-      }
-      __syncwarp();
-      if (overflow) break;  // warp-uniform
+    if (lane < kPtShare && open) {
+      const int at = top + 1 + __popc(some & below);
+      s_cell[warp][at] = cc >= 0 ? cc : 0;
+      s_mask[warp][at] = open * 0xfu;
     }
+    top += cnt;
+    __syncwarp();
   }
+  flush_cells(true);
+  flush_leaves(true);
   if (overflow && lane == 0) set_err(m.st, TREE2D_ERR_TIMEOUT);
-  if (valid) {
+  double u = phy.value() + ax.value(), v = phx.value() + ay.value();
+  for (int o = 1; o < kPtShare; o <<= 1) {
+    u += __shfl_xor_sync(0xffffffffu, u, o);
+    v += __shfl_xor_sync(0xffffffffu, v, o);
+  }
+  if (valid && sub == 0) {
     const double inv2pi = 0.15915494309189533577;
     const long o = out_idx ? out_idx[i] : i;
-    uv[2 * o] = overflow ? NAN : (phy + ax) * inv2pi;
-    uv[2 * o + 1] = overflow ? NAN : (phx + ay) * inv2pi;
+    uv[2 * o] = overflow ? NAN : u * inv2pi;
+    uv[2 * o + 1] = overflow ? NAN : v * inv2pi;
   }
+  unsigned long long m2p = valid && sub == 0 ? n_m2p : 0;
+  if (!valid) n_pairs = 0;
   for (int o = 16; o; o >>= 1) {
-    n_m2p += __shfl_xor_sync(0xffffffffu, n_m2p, o);
+    m2p += __shfl_xor_sync(0xffffffffu, m2p, o);
     n_pairs += __shfl_xor_sync(0xffffffffu, n_pairs, o);
   }
   if (lane == 0) {
-    atomicAdd(&m.st->n_m2s, n_m2p);
+    atomicAdd(&m.st->n_m2s, m2p);
     atomicAdd(&m.st->n_pairs, n_pairs);
   }
 }
@@ -2432,7 +2567,7 @@ int mixed_eval_points(Workspace &ws, int ntgt, const double *tx, const double *t
                       cudaStream_t s) {
   if (ntgt <= 0) return TREE2D_OK;
   if (!ws.mxv) return TREE2D_ERR_NO_TREE;
-  const int warps = (ntgt + 31) / 32;
+  const int warps = (ntgt + kPtTargets - 1) / kPtTargets;
   k_eval_points<<<(warps + kPtWarps - 1) / kPtWarps, kPtWarps * 32, 0, s>>>(*ws.mxv, ntgt, tx, ty, out_idx, uv);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());

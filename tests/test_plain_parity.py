@@ -274,3 +274,35 @@ def test_batch_lookup_in_order_device_chunks(gpu_lib):
         assert np.array_equal(P.biot_tree_batch(q.copy()), uv)
     finally:
         P.set_mode(P.MODE_PLAIN)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["plain", "mixed"])
+@pytest.mark.parametrize("n", [1, 40, 3000])
+def test_batch_places_queries_in_any_order(gpu_lib, mode, n):
+    """Queries at blobs in another order, repeated, at coincident blobs, with
+    the other zero's sign, next to blobs, far away and not finite: blob
+    answers equal the in-order ones bit for bit, the others single-point
+    calls."""
+    P = gpu_lib
+    rng = np.random.default_rng(n)
+    xy = rng.random((n, 2))
+    xy[0] = [0.0, 0.5]
+    if n > 3:
+        xy[2] = xy[1]  # coincident
+    cir, cor = rng.standard_normal(n), np.full(n, 0.01)
+    P.set_params(9, 33, 0.5)
+    P.set_mode(P.MODE_PLAIN if mode == "plain" else P.MODE_MIXED)
+    try:
+        P.make_tree(xy, cir, cor)
+        own = P.biot_tree_batch(xy)
+        pick = rng.integers(0, n, 2 * n + 1100)
+        q = np.concatenate([xy[pick], [[-0.0, 0.5], [0.25, np.nan], [7.0, -3.0]], xy[:5] + 1e-9])
+        uv = P.biot_tree_batch(q)
+        assert np.array_equal(uv[: len(pick)], own[pick])
+        for i in range(len(pick), len(q)):
+            u, v = P.biot_tree(*q[i])
+            assert np.array_equal(uv[i], [u, v], equal_nan=True), q[i]
+    finally:
+        P.set_mode(P.MODE_PLAIN)
+        P.clear_params()
