@@ -6,17 +6,17 @@
 //              that completes a cell's last child forms that cell (children
 //              in quadrant order 3,2,1,0).  The level-1 -> root shift is
 //              skipped as in the reference.
-//  k_eval      one warp per 8 consecutive targets (tree order, so the warp's
-//              targets are neighbours), four lanes per target.  The warp walks
+//  k_eval      one warp per 8 or 4 consecutive targets (tree order, so the warp's
+//              targets are neighbours), 4 or 8 lanes per target.  The warp walks
 //              the UNION of its targets' traversals with a shared LIFO of
 //              (cell, lane mask): restricted to one target, the visit order
 //              is that target's own LIFO order in fmm.c:90-112.  The opening
 //              test uses round-to-nearest FP64 operations without contraction
 //              (r = sqrt(dx*dx + dy*dy); region > theta*r), so each target
-//              takes exactly the reference's branch.  The four lanes of a
+//              takes exactly the reference's branch.  The lanes of a
 //              target share its accepted cells (M2S, fmm.c:60-67, by Horner in
 //              w = 1/(z - zc)) and its direct pairs (fmm.c:121-142); their
-//              four partial sums are added in a fixed order at the end.  Both
+//              partial sums are added in a fixed order at the end.  Both
 //              in 64-bit fixed point (fix64.cuh): FP64 runs at 1/64 of the
 //              FP32 rate here.
 #include "dev_common.cuh"
@@ -179,11 +179,7 @@ __global__ void __launch_bounds__(128) k_upward(Tree t, int nt) {
 
 constexpr int kEvalWarps = 4;
 constexpr int kStackCap = 160;
-constexpr int kShare = 4;                // lanes per target (one per child of a cell)
-constexpr int kEvalTargets = 32 / kShare;  // targets per warp
-constexpr unsigned kEachTarget = 0x11111111u;  // the first lane of each target
 constexpr int kQueue = 64;  // deferred M2S cells per target
-static_assert(kShare == 4 && kEvalTargets * kShare == 32, "the masks below are for four lanes per target");
 static_assert((kQueue & (kQueue - 1)) == 0, "the M2S queues are rings indexed by a mask");
 
 struct EvalArgs {
@@ -214,8 +210,11 @@ enum EvalForm { kFormFp64, kFormFull, kFormHalf };
 // fills four times the warps (20,000 blobs: 1.43 -> 1.07 ms per solve).
 // 80 registers, 24 warps per SM: 64 registers spill (24.0 against 21.4 ms
 // per solve), 2 or 8 warps per block are slower (23.6, 22.2).
-template <int kForm>
+template <int kForm, int kShare>
 __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
+  constexpr int kEvalTargets = 32 / kShare;  // per warp
+  constexpr unsigned kLanes = (1u << kShare) - 1u, kEachTarget = 0xffffffffu / kLanes;  // a target's lanes; the first of each
+  static_assert(kShare == 4 || kShare == 8, "a target's first four lanes test a cell's four children");
   __shared__ int s_cell[kEvalWarps][kStackCap];
   __shared__ unsigned s_mask[kEvalWarps][kStackCap];
   __shared__ int s_queue[kEvalWarps][kEvalTargets][kQueue];
@@ -246,9 +245,9 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
   // The targets accept cells at different depths, so an M2S evaluated where
   // it is accepted runs with the warp's other lanes idle.  Each target
   // instead queues its accepted cells (a ring: head qh, count nq, the same in
-  // its four lanes) and the warp evaluates the queues together, four entries
-  // per target and round.  Entry k of a target (counted over the whole
-  // traversal) is lane k mod 4's, so the partial sums do not depend on when
+  // its lanes) and the warp evaluates the queues together, an entry per lane
+  // and round.  Entry k of a target (counted over the whole
+  // traversal) is lane k mod kShare's, so the partial sums do not depend on when
   // the queues are emptied, nor on the warp's other targets.  A flush when
   // some queue could overflow evaluates only as many rounds as every target
   // can fill, or as the fullest one needs to make room for four entries, if
@@ -261,7 +260,7 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
       hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, o));
       lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, o));
     }
-    const int rounds = (all ? hi + kShare - 1 : max(lo, hi - (kQueue - kShare) + kShare - 1)) / kShare;
+    const int rounds = (all ? hi + kShare - 1 : max(lo, hi - (kQueue - 4) + kShare - 1)) / kShare;
     const int first = (int)((unsigned)(sub - (int)qh) & (kShare - 1));
     fix::settle(far);  // at most kQueue / kShare terms follow
     for (int r = 0; r < rounds; r++) {
@@ -348,9 +347,9 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
       __syncwarp();
     } else {
       // a cell's four children can add four entries to a target's queue
-      if (__any_sync(0xffffffffu, nq > kQueue - kShare)) flush(false);
-      // each of a target's lanes tests one child
-      const int cc = t.child[4 * (long)c + sub];
+      if (__any_sync(0xffffffffu, nq > kQueue - 4)) flush(false);
+      // each of a target's first four lanes tests one child
+      const int cc = sub < 4 ? t.child[4 * (long)c + sub] : -1;
       bool desc = false;
       if (act && cc >= 0) {
         // The reference's test is region > theta * sqrt(d2), each step
@@ -414,10 +413,10 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
         overflow = true;
         break;
       }
-      if (lane < kShare && open) {
+      if (lane < 4 && open) {
         const int at = top + 1 + __popc(some & ((1u << lane) - 1u));
         s_cell[warp][at] = cc;
-        s_mask[warp][at] = open * 0xfu;
+        s_mask[warp][at] = open * kLanes;
       }
       top += cnt;
       __syncwarp();
@@ -425,7 +424,7 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
   }
   flush(true);
   if (overflow && lane == 0) set_err(a.st, TREE2D_ERR_TIMEOUT);
-  // the four lanes' sums
+  // the lanes' sums
   double2 phi = kForm != kFormFp64 ? make_double2(fix::to_double(far.x, far.xl, far.e), fix::to_double(far.y, far.yl, far.e))
                                    : make_double2(0.0, 0.0);
   phi.x = __dadd_rn(phi.x, far64.x);
@@ -537,17 +536,26 @@ int plain_upward(Workspace &ws, const Tree &t, const Params &p, cudaStream_t s) 
   return TREE2D_OK;
 }
 
+// Trees of up to this many blobs are evaluated with eight lanes per target,
+// which leaves fewer targets to a warp and twice the warps to hide latencies.
+// Measured evaluation, 8 against 4 lanes: 4,096 uniform blobs 115 / 166 us,
+// 32,768 399 / 451, 65,536 752 / 729; Lamb-Oseen 65,536 1.10 / 1.12 ms,
+// 131,072 2.15 / 2.09.  By the tree's size, not the targets' number: a point's
+// sums do not depend on how many points are asked for.
+constexpr int kWideBlobs = 65536;
+
 int plain_evaluate(Workspace &ws, const Tree &t, const Params &p, int ntgt, const double *tx, const double *ty,
                    const int *out_idx, double *uv, cudaStream_t s) {
   if (ntgt <= 0) return TREE2D_OK;
   T2D_CUDA_TRY(mac_bounds(ws, t, p.theta, p.nterms, s));
   EvalArgs a{t, p.nterms, p.theta, ntgt, tx, ty, out_idx, uv, ws.status, fix::first_pair_term(p.theta),
              reinterpret_cast<const void *>(t.fix) != reinterpret_cast<const void *>(t.coef), fix::One()};
-  const int warps = (ntgt + kEvalTargets - 1) / kEvalTargets;
+  const bool wide = t.n <= kWideBlobs;
+  const int warps = (int)(((long)ntgt * (wide ? 8 : 4) + 31) / 32);
   const int blocks = (warps + kEvalWarps - 1) / kEvalWarps;
-  auto kernel = p.theta > kFixTheta           ? k_eval<kFormFp64>
-                : p.theta > fix::kHalfTheta ? k_eval<kFormFull>
-                                            : k_eval<kFormHalf>;
+  auto kernel = p.theta > kFixTheta         ? (wide ? k_eval<kFormFp64, 8> : k_eval<kFormFp64, 4>)
+                : p.theta > fix::kHalfTheta ? (wide ? k_eval<kFormFull, 8> : k_eval<kFormFull, 4>)
+                                            : (wide ? k_eval<kFormHalf, 8> : k_eval<kFormHalf, 4>);
   kernel<<<blocks, kEvalWarps * 32, 0, s>>>(a);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());

@@ -257,3 +257,28 @@ def test_coefficients_are_the_cells_moments(gpu_lib, nterms, n, num_p):
         scale = np.abs(g[s]).sum() * (1.5 * t["region"][c]) ** k
         err = np.abs(t["coef"][c] - exact).astype(float)
         assert (err <= 8 * (k + 1) * (t["level"].max() + 1) * 2.0**-53 * scale).all(), (c, err / scale)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("theta", [0.3, 0.5, 0.9])
+@pytest.mark.parametrize("n", [65536, 65537])
+def test_lanes_per_target_around_their_limit(gpu_lib, n, theta):
+    """The evaluation's two splits, eight lanes per target up to 65,536 blobs
+    and four beyond, in each of its arithmetics (theta up to 0.35, up to 0.7,
+    beyond): blobs and points off the blobs, ragged numbers of both, within
+    the parity bar of the oracle."""
+    P = gpu_lib
+    W = workloads()
+    b = W.uniform(n, seed=3)
+    rng = np.random.default_rng(7)
+    q = np.concatenate([b.xy[W.sample_targets(n, 509, seed=2)], rng.uniform(-1.2, 1.2, (33, 2))])
+    P.set_params(b.nterms, b.num_p, theta)
+    P.set_mode(P.MODE_PLAIN)
+    try:
+        P.make_tree(b.xy, b.cir, b.cor)
+        uv = P.biot_tree_batch(q)
+    finally:
+        P.clear_params()
+    o = oracle().Oracle(b.nterms, b.num_p, theta)
+    o.make_tree(b.xy, b.cir, b.cor)
+    assert_parity(uv, o.biot(q), q, ext_for(b.xy, b.cir, b.cor, b.nterms, b.num_p, theta), label=f"{n} theta {theta}")
