@@ -31,13 +31,18 @@
 namespace t2d {
 namespace {
 
-constexpr int kBoxBlocks = 1216;  // 8 x 152 SMs: enough loads in flight to stream the positions
+constexpr int kBoxBlocks = 1216;  // at most; 8 x 152 SMs: enough loads in flight to stream the positions
+inline int box_blocks(int n) { return (n + 255) / 256 < kBoxBlocks ? (n + 255) / 256 : kBoxBlocks; }
 
 struct __align__(16) Box4 {
   double x, y, z, w;  // xmax, xmin, ymax, ymin
 };
 constexpr int kScanThreads = 256;
-constexpr int kScanItems = 16;
+// Positions per thread of the cell scans, which walk them one after another:
+// few, so that a small tree fills more blocks (k_emit_cells at 50,000 blobs 26
+// us with 16 positions, 9 us so; a whole solve of 50,000 602 -> 580 us, of 4M
+// no change).
+constexpr int kScanItems = 4;
 constexpr int kScanTile = kScanThreads * kScanItems;
 
 __device__ __forceinline__ double warp_max(double v) {
@@ -819,7 +824,7 @@ size_t build_tmp_bytes(int n, int nsets) {
   tneed += Arena::bytes_for(n, 8) + Arena::bytes_for(n, 4) * 2;  // keys_alt, vals, vals_alt
   tneed += Arena::bytes_for(n, 1);                              // w
   tneed += radix_sort_temp_bytes(n) + 256;
-  tneed += Arena::bytes_for(kBoxBlocks, sizeof(Box4));
+  tneed += Arena::bytes_for(box_blocks(n), sizeof(Box4));
   tneed += Arena::bytes_for(ntiles + 1, 8) + 256;
   const int tlev = batched ? 12 : centre_levels(n);
   tneed += Arena::bytes_for(2 * centre_entries(tlev) * ns, 8);
@@ -883,9 +888,9 @@ int build_tree(Workspace &ws, int n, const double *d_xy, const double *d_cir, co
   uint64_t *keys_alt = ws.tmp_arena.take<uint64_t>(n);
   uint32_t *vals = ws.tmp_arena.take<uint32_t>(n);
   uint32_t *vals_alt = ws.tmp_arena.take<uint32_t>(n);
+  void *sort_tmp = ws.tmp_arena.take<char>(radix_sort_temp_bytes(n));  // right after vals_alt (see the sort)
   uint8_t *w = ws.tmp_arena.take<uint8_t>(n);
-  void *sort_tmp = ws.tmp_arena.take<char>(radix_sort_temp_bytes(n));
-  Box4 *bpart = ws.tmp_arena.take<Box4>(kBoxBlocks);
+  Box4 *bpart = ws.tmp_arena.take<Box4>(box_blocks(n));
   unsigned long long *part = ws.tmp_arena.take<unsigned long long>(ntiles + 1);
   unsigned long long *total = ws.tmp_arena.take<unsigned long long>(1);
   uint64_t *ctab = ws.tmp_arena.take<uint64_t>(2 * centre_entries(tlev) * t.nsets);
@@ -911,8 +916,8 @@ retry:
     k_roots_sets<<<(nsets + 127) / 128, 128, 0, s>>>(set_part, nsets, t.root);
     ::t2d::g_launches.fetch_add(2, std::memory_order_relaxed);
   } else {
-    k_bbox<<<kBoxBlocks, 256, 0, s>>>(d_xy, n, bpart, ws.status);
-    k_root<<<1, kRootThreads, 0, s>>>(bpart, kBoxBlocks, t.root);
+    k_bbox<<<box_blocks(n), 256, 0, s>>>(d_xy, n, bpart, ws.status);
+    k_root<<<1, kRootThreads, 0, s>>>(bpart, box_blocks(n), t.root);
     ::t2d::g_launches.fetch_add(2, std::memory_order_relaxed);
   }
   // 2. keys
@@ -934,8 +939,9 @@ retry:
   ::t2d::g_launches.fetch_add(2, std::memory_order_relaxed);
   // 3. sort
   if (packed)
+    // a packed sort has no use for vals_alt: its scratch starts there
     T2D_CUDA_TRY(radix_sort_packed(words, words == t.keys ? keys_alt : t.keys, n, 64 - 2 * total_levels, t.keys,
-                                   vals, sort_tmp, ws.status, s));
+                                   vals, vals_alt, Arena::bytes_for(n, 4) + radix_sort_temp_bytes(n), ws.status, s));
   else
     T2D_CUDA_TRY(radix_sort_pairs(t.keys, vals, keys_alt, vals_alt, n, 64 - 2 * total_levels, 64, sort_tmp, s));
   t.key_order = vals;
@@ -1021,12 +1027,12 @@ retry:
 
 int sort_targets(Workspace &ws, int n, const double *d_xy, const RootBox *d_root, int *d_order, cudaStream_t s) {
   if (n <= 0) return TREE2D_OK;
-  size_t need = Arena::bytes_for(n, 8) * 2 + radix_sort_temp_bytes(n) + 512;
-  T2D_CUDA_TRY(ws.tmp_arena.reserve(need));
+  const size_t tmp_bytes = Arena::bytes_for(n, 4) + radix_sort_temp_bytes(n);
+  T2D_CUDA_TRY(ws.tmp_arena.reserve(Arena::bytes_for(n, 8) * 2 + tmp_bytes + 512));
   ws.tmp_arena.reset();
   uint64_t *a = ws.tmp_arena.take<uint64_t>(n);
   uint64_t *b = ws.tmp_arena.take<uint64_t>(n);
-  void *tmp = ws.tmp_arena.take<char>(radix_sort_temp_bytes(n));
+  void *tmp = ws.tmp_arena.take<char>(tmp_bytes);
   // only for warps of neighbours: digits down to about one point per cell
   int levels = 4;
   while (levels < 16 && (1l << (2 * levels)) < 4l * n) levels++;
@@ -1039,7 +1045,7 @@ int sort_targets(Workspace &ws, int n, const double *d_xy, const RootBox *d_root
   }
   // the last pass reads `a` after an odd number of passes, `b` after an even one
   T2D_CUDA_TRY(radix_sort_packed(a, b, n, 64 - 2 * levels, odd ? b : a, reinterpret_cast<uint32_t *>(d_order), tmp,
-                                 ws.status, s));
+                                 tmp_bytes, ws.status, s));
   return TREE2D_OK;
 }
 

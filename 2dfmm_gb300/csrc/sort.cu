@@ -240,13 +240,15 @@ __global__ void __launch_bounds__(kThreads) k_hist_all(const uint64_t *__restric
 // counter (zero before the pass).  A look-back that polls `limit` times
 // without an answer records TREE2D_ERR_TIMEOUT and takes the missing count
 // as zero (the output is then wrong and the build reports the error).
+template <int kPer>
 __global__ void __launch_bounds__(kThreads) k_onesweep(const uint64_t *__restrict__ kin, uint64_t *__restrict__ kout,
                                                        uint32_t *__restrict__ vout, int n, int shift,
                                                        const unsigned *__restrict__ hist, unsigned *status,
                                                        unsigned *ctr, int ntiles, int split, long limit,
                                                        DevStatus *st) {
+  constexpr int kTileN = kThreads * kPer;
   extern __shared__ __align__(16) unsigned char stage[];
-  uint64_t *sk = reinterpret_cast<uint64_t *>(stage);  // kTile words, tile digit order
+  uint64_t *sk = reinterpret_cast<uint64_t *>(stage);  // kTileN words, tile digit order
   __shared__ unsigned wcount[kWarps][kBins];
   __shared__ unsigned lbase[kBins];
   __shared__ unsigned gbase[kBins];
@@ -259,13 +261,13 @@ __global__ void __launch_bounds__(kThreads) k_onesweep(const uint64_t *__restric
   for (int i = threadIdx.x; i < kWarps * kBins; i += kThreads) (&wcount[0][0])[i] = 0;
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const long tile0 = (long)tile * kTile;
-  const long base = tile0 + warp * (kItems * 32);
-  uint64_t k[kItems];
-  unsigned r[kItems];
+  const long tile0 = (long)tile * kTileN;
+  const long base = tile0 + warp * (kPer * 32);
+  uint64_t k[kPer];
+  unsigned r[kPer];
   const unsigned ltmask = lanemask_lt();
 #pragma unroll
-  for (int j = 0; j < kItems; j++) {
+  for (int j = 0; j < kPer; j++) {
     const long i = base + j * 32 + lane;
     const bool valid = i < n;
     k[j] = valid ? kin[i] : 0;
@@ -322,7 +324,7 @@ __global__ void __launch_bounds__(kThreads) k_onesweep(const uint64_t *__restric
   lbase[threadIdx.x] = lb;
   __syncthreads();
 #pragma unroll
-  for (int j = 0; j < kItems; j++) {
+  for (int j = 0; j < kPer; j++) {
     const long i = base + j * 32 + lane;
     if (i < n) {
       const unsigned d = (unsigned)((k[j] >> shift) & 0xff);
@@ -330,7 +332,7 @@ __global__ void __launch_bounds__(kThreads) k_onesweep(const uint64_t *__restric
     }
   }
   __syncthreads();
-  const int tile_n = (int)min((long)kTile, (long)n - tile0);
+  const int tile_n = (int)min((long)kTileN, (long)n - tile0);
   for (int p = threadIdx.x; p < tile_n; p += kThreads) {
     const uint64_t key = sk[p];
     const unsigned d = (unsigned)((key >> shift) & 0xff);
@@ -346,15 +348,23 @@ __global__ void __launch_bounds__(kThreads) k_onesweep(const uint64_t *__restric
 
 }  // namespace
 
-static size_t onesweep_temp_bytes(int n) {
-  const size_t ntiles = (size_t)(n > 0 ? (n + kTile - 1) / kTile : 1);
+// Small sorts take tiles of 4 words per thread instead of 16: a pass over few
+// tiles is bound by the steps one tile walks through, a pass over many by the
+// look-back.  Whole solves with 4 against 16 (us): static plain of 4,096 blobs
+// 319 / 353; mixed, uniform, 8,192 452 / 468, 32,768 532 / 555, 131,072
+// 650 / 660, 262,144 715 / 711, 524,288 1092 / 1073.
+constexpr int kSmallItems = 4;
+constexpr int kSmallSort = 131072;
+
+static size_t onesweep_temp_bytes(int n, int tile) {
+  const size_t ntiles = (size_t)(n > 0 ? (n + tile - 1) / tile : 1);
   return ((size_t)kMaxPasses * kBins + kMaxPasses + (size_t)kMaxPasses * ntiles * kBins) * sizeof(unsigned);
 }
 
 size_t radix_sort_temp_bytes(int n) {
   long ntiles = (n + kTile - 1) / kTile;
   const size_t classic = (size_t)kBins * (size_t)(ntiles > 0 ? ntiles : 1) * sizeof(unsigned) + kBins * sizeof(unsigned);
-  const size_t single = onesweep_temp_bytes(n);
+  const size_t single = onesweep_temp_bytes(n, kTile);
   return classic > single ? classic : single;
 }
 
@@ -392,29 +402,34 @@ cudaError_t radix_sort_pairs(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt,
 }
 
 cudaError_t radix_sort_packed(uint64_t *words, uint64_t *words_alt, int n, int begin_bit, uint64_t *keys_out,
-                              uint32_t *vals_out, void *temp, DevStatus *st, cudaStream_t s) {
+                              uint32_t *vals_out, void *temp, size_t temp_bytes, DevStatus *st, cudaStream_t s) {
   if (begin_bit < 32 || begin_bit >= 64 || n < 2) return cudaErrorInvalidValue;
   const int passes = (64 - begin_bit + 7) / 8;
-  const int ntiles = (n + kTile - 1) / kTile;
   uint64_t *ka = words, *kb = words_alt;
   if (n < (1 << 30) && st) {
     // single pass per digit: counts up to 2^30 - 1 fit a status word
+    constexpr int kSmallTile = kThreads * kSmallItems;
+    const bool small = n <= kSmallSort && onesweep_temp_bytes(n, kSmallTile) <= temp_bytes;
+    const int tile = small ? kSmallTile : kTile;
+    const int ntiles = (n + tile - 1) / tile;
     unsigned *hist = static_cast<unsigned *>(temp);
     unsigned *ctr = hist + kMaxPasses * kBins;
     unsigned *status = ctr + kMaxPasses;
     const size_t zero = ((size_t)kMaxPasses * kBins + kMaxPasses + (size_t)passes * ntiles * kBins) * sizeof(unsigned);
     cudaError_t e = cudaMemsetAsync(temp, 0, zero, s);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_onesweep, cudaFuncAttributeMaxDynamicSharedMemorySize, kStagePackedBytes);
+    e = cudaFuncSetAttribute(k_onesweep<kItems>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStagePackedBytes);
     if (e != cudaSuccess) return e;
     const int hblocks = ntiles < 152 * 4 ? ntiles : 152 * 4;
     k_hist_all<<<hblocks, kThreads, 0, s>>>(ka, n, begin_bit, passes, hist);
     ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
+    auto kernel = small ? k_onesweep<kSmallItems> : k_onesweep<kItems>;
     for (int p = 0; p < passes; p++) {
       const bool last = p == passes - 1;
-      k_onesweep<<<ntiles, kThreads, kStagePackedBytes, s>>>(
-          ka, last ? keys_out : kb, last ? vals_out : nullptr, n, begin_bit + 8 * p, hist + p * kBins,
-          status + (size_t)p * ntiles * kBins, ctr + p, ntiles, last ? 1 : 0, kLookbackLimit, st);
+      kernel<<<ntiles, kThreads, tile * 8, s>>>(ka, last ? keys_out : kb, last ? vals_out : nullptr, n,
+                                                begin_bit + 8 * p, hist + p * kBins,
+                                                status + (size_t)p * ntiles * kBins, ctr + p, ntiles, last ? 1 : 0,
+                                                kLookbackLimit, st);
       ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
       uint64_t *t = ka;
       ka = kb;
@@ -422,6 +437,7 @@ cudaError_t radix_sort_packed(uint64_t *words, uint64_t *words_alt, int n, int b
     }
     return cudaGetLastError();
   }
+  const int ntiles = (n + kTile - 1) / kTile;
   unsigned *counts = static_cast<unsigned *>(temp);
   unsigned *totals = counts + (size_t)kBins * ntiles;
   cudaError_t e = cudaFuncSetAttribute(k_downsweep<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,

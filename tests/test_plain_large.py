@@ -282,3 +282,22 @@ def test_lanes_per_target_around_their_limit(gpu_lib, n, theta):
     o = oracle().Oracle(b.nterms, b.num_p, theta)
     o.make_tree(b.xy, b.cir, b.cor)
     assert_parity(uv, o.biot(q), q, ext_for(b.xy, b.cir, b.cor, b.nterms, b.num_p, theta), label=f"{n} theta {theta}")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2, 1023, 1024, 1025, 4097, 131072, 131073])
+def test_tree_around_the_tiles(gpu_lib, n):
+    """The tree equals the oracle's where the number of blobs meets the edges
+    of a sort or scan tile and the largest sort of small tiles."""
+    P = gpu_lib
+    b = workloads().uniform(n, seed=n)
+    P.set_params(11, 33, 0.5)
+    P.set_mode(P.MODE_PLAIN)
+    try:
+        P.make_tree(b.xy, b.cir, b.cor)
+        d = P.export_tree(n, 11)
+    finally:
+        P.clear_params()
+    o = oracle().Oracle(11, 33, 0.5)
+    o.make_tree(b.xy, b.cir, b.cor)
+    assert_same_tree(d, o.dump(n))
