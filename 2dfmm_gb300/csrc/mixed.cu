@@ -1216,13 +1216,6 @@ __global__ void __launch_bounds__(256) k_l2l_f32(MixedView m, int lev) {
   }
 }
 
-__device__ __forceinline__ void kahan(float &s, float &cmp, float v) {
-  float y = v - cmp;
-  float t = s + y;
-  cmp = (t - s) - y;
-  s = t;
-}
-
 // Order of an M2P the network chose: class c >= 1 is order c + 3 (4..16),
 // raised by the margin, capped at P; class 0 of a W entry keeps P.
 __device__ __forceinline__ int chosen_order(int d, int margin, int P) {
@@ -1430,14 +1423,14 @@ struct GlobalSrc {
 };
 
 // Direct (U list) or correction (K list) sums of source blobs [j0, j1) for
-// one target per lane (leaf_pairs1), one pack of two (leaf_pairs2) or two
-// packs sharing every source record (leaf_pairs4); the targets are given
-// negated (see pair).  Each source leaf is summed in plain FP32 and then
+// one target per lane (leaf_pairs1), one pack of two (leaf_pairs2), or a pack
+// and a third target (leaf_pairs3) or two packs (leaf_pairs4) sharing every
+// source record; the targets are given negated (see pair).  Each source leaf is summed in plain FP32 and then
 // added with compensation (leaf_add), so the compensated sum costs once per
 // leaf, not once per pair.
-template <bool kCorrection, bool kScaled, class S>
+template <bool kCorrection, bool kScaled, int kUnroll, class S>
 __device__ __forceinline__ void leaf_pairs1(const S src, int j0, int j1, float ntx, float nty, float &a, float &b) {
-#pragma unroll 4
+#pragma unroll kUnroll
   for (int j = j0; j < j1; j++) pair<kCorrection, kScaled>(src[j], ntx, nty, a, b);
 }
 
@@ -1446,6 +1439,17 @@ __device__ __forceinline__ void leaf_pairs2(const S src, int j0, int j1, float2 
                                             float2 &b) {
 #pragma unroll kUnroll
   for (int j = j0; j < j1; j++) pair2<kCorrection, kScaled>(src[j], ntx, nty, a, b);
+}
+
+template <bool kCorrection, bool kScaled, int kUnroll, class S>
+__device__ __forceinline__ void leaf_pairs3(const S src, int j0, int j1, float2 ntx0, float2 nty0, float ntx1,
+                                            float nty1, float2 &a0, float2 &b0, float &a1, float &b1) {
+#pragma unroll kUnroll
+  for (int j = j0; j < j1; j++) {
+    const float4 sj = src[j];
+    pair2<kCorrection, kScaled>(sj, ntx0, nty0, a0, b0);
+    pair<kCorrection, kScaled>(sj, ntx1, nty1, a1, b1);
+  }
 }
 
 template <bool kCorrection, bool kScaled, int kUnroll, class S>
@@ -1491,22 +1495,11 @@ __device__ __forceinline__ float leaf_cutoff(const MixedView &m, int B) {
 
 constexpr unsigned kAllChunks = 0xffffffffu;
 
-// Pair counters of one warp, kept in shared memory by lane 0 (every count
-// is warp-uniform): target-source pairs evaluated, correction pairs
-// evaluated and correction pairs listed, over the current chunk of targets
-// and then summed over chunks.
+// Pair counters of one warp, kept in shared memory by lane 0: target-source
+// pairs evaluated, correction pairs evaluated and correction pairs listed.
 struct WarpCounts {
-  unsigned chunk[3];
   unsigned long long total[3];
 };
-
-__device__ __forceinline__ void counts_add(WarpCounts *c, int lane, unsigned done, unsigned done_k, unsigned listed) {
-  if (lane == 0) {
-    c->chunk[0] += done;
-    c->chunk[1] += done_k;
-    c->chunk[2] += listed;
-  }
-}
 
 __device__ __forceinline__ void counts_flush(WarpCounts *c, int lane, DevStatus *st) {
   if (lane == 0) {
@@ -1542,36 +1535,49 @@ __device__ __forceinline__ int next_run(unsigned &r0, unsigned &r1, int cnt, int
 }
 
 // Chunks of correction source leaf A whose pairs with a pack of targets can
-// lie within the correction radius: bit k of *m0 (*m1) for the kChunk-blob chunk
+// lie within the correction radius: bit k of m0 (m1) for the kChunk-blob chunk
 // k of A whose bounding box comes within rc of pack 0's (pack 1's) target
 // box, tb[0..3] (tb[4..7]), rc^2 in tb[8]; the boxes are offsets from the
 // target leaf's centre, (ox, oy) is A's centre seen from there.  Pairs
 // farther than rc from every target add terms below exp(-rc^2/sigma^2) of a
 // point vortex: the ones the correction list already leaves out beyond rc.
-// A leaf of more than 32 chunks is not culled (kAllChunks).  Warp-uniform.
+// A leaf of more than 32 chunks is not culled (kAllChunks).  A lane forms
+// every second chunk's bits, from chunk `first` on.
 template <int kPacks>
-__device__ __forceinline__ void chunk_mask(const MixedView &m, int A, float ox, float oy, const float *tb, int lane,
-                                           unsigned &m0, unsigned &m1) {
-  const int nch = (m.end[A] - m.begin[A] + kChunk - 1) >> kChunkShift;
+__device__ __forceinline__ void chunk_mask(const MixedView &m, int A, int cnt, float ox, float oy, const float *tb,
+                                           int first, unsigned &m0, unsigned &m1) {
+  const int nch = (cnt + kChunk - 1) >> kChunkShift;
   if (nch > 32 || nch > m.kchunks) {
     m0 = m1 = kAllChunks;
     return;
   }
-  bool keep[2] = {false, false};
-  if (lane < nch) {
-    const float rc2 = tb[8];
-    const float4 s = m.cbox[(size_t)A * m.kchunks + lane];
+  const float4 *box = m.cbox + (size_t)A * m.kchunks;
+  float4 T[kPacks];  // pack p's box in A's frame
+#pragma unroll
+  for (int p = 0; p < kPacks; p++)
+    T[p] = make_float4(__fadd_rn(tb[4 * p], ox), __fadd_rn(tb[4 * p + 1], oy), __fadd_rn(tb[4 * p + 2], ox),
+                       __fadd_rn(tb[4 * p + 3], oy));
+  const float rc2 = tb[8];
+  unsigned keep[2] = {0, 0};
+#pragma unroll 2
+  for (int k = first; k < nch; k += 2) {
+    const float4 s = box[k];
 #pragma unroll
     for (int p = 0; p < kPacks; p++) {
-      // pack p's box in A's frame: T + (ox, oy)
-      const float4 T = make_float4(tb[4 * p], tb[4 * p + 1], tb[4 * p + 2], tb[4 * p + 3]);
-      const float gx = fmaxf(fmaxf(__fsub_rn(s.x, __fadd_rn(T.z, ox)), __fsub_rn(__fadd_rn(T.x, ox), s.z)), 0.f);
-      const float gy = fmaxf(fmaxf(__fsub_rn(s.y, __fadd_rn(T.w, oy)), __fsub_rn(__fadd_rn(T.y, oy), s.w)), 0.f);
-      keep[p] = fmaf(gx, gx, __fmul_rn(gy, gy)) <= rc2;
+      const float gx = fmaxf(fmaxf(__fsub_rn(s.x, T[p].z), __fsub_rn(T[p].x, s.z)), 0.f);
+      const float gy = fmaxf(fmaxf(__fsub_rn(s.y, T[p].w), __fsub_rn(T[p].y, s.w)), 0.f);
+      if (fmaf(gx, gx, __fmul_rn(gy, gy)) <= rc2) keep[p] |= 1u << k;
     }
   }
-  m0 = __ballot_sync(0xffffffffu, keep[0]);
-  m1 = kPacks == 2 ? __ballot_sync(0xffffffffu, keep[1]) : m0;
+  m0 = keep[0];
+  m1 = kPacks == 2 ? keep[1] : keep[0];
+}
+
+// Blobs in the chunks of `mask`, of a leaf of cnt blobs.
+__device__ __forceinline__ unsigned mask_blobs(unsigned mask, int cnt) {
+  if (mask == kAllChunks) return (unsigned)cnt;
+  const int nch = (cnt + kChunk - 1) >> kChunkShift;
+  return (unsigned)((__popc(mask) << kChunkShift) - ((mask >> (nch - 1)) & 1u) * ((nch << kChunkShift) - cnt));
 }
 
 // The persistent near-field warps take target leaves in the order of
@@ -1599,7 +1605,7 @@ __global__ void k_leaf_cost(MixedView m, uint64_t *keys, uint32_t *vals) {
 }
 
 // Near field of every leaf: one warp per target leaf.  The leaf's targets
-// are taken in chunks of 128, 64 or 32 (4, 2 or 1 per lane, packed in
+// are taken in chunks of 128, 96, 64 or 32 (4, 3, 2 or 1 per lane, packed in
 // twos: a leaf of 97-128 blobs walks its source lists once with four
 // targets per lane instead of twice with two).  For each chunk the warp
 // walks its direct entries (U list, then K list; in the learned form the
@@ -1614,50 +1620,80 @@ __global__ void k_leaf_cost(MixedView m, uint64_t *keys, uint32_t *vals) {
 // the sources are read from global memory (through L1).  The compensated
 // per-target sums live in shared memory (written once per source leaf),
 // which keeps the pair loop's registers for the targets.
+//
+// What an entry needs -- its leaf's range, the offset of its centre, its
+// chunks within the correction radius -- is formed for kBatch entries at a
+// time, a lane pair per entry, and kept as a record in shared memory.  The
+// kernel is bound by issue slots, and with the warp forming one entry after
+// another those steps took about as many as the pairs (whole solves, one
+// entry after another against batches, with leaves of 65-96 blobs in chunks
+// of 64 and 32 against one of 96: 4M two-patch + sheet blobs 6.93 -> 6.41 ms,
+// 1M Lamb-Oseen, learned, 1.95 -> 1.83 ms, 512 sets 14.67 -> 14.00 ms).
 constexpr int kStage = 128;  // blobs per stage buffer: the largest leaf of the default leaf sizes
+constexpr int kBatch = 16;   // entries prepared at a time
 constexpr long kEvalWaitLimit = 1l << 22;  // polls; a healthy copy lands within microseconds
+
+// One source leaf with work: its centre's offset from the target leaf's, its
+// scale (1 without scaled records), its blobs, its kept chunks per pack.
+struct __align__(16) NearEntry {
+  float ox, oy, s;
+  int corr;
+  int j0, cnt;
+  unsigned r0, r1;
+};
 
 struct NearWarp {
   float4 *src;       // stage buffers [2][kStage] (kStaged)
   uint64_t *bar;     // their mbarriers [2]
   float *tbox;       // target boxes of the chunk's packs and rc^2
-  float4 *acc;       // compensated sums {ax, cx, ay, cy} [4][32]
+  float4 *acc;       // compensated sums [4][32], see leaf_add
+  NearEntry *list;   // [kBatch]
   WarpCounts *cnts;
   unsigned parity;   // bit b: parity of buffer b's next completion
   unsigned inflight; // bit b: a copy into buffer b not yet waited for
   bool staging;      // false after a wait gave up
 };
 
-// Adds one source leaf's sums (sa, sb of pair) to target slot k's
-// compensated sums: velocity (a, -b) for a direct leaf, (-a, b) for a
-// correction leaf.
-__device__ __forceinline__ void leaf_add(float4 *acc, int k, int lane, bool corr, float a, float b) {
-  float4 s = acc[32 * k + lane];
-  kahan(s.x, s.y, corr ? -a : a);
-  kahan(s.z, s.w, corr ? b : -b);
-  acc[32 * k + lane] = s;
+// Adds one source leaf's sums to a target's compensated sums: velocity
+// (a, -b) for a direct leaf, (-a, b) for a correction leaf, sg = 1 or -1.
+// `s` is a sum and `nc` its negated compensation; the steps are Kahan's,
+// y = v - c, t = s + y, c = (t - s) - y, with the signs folded into FMAs by
+// +-1 (exact).
+__device__ __forceinline__ void leaf_add(float &s, float &nc, float sg, float v) {
+  const float y = fmaf(sg, v, nc), t = __fadd_rn(s, y);
+  nc = __fsub_rn(y, __fsub_rn(t, s));
+  s = t;
+}
+__device__ __forceinline__ void leaf_add2(float2 &s, float2 &nc, float sg, float2 v) {
+  const float2 y = __ffma2_rn(f2(sg), v, nc), t = __fadd2_rn(s, y);
+  nc = __ffma2_rn(f2(-1.f), __ffma2_rn(f2(-1.f), s, t), y);
+  s = t;
 }
 
 // One chunk of a target leaf's targets: 32 kT of them from t0 on, kT per
-// lane (target t0 + 32 k + lane in slot k), in packs of two slots (k = 0, 1
-// and k = 2, 3), each pack with its own bounding box for the correction
+// lane (target t0 + 32 k + lane in slot k), in packs of up to two slots (k =
+// 0, 1 and k = 2, 3), each pack with its own bounding box for the correction
 // cull.  The tree's in-leaf order is spatial (k_leaf_setup), so a pack of
 // 64 consecutive targets is compact.
 template <bool kLearned, bool kStaged, int kT, int kUnroll, bool kScaled>
 __device__ __forceinline__ void near_chunk(const MixedView &m, const Decisions &dec, double *uv, const int *perm,
                                            long wait_limit, int l, int B, int t0, int lane, NearWarp &w) {
-  constexpr int kPacks = kT == 4 ? 2 : 1;
+  constexpr int kPacks = kT > 2 ? 2 : 1;
+  constexpr int kPairs = kT / 2;   // packs of two targets per lane
+  constexpr bool kOdd = kT & 1;    // the last pack has one
   const int tend = m.end[B];
   float bx[kPacks][4];
 #pragma unroll
   for (int p = 0; p < kPacks; p++) bx[p][0] = bx[p][1] = INFINITY, bx[p][2] = bx[p][3] = -INFINITY;
+  // target offsets from B's centre, held in registers for the chunk
+  float2 z[kT];
 #pragma unroll
   for (int k = 0; k < kT; k++) {
     const int t = t0 + 32 * k + lane, p = k >> 1;
-    const float2 zk = t < tend ? m.loc[t] : make_float2(0.f, 0.f);
+    z[k] = t < tend ? m.loc[t] : make_float2(0.f, 0.f);
     if (t < tend)
-      bx[p][0] = fminf(bx[p][0], zk.x), bx[p][1] = fminf(bx[p][1], zk.y), bx[p][2] = fmaxf(bx[p][2], zk.x),
-      bx[p][3] = fmaxf(bx[p][3], zk.y);
+      bx[p][0] = fminf(bx[p][0], z[k].x), bx[p][1] = fminf(bx[p][1], z[k].y), bx[p][2] = fmaxf(bx[p][2], z[k].x),
+      bx[p][3] = fmaxf(bx[p][3], z[k].y);
     w.acc[32 * k + lane] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   // each pack's target box (offsets from B's centre) and rc^2, in shared memory
@@ -1677,49 +1713,62 @@ __device__ __forceinline__ void near_chunk(const MixedView &m, const Decisions &
     w.tbox[8] = __fmul_rn(rc, rc);
   }
   __syncwarp();
-  // target offsets from B's centre, held in registers for the chunk
-  float2 zr[kT];
-#pragma unroll
-  for (int k = 0; k < kT; k++) {
-    const int t = t0 + 32 * k + lane;
-    zr[k] = t < tend ? m.loc[t] : make_float2(0.f, 0.f);
-  }
-  auto zof = [&](int k) { return zr[k]; };
-  // valid targets of each pack (the pair counts are per target)
-  const unsigned nt = (unsigned)min(tend - t0, 32 * kT);
-  const unsigned vp0 = kT == 4 ? min(nt, 64u) : nt, vp1 = kT == 4 ? nt - vp0 : 0u;
   const int u0 = m.u_off[l], nu = m.u_off[l + 1] - u0;
-  const int k0 = m.k_off[l], nk = m.k_off[l + 1] - k0;
-  auto src_leaf = [&](int q) { return q < nu ? m.u_idx[u0 + q] : m.k_idx[k0 + q - nu]; };
-  auto direct = [&](int q) {
-    if (!kLearned) return true;
-    return (q < nu ? dec.u[u0 + q] : dec.k[k0 + q - nu]) == 0;
-  };
-  // the next entry with work for these targets: a direct entry, and for a
-  // correction entry at least one chunk within rc of a pack (r0, r1: its
-  // chunks per pack, all for a U entry); culled correction entries are
-  // counted and skipped
-  auto next_work = [&](int q, unsigned &r0, unsigned &r1) {
-    for (; q < nu + nk; q++) {
-      if (!direct(q)) continue;
-      if (q < nu) {
-        r0 = r1 = kAllChunks;
-        return q;
+  const int k0 = m.k_off[l], nq = nu + m.k_off[l + 1] - k0;
+  // The next batch of entries with work for these targets: a direct entry,
+  // and for a correction entry at least one chunk within rc of a pack (r0,
+  // r1: its chunks per pack, all for a U entry).  Counts the batch's pairs,
+  // culled entries' too.  listed = 0 when the lists are done.
+  int qb = 0, listed = 0;
+  auto fill = [&]() {
+    listed = 0;
+    while (listed == 0 && qb < nq) {
+      const int q = qb + (lane >> 1), half = lane & 1;
+      bool take = q < nq;
+      if (kLearned && take) take = (q < nu ? dec.u[u0 + q] : dec.k[k0 + q - nu]) == 0;
+      NearEntry e{0.f, 0.f, 1.f, 0, 0, 0, 0u, 0u};
+      if (take) {
+        const int A = q < nu ? m.u_idx[u0 + q] : m.k_idx[k0 + q - nu];
+        // offset of the source leaf's centre from the two-float centres: FP32
+        // centres alone would carry ~3e-8 absolute error into every close pair
+        e.ox = centre_offset(m.cxf, m.cxl, B, A), e.oy = centre_offset(m.cyf, m.cyl, B, A);
+        e.j0 = m.begin[A], e.cnt = m.end[A] - e.j0;
+        if (kScaled) e.s = m.lscale[A];
+        e.corr = q >= nu;
+        e.r0 = e.r1 = kAllChunks;
+        if (e.corr) chunk_mask<kPacks>(m, A, e.cnt, e.ox, e.oy, w.tbox, half, e.r0, e.r1);
       }
-      const int A = m.k_idx[k0 + q - nu];
-      chunk_mask<kPacks>(m, A, centre_offset(m.cxf, m.cxl, B, A), centre_offset(m.cyf, m.cyl, B, A), w.tbox, lane,
-                         r0, r1);
-      if (r0 | r1) return q;
-      counts_add(w.cnts, lane, 0u, 0u, (unsigned)(m.end[A] - m.begin[A]) * nt);
+      e.r0 |= __shfl_xor_sync(0xffffffffu, e.r0, 1);
+      e.r1 |= __shfl_xor_sync(0xffffffffu, e.r1, 1);
+      // pairs of the chunk's valid targets (the pair counts are per target)
+      const unsigned nt = (unsigned)min(tend - t0, 32 * kT);
+      const unsigned vp0 = kPacks == 2 ? min(nt, 64u) : nt, vp1 = nt - vp0;
+      const bool count = take && half == 0;
+      const unsigned done = count ? mask_blobs(e.r0, e.cnt) * vp0 + (vp1 ? mask_blobs(e.r1, e.cnt) * vp1 : 0u) : 0u;
+      const unsigned c0 = __reduce_add_sync(0xffffffffu, done);
+      const unsigned c1 = __reduce_add_sync(0xffffffffu, e.corr ? done : 0u);
+      const unsigned c2 = __reduce_add_sync(0xffffffffu, count && e.corr ? (unsigned)e.cnt * nt : 0u);
+      if (lane == 0) w.cnts->total[0] += c0, w.cnts->total[1] += c1, w.cnts->total[2] += c2;
+      const bool keep = take && (e.r0 | e.r1);
+      const unsigned kept = __ballot_sync(0xffffffffu, keep) & 0x55555555u;
+      __syncwarp();  // every lane has read the last batch
+      if (keep) {
+        float4 *rec = reinterpret_cast<float4 *>(w.list + __popc(kept & ((1u << (lane & 30)) - 1u)));
+        if (half == 0)
+          rec[0] = make_float4(e.ox, e.oy, e.s, __int_as_float(e.corr));
+        else
+          rec[1] = make_float4(__int_as_float(e.j0), __int_as_float(e.cnt), __uint_as_float(e.r0),
+                               __uint_as_float(e.r1));
+      }
+      __syncwarp();
+      listed = __popc(kept);
+      qb += kBatch;
     }
-    r0 = r1 = 0;
-    return q;
   };
-  // copy source leaf of position q into buffer b (warp-uniform decision)
-  auto stage = [&](int q, int b) {
+  // copy the source leaf of list entry i into buffer b (warp-uniform decision)
+  auto stage = [&](int i, int b) {
     if (!kStaged) return false;
-    const int A = src_leaf(q);
-    const int j0 = m.begin[A], cnt = m.end[A] - j0;
+    const int j0 = w.list[i].j0, cnt = w.list[i].cnt;
     if (!w.staging || cnt > kStage) return false;
     if (lane == 0) {
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -1729,141 +1778,153 @@ __device__ __forceinline__ void near_chunk(const MixedView &m, const Decisions &
     w.inflight |= 1u << b;
     return true;
   };
-  unsigned r0 = 0, r1 = 0;
-  int q = next_work(0, r0, r1);
-  int buf = 0;
-  bool staged = q < nu + nk && stage(q, buf);
-  while (q < nu + nk) {
-    unsigned r0n = 0, r1n = 0;
-    const int qn = next_work(q + 1, r0n, r1n);
-    const bool staged_next = qn < nu + nk && stage(qn, buf ^ 1);
-    const int A = src_leaf(q);
-    // offset of the source leaf's centre from the two-float centres: FP32
-    // centres alone would carry ~3e-8 absolute error into every close pair
-    const float ox = centre_offset(m.cxf, m.cxl, B, A), oy = centre_offset(m.cyf, m.cyl, B, A);
-    const int j0 = m.begin[A], cnt = m.end[A] - j0;
-    bool use_smem = false;
-    if (staged) {
-      if (mbar_wait(&w.bar[buf], (w.parity >> buf) & 1u, wait_limit)) {
-        w.parity ^= 1u << buf;
-        w.inflight &= ~(1u << buf);
-        use_smem = true;
-      } else {
-        w.staging = false;  // the copy stays in flight; read global memory from now on
-        if (lane == 0) set_err(m.st, TREE2D_ERR_TIMEOUT);
+  // each turn stages the next entry (i of the list), then sums the current
+  // one (e0, e1, in buffer buf)
+  int i = 0, buf = 1;
+  bool current = false, staged = false;
+  float4 e0 = make_float4(0.f, 0.f, 0.f, 0.f), e1 = e0;
+  for (;;) {
+    if (i == listed) {
+      fill();
+      i = 0;
+    }
+    const bool staged_next = listed && stage(i, buf ^ 1);
+    if (current) {
+      const int j0 = __float_as_int(e1.x), cnt = __float_as_int(e1.y);
+      unsigned r0 = __float_as_uint(e1.z), r1 = __float_as_uint(e1.w);
+      const bool corr = __float_as_int(e0.w) != 0;
+      bool use_smem = false;
+      if (staged) {
+        if (mbar_wait(&w.bar[buf], (w.parity >> buf) & 1u, wait_limit)) {
+          w.parity ^= 1u << buf;
+          w.inflight &= ~(1u << buf);
+          use_smem = true;
+        } else {
+          w.staging = false;  // the copy stays in flight; read global memory from now on
+          if (lane == 0) set_err(m.st, TREE2D_ERR_TIMEOUT);
+        }
       }
-    }
-    const bool corr = q >= nu;
-    // the targets' offsets from A's centre, negated (see pair), and scaled
-    // by A's s with scaled records
-    const float sA = kScaled ? m.lscale[A] : 1.f;
-    float ntx[kT], nty[kT], sa[kT], sb[kT];
+      // the targets' offsets from A's centre, negated (see pair), and scaled
+      // by A's s with scaled records; an odd target is .x of the last pack
+      float2 ntx[kPairs + kOdd], nty[kPairs + kOdd], sa[kPairs + kOdd], sb[kPairs + kOdd];
 #pragma unroll
-    for (int k = 0; k < kT; k++) {
-      const float2 zk = zof(k);
-      ntx[k] = kScaled ? __fmul_rn(-__fadd_rn(zk.x, ox), sA) : -__fadd_rn(zk.x, ox);
-      nty[k] = kScaled ? __fmul_rn(-__fadd_rn(zk.y, oy), sA) : -__fadd_rn(zk.y, oy);
-      sa[k] = 0.f;
-      sb[k] = 0.f;
-    }
-    unsigned done = 0;  // pairs evaluated for the chunk's valid targets
-    auto runs = [&](const auto src) {
-    while (r0 | r1) {
-      int s0, s1;
-      const int packs = next_run(r0, r1, cnt, s0, s1);
-      done += (unsigned)(s1 - s0) * ((packs & 1 ? vp0 : 0u) + (packs & 2 ? vp1 : 0u));
-      if (kT == 1) {
-        if (!corr)
-          leaf_pairs1<false, kScaled>(src, s0, s1, ntx[0], nty[0], sa[0], sb[0]);
-        else
-          leaf_pairs1<true, kScaled>(src, s0, s1, ntx[0], nty[0], sa[0], sb[0]);
-      } else if (kT == 2 || packs != 3) {
-        // one pack: slots 0, 1, or in a four-slot chunk 2, 3 when the run is
-        // pack 1's alone (constant indices keep the slots in registers)
-        auto one_pack = [&](auto k_) {
-          constexpr int k = decltype(k_)::value;
-          const float2 tx = make_float2(ntx[k], ntx[k + 1]), ty = make_float2(nty[k], nty[k + 1]);
-          float2 a = make_float2(sa[k], sa[k + 1]), b = make_float2(sb[k], sb[k + 1]);
-          if (!corr)
-            leaf_pairs2<false, kScaled, kUnroll>(src, s0, s1, tx, ty, a, b);
-          else
-            leaf_pairs2<true, kScaled, kUnroll>(src, s0, s1, tx, ty, a, b);
-          sa[k] = a.x, sa[k + 1] = a.y, sb[k] = b.x, sb[k + 1] = b.y;
-        };
-        if (kT == 4 && packs == 2)
-          one_pack(std::integral_constant<int, kT - 2>{});
-        else
-          one_pack(std::integral_constant<int, 0>{});
-      } else {
-        const float2 tx0 = make_float2(ntx[0], ntx[1]), ty0 = make_float2(nty[0], nty[1]);
-        const float2 tx1 = make_float2(ntx[kT - 2], ntx[kT - 1]), ty1 = make_float2(nty[kT - 2], nty[kT - 1]);
-        float2 a0 = make_float2(sa[0], sa[1]), b0 = make_float2(sb[0], sb[1]);
-        float2 a1 = make_float2(sa[kT - 2], sa[kT - 1]), b1 = make_float2(sb[kT - 2], sb[kT - 1]);
-        if (!corr)
-          leaf_pairs4<false, kScaled, kUnroll>(src, s0, s1, tx0, ty0, tx1, ty1, a0, b0, a1, b1);
-        else
-          leaf_pairs4<true, kScaled, kUnroll>(src, s0, s1, tx0, ty0, tx1, ty1, a0, b0, a1, b1);
-        sa[0] = a0.x, sa[1] = a0.y, sb[0] = b0.x, sb[1] = b0.y;
-        sa[kT - 2] = a1.x, sa[kT - 1] = a1.y, sb[kT - 2] = b1.x, sb[kT - 1] = b1.y;
+      for (int p = 0; p < kPairs + kOdd; p++) {
+        const int k1 = 2 * p + 1 < kT ? 2 * p + 1 : 2 * p;
+        const float2 dx = __fadd2_rn(make_float2(z[2 * p].x, z[k1].x), f2(e0.x));
+        const float2 dy = __fadd2_rn(make_float2(z[2 * p].y, z[k1].y), f2(e0.y));
+        ntx[p] = kScaled ? __fmul2_rn(dx, f2(-e0.z)) : neg2(dx);
+        nty[p] = kScaled ? __fmul2_rn(dy, f2(-e0.z)) : neg2(dy);
+        sa[p] = sb[p] = f2(0.f);
       }
-    }
-    };
-    if (use_smem)
-      runs(SmemSrc{smem_u32(w.src + buf * kStage)});
-    else
-      runs(GlobalSrc{(kScaled ? m.src4s : m.src4) + j0});
+      auto runs = [&](const auto src, auto corr_, auto unroll_) {
+        constexpr bool kCorr = decltype(corr_)::value;
+        constexpr int kU = decltype(unroll_)::value;
+        while (r0 | r1) {
+          int s0, s1;
+          const int packs = next_run(r0, r1, cnt, s0, s1);
+          if constexpr (kT == 1) {
+            leaf_pairs1<kCorr, kScaled, kU>(src, s0, s1, ntx[0].x, nty[0].x, sa[0].x, sb[0].x);
+          } else if constexpr (kT == 2) {
+            leaf_pairs2<kCorr, kScaled, kU>(src, s0, s1, ntx[0], nty[0], sa[0], sb[0]);
+          } else {
+            if (packs == 1)
+              leaf_pairs2<kCorr, kScaled, kU>(src, s0, s1, ntx[0], nty[0], sa[0], sb[0]);
+            else if (packs == 2) {
+              if constexpr (kOdd)
+                leaf_pairs1<kCorr, kScaled, kU>(src, s0, s1, ntx[1].x, nty[1].x, sa[1].x, sb[1].x);
+              else
+                leaf_pairs2<kCorr, kScaled, kU>(src, s0, s1, ntx[1], nty[1], sa[1], sb[1]);
+            } else {
+              if constexpr (kOdd)
+                leaf_pairs3<kCorr, kScaled, kU>(src, s0, s1, ntx[0], nty[0], ntx[1].x, nty[1].x, sa[0], sb[0], sa[1].x,
+                                                sb[1].x);
+              else
+                leaf_pairs4<kCorr, kScaled, kU>(src, s0, s1, ntx[0], nty[0], ntx[1], nty[1], sa[0], sb[0], sa[1],
+                                                sb[1]);
+            }
+          }
+        }
+      };
+      using Corr = std::integral_constant<bool, true>;
+      using Direct = std::integral_constant<bool, false>;
+      const GlobalSrc global{(kScaled ? m.src4s : m.src4) + j0};
+      if (kStaged && use_smem) {
+        const SmemSrc smem{smem_u32(w.src + buf * kStage)};
+        if (corr)
+          runs(smem, Corr{}, std::integral_constant<int, kUnroll>{});
+        else
+          runs(smem, Direct{}, std::integral_constant<int, kUnroll>{});
+      } else {
+        // the rare path of a staged variant: kept small
+        if (corr)
+          runs(global, Corr{}, std::integral_constant<int, kStaged ? 1 : kUnroll>{});
+        else
+          runs(global, Direct{}, std::integral_constant<int, kStaged ? 1 : kUnroll>{});
+      }
+      const float sg = corr ? -1.f : 1.f;
 #pragma unroll
-    for (int k = 0; k < kT; k++) leaf_add(w.acc, k, lane, corr, sa[k], sb[k]);
-    counts_add(w.cnts, lane, done, corr ? done : 0u, corr ? (unsigned)cnt * nt : 0u);
-    __syncwarp();  // every lane is done with this buffer before it is refilled
-    q = qn;
-    r0 = r0n;
-    r1 = r1n;
+      for (int p = 0; p < kPairs; p++) {
+        float4 *acc = w.acc + 64 * p + lane;
+        float4 s = acc[0], t = acc[32];
+        float2 sx = make_float2(s.x, s.y), cx = make_float2(s.z, s.w), sy = make_float2(t.x, t.y),
+               cy = make_float2(t.z, t.w);
+        leaf_add2(sx, cx, sg, sa[p]);
+        leaf_add2(sy, cy, -sg, sb[p]);
+        acc[0] = make_float4(sx.x, sx.y, cx.x, cx.y);
+        acc[32] = make_float4(sy.x, sy.y, cy.x, cy.y);
+      }
+      if (kOdd) {
+        float4 s = w.acc[64 * kPairs + lane];
+        leaf_add(s.x, s.z, sg, sa[kPairs].x);
+        leaf_add(s.y, s.w, -sg, sb[kPairs].x);
+        w.acc[64 * kPairs + lane] = s;
+      }
+      __syncwarp();  // every lane is done with this buffer before it is refilled
+    }
+    if (!listed) break;
+    e0 = reinterpret_cast<const float4 *>(w.list + i)[0];
+    e1 = reinterpret_cast<const float4 *>(w.list + i)[1];
+    i++;
+    current = true;
     buf ^= 1;
     staged = staged_next;
   }
   // far field: L2P of B's local expansion and the W list's M2P, then in the
   // learned form the accepted U entries' multipoles at the chosen order
-  float2 phi[kT], z[kT];
-#pragma unroll
-  for (int k = 0; k < kT; k++) z[k] = zof(k);
+  float2 phi[kT];
   const unsigned char *wdec = kLearned ? dec.w : nullptr;
-  if (kT == 1) {
-    far_field(m, l, B, z[0], phi[0], wdec, dec.margin);
-  } else {
 #pragma unroll
-    for (int k = 0; k < kT; k += 2)
-      far_field2(m, l, B, z[k], z[(k + 1) % kT], phi[k], phi[(k + 1) % kT], wdec, dec.margin);
-  }
+  for (int k = 0; k + 1 < kT; k += 2) far_field2(m, l, B, z[k], z[k + 1], phi[k], phi[k + 1], wdec, dec.margin);
+  if (kOdd) far_field(m, l, B, z[kT - 1], phi[kT - 1], wdec, dec.margin);
   if (kLearned) {
     for (int e = u0; e < u0 + nu; e++) {
       const int d = dec.u[e];
       if (d > 0) {
         const int A = m.u_idx[e];
         const int p = min(min(class_order(d) + dec.margin, 16), m.P);
-        if (kT == 1) {
-          m2p_order(m, B, A, p, z[0], phi[0]);
-        } else {
 #pragma unroll
-          for (int k = 0; k < kT; k += 2) m2p_order2(m, B, A, p, z[k], z[(k + 1) % kT], phi[k], phi[(k + 1) % kT]);
-        }
+        for (int k = 0; k + 1 < kT; k += 2) m2p_order2(m, B, A, p, z[k], z[k + 1], phi[k], phi[k + 1]);
+        if (kOdd) m2p_order(m, B, A, p, z[kT - 1], phi[kT - 1]);
       }
     }
   }
-  if (lane == 0)
-    for (int c = 0; c < 3; c++) {
-      w.cnts->total[c] += w.cnts->chunk[c];
-      w.cnts->chunk[c] = 0;
-    }
   // FP64 final reduction: u = Im(phi)/2pi + ax/2pi, v = Re(phi)/2pi + ay/2pi
   const double inv2pi = 0.15915494309189533577;
 #pragma unroll
   for (int k = 0; k < kT; k++)
     if (t0 + 32 * k + lane < tend) {
-      const float4 sacc = w.acc[32 * k + lane];
+      // slot k: .x or .y of its pack's records
+      const float4 s = w.acc[64 * (k >> 1) + lane];
+      float ax, cx, ay, cy;
+      if (kOdd && k == kT - 1) {
+        ax = s.x, ay = s.y, cx = s.z, cy = s.w;
+      } else {
+        const float4 t = w.acc[64 * (k >> 1) + 32 + lane];
+        ax = k & 1 ? s.y : s.x, cx = k & 1 ? s.w : s.z, ay = k & 1 ? t.y : t.x, cy = k & 1 ? t.w : t.z;
+      }
       const int o = perm[t0 + 32 * k + lane];
-      uv[2 * (size_t)o] = ((double)phi[k].y + (double)sacc.x - (double)sacc.y) * inv2pi;
-      uv[2 * (size_t)o + 1] = ((double)phi[k].x + (double)sacc.z - (double)sacc.w) * inv2pi;
+      uv[2 * (size_t)o] = ((double)phi[k].y + (double)ax + (double)cx) * inv2pi;
+      uv[2 * (size_t)o + 1] = ((double)phi[k].x + (double)ay + (double)cy) * inv2pi;
     }
   __syncwarp();
 }
@@ -1875,12 +1936,13 @@ __global__ void __launch_bounds__(32 * kWarps, (kWide ? 24 : 32) / kWarps) k_eva
   __shared__ __align__(8) uint64_t s_bar[kWarps][2];
   __shared__ float s_tb[kWarps][9];
   __shared__ __align__(16) float4 s_acc[kWarps][4 * 32];
+  __shared__ NearEntry s_list[kWarps][kBatch];
   __shared__ WarpCounts s_cnt[kWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int i = next_leaf(m.st, lane);
   if (i >= m.nleaf) return;  // uniform over the warp; nothing below syncs the block
-  NearWarp w{s_src + (kStaged ? warp * 2 * kStage : 0), s_bar[warp], s_tb[warp], s_acc[warp], &s_cnt[warp], 0u, 0u,
-             true};
+  NearWarp w{s_src + (kStaged ? warp * 2 * kStage : 0), s_bar[warp], s_tb[warp], s_acc[warp], s_list[warp],
+             &s_cnt[warp], 0u, 0u, true};
   if (kStaged && lane == 0) {
     mbar_init(&w.bar[0], 1);
     mbar_init(&w.bar[1], 1);
@@ -1896,6 +1958,9 @@ __global__ void __launch_bounds__(32 * kWarps, (kWide ? 24 : 32) / kWarps) k_eva
       if (rem > 96) {
         near_chunk<kLearned, kStaged, 4, kWide ? 4 : 2, kScaled>(m, dec, uv, perm, wait_limit, l, B, t0, lane, w);
         t0 += 128;
+      } else if (rem > 64) {
+        near_chunk<kLearned, kStaged, 3, kWide ? 4 : 2, kScaled>(m, dec, uv, perm, wait_limit, l, B, t0, lane, w);
+        t0 += 96;
       } else if (rem > 32) {
         near_chunk<kLearned, kStaged, 2, kWide ? 4 : 2, kScaled>(m, dec, uv, perm, wait_limit, l, B, t0, lane, w);
         t0 += 64;

@@ -324,3 +324,47 @@ def test_mixed_expansion_lengths(gpu_lib):
         P.set_mixed_params(16, 2.5, True)
     assert rel[24] <= REL_L2 and rel[16] <= REL_L2, rel
     assert rel[8] > rel[16] and rel[8] <= 1e-2, rel
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("uniform_cores", [True, False])
+@pytest.mark.parametrize("leaf", [15, 32, 64, 96, 128, 300])
+def test_near_field_over_leaf_sizes(gpu_lib, leaf, uniform_cores):
+    """Leaves of one to four targets per lane and beyond a stage buffer, with
+    correction lists of many entries, one core radius or many: every
+    near-field variant gives the same bits and pair counts, and meets the
+    accuracy bar.  32 terms and a cutoff of 5.5 radii leave FP32's rounding
+    only: a pair's factor is within a few 2^-22 of exact, and the bar is 1e-6."""
+    torch = pytest.importorskip("torch")
+    P = gpu_lib
+    rng = np.random.default_rng(leaf)
+    n = 9000
+    xy = rng.normal(size=(n, 2))
+    cir = rng.uniform(0.5, 1.5, n) / n
+    cor = np.full(n, 0.12) if uniform_cores else rng.uniform(0.06, 0.12, n)
+    dev = torch.device("cuda:0")
+    t = [torch.from_numpy(np.ascontiguousarray(a)).to(dev) for a in (xy, cir, cor)]
+    ref = torch.empty_like(t[0])
+    P.direct_device(t[0].data_ptr(), n, t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), n, ref.data_ptr())
+    P.set_params(11, 33, 0.5)
+    P.set_mode(P.MODE_MIXED)
+    P.set_mixed_params(32, 5.5, True)
+    P.set_mixed_leaf(leaf)
+    outs = []
+    try:
+        for v in range(P.EVAL_VARIANTS):
+            P.set_tuning(False, v)
+            uv = torch.empty_like(ref)
+            P.solve_device(t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), uv.data_ptr(), n)
+            torch.cuda.synchronize()
+            s = P.stats()
+            outs.append((uv, [s[k] for k in ("n_pairs", "n_pairs_k", "n_pairs_k_listed")]))
+    finally:
+        P.set_tuning(True, -1)
+        P.set_mixed_leaf(-1)
+        P.set_mixed_params()
+        P.set_mode(P.MODE_PLAIN)
+        P.clear_params()
+    for uv, counts in outs:
+        assert torch.equal(uv, outs[0][0]) and counts == outs[0][1]
+    assert float(torch.linalg.norm(uv - ref) / torch.linalg.norm(ref)) <= REL_L2
