@@ -1335,6 +1335,8 @@ __device__ __forceinline__ float sfu_rcp(float x) {
 //                   1 - e^-x is taken from its series x (1 - x/2) =
 //                   t (-ln2 - (ln2)^2/2 t) below x = 1e-3, where the
 //                   subtraction would cancel;
+//   direct, far:    the same without the series, for leaves none of whose
+//                   pairs is that close (scaled records only);
 //   correction (K): f = G exp(-r^2/s^2) / r^2, velocity (-a, b): the
 //                   correction -G exp(-r^2/s^2) / r^2 of every pair of the
 //                   two leaves (the list holds the leaves within rc; pairs
@@ -1355,7 +1357,9 @@ constexpr float kSerT = -1.44269504e-3f;  // t at x = 1e-3
 // q = r^2 log2(e) / sigma^2 itself, the Gaussian exp2(-q) needs no product
 // per pair, and G s / q carries the 1 / r^2 (G s / q (y s) = G / r^2 y).
 // One FP32 operation fewer per pair, the same quantities up to rounding.
-template <bool kCorrection, bool kScaled = false>
+enum PairForm { kDirect, kCorrection, kDirectFar };
+
+template <int kForm, bool kScaled = false>
 __device__ __forceinline__ void pair(const float4 sj, float ntx, float nty, float &a, float &b) {
   const float nrx = __fadd_rn(sj.x, ntx), nry = __fadd_rn(sj.y, nty);
   const float r2 = fmaf(nrx, nrx, fmaf(nry, nry, 1e-30f));
@@ -1364,7 +1368,9 @@ __device__ __forceinline__ void pair(const float4 sj, float ntx, float nty, floa
   const float e = sfu_exp2(kScaled ? -r2 : t);
   const float ir2 = sfu_rcp(r2);
   float f;
-  if (!kCorrection) {
+  if (kForm == kDirectFar) {
+    f = __fmul_rn(__fmul_rn(sj.z, fmaf(-1.f, e, 1.f)), ir2);
+  } else if (kForm == kDirect) {
     // x (1 - x/2) = t (-ln2 - (ln2)^2/2 t) = q (ln2 - (ln2)^2/2 q), the same bits
     const float ser = kScaled ? __fmul_rn(r2, fmaf(kSer2, r2, -kSer1)) : __fmul_rn(t, fmaf(kSer2, t, kSer1));
     const float ome = fmaf(-1.f, e, 1.f);
@@ -1381,7 +1387,7 @@ __device__ __forceinline__ void pair(const float4 sj, float ntx, float nty, floa
 // instruction forms both targets' value of every step, with the rounding
 // of the scalar step (each component rounds as the scalar operation does),
 // so a target's sum does not depend on how many targets its lane holds.
-template <bool kCorrection, bool kScaled = false>
+template <int kForm, bool kScaled = false>
 __device__ __forceinline__ void pair2(const float4 sj, float2 ntx, float2 nty, float2 &a, float2 &b) {
   const float2 nrx = __fadd2_rn(f2(sj.x), ntx), nry = __fadd2_rn(f2(sj.y), nty);
   const float2 r2 = __ffma2_rn(nrx, nrx, __ffma2_rn(nry, nry, f2(1e-30f)));
@@ -1389,7 +1395,9 @@ __device__ __forceinline__ void pair2(const float4 sj, float2 ntx, float2 nty, f
   const float2 e = kScaled ? make_float2(sfu_exp2(-r2.x), sfu_exp2(-r2.y)) : make_float2(sfu_exp2(t.x), sfu_exp2(t.y));
   const float2 ir2 = make_float2(sfu_rcp(r2.x), sfu_rcp(r2.y));
   float2 f;
-  if (!kCorrection) {
+  if (kForm == kDirectFar) {
+    f = __fmul2_rn(__fmul2_rn(f2(sj.z), __ffma2_rn(f2(-1.f), e, f2(1.f))), ir2);
+  } else if (kForm == kDirect) {
     const float2 ser = kScaled ? __fmul2_rn(r2, __ffma2_rn(f2(kSer2), r2, f2(-kSer1)))
                                : __fmul2_rn(t, __ffma2_rn(f2(kSer2), t, f2(kSer1)));
     const float2 ome = __ffma2_rn(f2(-1.f), e, f2(1.f));
@@ -1428,38 +1436,38 @@ struct GlobalSrc {
 // source record; the targets are given negated (see pair).  Each source leaf is summed in plain FP32 and then
 // added with compensation (leaf_add), so the compensated sum costs once per
 // leaf, not once per pair.
-template <bool kCorrection, bool kScaled, int kUnroll, class S>
+template <int kForm, bool kScaled, int kUnroll, class S>
 __device__ __forceinline__ void leaf_pairs1(const S src, int j0, int j1, float ntx, float nty, float &a, float &b) {
 #pragma unroll kUnroll
-  for (int j = j0; j < j1; j++) pair<kCorrection, kScaled>(src[j], ntx, nty, a, b);
+  for (int j = j0; j < j1; j++) pair<kForm, kScaled>(src[j], ntx, nty, a, b);
 }
 
-template <bool kCorrection, bool kScaled, int kUnroll, class S>
+template <int kForm, bool kScaled, int kUnroll, class S>
 __device__ __forceinline__ void leaf_pairs2(const S src, int j0, int j1, float2 ntx, float2 nty, float2 &a,
                                             float2 &b) {
 #pragma unroll kUnroll
-  for (int j = j0; j < j1; j++) pair2<kCorrection, kScaled>(src[j], ntx, nty, a, b);
+  for (int j = j0; j < j1; j++) pair2<kForm, kScaled>(src[j], ntx, nty, a, b);
 }
 
-template <bool kCorrection, bool kScaled, int kUnroll, class S>
+template <int kForm, bool kScaled, int kUnroll, class S>
 __device__ __forceinline__ void leaf_pairs3(const S src, int j0, int j1, float2 ntx0, float2 nty0, float ntx1,
                                             float nty1, float2 &a0, float2 &b0, float &a1, float &b1) {
 #pragma unroll kUnroll
   for (int j = j0; j < j1; j++) {
     const float4 sj = src[j];
-    pair2<kCorrection, kScaled>(sj, ntx0, nty0, a0, b0);
-    pair<kCorrection, kScaled>(sj, ntx1, nty1, a1, b1);
+    pair2<kForm, kScaled>(sj, ntx0, nty0, a0, b0);
+    pair<kForm, kScaled>(sj, ntx1, nty1, a1, b1);
   }
 }
 
-template <bool kCorrection, bool kScaled, int kUnroll, class S>
+template <int kForm, bool kScaled, int kUnroll, class S>
 __device__ __forceinline__ void leaf_pairs4(const S src, int j0, int j1, float2 ntx0, float2 nty0, float2 ntx1,
                                             float2 nty1, float2 &a0, float2 &b0, float2 &a1, float2 &b1) {
 #pragma unroll kUnroll
   for (int j = j0; j < j1; j++) {
     const float4 sj = src[j];
-    pair2<kCorrection, kScaled>(sj, ntx0, nty0, a0, b0);
-    pair2<kCorrection, kScaled>(sj, ntx1, nty1, a1, b1);
+    pair2<kForm, kScaled>(sj, ntx0, nty0, a0, b0);
+    pair2<kForm, kScaled>(sj, ntx1, nty1, a1, b1);
   }
 }
 
@@ -1534,18 +1542,19 @@ __device__ __forceinline__ int next_run(unsigned &r0, unsigned &r1, int cnt, int
   return packs;
 }
 
-// Chunks of correction source leaf A whose pairs with a pack of targets can
-// lie within the correction radius: bit k of m0 (m1) for the kChunk-blob chunk
-// k of A whose bounding box comes within rc of pack 0's (pack 1's) target
-// box, tb[0..3] (tb[4..7]), rc^2 in tb[8]; the boxes are offsets from the
-// target leaf's centre, (ox, oy) is A's centre seen from there.  Pairs
-// farther than rc from every target add terms below exp(-rc^2/sigma^2) of a
-// point vortex: the ones the correction list already leaves out beyond rc.
+// Chunks of source leaf A whose pairs with a pack of targets can lie within
+// a distance r, lim = r^2: bit k of m0 (m1) for the kChunk-blob chunk k of A
+// whose bounding box comes within r of pack 0's (pack 1's) target box, tb[0..3]
+// (tb[4..7]); the boxes are offsets from the target leaf's centre, (ox, oy) is
+// A's centre seen from there.  For a correction entry r is the correction
+// radius rc: pairs farther than rc from every target add terms below
+// exp(-rc^2/sigma^2) of a point vortex, the ones the correction list already
+// leaves out beyond rc.  For a direct entry see series_limit.
 // A leaf of more than 32 chunks is not culled (kAllChunks).  A lane forms
 // every second chunk's bits, from chunk `first` on.
 template <int kPacks>
 __device__ __forceinline__ void chunk_mask(const MixedView &m, int A, int cnt, float ox, float oy, const float *tb,
-                                           int first, unsigned &m0, unsigned &m1) {
+                                           float lim, int first, unsigned &m0, unsigned &m1) {
   const int nch = (cnt + kChunk - 1) >> kChunkShift;
   if (nch > 32 || nch > m.kchunks) {
     m0 = m1 = kAllChunks;
@@ -1557,7 +1566,6 @@ __device__ __forceinline__ void chunk_mask(const MixedView &m, int A, int cnt, f
   for (int p = 0; p < kPacks; p++)
     T[p] = make_float4(__fadd_rn(tb[4 * p], ox), __fadd_rn(tb[4 * p + 1], oy), __fadd_rn(tb[4 * p + 2], ox),
                        __fadd_rn(tb[4 * p + 3], oy));
-  const float rc2 = tb[8];
   unsigned keep[2] = {0, 0};
 #pragma unroll 2
   for (int k = first; k < nch; k += 2) {
@@ -1566,11 +1574,23 @@ __device__ __forceinline__ void chunk_mask(const MixedView &m, int A, int cnt, f
     for (int p = 0; p < kPacks; p++) {
       const float gx = fmaxf(fmaxf(__fsub_rn(s.x, T[p].z), __fsub_rn(T[p].x, s.z)), 0.f);
       const float gy = fmaxf(fmaxf(__fsub_rn(s.y, T[p].w), __fsub_rn(T[p].y, s.w)), 0.f);
-      if (fmaf(gx, gx, __fmul_rn(gy, gy)) <= rc2) keep[p] |= 1u << k;
+      if (fmaf(gx, gx, __fmul_rn(gy, gy)) <= lim) keep[p] |= 1u << k;
     }
   }
   m0 = keep[0];
   m1 = kPacks == 2 ? keep[1] : keep[0];
+}
+
+// The square of a distance beyond which no pair of a direct entry takes the
+// series (q >= -kSerT in its FP32 evaluation), q = (s d)^2 with scale s: s d
+// is formed from coordinates of at most `extent` with four roundings, so that
+// it is off by less than 2^-22 s extent, and q by a few 2^-24 of itself;
+// 0.0384^2 is 2% above -kSerT.  Without the series a direct pair takes 6.5
+// issue slots instead of 9.5: whole solves of 512 sets 14.00 -> 13.42 ms, of 4M
+// two-patch + sheet blobs 6.41 -> 6.28.
+__device__ __forceinline__ float series_limit(float s, float extent) {
+  const float r = (0.0384f + 0x1p-20f * s * extent) / s;
+  return r * r;
 }
 
 // Blobs in the chunks of `mask`, of a leaf of cnt blobs.
@@ -1634,10 +1654,11 @@ constexpr int kBatch = 16;   // entries prepared at a time
 constexpr long kEvalWaitLimit = 1l << 22;  // polls; a healthy copy lands within microseconds
 
 // One source leaf with work: its centre's offset from the target leaf's, its
-// scale (1 without scaled records), its blobs, its kept chunks per pack.
+// scale (1 without scaled records), its pairs' form, its blobs, its kept
+// chunks per pack.
 struct __align__(16) NearEntry {
   float ox, oy, s;
-  int corr;
+  int form;
   int j0, cnt;
   unsigned r0, r1;
 };
@@ -1726,7 +1747,7 @@ __device__ __forceinline__ void near_chunk(const MixedView &m, const Decisions &
       const int q = qb + (lane >> 1), half = lane & 1;
       bool take = q < nq;
       if (kLearned && take) take = (q < nu ? dec.u[u0 + q] : dec.k[k0 + q - nu]) == 0;
-      NearEntry e{0.f, 0.f, 1.f, 0, 0, 0, 0u, 0u};
+      NearEntry e{0.f, 0.f, 1.f, kDirect, 0, 0, 0u, 0u};
       if (take) {
         const int A = q < nu ? m.u_idx[u0 + q] : m.k_idx[k0 + q - nu];
         // offset of the source leaf's centre from the two-float centres: FP32
@@ -1734,20 +1755,28 @@ __device__ __forceinline__ void near_chunk(const MixedView &m, const Decisions &
         e.ox = centre_offset(m.cxf, m.cxl, B, A), e.oy = centre_offset(m.cyf, m.cyl, B, A);
         e.j0 = m.begin[A], e.cnt = m.end[A] - e.j0;
         if (kScaled) e.s = m.lscale[A];
-        e.corr = q >= nu;
+        e.form = q >= nu ? kCorrection : kDirect;
         e.r0 = e.r1 = kAllChunks;
-        if (e.corr) chunk_mask<kPacks>(m, A, e.cnt, e.ox, e.oy, w.tbox, half, e.r0, e.r1);
+        if (kScaled || e.form == kCorrection) {
+          const float side = 2.f * (fabsf(e.ox) + fabsf(e.oy)) + 2.f * (m.h[A] + m.h[B]);
+          chunk_mask<kPacks>(m, A, e.cnt, e.ox, e.oy, w.tbox,
+                             e.form == kCorrection ? w.tbox[8] : series_limit(e.s, side), half, e.r0, e.r1);
+        }
       }
       e.r0 |= __shfl_xor_sync(0xffffffffu, e.r0, 1);
       e.r1 |= __shfl_xor_sync(0xffffffffu, e.r1, 1);
+      if (kScaled && take && e.form == kDirect) {  // every chunk; with the series if some may need it
+        if ((e.r0 | e.r1) == 0u) e.form = kDirectFar;
+        e.r0 = e.r1 = kAllChunks;
+      }
       // pairs of the chunk's valid targets (the pair counts are per target)
       const unsigned nt = (unsigned)min(tend - t0, 32 * kT);
       const unsigned vp0 = kPacks == 2 ? min(nt, 64u) : nt, vp1 = nt - vp0;
       const bool count = take && half == 0;
       const unsigned done = count ? mask_blobs(e.r0, e.cnt) * vp0 + (vp1 ? mask_blobs(e.r1, e.cnt) * vp1 : 0u) : 0u;
       const unsigned c0 = __reduce_add_sync(0xffffffffu, done);
-      const unsigned c1 = __reduce_add_sync(0xffffffffu, e.corr ? done : 0u);
-      const unsigned c2 = __reduce_add_sync(0xffffffffu, count && e.corr ? (unsigned)e.cnt * nt : 0u);
+      const unsigned c1 = __reduce_add_sync(0xffffffffu, e.form == kCorrection ? done : 0u);
+      const unsigned c2 = __reduce_add_sync(0xffffffffu, count && e.form == kCorrection ? (unsigned)e.cnt * nt : 0u);
       if (lane == 0) w.cnts->total[0] += c0, w.cnts->total[1] += c1, w.cnts->total[2] += c2;
       const bool keep = take && (e.r0 | e.r1);
       const unsigned kept = __ballot_sync(0xffffffffu, keep) & 0x55555555u;
@@ -1755,7 +1784,7 @@ __device__ __forceinline__ void near_chunk(const MixedView &m, const Decisions &
       if (keep) {
         float4 *rec = reinterpret_cast<float4 *>(w.list + __popc(kept & ((1u << (lane & 30)) - 1u)));
         if (half == 0)
-          rec[0] = make_float4(e.ox, e.oy, e.s, __int_as_float(e.corr));
+          rec[0] = make_float4(e.ox, e.oy, e.s, __int_as_float(e.form));
         else
           rec[1] = make_float4(__int_as_float(e.j0), __int_as_float(e.cnt), __uint_as_float(e.r0),
                                __uint_as_float(e.r1));
@@ -1792,7 +1821,7 @@ __device__ __forceinline__ void near_chunk(const MixedView &m, const Decisions &
     if (current) {
       const int j0 = __float_as_int(e1.x), cnt = __float_as_int(e1.y);
       unsigned r0 = __float_as_uint(e1.z), r1 = __float_as_uint(e1.w);
-      const bool corr = __float_as_int(e0.w) != 0;
+      const int form = __float_as_int(e0.w);
       bool use_smem = false;
       if (staged) {
         if (mbar_wait(&w.bar[buf], (w.parity >> buf) & 1u, wait_limit)) {
@@ -1816,52 +1845,63 @@ __device__ __forceinline__ void near_chunk(const MixedView &m, const Decisions &
         nty[p] = kScaled ? __fmul2_rn(dy, f2(-e0.z)) : neg2(dy);
         sa[p] = sb[p] = f2(0.f);
       }
-      auto runs = [&](const auto src, auto corr_, auto unroll_) {
-        constexpr bool kCorr = decltype(corr_)::value;
+      auto runs = [&](const auto src, auto form_, auto unroll_) {
+        constexpr int kForm = decltype(form_)::value;
         constexpr int kU = decltype(unroll_)::value;
         while (r0 | r1) {
           int s0, s1;
           const int packs = next_run(r0, r1, cnt, s0, s1);
           if constexpr (kT == 1) {
-            leaf_pairs1<kCorr, kScaled, kU>(src, s0, s1, ntx[0].x, nty[0].x, sa[0].x, sb[0].x);
+            leaf_pairs1<kForm, kScaled, kU>(src, s0, s1, ntx[0].x, nty[0].x, sa[0].x, sb[0].x);
           } else if constexpr (kT == 2) {
-            leaf_pairs2<kCorr, kScaled, kU>(src, s0, s1, ntx[0], nty[0], sa[0], sb[0]);
+            leaf_pairs2<kForm, kScaled, kU>(src, s0, s1, ntx[0], nty[0], sa[0], sb[0]);
           } else {
             if (packs == 1)
-              leaf_pairs2<kCorr, kScaled, kU>(src, s0, s1, ntx[0], nty[0], sa[0], sb[0]);
+              leaf_pairs2<kForm, kScaled, kU>(src, s0, s1, ntx[0], nty[0], sa[0], sb[0]);
             else if (packs == 2) {
               if constexpr (kOdd)
-                leaf_pairs1<kCorr, kScaled, kU>(src, s0, s1, ntx[1].x, nty[1].x, sa[1].x, sb[1].x);
+                leaf_pairs1<kForm, kScaled, kU>(src, s0, s1, ntx[1].x, nty[1].x, sa[1].x, sb[1].x);
               else
-                leaf_pairs2<kCorr, kScaled, kU>(src, s0, s1, ntx[1], nty[1], sa[1], sb[1]);
+                leaf_pairs2<kForm, kScaled, kU>(src, s0, s1, ntx[1], nty[1], sa[1], sb[1]);
             } else {
               if constexpr (kOdd)
-                leaf_pairs3<kCorr, kScaled, kU>(src, s0, s1, ntx[0], nty[0], ntx[1].x, nty[1].x, sa[0], sb[0], sa[1].x,
+                leaf_pairs3<kForm, kScaled, kU>(src, s0, s1, ntx[0], nty[0], ntx[1].x, nty[1].x, sa[0], sb[0], sa[1].x,
                                                 sb[1].x);
               else
-                leaf_pairs4<kCorr, kScaled, kU>(src, s0, s1, ntx[0], nty[0], ntx[1], nty[1], sa[0], sb[0], sa[1],
+                leaf_pairs4<kForm, kScaled, kU>(src, s0, s1, ntx[0], nty[0], ntx[1], nty[1], sa[0], sb[0], sa[1],
                                                 sb[1]);
             }
           }
         }
       };
-      using Corr = std::integral_constant<bool, true>;
-      using Direct = std::integral_constant<bool, false>;
+      using Direct = std::integral_constant<int, kDirect>;
+      using DirectFar = std::integral_constant<int, kDirectFar>;
+      using Correction = std::integral_constant<int, kCorrection>;
+      using Unroll = std::integral_constant<int, kUnroll>;
       const GlobalSrc global{(kScaled ? m.src4s : m.src4) + j0};
       if (kStaged && use_smem) {
         const SmemSrc smem{smem_u32(w.src + buf * kStage)};
-        if (corr)
-          runs(smem, Corr{}, std::integral_constant<int, kUnroll>{});
+        if (form == kCorrection)
+          runs(smem, Correction{}, Unroll{});
+        else if (kScaled && form == kDirectFar)
+          runs(smem, DirectFar{}, Unroll{});
         else
-          runs(smem, Direct{}, std::integral_constant<int, kUnroll>{});
+          runs(smem, Direct{}, Unroll{});
+      } else if (kStaged) {  // rare: kept small
+        using One = std::integral_constant<int, 1>;
+        if (form == kCorrection)
+          runs(global, Correction{}, One{});
+        else
+          runs(global, Direct{}, One{});
       } else {
-        // the rare path of a staged variant: kept small
-        if (corr)
-          runs(global, Corr{}, std::integral_constant<int, kStaged ? 1 : kUnroll>{});
+        if (form == kCorrection)
+          runs(global, Correction{}, Unroll{});
+        else if (kScaled && form == kDirectFar)
+          runs(global, DirectFar{}, Unroll{});
         else
-          runs(global, Direct{}, std::integral_constant<int, kStaged ? 1 : kUnroll>{});
+          runs(global, Direct{}, Unroll{});
       }
-      const float sg = corr ? -1.f : 1.f;
+      const float sg = form == kCorrection ? -1.f : 1.f;
 #pragma unroll
       for (int p = 0; p < kPairs; p++) {
         float4 *acc = w.acc + 64 * p + lane;
@@ -2153,7 +2193,7 @@ __global__ void __launch_bounds__(kPtWarps * 32) k_eval_points(MixedView m, int 
         const float nfx = -(float)dx, nfy = -(float)dy;
         float sa = 0.f, sb = 0.f;  // velocity (sa, -sb), see pair
         const int e = m.end[c];
-        for (int j = m.begin[c]; j < e; j++) pair<false>(m.src4[j], nfx, nfy, sa, sb);
+        for (int j = m.begin[c]; j < e; j++) pair<kDirect>(m.src4[j], nfx, nfy, sa, sb);
         ax.add(sa);
         ay.add(-sb);
         n_pairs += (unsigned)(e - m.begin[c]);

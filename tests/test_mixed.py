@@ -368,3 +368,45 @@ def test_near_field_over_leaf_sizes(gpu_lib, leaf, uniform_cores):
     for uv, counts in outs:
         assert torch.equal(uv, outs[0][0]) and counts == outs[0][1]
     assert float(torch.linalg.norm(uv - ref) / torch.linalg.norm(ref)) <= REL_L2
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("gap", [0.0016, 0.02, 0.037, 0.0385, 0.05, 0.4])
+def test_close_leaves_take_the_series(gpu_lib, gap):
+    """Two clusters on either side of a cell edge, `gap` core radii apart:
+    pairs closer than 0.0316 radii lose 1 - exp(-x) to cancellation unless
+    they take its series, which pairs of leaves far enough apart skip.
+    Bound per blob, in units of the magnitudes of its terms: beyond the
+    series' border x = 1e-3, 1 - e is off by e's 2^-22 + 2^-24, 3.0e-4 of it;
+    offsets of 0.1 rounded to FP32 move distances of 5e-4 by 5e-5."""
+    torch = pytest.importorskip("torch")
+    P = gpu_lib
+    rng = np.random.default_rng(3)
+    c = rng.uniform(-4e-4, 4e-4, (2, 20, 2)) + np.array([[[gap / 2 + 4e-4, 0.05]], [[-gap / 2 - 4e-4, 0.05]]])
+    w = max(0.1, gap)
+    xy = np.concatenate([c.reshape(-1, 2), w * np.array([[1, 1], [-1, 1], [1, -1], [-1, -1]])])
+    n = len(xy)
+    cir = np.concatenate([rng.uniform(0.5, 1.5, n - 4), np.zeros(4)])
+    cor = np.ones(n)
+    d = xy[:, None] - xy[None]
+    r2 = (d ** 2).sum(-1)
+    np.fill_diagonal(r2, 1.0)
+    f = -cir[None] * np.expm1(-r2) / r2 / (2 * np.pi)
+    np.fill_diagonal(f, 0.0)
+    ref = np.stack([-(f * d[..., 1]).sum(1), (f * d[..., 0]).sum(1)], axis=1)
+    mag = (f * np.sqrt(r2)).sum(1)
+    dev = torch.device("cuda:0")
+    t = [torch.from_numpy(np.ascontiguousarray(a)).to(dev) for a in (xy, cir, cor)]
+    P.set_params(11, 33, 0.5)
+    P.set_mode(P.MODE_MIXED)
+    P.set_mixed_leaf(32)
+    try:
+        uv = torch.empty_like(t[0])
+        P.solve_device(t[0].data_ptr(), t[1].data_ptr(), t[2].data_ptr(), uv.data_ptr(), n)
+        torch.cuda.synchronize()
+    finally:
+        P.set_mixed_leaf(-1)
+        P.set_mode(P.MODE_PLAIN)
+        P.clear_params()
+    err = np.linalg.norm(uv.cpu().numpy() - ref, axis=1)
+    assert (err <= 4e-4 * mag)[:n - 4].all(), (err / mag)[:n - 4].max()
