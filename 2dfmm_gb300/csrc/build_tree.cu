@@ -112,6 +112,7 @@ struct Extremes {
 // circulations and core radii are checked where they are first read, in
 // k_gather).
 __global__ void __launch_bounds__(256) k_bbox(const double *__restrict__ xy, int n, Box4 *part, DevStatus *st) {
+  chain_wait();
   Extremes ex;
   ex.init();
   bool bad = false;
@@ -144,6 +145,7 @@ __device__ __forceinline__ RootBox root_from_box(const Box4 &r) {
 // The root box from the blocks' extremes: one block of kRootThreads.
 constexpr int kRootThreads = 256;
 __global__ void __launch_bounds__(kRootThreads) k_root(const Box4 *part, int nparts, RootBox *root) {
+  chain_wait();
   uint64_t e[4] = {okey(-INFINITY), okey(INFINITY), okey(-INFINITY), okey(INFINITY)};
   for (int k = threadIdx.x; k < nparts; k += kRootThreads) {
     const Box4 p = part[k];
@@ -175,6 +177,7 @@ constexpr int kSetSlices = 16;
 
 __global__ void __launch_bounds__(256) k_bbox_sets(const double *__restrict__ xy, const int *__restrict__ off,
                                                    Box4 *part, int *set_of, DevStatus *st) {
+  chain_wait();
   const int set = blockIdx.x;
   const int n0 = off[set], len = off[set + 1] - n0;
   const int per = (len + kSetSlices - 1) / kSetSlices;
@@ -194,6 +197,7 @@ __global__ void __launch_bounds__(256) k_bbox_sets(const double *__restrict__ xy
 }
 
 __global__ void k_roots_sets(const Box4 *part, int nsets, RootBox *roots) {
+  chain_wait();
   const int set = blockIdx.x * blockDim.x + threadIdx.x;
   if (set >= nsets) return;
   Box4 r = part[(size_t)set * kSetSlices];
@@ -231,6 +235,7 @@ inline size_t centre_entries(int lt) { return ((size_t)1 << lt) - 1; }
 
 __global__ void __launch_bounds__(256) k_centre_table(const RootBox *__restrict__ root, uint64_t *__restrict__ tab,
                                                       int lt) {
+  chain_wait();
   const int per = (1 << lt) - 1;
   root += blockIdx.y;  // batched sets: one table per set root
   tab += (size_t)blockIdx.y * 2 * per;
@@ -261,6 +266,7 @@ __global__ void __launch_bounds__(256) k_centre_table(const RootBox *__restrict_
 constexpr int kSetTableLevels = 12;
 __global__ void __launch_bounds__(256) k_centre_table_sets(const RootBox *__restrict__ root,
                                                            uint64_t *__restrict__ tab, int lt) {
+  chain_wait();
   __shared__ double c[(1 << kSetTableLevels) - 1];
   const int per = (1 << lt) - 1;
   const int set = blockIdx.x >> 1, axis = blockIdx.x & 1;
@@ -334,6 +340,7 @@ __global__ void __launch_bounds__(256) k_keys(const double *__restrict__ xy, int
                                               const uint64_t *__restrict__ tab, int tlev, uint64_t *__restrict__ keys,
                                               uint32_t *__restrict__ vals, int levels, const int *__restrict__ set_of,
                                               int lev0, int packed) {
+  chain_wait();
   long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   double x = xy[2 * i], y = xy[2 * i + 1];
@@ -392,6 +399,7 @@ __global__ void __launch_bounds__(256) k_keys(const double *__restrict__ xy, int
 // position's fraction of the root box, packed over the point's index.
 __global__ void __launch_bounds__(256) k_point_keys(const double *__restrict__ xy, int n, const RootBox *__restrict__ root,
                                                     int levels, uint64_t *__restrict__ words) {
+  chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float rinv = __frcp_rn((float)root->region), span = (float)(1 << levels);
@@ -405,6 +413,7 @@ __global__ void __launch_bounds__(256) k_point_keys(const double *__restrict__ x
 
 __global__ void __launch_bounds__(256) k_cpl(const uint64_t *__restrict__ keys, int n, int num_p,
                                              uint8_t *__restrict__ cpl, uint8_t *__restrict__ w) {
+  chain_wait();
   long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i + 1 < n) cpl[i] = (uint8_t)common_levels(keys[i], keys[i + 1]);
   if (i + num_p - 1 < n) w[i] = (uint8_t)common_levels(keys[i], keys[i + num_p - 1]);
@@ -420,6 +429,7 @@ constexpr int kLLTile = 2048;
 __global__ void __launch_bounds__(256) k_leaf_level(const uint8_t *__restrict__ w, int n, int num_p,
                                                     uint8_t *__restrict__ leaf_level, DevStatus *st, int levels,
                                                     int lev0) {
+  chain_wait();
   extern __shared__ uint8_t sbuf[];
   const int H = num_p - 1;
   const long tile0 = (long)blockIdx.x * kLLTile;
@@ -486,6 +496,7 @@ __device__ __forceinline__ void cell_counts(const uint8_t *cpl, const uint8_t *l
 // pack: cells in the high 32 bits, leaves in the low 32 bits
 __global__ void __launch_bounds__(kScanThreads) k_cells_reduce(const uint8_t *cpl, const uint8_t *leaf_level, int n,
                                                                unsigned long long *part) {
+  chain_wait();
   unsigned long long s = 0;
   long base = (long)blockIdx.x * kScanTile;
   for (int k = threadIdx.x; k < kScanTile; k += kScanThreads) {
@@ -506,6 +517,7 @@ __global__ void __launch_bounds__(kScanThreads) k_cells_reduce(const uint8_t *cp
 
 // exclusive scan of the tile partials (one block); total -> *total
 __global__ void __launch_bounds__(1024) k_scan_part(unsigned long long *part, int len, unsigned long long *total) {
+  chain_wait();
   __shared__ unsigned long long s[1024];
   const int t = threadIdx.x;
   const int per = (len + 1023) / 1024;
@@ -602,6 +614,7 @@ __device__ __forceinline__ void cell_geometry(const EmitArgs &a, uint64_t key, i
 }
 
 __global__ void __launch_bounds__(kScanThreads) k_emit_cells(EmitArgs a) {
+  chain_wait();
   const long base = (long)blockIdx.x * kScanTile + (long)threadIdx.x * kScanItems;
   unsigned c[kScanItems], l[kScanItems];
   unsigned long long mine = 0;
@@ -665,6 +678,7 @@ __global__ void __launch_bounds__(kScanThreads) k_emit_cells(EmitArgs a) {
 __global__ void __launch_bounds__(256) k_cell_end(const uint64_t *__restrict__ keys, int n, int ncell,
                                                   const int *__restrict__ level, const int *__restrict__ begin,
                                                   int *__restrict__ end) {
+  chain_wait();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncell) return;
   if (c == 0) {
@@ -693,6 +707,7 @@ __global__ void __launch_bounds__(256) k_children(const uint64_t *__restrict__ k
                                                   const int *__restrict__ level, const int *__restrict__ begin,
                                                   const int *__restrict__ end, const unsigned char *__restrict__ leaf,
                                                   int *__restrict__ child) {
+  chain_wait();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncell) return;
   int4 ch = make_int4(-1, -1, -1, -1);
@@ -762,6 +777,7 @@ __device__ __forceinline__ void leaf_sort(const uint32_t *__restrict__ vals, int
 __global__ void __launch_bounds__(256) k_leaf_order(const uint32_t *__restrict__ vals, int nleaf,
                                                     const int *__restrict__ leaf_cell, const int *__restrict__ begin,
                                                     const int *__restrict__ end, int *__restrict__ perm) {
+  chain_wait();
   int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   int lane = threadIdx.x & 31;
   if (wid >= nleaf) return;
@@ -790,6 +806,7 @@ __global__ void __launch_bounds__(256) k_gather(const double *__restrict__ xy, c
                                                 const double *__restrict__ cor, const int *__restrict__ perm, int n,
                                                 double *x, double *y, double *c, double *r, double *icor2,
                                                 DevStatus *st) {
+  chain_wait();
   long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   int p = perm[i];
@@ -912,20 +929,20 @@ retry:
 
   // 1. root box (per set)
   if (batched) {
-    k_bbox_sets<<<dim3((unsigned)nsets, kSetSlices), 256, 0, s>>>(d_xy, d_set_off, set_part, set_of, ws.status);
-    k_roots_sets<<<(nsets + 127) / 128, 128, 0, s>>>(set_part, nsets, t.root);
+    chained(k_bbox_sets, dim3((unsigned)nsets, kSetSlices), 256, 0, s)(d_xy, d_set_off, set_part, set_of, ws.status);
+    chained(k_roots_sets, (nsets + 127) / 128, 128, 0, s)(set_part, nsets, t.root);
     ::t2d::g_launches.fetch_add(2, std::memory_order_relaxed);
   } else {
-    k_bbox<<<box_blocks(n), 256, 0, s>>>(d_xy, n, bpart, ws.status);
-    k_root<<<1, kRootThreads, 0, s>>>(bpart, box_blocks(n), t.root);
+    chained(k_bbox, box_blocks(n), 256, 0, s)(d_xy, n, bpart, ws.status);
+    chained(k_root, 1, kRootThreads, 0, s)(bpart, box_blocks(n), t.root);
     ::t2d::g_launches.fetch_add(2, std::memory_order_relaxed);
   }
   // 2. keys
   const int total_levels = levels + lev0;
   if (batched && tlev <= kSetTableLevels)
-    k_centre_table_sets<<<2 * (unsigned)t.nsets, 256, 0, s>>>(t.root, ctab, tlev);
+    chained(k_centre_table_sets, 2 * (unsigned)t.nsets, 256, 0, s)(t.root, ctab, tlev);
   else
-    k_centre_table<<<dim3((unsigned)((2 * centre_entries(tlev) + 255) / 256), (unsigned)t.nsets), 256, 0, s>>>(
+    chained(k_centre_table, dim3((unsigned)((2 * centre_entries(tlev) + 255) / 256), (unsigned)t.nsets), 256, 0, s)(
         t.root, ctab, tlev);
   // Up to 16 digits the key and the blob index share one word: the sort
   // then moves 8 bytes per blob and pass instead of 12, and its last pass
@@ -934,7 +951,7 @@ retry:
   const bool packed = 2 * total_levels <= 32 && n >= 2;
   const int passes = (2 * total_levels + 7) / 8;
   uint64_t *words = packed && (passes & 1) ? keys_alt : t.keys;
-  k_keys<<<(n + 255) / 256, 256, 0, s>>>(d_xy, n, t.root, ctab, tlev, words, vals, levels, set_of, lev0,
+  chained(k_keys, (n + 255) / 256, 256, 0, s)(d_xy, n, t.root, ctab, tlev, words, vals, levels, set_of, lev0,
                                          packed ? 1 : 0);
   ::t2d::g_launches.fetch_add(2, std::memory_order_relaxed);
   // 3. sort
@@ -946,20 +963,20 @@ retry:
     T2D_CUDA_TRY(radix_sort_pairs(t.keys, vals, keys_alt, vals_alt, n, 64 - 2 * total_levels, 64, sort_tmp, s));
   t.key_order = vals;
   // 4-5. leaf levels
-  k_cpl<<<(n + 255) / 256, 256, 0, s>>>(t.keys, n, p.num_p, cpl, w);
+  chained(k_cpl, (n + 255) / 256, 256, 0, s)(t.keys, n, p.num_p, cpl, w);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   {
     const int H = p.num_p - 1;
     size_t smem = 2 * (size_t)(kLLTile + H);
     if (smem > 48 * 1024) T2D_CUDA_TRY(cudaFuncSetAttribute(k_leaf_level, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_leaf_level<<<(n + kLLTile - 1) / kLLTile, 256, smem, s>>>(w, n, p.num_p, leaf_level, ws.status, total_levels,
+    chained(k_leaf_level, (n + kLLTile - 1) / kLLTile, 256, smem, s)(w, n, p.num_p, leaf_level, ws.status, total_levels,
                                                                 lev0);
     ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   }
   // 6. counts and scan
-  k_cells_reduce<<<ntiles, kScanThreads, 0, s>>>(cpl, leaf_level, n, part);
+  chained(k_cells_reduce, ntiles, kScanThreads, 0, s)(cpl, leaf_level, n, part);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_scan_part<<<1, 1024, 0, s>>>(part, ntiles, total);
+  chained(k_scan_part, 1, 1024, 0, s)(part, ntiles, total);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   T2D_CUDA_TRY(cudaMemcpyAsync(ws.h_status, ws.status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
@@ -1004,21 +1021,21 @@ retry:
   // 7. cells
   EmitArgs ea{t.keys, cpl, leaf_level, part, t.root, n, cellbase, t.level, t.begin, t.leaf, t.cx, t.cy, t.region,
               t.leaf_cell, ctab, tlev, lev0};
-  k_emit_cells<<<ntiles, kScanThreads, 0, s>>>(ea);
+  chained(k_emit_cells, ntiles, kScanThreads, 0, s)(ea);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_cell_end<<<(t.ncell + 255) / 256, 256, 0, s>>>(t.keys, n, t.ncell, t.level, t.begin, t.end);
+  chained(k_cell_end, (t.ncell + 255) / 256, 256, 0, s)(t.keys, n, t.ncell, t.level, t.begin, t.end);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
-  k_children<<<(t.ncell + 255) / 256, 256, 0, s>>>(t.keys, cpl, cellbase, t.ncell, t.level, t.begin, t.end, t.leaf,
+  chained(k_children, (t.ncell + 255) / 256, 256, 0, s)(t.keys, cpl, cellbase, t.ncell, t.level, t.begin, t.end, t.leaf,
                                                     t.child);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   // 8. in-leaf order, 9. gather
   if (t.nleaf > 0) {
-    k_leaf_order<<<(int)(((long)t.nleaf * 32 + 255) / 256), 256, 0, s>>>(vals, t.nleaf, t.leaf_cell, t.begin, t.end,
-                                                                          t.perm);
+    chained(k_leaf_order, (int)(((long)t.nleaf * 32 + 255) / 256), 256, 0, s)(
+        vals, t.nleaf, t.leaf_cell, t.begin, t.end,                                                                  t.perm);
     ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   }
   if (cir_cor_ready) T2D_CUDA_TRY(cudaStreamWaitEvent(s, cir_cor_ready, 0));
-  k_gather<<<(n + 255) / 256, 256, 0, s>>>(d_xy, d_cir, d_cor, t.perm, n, t.x, t.y, t.cir, t.cor, t.icor2,
+  chained(k_gather, (n + 255) / 256, 256, 0, s)(d_xy, d_cir, d_cor, t.perm, n, t.x, t.y, t.cir, t.cor, t.icor2,
                                            ws.status);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
@@ -1037,7 +1054,7 @@ int sort_targets(Workspace &ws, int n, const double *d_xy, const RootBox *d_root
   int levels = 4;
   while (levels < 16 && (1l << (2 * levels)) < 4l * n) levels++;
   const bool odd = ((2 * levels + 7) / 8) & 1;
-  k_point_keys<<<(n + 255) / 256, 256, 0, s>>>(d_xy, n, d_root, levels, a);
+  chained(k_point_keys, (n + 255) / 256, 256, 0, s)(d_xy, n, d_root, levels, a);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   if (n < 2) {
     T2D_CUDA_TRY(cudaMemsetAsync(d_order, 0, sizeof(int), s));
@@ -1055,6 +1072,7 @@ namespace t2d {
 namespace {
 __global__ void k_gather_targets(const double *__restrict__ xy, const int *__restrict__ order, int n,
                                  double *__restrict__ tx, double *__restrict__ ty, int *__restrict__ out_idx) {
+  chain_wait();
   long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   int o = order ? order[i] : (int)i;
@@ -1067,7 +1085,7 @@ __global__ void k_gather_targets(const double *__restrict__ xy, const int *__res
 int gather_targets(int n, const double *d_xy, const int *d_order, double *tx, double *ty, int *out_idx,
                    cudaStream_t s) {
   if (n <= 0) return TREE2D_OK;
-  k_gather_targets<<<(n + 255) / 256, 256, 0, s>>>(d_xy, d_order, n, tx, ty, out_idx);
+  chained(k_gather_targets, (n + 255) / 256, 256, 0, s)(d_xy, d_order, n, tx, ty, out_idx);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;

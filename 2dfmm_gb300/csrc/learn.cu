@@ -30,6 +30,7 @@ namespace t2d {
 namespace {
 
 __global__ void k_leaf_stats(MixedView m, LeafStats *out) {
+  chain_wait();
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= m.nleaf) return;
   const int c = m.leaf_cell[w];
@@ -70,6 +71,7 @@ __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
 // [3*i+1] = kind (0 U, 1 K), [3*i+2] = entry index in that list.
 __global__ void k_labels(MixedView m, const LeafStats *st, const float *u_ref_ptr, double tol, int ns,
                          const int *samples, float *features, int *labels) {
+  chain_wait();
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= ns) return;
   const int l = samples[3 * w], kind = samples[3 * w + 1], e = samples[3 * w + 2];
@@ -302,6 +304,7 @@ __device__ __forceinline__ void load_weights(const float *theta, float (*W)[S]) 
 // the order of a plain loop, so the values do not depend on the tiling.
 __global__ void __launch_bounds__(256) k_rows(Rows rows, const float *__restrict__ theta, Pass p, float *logits,
                                               float *loss) {
+  chain_wait();
   extern __shared__ float4 shared_rows[];
   RowsShared &s = *reinterpret_cast<RowsShared *>(shared_rows);
   const int i0 = blockIdx.x * kRowsPerBlock, left = min(kRowsPerBlock, rows.bt - i0);
@@ -398,6 +401,7 @@ __device__ __forceinline__ void adam(const Adam &a, int i, float g) {
 }
 
 __global__ void __launch_bounds__(128) k_weights(int bt, Pass p, float *grad, Adam a) {
+  chain_wait();
   __shared__ __align__(16) float cols[kStages][kStage][32];  // [buffer][row][16 columns of D, 16 of A, or 32 of D]
   const bool copier = threadIdx.x >= 64;
   const int t = threadIdx.x & 63;
@@ -490,7 +494,7 @@ __global__ void __launch_bounds__(128) k_weights(int bt, Pass p, float *grad, Ad
 }
 
 cudaError_t run_weights(int bt, const Pass &p, float *grad, const Adam &a, cudaStream_t s) {
-  k_weights<<<kWeightBlocks, 128, 0, s>>>(bt, p, grad, a);
+  chained(k_weights, kWeightBlocks, 128, 0, s)(bt, p, grad, a);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return cudaGetLastError();
 }
@@ -508,7 +512,7 @@ cudaError_t run_rows(const Rows &rows, const float *theta, const Pass &p, float 
   const int bytes = (int)sizeof(RowsShared);
   cudaError_t e = cudaFuncSetAttribute(k_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) return e;
-  k_rows<<<(rows.bt + kRowsPerBlock - 1) / kRowsPerBlock, 256, bytes, s>>>(rows, theta, p, logits, loss);
+  chained(k_rows, (rows.bt + kRowsPerBlock - 1) / kRowsPerBlock, 256, bytes, s)(rows, theta, p, logits, loss);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return cudaGetLastError();
 }
@@ -517,6 +521,7 @@ cudaError_t run_rows(const Rows &rows, const float *theta, const Pass &p, float 
 
 // u_ref = sum |G| / R0 (deterministic: fixed per-thread ranges, tree sum).
 __global__ void __launch_bounds__(1024) k_uref(MixedView m, const LeafStats *st, const RootBox *root, float *out) {
+  chain_wait();
   __shared__ float part[1024];
   const int t = threadIdx.x;
   const int per = (m.nleaf + 1023) / 1024;
@@ -534,6 +539,7 @@ __global__ void __launch_bounds__(1024) k_uref(MixedView m, const LeafStats *st,
 // The leaves of each set of a batched tree: one contiguous range of the
 // leaf order (a set's cells are the subtree of its root), [lo[k], hi[k]).
 __global__ void k_set_leaf_ranges(MixedView m, int *lo, int *hi) {
+  chain_wait();
   const int l = blockIdx.x * blockDim.x + threadIdx.x;
   if (l >= m.nleaf) return;
   const int k = set_of_cell(m, m.leaf_cell[l]);
@@ -546,6 +552,7 @@ __global__ void k_set_leaf_ranges(MixedView m, int *lo, int *hi) {
 // a set's u_ref is the one it gets alone, bit for bit.
 __global__ void __launch_bounds__(1024) k_uref_sets(MixedView m, const LeafStats *st, const RootBox *root,
                                                     const int *lo, const int *hi, float *out) {
+  chain_wait();
   __shared__ float part[1024];
   const int k = blockIdx.x, t = threadIdx.x;
   const int l0 = lo[k], cnt = max(hi[k] - l0, 0);
@@ -566,22 +573,22 @@ int learned_uref_sets(MixedView &m, const LeafStats *stats, const RootBox *roots
   if (nsets <= 0) return TREE2D_OK;
   T2D_CUDA_TRY(cudaMemsetAsync(leaf_lo, 0, sizeof(int) * (size_t)nsets, s));
   T2D_CUDA_TRY(cudaMemsetAsync(leaf_hi, 0, sizeof(int) * (size_t)nsets, s));
-  if (m.nleaf > 0) k_set_leaf_ranges<<<(m.nleaf + 255) / 256, 256, 0, s>>>(m, leaf_lo, leaf_hi);
-  k_uref_sets<<<nsets, 1024, 0, s>>>(m, stats, roots, leaf_lo, leaf_hi, out);
+  if (m.nleaf > 0) chained(k_set_leaf_ranges, (m.nleaf + 255) / 256, 256, 0, s)(m, leaf_lo, leaf_hi);
+  chained(k_uref_sets, nsets, 1024, 0, s)(m, stats, roots, leaf_lo, leaf_hi, out);
   g_launches.fetch_add(2, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;
 }
 
 int learned_uref(MixedView &m, const LeafStats *stats, const RootBox *root, float *out, cudaStream_t s) {
-  k_uref<<<1, 1024, 0, s>>>(m, stats, root, out);
+  chained(k_uref, 1, 1024, 0, s)(m, stats, root, out);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;
 }
 
 int learned_leaf_stats(MixedView &m, LeafStats *stats, cudaStream_t s) {
-  k_leaf_stats<<<(int)(((long)m.nleaf * 32 + 255) / 256), 256, 0, s>>>(m, stats);
+  chained(k_leaf_stats, (int)(((long)m.nleaf * 32 + 255) / 256), 256, 0, s)(m, stats);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;
@@ -590,7 +597,7 @@ int learned_leaf_stats(MixedView &m, LeafStats *stats, cudaStream_t s) {
 int learned_labels(MixedView &m, const LeafStats *stats, const float *u_ref_ptr, double tol, int ns,
                    const int *samples, float *features, int *labels, cudaStream_t s) {
   if (ns <= 0) return TREE2D_OK;
-  k_labels<<<(int)(((long)ns * 32 + 255) / 256), 256, 0, s>>>(m, stats, u_ref_ptr, tol, ns, samples, features,
+  chained(k_labels, (int)(((long)ns * 32 + 255) / 256), 256, 0, s)(m, stats, u_ref_ptr, tol, ns, samples, features,
                                                                labels);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());

@@ -88,6 +88,7 @@ __device__ __forceinline__ void store_row(unsigned char *tile, int r, const floa
 }
 
 __global__ void __launch_bounds__(kTile) k_mlp_infer(InferArgs a) {
+  chain_wait();
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint64_t bar_w, bar_mma;
   __shared__ uint32_t s_tmem;
@@ -291,7 +292,7 @@ static int launch_infer(InferArgs &a, long total, cudaStream_t s) {
   // and 16 tiles measured 11.15, 11.05 and 11.05 ms against 11.02 ms)
   const long grid = (ntiles + kTilesPerCta - 1) / kTilesPerCta;
   a.wait_limit = 1l << 22;
-  k_mlp_infer<<<(unsigned)grid, kTile, smem, s>>>(a);
+  chained(k_mlp_infer, (unsigned)grid, kTile, smem, s)(a);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;

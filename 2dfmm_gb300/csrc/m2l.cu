@@ -35,6 +35,7 @@ namespace {
 
 // One warp per cell, lane l owns b_l.  The reference form for checking.
 __global__ void __launch_bounds__(256) k_m2l_cc(MixedView m, const float2 *__restrict__ T) {
+  chain_wait();
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (c >= m.ncell) return;
   if (m.level[c] - m.lev0 < 2) return;
@@ -89,6 +90,7 @@ constexpr int kMaxKc4 = 2 * kMaxP / 4;  // float4s in one multipole row (2P floa
 // operator images are in flight by bulk copy, so the gather latency is
 // paid once per tile rather than once per slot.
 __global__ void __launch_bounds__(kThreadsTC) k_m2l_tc(TcArgs a) {
+  chain_wait();
   extern __shared__ __align__(1024) unsigned char smem[];
   __shared__ uint64_t bar_mma[2], bar_b[3];
   __shared__ uint32_t s_tmem;
@@ -338,6 +340,7 @@ __global__ void __launch_bounds__(kThreadsTC) k_m2l_tc(TcArgs a) {
 // One atomic per warp and class (the lanes of a class take consecutive
 // positions in ballot order).
 __global__ void k_class_lists(MixedView m, int *list, int *count) {
+  chain_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const bool in = c < m.ncell && m.level[c] - m.lev0 >= 2;
@@ -363,7 +366,7 @@ uint32_t tf32_round_host(float x) {
 }  // namespace
 
 int m2l_cuda_cores(MixedView &m, const float *tables, cudaStream_t s) {
-  k_m2l_cc<<<(int)(((long)m.ncell * 32 + 255) / 256), 256, 0, s>>>(m, reinterpret_cast<const float2 *>(tables));
+  chained(k_m2l_cc, (int)(((long)m.ncell * 32 + 255) / 256), 256, 0, s)(m, reinterpret_cast<const float2 *>(tables));
   g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;
@@ -407,7 +410,7 @@ int m2l_tensor_cores(MixedView &m, const float *bimg, int *cls_list, int *cls_co
   const int P = m.P, Kc = 2 * P, Npad = m2l_npad(P);
   if (Kc % 8 != 0) return TREE2D_ERR_BAD_PARAMS;  // K of one MMA is 8 TF32 elements
   T2D_CUDA_TRY(cudaMemsetAsync(cls_count, 0, 4 * sizeof(int), s));
-  k_class_lists<<<(m.ncell + 255) / 256, 256, 0, s>>>(m, cls_list, cls_count);
+  chained(k_class_lists, (m.ncell + 255) / 256, 256, 0, s)(m, cls_list, cls_count);
   TcArgs a;
   a.m = m;
   a.cls_list = cls_list;
@@ -426,7 +429,7 @@ int m2l_tensor_cores(MixedView &m, const float *bimg, int *cls_list, int *cls_co
   const size_t smem = fixed + (size_t)a.nbs * bst;
   T2D_CUDA_TRY(cudaFuncSetAttribute(k_m2l_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((m.ncell + rows - 1) / rows, 4);
-  k_m2l_tc<<<grid, kThreadsTC, smem, s>>>(a);
+  chained(k_m2l_tc, grid, kThreadsTC, smem, s)(a);
   g_launches.fetch_add(2, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;

@@ -120,6 +120,7 @@ __device__ __forceinline__ bool adj_cells(const MixedView &m, int a, int b) {
 // ------------------------------------------------------------ cell setup
 
 __global__ void k_cell_info(MixedView m) {
+  chain_wait();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.ncell) return;
   int lev = m.level[c];
@@ -169,6 +170,7 @@ __device__ __forceinline__ unsigned spread3(unsigned v) {  // 3 bits -> even bit
 __global__ void __launch_bounds__(32 * kSetupWarps, 8) k_leaf_setup(MixedView m, const double *x, const double *y,
                                                                  const double *cir, const double *cor,
                                                                  const int *perm) {
+  chain_wait();
   __shared__ int s_cnt[kSetupWarps][kSubCells];
   __shared__ float2 s_lc[kSetupWarps][kSetupStage];   // offsets, in tree order
   __shared__ float2 s_out[kSetupWarps][kSetupStage];  // offsets, in the new order
@@ -297,6 +299,7 @@ __global__ void __launch_bounds__(32 * kSetupWarps, 8) k_leaf_setup(MixedView m,
 
 // Same-level 3x3 neighbourhood of every cell: exact cells and coarser leaves.
 __global__ void k_colleagues(MixedView m) {
+  chain_wait();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.ncell) return;
   const int lev = m.level[c];
@@ -333,6 +336,7 @@ __constant__ signed char c_slot[4][6][6];  // [class][dy+2+qy][dx+2+qx] -> slot 
 //      coarser leaf seen at several positions is kept once), in position
 //      order.
 __global__ void __launch_bounds__(256) k_vx_lists(MixedView m) {
+  chain_wait();
   // the slot table in shared memory: the lanes index it divergently, which
   // constant memory would serialise
   __shared__ signed char slot[4][6][6];
@@ -427,6 +431,7 @@ __device__ __forceinline__ unsigned warp_max_as_float_bits(unsigned long long mx
   return __float_as_uint((float)__longlong_as_double((long long)mx));
 }
 __global__ void k_sigma_max(const double *cor, int n, unsigned *out) {
+  chain_wait();
   unsigned long long mx = 0;
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const unsigned long long u = abs_bits(cor[i]);
@@ -437,6 +442,7 @@ __global__ void k_sigma_max(const double *cor, int n, unsigned *out) {
 }
 
 __global__ void k_cutoff(unsigned *bits, float cutoff, int count) {
+  chain_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   float s = __uint_as_float(bits[i]);
@@ -448,6 +454,7 @@ __global__ void k_cutoff(unsigned *bits, float cutoff, int count) {
 // `slice` of the set's input range.
 constexpr int kSigmaSlices = 16;
 __global__ void k_sigma_max_sets(const double *cor, const int *off, unsigned *out) {
+  chain_wait();
   const int set = blockIdx.x;
   const int n0 = off[set], len = off[set + 1] - n0;
   const int per = (len + kSigmaSlices - 1) / kSigmaSlices;
@@ -466,6 +473,7 @@ __global__ void k_sigma_max_sets(const double *cor, const int *off, unsigned *ou
 // the count of level l-1 first, then the exclusive offsets, and
 // level_off[kKeyLevels + 2 + l] is the fill cursor of level l.
 __global__ void k_level_hist(MixedView m) {
+  chain_wait();
   __shared__ int h[kKeyLevels + 1];
   for (int i = threadIdx.x; i <= kKeyLevels; i += blockDim.x) h[i] = 0;
   __syncthreads();
@@ -477,6 +485,7 @@ __global__ void k_level_hist(MixedView m) {
 }
 
 __global__ void k_level_scan(MixedView m) {
+  chain_wait();
   if (threadIdx.x != 0) return;
   int run = 0;
   for (int l = 0; l <= kKeyLevels; l++) {
@@ -488,6 +497,7 @@ __global__ void k_level_scan(MixedView m) {
 
 // One atomic per warp and level: lanes of equal level share a reservation.
 __global__ void k_level_fill(MixedView m) {
+  chain_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const int lane = threadIdx.x & 31;
   const int lev = c < m.ncell ? m.level[c] : -1;
@@ -500,6 +510,7 @@ __global__ void k_level_fill(MixedView m) {
 }
 
 __global__ void k_parent(MixedView m) {
+  chain_wait();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= m.ncell) return;
   if (m.leaf[c]) return;
@@ -546,6 +557,7 @@ constexpr unsigned kTagK = 0x80000000u;
 // turns into the same lists without a second walk.
 template <int kMode>
 __global__ void __launch_bounds__(32 * kWalkWarps) k_lists(MixedView m) {
+  chain_wait();
   constexpr bool kFill = kMode == 1;
   __shared__ unsigned s_stack[kWalkWarps][kWalkStack];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -683,6 +695,7 @@ __global__ void __launch_bounds__(32 * kWalkWarps) k_lists(MixedView m) {
 // emission order and writes each kind at its scanned offsets, in the order
 // the filling walk would (lane order within an emission).
 __global__ void __launch_bounds__(256) k_lists_compact(MixedView m) {
+  chain_wait();
   const int l = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (l >= m.nleaf) return;
   const unsigned lt = (1u << lane) - 1u;
@@ -740,6 +753,7 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int *sh, int &total) 
 
 __global__ void __launch_bounds__(kScan3Threads) k_scan3_tiles(const int *a, const int *b, const int *c, int len,
                                                                int *tile_sums, int ntiles) {
+  chain_wait();
   __shared__ int sh[32];
   const int *arr[3] = {a, b, c};
   for (int k = 0; k < 3; k++) {
@@ -757,6 +771,7 @@ __global__ void __launch_bounds__(kScan3Threads) k_scan3_tiles(const int *a, con
 // positions are ints, so a total beyond INT_MAX is reported as -1 (the host
 // then stops before any list is filled).
 __global__ void k_scan3_sums(int *tile_sums, int ntiles) {
+  chain_wait();
   const int k = threadIdx.x;
   if (k >= 3) return;
   int *t = tile_sums + k * (ntiles + 1);
@@ -771,6 +786,7 @@ __global__ void k_scan3_sums(int *tile_sums, int ntiles) {
 
 __global__ void __launch_bounds__(kScan3Threads) k_scan3_apply(int *a, int *b, int *c, int len, const int *tile_sums,
                                                                int ntiles) {
+  chain_wait();
   __shared__ int sh[32];
   int *arr[3] = {a, b, c};
   for (int k = 0; k < 3; k++) {
@@ -834,6 +850,7 @@ __device__ __forceinline__ float warp_chunk_sum(const float (&acc)[2 * kCoefChun
 
 // S2M: one warp per leaf, a_k = sum_j G_j ((z_j - c)/h)^k.
 __global__ void __launch_bounds__(256) k_s2m_f32(MixedView m) {
+  chain_wait();
   __shared__ float sh[8][32 * kCoefPitch];
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (wid >= m.nleaf) return;
@@ -881,6 +898,7 @@ __device__ __forceinline__ void stage_translation(const float2 *__restrict__ tab
 // sums are independent chains, ((q0 + q1) + (q2 + q3)) at the end.
 template <int kG>
 __global__ void __launch_bounds__(256) k_m2m_f32(MixedView m, int lev) {
+  chain_wait();
   extern __shared__ float2 s_tab[];  // [4][P][P]: [q][n][k]
   const int P = m.P;
   stage_translation(m.m2m, P, s_tab);
@@ -931,6 +949,7 @@ __global__ void __launch_bounds__(256) k_m2m_f32(MixedView m, int lev) {
 // z the blob's offset from c's centre in units of c's side.  One warp per
 // cell, lanes over blobs, chunked coefficients as S2M.
 __global__ void __launch_bounds__(256) k_p2l(MixedView m) {
+  chain_wait();
   __shared__ float sh[8][32 * kCoefPitch];
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (c >= m.ncell) return;
@@ -1105,6 +1124,7 @@ __device__ __forceinline__ void l2l_quad_level(const MixedView &m, const float2 
 
 template <int kP>
 __global__ void __launch_bounds__(kQuadThreads) k_m2m_quad(MixedView m, int lev) {
+  chain_wait();
   __shared__ float2 s_tab[4 * (kP * kP + 1)];  // [q][n][k], padded per q
   stage_translation_padded<kP>(m.m2m, s_tab);
   m2m_quad_level<kP, false>(m, s_tab, lev, (blockIdx.x * blockDim.x + threadIdx.x) >> 2,
@@ -1113,6 +1133,7 @@ __global__ void __launch_bounds__(kQuadThreads) k_m2m_quad(MixedView m, int lev)
 
 template <int kP>
 __global__ void __launch_bounds__(kQuadThreads) k_l2l_quad(MixedView m, int lev) {
+  chain_wait();
   __shared__ float2 s_tab[4 * (kP * kP + 1)];  // [q][k][l], padded per q
   stage_translation_padded<kP>(m.l2l, s_tab);
   l2l_quad_level<kP, false>(m, s_tab, lev, (blockIdx.x * blockDim.x + threadIdx.x) >> 2,
@@ -1156,6 +1177,7 @@ __device__ bool grid_barrier(DevStatus *st, unsigned nblocks, long limit, bool &
 // meet at the grid barrier before the next level reads what this one wrote.
 template <int kP, bool kUp>
 __global__ void __launch_bounds__(kQuadThreads) k_chain_quad(MixedView m, int lev_first, int lev_last, long limit) {
+  chain_wait();
   __shared__ float2 s_tab[4 * (kP * kP + 1)];
   stage_translation_padded<kP>(kUp ? m.m2m : m.l2l, s_tab);
   const int i0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, stride = (gridDim.x * blockDim.x) >> 2;
@@ -1176,6 +1198,7 @@ __global__ void __launch_bounds__(kQuadThreads) k_chain_quad(MixedView m, int le
 // each half-warp translates two of the four children, lane = coefficient.
 template <int kG>
 __global__ void __launch_bounds__(256) k_l2l_f32(MixedView m, int lev) {
+  chain_wait();
   extern __shared__ float2 s_tab[];  // [4][P][P]: [q][k][l]
   const int P = m.P;
   stage_translation(m.l2l, P, s_tab);
@@ -1609,6 +1632,7 @@ __device__ __forceinline__ unsigned mask_blobs(unsigned mask, int cnt) {
 // one stable radix pass orders the keys (ties by leaf ordinal).  The order
 // changes only which warp evaluates a leaf, never a result.
 __global__ void k_leaf_cost(MixedView m, uint64_t *keys, uint32_t *vals) {
+  chain_wait();
   const int l = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (l >= m.nleaf) return;
   const int B = m.leaf_cell[l];
@@ -1972,6 +1996,7 @@ __device__ __forceinline__ void near_chunk(const MixedView &m, const Decisions &
 template <bool kLearned, bool kStaged, int kWarps, bool kWide, bool kScaled>
 __global__ void __launch_bounds__(32 * kWarps, (kWide ? 24 : 32) / kWarps) k_eval_near(MixedView m, double *uv, const int *perm,
                                                                          Decisions dec, long wait_limit) {
+  chain_wait();
   extern __shared__ __align__(128) float4 s_src[];  // kStaged: [kWarps][2 * kStage]
   __shared__ __align__(8) uint64_t s_bar[kWarps][2];
   __shared__ float s_tb[kWarps][9];
@@ -2101,6 +2126,7 @@ __device__ __forceinline__ bool far_from(const MixedView &m, int c, double x, do
 
 __global__ void __launch_bounds__(kPtWarps * 32) k_eval_points(MixedView m, int ntgt, const double *tx,
                                                                const double *ty, const int *out_idx, double *uv) {
+  chain_wait();
   __shared__ int s_cell[kPtWarps][kPtStack];
   __shared__ unsigned s_mask[kPtWarps][kPtStack];
   __shared__ int s_queue[kPtWarps][kPtTargets][kPtQueue];
@@ -2377,23 +2403,23 @@ cudaError_t mixed_tables(int P, float *h_m2l, float *h_m2m, float *h_l2l) {
 
 int mixed_lists(MixedView &m, cudaStream_t s) {
   const int cb = (m.ncell + 255) / 256;
-  k_cell_info<<<cb, 256, 0, s>>>(m);
+  chained(k_cell_info, cb, 256, 0, s)(m);
   T2D_CUDA_TRY(cudaMemsetAsync(m.level_off, 0, sizeof(int) * (2 * kKeyLevels + 4), s));
-  k_level_hist<<<cb, 256, 0, s>>>(m);
-  k_level_scan<<<1, 32, 0, s>>>(m);
-  k_level_fill<<<cb, 256, 0, s>>>(m);
+  chained(k_level_hist, cb, 256, 0, s)(m);
+  chained(k_level_scan, 1, 32, 0, s)(m);
+  chained(k_level_fill, cb, 256, 0, s)(m);
   g_launches.fetch_add(3, std::memory_order_relaxed);
-  k_parent<<<cb, 256, 0, s>>>(m);
-  k_colleagues<<<cb, 256, 0, s>>>(m);
-  k_vx_lists<<<(int)(((long)m.ncell * 32 + 255) / 256), 256, 0, s>>>(m);
+  chained(k_parent, cb, 256, 0, s)(m);
+  chained(k_colleagues, cb, 256, 0, s)(m);
+  chained(k_vx_lists, (int)(((long)m.ncell * 32 + 255) / 256), 256, 0, s)(m);
   if (m.list_scratch)
-    k_lists<2><<<(m.nleaf + kWalkWarps - 1) / kWalkWarps, 32 * kWalkWarps, 0, s>>>(m);
+    chained(k_lists<2>, (m.nleaf + kWalkWarps - 1) / kWalkWarps, 32 * kWalkWarps, 0, s)(m);
   else
-    k_lists<0><<<(m.nleaf + kWalkWarps - 1) / kWalkWarps, 32 * kWalkWarps, 0, s>>>(m);
+    chained(k_lists<0>, (m.nleaf + kWalkWarps - 1) / kWalkWarps, 32 * kWalkWarps, 0, s)(m);
   const int ntiles = max(1, (m.nleaf + kScanTile3 - 1) / kScanTile3);
-  k_scan3_tiles<<<ntiles, kScan3Threads, 0, s>>>(m.u_off, m.w_off, m.k_off, m.nleaf, m.scan_tmp, ntiles);
-  k_scan3_sums<<<1, 32, 0, s>>>(m.scan_tmp, ntiles);
-  k_scan3_apply<<<ntiles, kScan3Threads, 0, s>>>(m.u_off, m.w_off, m.k_off, m.nleaf, m.scan_tmp, ntiles);
+  chained(k_scan3_tiles, ntiles, kScan3Threads, 0, s)(m.u_off, m.w_off, m.k_off, m.nleaf, m.scan_tmp, ntiles);
+  chained(k_scan3_sums, 1, 32, 0, s)(m.scan_tmp, ntiles);
+  chained(k_scan3_apply, ntiles, kScan3Threads, 0, s)(m.u_off, m.w_off, m.k_off, m.nleaf, m.scan_tmp, ntiles);
   g_launches.fetch_add(8, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;
@@ -2401,16 +2427,16 @@ int mixed_lists(MixedView &m, cudaStream_t s) {
 
 int mixed_fill_lists(MixedView &m, bool from_scratch, cudaStream_t s) {
   if (from_scratch)
-    k_lists_compact<<<(int)(((long)m.nleaf * 32 + 255) / 256), 256, 0, s>>>(m);
+    chained(k_lists_compact, (int)(((long)m.nleaf * 32 + 255) / 256), 256, 0, s)(m);
   else
-    k_lists<1><<<(m.nleaf + kWalkWarps - 1) / kWalkWarps, 32 * kWalkWarps, 0, s>>>(m);
+    chained(k_lists<1>, (m.nleaf + kWalkWarps - 1) / kWalkWarps, 32 * kWalkWarps, 0, s)(m);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;
 }
 
 int mixed_leaf_setup(MixedView &m, const Tree &t, cudaStream_t s) {
-  k_leaf_setup<<<(m.nleaf + kSetupWarps - 1) / kSetupWarps, 32 * kSetupWarps, 0, s>>>(m, t.x, t.y, t.cir, t.cor,
+  chained(k_leaf_setup, (m.nleaf + kSetupWarps - 1) / kSetupWarps, 32 * kSetupWarps, 0, s)(m, t.x, t.y, t.cir, t.cor,
                                                                                         t.perm);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
@@ -2472,7 +2498,7 @@ bool launch_chain(MixedView &m, int lev_first, int lev_last, cudaStream_t s) {
 }
 
 int mixed_upward(MixedView &m, int depth, const int *lev_off, cudaStream_t s, bool chain) {
-  k_s2m_f32<<<(int)(((long)m.nleaf * 32 + 255) / 256), 256, 0, s>>>(m);
+  chained(k_s2m_f32, (int)(((long)m.nleaf * 32 + 255) / 256), 256, 0, s)(m);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   const size_t tab_bytes = 4 * sizeof(float2) * m.P * m.P;
   if (chain && m.P == 16 && depth - 1 > 2 + m.lev0 && launch_chain<true>(m, depth - 1, 2 + m.lev0, s)) {
@@ -2481,11 +2507,11 @@ int mixed_upward(MixedView &m, int depth, const int *lev_off, cudaStream_t s, bo
   }
   for (int lev = depth - 1; lev >= 2 + m.lev0; lev--) {
     if (m.P == 16)
-      k_m2m_quad<16><<<quad_blocks(lev_off, lev), kQuadThreads, 0, s>>>(m, lev);
+      chained(k_m2m_quad<16>, quad_blocks(lev_off, lev), kQuadThreads, 0, s)(m, lev);
     else if (m.P < 16)
-      k_m2m_f32<16><<<level_blocks(lev_off, lev), 256, tab_bytes, s>>>(m, lev);
+      chained(k_m2m_f32<16>, level_blocks(lev_off, lev), 256, tab_bytes, s)(m, lev);
     else
-      k_m2m_f32<32><<<level_blocks(lev_off, lev), 256, tab_bytes, s>>>(m, lev);
+      chained(k_m2m_f32<32>, level_blocks(lev_off, lev), 256, tab_bytes, s)(m, lev);
     g_launches.fetch_add(1, std::memory_order_relaxed);
   }
   T2D_CUDA_TRY(cudaGetLastError());
@@ -2493,7 +2519,7 @@ int mixed_upward(MixedView &m, int depth, const int *lev_off, cudaStream_t s, bo
 }
 
 int mixed_downward(MixedView &m, int depth, const int *lev_off, cudaStream_t s, bool chain) {
-  k_p2l<<<(int)(((long)m.ncell * 32 + 255) / 256), 256, 0, s>>>(m);
+  chained(k_p2l, (int)(((long)m.ncell * 32 + 255) / 256), 256, 0, s)(m);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   const size_t tab_bytes = 4 * sizeof(float2) * m.P * m.P;
   if (chain && m.P == 16 && depth > 3 + m.lev0 && launch_chain<false>(m, 3 + m.lev0, depth, s)) {
@@ -2502,11 +2528,11 @@ int mixed_downward(MixedView &m, int depth, const int *lev_off, cudaStream_t s, 
   }
   for (int lev = 3 + m.lev0; lev <= depth; lev++) {
     if (m.P == 16)
-      k_l2l_quad<16><<<quad_blocks(lev_off, lev - 1), kQuadThreads, 0, s>>>(m, lev);
+      chained(k_l2l_quad<16>, quad_blocks(lev_off, lev - 1), kQuadThreads, 0, s)(m, lev);
     else if (m.P < 16)
-      k_l2l_f32<16><<<level_blocks(lev_off, lev - 1), 256, tab_bytes, s>>>(m, lev);
+      chained(k_l2l_f32<16>, level_blocks(lev_off, lev - 1), 256, tab_bytes, s)(m, lev);
     else
-      k_l2l_f32<32><<<level_blocks(lev_off, lev - 1), 256, tab_bytes, s>>>(m, lev);
+      chained(k_l2l_f32<32>, level_blocks(lev_off, lev - 1), 256, tab_bytes, s)(m, lev);
     g_launches.fetch_add(1, std::memory_order_relaxed);
   }
   T2D_CUDA_TRY(cudaGetLastError());
@@ -2549,7 +2575,8 @@ cudaError_t launch_near(const MixedView &m, double *uv, const int *perm, Decisio
     const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  k<<<persistent_blocks(k, kWarps, smem, m.nleaf, resident), 32 * kWarps, smem, s>>>(m, uv, perm, d, kEvalWaitLimit);
+  chained(k, persistent_blocks(k, kWarps, smem, m.nleaf, resident), 32 * kWarps, smem, s)(m, uv, perm, d,
+                                                                                          kEvalWaitLimit);
   return cudaSuccess;
 }
 
@@ -2673,7 +2700,7 @@ int mixed_eval_points(Workspace &ws, int ntgt, const double *tx, const double *t
   if (ntgt <= 0) return TREE2D_OK;
   if (!ws.mxv) return TREE2D_ERR_NO_TREE;
   const int warps = (ntgt + kPtTargets - 1) / kPtTargets;
-  k_eval_points<<<(warps + kPtWarps - 1) / kPtWarps, kPtWarps * 32, 0, s>>>(*ws.mxv, ntgt, tx, ty, out_idx, uv);
+  chained(k_eval_points, (warps + kPtWarps - 1) / kPtWarps, kPtWarps * 32, 0, s)(*ws.mxv, ntgt, tx, ty, out_idx, uv);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;
@@ -2819,13 +2846,13 @@ int mixed_solve(Workspace &ws, const Tree &t, const MixedParams &mp, double *d_u
   m.st = ws.status;
   T2D_CUDA_TRY(cudaMemsetAsync(m.parent, 0xff, sizeof(int) * (size_t)nc, s));
   T2D_CUDA_TRY(cudaMemsetAsync(rc_bits, 0, 4, s));
-  k_sigma_max<<<304, 256, 0, s>>>(t.cor, n, rc_bits);
-  k_cutoff<<<1, 32, 0, s>>>(rc_bits, (float)mp.cutoff, 1);
+  chained(k_sigma_max, 304, 256, 0, s)(t.cor, n, rc_bits);
+  chained(k_cutoff, 1, 32, 0, s)(rc_bits, (float)mp.cutoff, 1);
   g_launches.fetch_add(2, std::memory_order_relaxed);
   if (rc_set_bits) {
     T2D_CUDA_TRY(cudaMemsetAsync(rc_set_bits, 0, 4 * (size_t)t.nsets, s));
-    k_sigma_max_sets<<<dim3((unsigned)t.nsets, kSigmaSlices), 256, 0, s>>>(t.set_cor, t.set_off, rc_set_bits);
-    k_cutoff<<<(t.nsets + 255) / 256, 256, 0, s>>>(rc_set_bits, (float)mp.cutoff, t.nsets);
+    chained(k_sigma_max_sets, dim3((unsigned)t.nsets, kSigmaSlices), 256, 0, s)(t.set_cor, t.set_off, rc_set_bits);
+    chained(k_cutoff, (t.nsets + 255) / 256, 256, 0, s)(rc_set_bits, (float)mp.cutoff, t.nsets);
     g_launches.fetch_add(2, std::memory_order_relaxed);
   }
 
@@ -2870,7 +2897,7 @@ int mixed_solve(Workspace &ws, const Tree &t, const MixedParams &mp, double *d_u
   if (nl > 1) m.leaf_order = reinterpret_cast<const int *>(ord_vals);
   auto schedule = [&](cudaStream_t q) -> cudaError_t {
     if (nl <= 1) return cudaSuccess;
-    k_leaf_cost<<<(int)(((long)nl * 32 + 255) / 256), 256, 0, q>>>(m, ord_keys, ord_vals);
+    chained(k_leaf_cost, (int)(((long)nl * 32 + 255) / 256), 256, 0, q)(m, ord_keys, ord_vals);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return radix_sort_pairs(ord_keys, ord_vals, ord_keys2, ord_vals2, nl, 56, 64, ord_tmp, q);
   };

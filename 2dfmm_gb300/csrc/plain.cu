@@ -56,6 +56,7 @@ struct Climb {
 static_assert(sizeof(Climb) == sizeof(double2), "the climbing state replaces the opening bounds");
 
 __global__ void __launch_bounds__(256) k_climb_init(Tree t, int nt) {
+  chain_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= t.ncell) return;
   Climb *climb = reinterpret_cast<Climb *>(t.mac);
@@ -138,6 +139,7 @@ __device__ __forceinline__ double2 shift_coef(double2 a, double2 d, int nt, int 
 // ms at 20,000 uniform ones; this takes 0.42 and 0.05 (solves 21.5 -> 19.0
 // and 1.03 -> 0.63 ms).
 __global__ void __launch_bounds__(128) k_upward(Tree t, int nt) {
+  chain_wait();
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (wid >= t.nleaf) return;
@@ -212,6 +214,7 @@ enum EvalForm { kFormFp64, kFormFull, kFormHalf };
 // per solve), 2 or 8 warps per block are slower (23.6, 22.2).
 template <int kForm, int kShare>
 __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
+  chain_wait();
   constexpr int kEvalTargets = 32 / kShare;  // per warp
   constexpr unsigned kLanes = (1u << kShare) - 1u, kEachTarget = 0xffffffffu / kLanes;  // a target's lanes; the first of each
   static_assert(kShare == 4 || kShare == 8, "a target's first four lanes test a cell's four children");
@@ -471,6 +474,7 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
 // FP32; a lower bound below 1e-30 becomes -1 and an upper one below 1e-30
 // +inf (no sure answer: the FP32 error bound does not cover subnormals).
 __global__ void k_mac_bounds(Tree t, double theta, int nt, int fixed) {
+  chain_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= t.ncell) return;
   const double r2 = t.region[c] * t.region[c], th2 = theta * theta;
@@ -516,7 +520,7 @@ constexpr double kFixTheta = 2.0 * fix::kHalfTheta;
 
 cudaError_t mac_bounds(Workspace &ws, const Tree &t, double theta, int nt, cudaStream_t s) {
   if (ws.mac_theta == theta || t.ncell <= 0) return cudaSuccess;
-  k_mac_bounds<<<(t.ncell + 63) / 64, 64, 0, s>>>(t, theta, nt, theta <= kFixTheta);
+  chained(k_mac_bounds, (t.ncell + 63) / 64, 64, 0, s)(t, theta, nt, theta <= kFixTheta);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   const cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) ws.mac_theta = theta;
@@ -529,8 +533,8 @@ int plain_upward(Workspace &ws, const Tree &t, const Params &p, cudaStream_t s) 
   const int nt = p.nterms;
   if (nt <= 0 || t.ncell <= 0) return TREE2D_OK;
   ws.mac_theta = -1.0;  // the climb uses the bounds' memory
-  k_climb_init<<<(t.ncell + 255) / 256, 256, 0, s>>>(t, nt);
-  if (t.nleaf > 0) k_upward<<<(t.nleaf + 3) / 4, 128, 0, s>>>(t, nt);
+  chained(k_climb_init, (t.ncell + 255) / 256, 256, 0, s)(t, nt);
+  if (t.nleaf > 0) chained(k_upward, (t.nleaf + 3) / 4, 128, 0, s)(t, nt);
   ::t2d::g_launches.fetch_add(2, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;
@@ -556,7 +560,7 @@ int plain_evaluate(Workspace &ws, const Tree &t, const Params &p, int ntgt, cons
   auto kernel = p.theta > kFixTheta         ? (wide ? k_eval<kFormFp64, 8> : k_eval<kFormFp64, 4>)
                 : p.theta > fix::kHalfTheta ? (wide ? k_eval<kFormFull, 8> : k_eval<kFormFull, 4>)
                                             : (wide ? k_eval<kFormHalf, 8> : k_eval<kFormHalf, 4>);
-  kernel<<<blocks, kEvalWarps * 32, 0, s>>>(a);
+  chained(kernel, blocks, kEvalWarps * 32, 0, s)(a);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;

@@ -42,6 +42,7 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 
 __global__ void __launch_bounds__(kThreads) k_upsweep(const uint64_t *__restrict__ keys, int n, int shift,
                                                       unsigned *__restrict__ counts, int ntiles) {
+  chain_wait();
   __shared__ unsigned hist[kBins];
   for (int i = threadIdx.x; i < kBins; i += kThreads) hist[i] = 0;
   __syncthreads();
@@ -62,6 +63,7 @@ __global__ void __launch_bounds__(kThreads) k_upsweep(const uint64_t *__restrict
 // One block per digit: exclusive scan of counts[d][0..ntiles) in place,
 // total -> totals[d].
 __global__ void __launch_bounds__(1024) k_scan_digit(unsigned *counts, int ntiles, unsigned *totals) {
+  chain_wait();
   __shared__ unsigned part[1024];
   unsigned *c = counts + (size_t)blockIdx.x * ntiles;
   const int t = threadIdx.x;
@@ -117,6 +119,7 @@ __global__ void __launch_bounds__(kThreads) k_downsweep(const uint64_t *__restri
                                                         uint64_t *__restrict__ kout, uint32_t *__restrict__ vout,
                                                         int n, int shift, const unsigned *__restrict__ offs,
                                                         int ntiles, const unsigned *__restrict__ totals, int split) {
+  chain_wait();
   extern __shared__ __align__(16) unsigned char stage[];
   uint64_t *sk = reinterpret_cast<uint64_t *>(stage);             // kTile keys, tile digit order
   uint32_t *sv = reinterpret_cast<uint32_t *>(stage + kTile * 8);  // kTile values (unpacked only)
@@ -207,6 +210,7 @@ constexpr long kLookbackLimit = 1l << 22;     // polls; a healthy look-back ends
 // shared memory, then added to hist[pass][digit].
 __global__ void __launch_bounds__(kThreads) k_hist_all(const uint64_t *__restrict__ words, int n, int begin_bit,
                                                        int passes, unsigned *__restrict__ hist) {
+  chain_wait();
   __shared__ unsigned hw[kWarps][kMaxPasses][kBins];  // per warp: no atomics collide across warps
   for (int i = threadIdx.x; i < kWarps * kMaxPasses * kBins; i += kThreads) (&hw[0][0][0])[i] = 0;
   __syncthreads();
@@ -246,6 +250,7 @@ __global__ void __launch_bounds__(kThreads) k_onesweep(const uint64_t *__restric
                                                        const unsigned *__restrict__ hist, unsigned *status,
                                                        unsigned *ctr, int ntiles, int split, long limit,
                                                        DevStatus *st) {
+  chain_wait();
   constexpr int kTileN = kThreads * kPer;
   extern __shared__ __align__(16) unsigned char stage[];
   uint64_t *sk = reinterpret_cast<uint64_t *>(stage);  // kTileN words, tile digit order
@@ -380,11 +385,11 @@ cudaError_t radix_sort_pairs(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt,
   cudaError_t e = cudaFuncSetAttribute(k_downsweep<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes);
   if (e != cudaSuccess) return e;
   for (int shift = begin_bit; shift < end_bit; shift += 8, passes++) {
-    k_upsweep<<<ntiles, kThreads, 0, s>>>(ka, n, shift, counts, ntiles);
+    chained(k_upsweep, ntiles, kThreads, 0, s)(ka, n, shift, counts, ntiles);
     ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
-    k_scan_digit<<<kBins, 1024, 0, s>>>(counts, ntiles, totals);
+    chained(k_scan_digit, kBins, 1024, 0, s)(counts, ntiles, totals);
     ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
-    k_downsweep<false><<<ntiles, kThreads, kStageBytes, s>>>(ka, va, kb, vb, n, shift, counts, ntiles, totals, 0);
+    chained(k_downsweep<false>, ntiles, kThreads, kStageBytes, s)(ka, va, kb, vb, n, shift, counts, ntiles, totals, 0);
     ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
     uint64_t *tk = ka;
     ka = kb;
@@ -421,12 +426,12 @@ cudaError_t radix_sort_packed(uint64_t *words, uint64_t *words_alt, int n, int b
     e = cudaFuncSetAttribute(k_onesweep<kItems>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStagePackedBytes);
     if (e != cudaSuccess) return e;
     const int hblocks = ntiles < 152 * 4 ? ntiles : 152 * 4;
-    k_hist_all<<<hblocks, kThreads, 0, s>>>(ka, n, begin_bit, passes, hist);
+    chained(k_hist_all, hblocks, kThreads, 0, s)(ka, n, begin_bit, passes, hist);
     ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
     auto kernel = small ? k_onesweep<kSmallItems> : k_onesweep<kItems>;
     for (int p = 0; p < passes; p++) {
       const bool last = p == passes - 1;
-      kernel<<<ntiles, kThreads, tile * 8, s>>>(ka, last ? keys_out : kb, last ? vals_out : nullptr, n,
+      chained(kernel, ntiles, kThreads, tile * 8, s)(ka, last ? keys_out : kb, last ? vals_out : nullptr, n,
                                                 begin_bit + 8 * p, hist + p * kBins,
                                                 status + (size_t)p * ntiles * kBins, ctr + p, ntiles, last ? 1 : 0,
                                                 kLookbackLimit, st);
@@ -446,9 +451,9 @@ cudaError_t radix_sort_packed(uint64_t *words, uint64_t *words_alt, int n, int b
   for (int p = 0; p < passes; p++) {
     const int shift = begin_bit + 8 * p;
     const bool last = p == passes - 1;
-    k_upsweep<<<ntiles, kThreads, 0, s>>>(ka, n, shift, counts, ntiles);
-    k_scan_digit<<<kBins, 1024, 0, s>>>(counts, ntiles, totals);
-    k_downsweep<true><<<ntiles, kThreads, kStagePackedBytes, s>>>(ka, nullptr, last ? keys_out : kb,
+    chained(k_upsweep, ntiles, kThreads, 0, s)(ka, n, shift, counts, ntiles);
+    chained(k_scan_digit, kBins, 1024, 0, s)(counts, ntiles, totals);
+    chained(k_downsweep<true>, ntiles, kThreads, kStagePackedBytes, s)(ka, nullptr, last ? keys_out : kb,
                                                                   last ? vals_out : nullptr, n, shift, counts,
                                                                   ntiles, totals, last ? 1 : 0);
     ::t2d::g_launches.fetch_add(3, std::memory_order_relaxed);
