@@ -301,3 +301,22 @@ def test_tree_around_the_tiles(gpu_lib, n):
     o = oracle().Oracle(11, 33, 0.5)
     o.make_tree(b.xy, b.cir, b.cor)
     assert_same_tree(d, o.dump(n))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,num_p", [(5000, 511), (5000, 513), (5000, 514), (311295, 33), (311296, 33)])
+def test_leaf_levels_around_the_tile_rule(gpu_lib, n, num_p):
+    """Leaf levels from tiles of 512 positions (fewer than 152 x 2048 blobs and
+    an overlap below 512) and of 2048: the tree equals the oracle's."""
+    P = gpu_lib
+    b = workloads().uniform(n, seed=n + num_p)
+    P.set_params(11, num_p, 0.5)
+    P.set_mode(P.MODE_PLAIN)
+    try:
+        P.make_tree(b.xy, b.cir, b.cor)
+        d = P.export_tree(n, 11)
+    finally:
+        P.clear_params()
+    o = oracle().Oracle(11, num_p, 0.5)
+    o.make_tree(b.xy, b.cir, b.cor)
+    assert_same_tree(d, o.dump(n))
