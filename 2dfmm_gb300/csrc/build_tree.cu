@@ -856,7 +856,7 @@ size_t build_tmp_bytes(int n, int nsets) {
   tneed += Arena::bytes_for(n, 1);                              // w
   tneed += radix_sort_temp_bytes(n) + 256;
   tneed += Arena::bytes_for(box_blocks(n), sizeof(Box4));
-  tneed += Arena::bytes_for(ntiles + 1, 8) + 256;
+  tneed += Arena::bytes_for(ntiles + 1, 8);
   const int tlev = batched ? 12 : centre_levels(n);
   tneed += Arena::bytes_for(2 * centre_entries(tlev) * ns, 8);
   if (batched) tneed += Arena::bytes_for(n, 4) + Arena::bytes_for((size_t)nsets * kSetSlices, sizeof(Box4));
@@ -923,7 +923,6 @@ int build_tree(Workspace &ws, int n, const double *d_xy, const double *d_cir, co
   uint8_t *w = ws.tmp_arena.take<uint8_t>(n);
   Box4 *bpart = ws.tmp_arena.take<Box4>(box_blocks(n));
   unsigned long long *part = ws.tmp_arena.take<unsigned long long>(ntiles + 1);
-  unsigned long long *total = ws.tmp_arena.take<unsigned long long>(1);
   uint64_t *ctab = ws.tmp_arena.take<uint64_t>(2 * centre_entries(tlev) * t.nsets);
   int *set_of = batched ? ws.tmp_arena.take<int>(n) : nullptr;
   Box4 *set_part = batched ? ws.tmp_arena.take<Box4>((size_t)nsets * kSetSlices) : nullptr;
@@ -991,12 +990,10 @@ retry:
   // 6. counts and scan
   chained(k_cells_reduce, ntiles, kScanThreads, 0, s)(cpl, leaf_level, n, part);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
-  chained(k_scan_part, 1, 1024, 0, s)(part, ntiles, total);
+  chained(k_scan_part, 1, 1024, 0, s)(part, ntiles, &ws.status->cells);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   T2D_CUDA_TRY(cudaMemcpyAsync(ws.h_status, ws.status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
-  unsigned long long *h_total = reinterpret_cast<unsigned long long *>(ws.h_status + 1);
-  T2D_CUDA_TRY(cudaMemcpyAsync(h_total, total, 8, cudaMemcpyDeviceToHost, s));
   T2D_CUDA_TRY(cudaStreamSynchronize(s));
   if (ws.h_status->err) return ws.h_status->err;
   if (ws.h_status->deeper && total_levels < kKeyLevels) {
@@ -1005,7 +1002,7 @@ retry:
   }
   t.key_levels = total_levels;
   ws.last_depth = ws.h_status->depth;
-  unsigned long long tot = *h_total;
+  const unsigned long long tot = ws.h_status->cells;
   long long ncell = 1 + (long long)(tot >> 32);
   long long nleaf = (long long)(tot & 0xffffffffu);
   if (ncell > (1ll << 31) - 1) return TREE2D_ERR_TOO_DEEP;

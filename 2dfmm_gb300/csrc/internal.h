@@ -88,6 +88,9 @@ struct DevStatus {
   unsigned bar_count;      // mixed: arrivals at the level chain's grid barrier (zeroed before a launch)
   unsigned bar_gen;        // mixed: generation of that barrier
   int nonuniform;          // mixed: some leaf's blobs have different core radii
+  unsigned long long cells;         // build: cells (high 32 bits) and leaves (low) below the root
+  int list_total[3];                // mixed: U, W and K list entries of all leaves (-1: beyond 2^31 - 1)
+  int level_off[kKeyLevels + 2];    // mixed: start of each level in MixedView::by_level
 };
 
 // Bump allocator over one device allocation.  Buffers are 256-byte aligned.
@@ -185,7 +188,7 @@ struct Workspace {
   int list_cap = 256;  // entries per leaf of the one-walk list scratch (from the last solve)
   DevStatus *status = nullptr;   // device
   DevStatus *h_status = nullptr; // pinned host mirror
-  int *h_levels = nullptr;        // pinned: the mixed form's per-level cell offsets (kKeyLevels + 2)
+  int h_levels[kKeyLevels + 2] = {};  // the mixed form's per-level cell offsets
   cudaEvent_t ev[8] = {};
   cudaStream_t side = nullptr;    // second stream (learned decisions beside the expansions)
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr;

@@ -405,12 +405,18 @@ void m2l_b_images(int P, const float *h_m2l, std::vector<float> &img) {
     }
 }
 
-int m2l_tensor_cores(MixedView &m, const float *bimg, int *cls_list, int *cls_count, int rows, cudaStream_t s) {
+int m2l_class_lists(MixedView &m, int *cls_list, int *cls_count, cudaStream_t s) {
+  chained(k_class_lists, (m.ncell + 255) / 256, 256, 0, s)(m, cls_list, cls_count);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
+  T2D_CUDA_TRY(cudaGetLastError());
+  return TREE2D_OK;
+}
+
+int m2l_tensor_cores(MixedView &m, const float *bimg, const int *cls_list, const int *cls_count, int rows,
+                     cudaStream_t s) {
   if (rows != kRows && rows != kRows / 2) return TREE2D_ERR_BAD_PARAMS;
   const int P = m.P, Kc = 2 * P, Npad = m2l_npad(P);
   if (Kc % 8 != 0) return TREE2D_ERR_BAD_PARAMS;  // K of one MMA is 8 TF32 elements
-  T2D_CUDA_TRY(cudaMemsetAsync(cls_count, 0, 4 * sizeof(int), s));
-  chained(k_class_lists, (m.ncell + 255) / 256, 256, 0, s)(m, cls_list, cls_count);
   TcArgs a;
   a.m = m;
   a.cls_list = cls_list;
@@ -430,7 +436,7 @@ int m2l_tensor_cores(MixedView &m, const float *bimg, int *cls_list, int *cls_co
   T2D_CUDA_TRY(cudaFuncSetAttribute(k_m2l_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((m.ncell + rows - 1) / rows, 4);
   chained(k_m2l_tc, grid, kThreadsTC, smem, s)(a);
-  g_launches.fetch_add(2, std::memory_order_relaxed);
+  g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;
 }

@@ -35,6 +35,7 @@
 // centre, formed from the FP64 centres), compensated (Kahan) sums for the
 // direct and correction terms, FP64 for the final per-target reduction.
 #include <cmath>
+#include <cstring>
 #include <type_traits>
 #include <vector>
 
@@ -72,10 +73,21 @@ __device__ __forceinline__ bool adj_cells(const MixedView &m, int a, int b) {
 
 // ------------------------------------------------------------ cell setup
 
-__global__ void k_cell_info(MixedView m) {
+// Also clears what the kernels after it count into or fill (memsets of their
+// own would each stand between two kernels of the chain).
+__global__ void __launch_bounds__(256) k_cell_info(MixedView m, unsigned *rc_bits, unsigned *rc_set_bits, int nsets,
+                                                   int *cls_count) {
   chain_wait();
   int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.x == 0) {
+    for (int i = c; i < 2 * kKeyLevels + 4; i += blockDim.x) m.level_off[i] = 0;
+    if (c < 4) cls_count[c] = 0;
+    if (c == 0) *rc_bits = 0u;
+    if (rc_set_bits)
+      for (int i = c; i < nsets; i += blockDim.x) rc_set_bits[i] = 0u;
+  }
   if (c >= m.ncell) return;
+  m.parent[c] = -1;
   int lev = m.level[c];
   uint64_t k = m.keys[m.begin[c]];
   unsigned ix = 0, iy = 0;
@@ -457,6 +469,7 @@ __global__ void k_level_scan(MixedView m) {
     m.level_off[l + 1] = run;
     m.level_off[kKeyLevels + 2 + l] = m.level_off[l];
   }
+  for (int l = 0; l < kKeyLevels + 2; l++) m.st->level_off[l] = m.level_off[l];
 }
 
 // One atomic per warp and level: lanes of equal level share a reservation.
@@ -734,7 +747,7 @@ __global__ void __launch_bounds__(kScan3Threads) k_scan3_tiles(const int *a, con
 // One thread per array: 64-bit running sums over the tile sums.  List
 // positions are ints, so a total beyond INT_MAX is reported as -1 (the host
 // then stops before any list is filled).
-__global__ void k_scan3_sums(int *tile_sums, int ntiles) {
+__global__ void k_scan3_sums(int *tile_sums, int ntiles, DevStatus *st) {
   chain_wait();
   const int k = threadIdx.x;
   if (k >= 3) return;
@@ -746,6 +759,7 @@ __global__ void k_scan3_sums(int *tile_sums, int ntiles) {
     run += v;
   }
   t[ntiles] = run > 2147483647ll ? -1 : (int)run;
+  st->list_total[k] = t[ntiles];
 }
 
 __global__ void __launch_bounds__(kScan3Threads) k_scan3_apply(int *a, int *b, int *c, int len, const int *tile_sums,
@@ -1467,7 +1481,8 @@ struct Decisions {
 
 // Persistent near-field warps: the grid holds as many warps as fit on the
 // GPU at once, and each warp takes the next target leaf from a counter
-// (DevStatus::eval_next, zeroed before each launch) until none is left.
+// (DevStatus::eval_next, zero since the build cleared the status, or cleared
+// again between the tuner's runs) until none is left.
 // Leaves differ widely in work, so a warp that finishes early takes more
 // instead of idling beside the slowest warp of a resident block.
 __device__ __forceinline__ int next_leaf(DevStatus *st, int lane) {
@@ -2367,8 +2382,6 @@ cudaError_t mixed_tables(int P, float *h_m2l, float *h_m2m, float *h_l2l) {
 
 int mixed_lists(MixedView &m, cudaStream_t s) {
   const int cb = (m.ncell + 255) / 256;
-  chained(k_cell_info, cb, 256, 0, s)(m);
-  T2D_CUDA_TRY(cudaMemsetAsync(m.level_off, 0, sizeof(int) * (2 * kKeyLevels + 4), s));
   chained(k_level_hist, cb, 256, 0, s)(m);
   chained(k_level_scan, 1, 32, 0, s)(m);
   chained(k_level_fill, cb, 256, 0, s)(m);
@@ -2382,7 +2395,7 @@ int mixed_lists(MixedView &m, cudaStream_t s) {
     chained(k_lists<0>, (m.nleaf + kWalkWarps - 1) / kWalkWarps, 32 * kWalkWarps, 0, s)(m);
   const int ntiles = max(1, (m.nleaf + kScanTile3 - 1) / kScanTile3);
   chained(k_scan3_tiles, ntiles, kScan3Threads, 0, s)(m.u_off, m.w_off, m.k_off, m.nleaf, m.scan_tmp, ntiles);
-  chained(k_scan3_sums, 1, 32, 0, s)(m.scan_tmp, ntiles);
+  chained(k_scan3_sums, 1, 32, 0, s)(m.scan_tmp, ntiles, m.st);
   chained(k_scan3_apply, ntiles, kScan3Threads, 0, s)(m.u_off, m.w_off, m.k_off, m.nleaf, m.scan_tmp, ntiles);
   g_launches.fetch_add(8, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
@@ -2547,8 +2560,7 @@ cudaError_t launch_near(const MixedView &m, double *uv, const int *perm, Decisio
 template <bool kLearned, bool kScaled>
 cudaError_t launch_eval(int v, const MixedView &m, double *uv, const int *perm, Decisions d, cudaStream_t s) {
   static int resident[kEvalVariants] = {};  // per variant (the devices here are all one model)
-  cudaError_t e = cudaMemsetAsync(&m.st->eval_next, 0, sizeof(unsigned), s);
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
   switch (v) {
     case 0: e = launch_near<kLearned, kScaled, false, 4>(m, uv, perm, d, s, &resident[0]); break;
     case 1: e = launch_near<kLearned, kScaled, false, 8>(m, uv, perm, d, s, &resident[1]); break;
@@ -2593,6 +2605,7 @@ int near_field(Workspace &ws, const MixedParams &mp, MixedView &m, bool learned,
       for (int r = 0; r < 2 * kEvalVariants; r++) {
         const int c = r < kEvalVariants ? r : 2 * kEvalVariants - 1 - r;
         T2D_CUDA_TRY(cudaMemsetAsync(&ws.status->n_pairs, 0, sizeof(unsigned long long), s));
+        T2D_CUDA_TRY(cudaMemsetAsync(&ws.status->eval_next, 0, sizeof(unsigned), s));
         T2D_CUDA_TRY(cudaEventRecord(ws.ev[6], s));
         T2D_CUDA_TRY(run(c));
         T2D_CUDA_TRY(cudaEventRecord(ws.ev[7], s));
@@ -2744,9 +2757,6 @@ int mixed_solve(Workspace &ws, const Tree &t, const MixedParams &mp, double *d_u
   m.nleaf = nl;
   m.P = P;
   m.keys = t.keys;
-  m.cpl = t.cpl;
-  m.leaf_level = t.leaf_level;
-  m.cellbase = t.cellbase;
   m.level = t.level;
   m.begin = t.begin;
   m.end = t.end;
@@ -2808,13 +2818,11 @@ int mixed_solve(Workspace &ws, const Tree &t, const MixedParams &mp, double *d_u
   m.m2m = reinterpret_cast<const float2 *>(dm2m);
   m.l2l = reinterpret_cast<const float2 *>(dl2l);
   m.st = ws.status;
-  T2D_CUDA_TRY(cudaMemsetAsync(m.parent, 0xff, sizeof(int) * (size_t)nc, s));
-  T2D_CUDA_TRY(cudaMemsetAsync(rc_bits, 0, 4, s));
+  chained(k_cell_info, (nc + 255) / 256, 256, 0, s)(m, rc_bits, rc_set_bits, t.nsets, cls_count);
   chained(k_sigma_max, 304, 256, 0, s)(t.cor, n, rc_bits);
   chained(k_cutoff, 1, 32, 0, s)(rc_bits, (float)mp.cutoff, 1);
   g_launches.fetch_add(2, std::memory_order_relaxed);
   if (rc_set_bits) {
-    T2D_CUDA_TRY(cudaMemsetAsync(rc_set_bits, 0, 4 * (size_t)t.nsets, s));
     chained(k_sigma_max_sets, dim3((unsigned)t.nsets, kSigmaSlices), 256, 0, s)(t.set_cor, t.set_off, rc_set_bits);
     chained(k_cutoff, (t.nsets + 255) / 256, 256, 0, s)(rc_set_bits, (float)mp.cutoff, t.nsets);
     g_launches.fetch_add(2, std::memory_order_relaxed);
@@ -2824,14 +2832,18 @@ int mixed_solve(Workspace &ws, const Tree &t, const MixedParams &mp, double *d_u
   if (rc) return rc;
   rc = mixed_lists(m, s);
   if (rc) return rc;
-  int tot[3];
-  T2D_CUDA_TRY(cudaMemcpyAsync(&tot[0], m.u_off + nl, 4, cudaMemcpyDeviceToHost, s));
-  T2D_CUDA_TRY(cudaMemcpyAsync(&tot[1], m.w_off + nl, 4, cudaMemcpyDeviceToHost, s));
-  T2D_CUDA_TRY(cudaMemcpyAsync(&tot[2], m.k_off + nl, 4, cudaMemcpyDeviceToHost, s));
+  // the lists' sizes and the levels, with the status; what the expansions
+  // need besides the lists runs while the host wakes up
   T2D_CUDA_TRY(cudaMemcpyAsync(ws.h_status, ws.status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
-  if (ws.h_levels)
-    T2D_CUDA_TRY(cudaMemcpyAsync(ws.h_levels, m.level_off, sizeof(int) * (kKeyLevels + 2), cudaMemcpyDeviceToHost, s));
-  T2D_CUDA_TRY(cudaStreamSynchronize(s));
+  T2D_CUDA_TRY(cudaEventRecord(ws.fork_ev, s));
+  T2D_CUDA_TRY(cudaMemsetAsync(m.L, 0, sizeof(float) * (size_t)nc * 2 * P, s));
+  if (tc) {
+    rc = m2l_class_lists(m, cls_list, cls_count, s);
+    if (rc) return rc;
+  }
+  T2D_CUDA_TRY(cudaEventSynchronize(ws.fork_ev));
+  const int tot[3] = {ws.h_status->list_total[0], ws.h_status->list_total[1], ws.h_status->list_total[2]};
+  std::memcpy(ws.h_levels, ws.h_status->level_off, sizeof(ws.h_levels));
   const bool from_scratch = one_walk && !ws.h_status->list_overflow;
   {
     // the next solve's scratch rows: 1.25 x this solve's largest leaf
@@ -2971,7 +2983,6 @@ int mixed_solve(Workspace &ws, const Tree &t, const MixedParams &mp, double *d_u
   }
   rc = mixed_upward(m, t.depth, ws.h_levels, su, mp.level_chain != 0);
   if (rc) return drain(rc);
-  T2D_TRY_DRAIN(cudaMemsetAsync(m.L, 0, sizeof(float) * (size_t)nc * 2 * P, su));
   rc = tc ? m2l_tc_tuned(ws, mp, m, dimg, cls_list, cls_count, su, st) : m2l_cuda_cores(m, dm2l, su);
   if (rc) return drain(rc);
   st.m2l_path = tc ? 2 : 1;

@@ -25,8 +25,6 @@ struct MixedView {
   int lev0;             // batched sets: levels of container cells above the set roots
   // from the tree
   const uint64_t *keys;
-  const uint8_t *cpl, *leaf_level;
-  const unsigned *cellbase;
   const int *level, *begin, *end, *child, *leaf_cell;
   const unsigned char *leaf;
   const double *cx, *cy, *region;
@@ -96,7 +94,10 @@ int m2l_cuda_cores(MixedView &m, const float *tables, cudaStream_t s);
 // Tensor-core form: needs P % 4 == 0.  `bimg` are the B operator images
 // (m2l_b_images), cls_list/cls_count scratch of 4*ncell and 4 ints.
 // rows: cells per CTA, 128 or 64 (bit-identical results)
-int m2l_tensor_cores(MixedView &m, const float *bimg, int *cls_list, int *cls_count, int rows, cudaStream_t s);
+int m2l_tensor_cores(MixedView &m, const float *bimg, const int *cls_list, const int *cls_count, int rows,
+                     cudaStream_t s);
+// The cells of each class (cls_count: 4 zeros before), for m2l_tensor_cores.
+int m2l_class_lists(MixedView &m, int *cls_list, int *cls_count, cudaStream_t s);
 int m2l_npad(int P);
 void m2l_b_images(int P, const float *h_m2l, std::vector<float> &img);
 
