@@ -89,6 +89,16 @@ constexpr int kMaxKc4 = 2 * kMaxP / 4;  // float4s in one multipole row (2P floa
 // i+1's multipole row in registers, and (with 3 B stages) slot i+1's
 // operator images are in flight by bulk copy, so the gather latency is
 // paid once per tile rather than once per slot.
+//
+// kWhole (Kc = 32, the default 16 terms): a row is one 128-byte line, and
+// eight lanes load one whole, a 16-byte piece each, so that a warp's load
+// touches four lines; with a row per thread it touched 32, and looking those up
+// in L1 was what a slot waited for (M2L of 16M pairs, 512 sets: 1.42 -> 1.10
+// ms; of 2M pairs, 4M blobs: 214 -> 164 us).  The eight pieces of a row are then
+// stored by neighbouring lanes, without bank conflicts because the core
+// matrices of a row lie 144 bytes apart (kLboWhole) instead of 128.
+constexpr uint32_t kLboWhole = 144;
+template <bool kWhole>
 __global__ void __launch_bounds__(kThreadsTC) k_m2l_tc(TcArgs a) {
   chain_wait();
   extern __shared__ __align__(1024) unsigned char smem[];
@@ -103,8 +113,9 @@ __global__ void __launch_bounds__(kThreadsTC) k_m2l_tc(TcArgs a) {
   if (row0 >= count) return;  // uniform for the block
   const MixedView &m = a.m;
   const int P = a.P, Kc = a.Kc, Npad = a.Npad, nbs = a.nbs;
-  const uint32_t a_bytes = kRows * Kc * 4, b_bytes = Npad * Kc * 4;
-  const uint32_t sbo_a = (Kc / 4) * 128, sbo_b = sbo_a, lbo = 128;
+  const uint32_t lbo = 128, lbo_a = kWhole ? kLboWhole : lbo;
+  const uint32_t sbo_a = (Kc / 4) * lbo_a, sbo_b = (Kc / 4) * lbo;
+  const uint32_t a_bytes = kRows / 8 * sbo_a, b_bytes = Npad * Kc * 4;
   const int tid = threadIdx.x, warp = tid >> 5;
   int *sV = reinterpret_cast<int *>(smem);                       // [27][kRows]
   unsigned char *astage = smem + 27 * kRows * 4;                 // 2 x (hi, lo)
@@ -149,25 +160,35 @@ __global__ void __launch_bounds__(kThreadsTC) k_m2l_tc(TcArgs a) {
   const uint32_t idesc = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(Npad >> 3) << 17) | ((uint32_t)(kRows >> 4) << 24);
   const float *bbase = a.bimg + (size_t)cls * 27 * 2 * (Npad * Kc);
 
-  uint32_t phase_mma[2] = {0, 0}, phase_b[3] = {0, 0, 0};
-  bool pending[2] = {false, false};
-  bool b_inflight[3] = {false, false, false};  // thread 0: bulk copy issued, not yet waited for
+  // bit k: phase and state of stage k (in registers, where arrays indexed by
+  // the stage would be in local memory)
+  uint32_t phase_mma = 0, phase_b = 0, pending = 0;
+  uint32_t b_inflight = 0;  // thread 0: bulk copy issued, not yet waited for
   // Slots are spread over `ngroups` accumulators (TMEM column blocks of
   // Npad) by slot number, slot % ngroups; each accumulates few MMAs and the
   // partial sums are added in FP32 registers at the end, in group order,
   // which keeps the accumulation error small.  A row's sums depend only on
   // its own slots (a slot another row of the tile uses adds exact zeros),
   // so the result does not depend on which cells share the tile.
-  bool gfirst[8] = {true, true, true, true, true, true, true, true};
+  uint32_t gseen = 0;  // bit g: accumulator g has been written
   int issued = 0;  // steps whose MMAs were committed (or attempted)
   auto slot_at = [&](unsigned rest) { return __ffs(rest) - 1; };  // lowest remaining slot
   auto copy_b = [&](int slot, int bs) {
     if (tid != 0) return;
     mbar_expect_tx(&bar_b[bs], 2 * b_bytes);
     bulk_g2s(bstage + (size_t)bs * 2 * b_bytes, bbase + (size_t)slot * 2 * (Npad * Kc), 2 * b_bytes, &bar_b[bs]);
-    b_inflight[bs] = true;
+    b_inflight |= 1u << bs;
   };
   auto load_row = [&](int slot, float4 (&r)[kMaxKc4]) {
+    if (kWhole) {  // piece tid & 7 of the warp's rows 4 j + (lane >> 3)
+#pragma unroll
+      for (int j = 0; j < 8; j++) {
+        const int src = sV[slot * kRows + (tid & ~31) + 4 * j + ((tid & 31) >> 3)];
+        r[j] = src >= 0 ? reinterpret_cast<const float4 *>(m.M + (size_t)src * 2 * P)[tid & 7]
+                        : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      return;
+    }
     const int src = sV[slot * kRows + tid];
     const float4 *msrc = src >= 0 ? reinterpret_cast<const float4 *>(m.M + (size_t)src * 2 * P) : nullptr;
 #pragma unroll
@@ -186,10 +207,10 @@ __global__ void __launch_bounds__(kThreadsTC) k_m2l_tc(TcArgs a) {
     if (next >= 0) load_row(next, fill);
     // the MMAs that last read this A stage (and, with 3 B stages, the B
     // stage of the next slot) must be done before they are rewritten
-    if (pending[ast]) {
-      if (mbar_wait(&bar_mma[ast], phase_mma[ast], a.wait_limit)) {
-        phase_mma[ast] ^= 1;
-        pending[ast] = false;
+    if (pending >> ast & 1u) {
+      if (mbar_wait(&bar_mma[ast], phase_mma >> ast & 1u, a.wait_limit)) {
+        phase_mma ^= 1u << ast;
+        pending &= ~(1u << ast);
       } else {
         s_fail = 1;
       }
@@ -201,7 +222,7 @@ __global__ void __launch_bounds__(kThreadsTC) k_m2l_tc(TcArgs a) {
       float *Alo = reinterpret_cast<float *>(astage + (size_t)ast * 2 * a_bytes + a_bytes);
       const uint32_t rbase = (uint32_t)(tid >> 3) * sbo_a + (uint32_t)(tid & 7) * 16;
 #pragma unroll
-      for (int kk = 0; kk < kMaxKc4; kk++) {
+      for (int kk = 0; kk < (kWhole ? 8 : kMaxKc4); kk++) {
         if (kk >= Kc / 4) break;
         const float4 v = use[kk];
         float4 h, l;
@@ -213,7 +234,9 @@ __global__ void __launch_bounds__(kThreadsTC) k_m2l_tc(TcArgs a) {
         l.y = v.y - h.y;
         l.z = v.z - h.z;
         l.w = v.w - h.w;
-        const uint32_t off = rbase + (uint32_t)kk * lbo;
+        const uint32_t row = (uint32_t)((tid & ~31) + 4 * kk + ((tid & 31) >> 3));  // kWhole
+        const uint32_t off = kWhole ? (row >> 3) * sbo_a + (row & 7) * 16 + (uint32_t)(tid & 7) * kLboWhole
+                                    : rbase + (uint32_t)kk * lbo;
         *reinterpret_cast<float4 *>(reinterpret_cast<unsigned char *>(Ahi) + off) = h;
         *reinterpret_cast<float4 *>(reinterpret_cast<unsigned char *>(Alo) + off) = l;
       }
@@ -221,20 +244,20 @@ __global__ void __launch_bounds__(kThreadsTC) k_m2l_tc(TcArgs a) {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (__syncthreads_or(s_fail)) return false;
     if (tid == 0) {
-      if (mbar_wait(&bar_b[bs], phase_b[bs], a.wait_limit)) {
-        phase_b[bs] ^= 1;
-        b_inflight[bs] = false;
+      if (mbar_wait(&bar_b[bs], phase_b >> bs & 1u, a.wait_limit)) {
+        phase_b ^= 1u << bs;
+        b_inflight &= ~(1u << bs);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t ah = smem_u32(astage + (size_t)ast * 2 * a_bytes), al = ah + a_bytes;
         const uint32_t bh = smem_u32(bstage + (size_t)bs * 2 * b_bytes), bl = bh + b_bytes;
         const int g = slot % a.ngroups;
         const uint32_t dcol = tmem + (uint32_t)(g * Npad);
         for (int t = 0; t < Kc / 8; t++) {
-          const uint32_t ko = (uint32_t)t * 2 * lbo;
-          const uint64_t dah = smem_desc(ah + ko, lbo, sbo_a), dal = smem_desc(al + ko, lbo, sbo_a);
+          const uint32_t ko = (uint32_t)t * 2 * lbo, ka = (uint32_t)t * 2 * lbo_a;
+          const uint64_t dah = smem_desc(ah + ka, lbo_a, sbo_a), dal = smem_desc(al + ka, lbo_a, sbo_a);
           const uint64_t dbh = smem_desc(bh + ko, lbo, sbo_b), dbl = smem_desc(bl + ko, lbo, sbo_b);
-          mma_tf32(dcol, dah, dbh, idesc, gfirst[g] ? 0u : 1u);
-          gfirst[g] = false;
+          mma_tf32(dcol, dah, dbh, idesc, gseen >> g & 1u);
+          gseen |= 1u << g;
           mma_tf32(dcol, dah, dbl, idesc, 1u);
           mma_tf32(dcol, dal, dbh, idesc, 1u);
         }
@@ -245,7 +268,7 @@ __global__ void __launch_bounds__(kThreadsTC) k_m2l_tc(TcArgs a) {
         s_fail = 1;
       }
     }
-    pending[ast] = true;
+    pending |= 1u << ast;
     issued = i + 1;
     return true;
   };
@@ -275,10 +298,10 @@ __global__ void __launch_bounds__(kThreadsTC) k_m2l_tc(TcArgs a) {
   // drain: every stage with MMAs in flight (bounded; a failed wait is
   // retried once more below before TMEM and shared memory are released)
   for (int st = 0; st < 2; st++) {
-    if (pending[st]) {
-      if (mbar_wait(&bar_mma[st], phase_mma[st], a.wait_limit)) {
-        phase_mma[st] ^= 1;
-        pending[st] = false;
+    if (pending >> st & 1u) {
+      if (mbar_wait(&bar_mma[st], phase_mma >> st & 1u, a.wait_limit)) {
+        phase_mma ^= 1u << st;
+        pending &= ~(1u << st);
       } else {
         s_fail = 1;
       }
@@ -324,9 +347,9 @@ __global__ void __launch_bounds__(kThreadsTC) k_m2l_tc(TcArgs a) {
     // a wait gave up: give MMAs and copies still in flight one more bounded
     // wait before the TMEM and shared memory are released
     for (int st = 0; st < 2; st++)
-      if (pending[st]) mbar_wait(&bar_mma[st], phase_mma[st], a.wait_limit);
+      if (pending >> st & 1u) mbar_wait(&bar_mma[st], phase_mma >> st & 1u, a.wait_limit);
     for (int bs = 0; bs < 3; bs++)
-      if (tid == 0 && b_inflight[bs]) mbar_wait(&bar_b[bs], phase_b[bs], a.wait_limit);
+      if (tid == 0 && (b_inflight >> bs & 1u)) mbar_wait(&bar_b[bs], phase_b >> bs & 1u, a.wait_limit);
   }
   if (s_fail && tid == 0) set_err(m.st, TREE2D_ERR_TIMEOUT);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -429,13 +452,15 @@ int m2l_tensor_cores(MixedView &m, const float *bimg, const int *cls_list, const
   a.ngroups = 256 / Npad < 8 ? 256 / Npad : 8;
   a.rows = rows;
   a.wait_limit = 1l << 22;  // polls; a healthy wait ends within microseconds
-  const size_t fixed = (size_t)27 * kRows * 4 + 2 * (2 * (size_t)kRows * Kc * 4);
+  const bool whole = Kc == 32;
+  const size_t fixed = (size_t)27 * kRows * 4 + 2 * (2 * (size_t)(kRows / 8) * (Kc / 4) * (whole ? kLboWhole : 128));
   const size_t bst = 2 * (size_t)Npad * Kc * 4;
   a.nbs = fixed + 3 * bst <= 110 * 1024 ? 3 : 2;  // 3 B stages while two CTAs still fit an SM
   const size_t smem = fixed + (size_t)a.nbs * bst;
-  T2D_CUDA_TRY(cudaFuncSetAttribute(k_m2l_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  auto kernel = whole ? k_m2l_tc<true> : k_m2l_tc<false>;
+  T2D_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   dim3 grid((m.ncell + rows - 1) / rows, 4);
-  chained(k_m2l_tc, grid, kThreadsTC, smem, s)(a);
+  chained(kernel, grid, kThreadsTC, smem, s)(a);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;
