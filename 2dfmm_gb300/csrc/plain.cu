@@ -6,8 +6,8 @@
 //              that completes a cell's last child forms that cell (children
 //              in quadrant order 3,2,1,0).  The level-1 -> root shift is
 //              skipped as in the reference.
-//  k_eval      one warp per 8 or 4 consecutive targets (tree order, so the warp's
-//              targets are neighbours), 4 or 8 lanes per target.  The warp walks
+//  k_eval      one warp per 8, 4 or 2 consecutive targets (tree order, so the
+//              targets are neighbours), 4, 8 or 16 lanes per target.  The warp walks
 //              the UNION of its targets' traversals with a shared LIFO of
 //              (cell, lane mask): restricted to one target, the visit order
 //              is that target's own LIFO order in fmm.c:90-112.  The opening
@@ -216,8 +216,8 @@ template <int kForm, int kShare>
 __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
   chain_wait();
   constexpr int kEvalTargets = 32 / kShare;  // per warp
-  constexpr unsigned kLanes = (1u << kShare) - 1u, kEachTarget = 0xffffffffu / kLanes;  // a target's lanes; the first of each
-  static_assert(kShare == 4 || kShare == 8, "a target's first four lanes test a cell's four children");
+  constexpr unsigned kLanes = 0xffffffffu >> (32 - kShare), kEachTarget = 0xffffffffu / kLanes;  // a target's; each's first
+  static_assert(kShare >= 4 && (kShare & (kShare - 1)) == 0, "a target's first four lanes test a cell's four children");
   __shared__ int s_cell[kEvalWarps][kStackCap];
   __shared__ unsigned s_mask[kEvalWarps][kStackCap];
   __shared__ int s_queue[kEvalWarps][kEvalTargets][kQueue];
@@ -540,13 +540,32 @@ int plain_upward(Workspace &ws, const Tree &t, const Params &p, cudaStream_t s) 
   return TREE2D_OK;
 }
 
-// Trees of up to this many blobs are evaluated with eight lanes per target,
-// which leaves fewer targets to a warp and twice the warps to hide latencies.
-// Measured evaluation, 8 against 4 lanes: 4,096 uniform blobs 115 / 166 us,
-// 32,768 399 / 451, 65,536 752 / 729; Lamb-Oseen 65,536 1.10 / 1.12 ms,
-// 131,072 2.15 / 2.09.  By the tree's size, not the targets' number: a point's
-// sums do not depend on how many points are asked for.
-constexpr int kWideBlobs = 65536;
+// Lanes per target.  A small tree's evaluation has few warps and waits on
+// latencies: more lanes leave fewer targets to a warp, for more warps; a large
+// one's fills the chip anyway, and sharing a target costs.  The lines grow with
+// the leaf size, as a target's work does.  Measured evaluation, us, with 4 / 8
+// / 16 lanes, Lamb-Oseen blobs:
+//    num_p        33                65                250                500
+//    4,096   247 / 157 / 114   296 / 183 / 112   593 / 318 / 179    699 / 368 / 206
+//    8,192   286 / 181 / 169   337 / 218 / 169   808 / 429 / 296   1017 / 540 / 357
+//   12,288   307 / 223 / 244   371 / 268 / 262   855 / 524 / 440   1536 / 870 / 670
+//   32,768   531 / 507 / 589   620 / 558 / 607  1136 / 953 / 943   2258 / 1844 / 1644
+//   65,536   963 / 985 / 1169 1122 / 1092 / 1233 2346 / 2032 / 2043 3971 / 3333 / 3205
+//  131,072  1797 / 1938 / -   2070 / 2138 / -   3608 / 3423 / 3690 6871 / 6301 / 6465
+// By the tree, not the targets' number: a point's sums do not depend on how
+// many points are asked for.
+int eval_share(int n, int num_p) {
+  if (n <= 8192 || (n <= 65536 && n <= 200l * num_p)) return 16;
+  if (n <= 65536 || (n <= 131072 && n <= 1024l * num_p)) return 8;
+  return 4;
+}
+
+template <int kShare>
+auto eval_kernel(double theta) {
+  return theta > kFixTheta         ? k_eval<kFormFp64, kShare>
+         : theta > fix::kHalfTheta ? k_eval<kFormFull, kShare>
+                                   : k_eval<kFormHalf, kShare>;
+}
 
 int plain_evaluate(Workspace &ws, const Tree &t, const Params &p, int ntgt, const double *tx, const double *ty,
                    const int *out_idx, double *uv, cudaStream_t s) {
@@ -554,12 +573,10 @@ int plain_evaluate(Workspace &ws, const Tree &t, const Params &p, int ntgt, cons
   T2D_CUDA_TRY(mac_bounds(ws, t, p.theta, p.nterms, s));
   EvalArgs a{t, p.nterms, p.theta, ntgt, tx, ty, out_idx, uv, ws.status, fix::first_pair_term(p.theta),
              reinterpret_cast<const void *>(t.fix) != reinterpret_cast<const void *>(t.coef), fix::One()};
-  const bool wide = t.n <= kWideBlobs;
-  const int warps = (int)(((long)ntgt * (wide ? 8 : 4) + 31) / 32);
+  const int share = eval_share(t.n, p.num_p);
+  const int warps = (int)(((long)ntgt * share + 31) / 32);
   const int blocks = (warps + kEvalWarps - 1) / kEvalWarps;
-  auto kernel = p.theta > kFixTheta         ? (wide ? k_eval<kFormFp64, 8> : k_eval<kFormFp64, 4>)
-                : p.theta > fix::kHalfTheta ? (wide ? k_eval<kFormFull, 8> : k_eval<kFormFull, 4>)
-                                            : (wide ? k_eval<kFormHalf, 8> : k_eval<kFormHalf, 4>);
+  auto kernel = share == 16 ? eval_kernel<16>(p.theta) : share == 8 ? eval_kernel<8>(p.theta) : eval_kernel<4>(p.theta);
   chained(kernel, blocks, kEvalWarps * 32, 0, s)(a);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());

@@ -320,3 +320,26 @@ def test_leaf_levels_around_the_tile_rule(gpu_lib, n, num_p):
     o = oracle().Oracle(11, num_p, 0.5)
     o.make_tree(b.xy, b.cir, b.cor)
     assert_same_tree(d, o.dump(n))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,num_p", [(8192, 33), (8193, 33), (13000, 65), (13001, 65), (65536, 400), (131072, 128)])
+def test_lanes_per_target_at_the_other_limits(gpu_lib, n, num_p):
+    """Sixteen lanes per target up to 8,192 blobs, or 200 per num_p, and eight
+    up to 131,072 with long leaves: blobs and points off the blobs, ragged
+    numbers of both, within the parity bar of the oracle."""
+    P = gpu_lib
+    W = workloads()
+    b = W.uniform(n, seed=4)
+    rng = np.random.default_rng(8)
+    q = np.concatenate([b.xy[W.sample_targets(n, 253, seed=2)], rng.uniform(-1.2, 1.2, (17, 2))])
+    P.set_params(13, num_p, 0.5)
+    P.set_mode(P.MODE_PLAIN)
+    try:
+        P.make_tree(b.xy, b.cir, b.cor)
+        uv = P.biot_tree_batch(q)
+    finally:
+        P.clear_params()
+    o = oracle().Oracle(13, num_p, 0.5)
+    o.make_tree(b.xy, b.cir, b.cor)
+    assert_parity(uv, o.biot(q), q, ext_for(b.xy, b.cir, b.cor, 13, num_p, 0.5), label=f"{n} leaf {num_p}")
