@@ -818,19 +818,17 @@ __global__ void __launch_bounds__(256) k_leaf_order(const uint32_t *__restrict__
 // non-finite circulation or a NaN core radius is bad input.
 __global__ void __launch_bounds__(256) k_gather(const double *__restrict__ xy, const double *__restrict__ cir,
                                                 const double *__restrict__ cor, const int *__restrict__ perm, int n,
-                                                double *x, double *y, double *c, double *r, double *icor2,
-                                                DevStatus *st) {
+                                                double *x, double *y, double *c, double *r, DevStatus *st) {
   chain_wait();
   long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (i >= n) return;
   int p = perm[i];
   const double g = cir[p], rc = cor[p];
-  if (!isfinite(g) || isnan(rc)) set_err(st, TREE2D_ERR_BAD_INPUT);
+  if (!finite_bits(g) || nan_bits(rc)) set_err(st, TREE2D_ERR_BAD_INPUT);
   x[i] = xy[2 * (long)p];
   y[i] = xy[2 * (long)p + 1];
   c[i] = g;
   r[i] = rc;
-  icor2[i] = 1.0 / (rc * rc);
 }
 
 }  // namespace
@@ -1047,8 +1045,7 @@ retry:
     ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   }
   if (cir_cor_ready) T2D_CUDA_TRY(cudaStreamWaitEvent(s, cir_cor_ready, 0));
-  chained(k_gather, (n + 255) / 256, 256, 0, s)(d_xy, d_cir, d_cor, t.perm, n, t.x, t.y, t.cir, t.cor, t.icor2,
-                                           ws.status);
+  chained(k_gather, (n + 255) / 256, 256, 0, s)(d_xy, d_cir, d_cor, t.perm, n, t.x, t.y, t.cir, t.cor, ws.status);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;

@@ -66,6 +66,14 @@ __device__ __forceinline__ double2 shfl_d2(double2 v, int src) {
   return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
 
+// Tests on a double's bits: FP64 comparisons run at 1/64 of the integer rate.
+__device__ __forceinline__ bool finite_bits(double v) {
+  return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000;
+}
+__device__ __forceinline__ bool nan_bits(double v) {
+  return (unsigned long long)(__double_as_longlong(v) & 0x7fffffffffffffffll) > 0x7ff0000000000000ull;
+}
+
 // Number of leading base-4 digits shared by two keys (32 if equal).
 __device__ __forceinline__ int common_levels(uint64_t a, uint64_t b) {
   uint64_t d = a ^ b;

@@ -137,7 +137,7 @@ class Arena {
 struct Tree {
   int n = 0, ncell = 0, nleaf = 0, depth = 0, nterms = 0;
   double *x = nullptr, *y = nullptr, *cir = nullptr, *cor = nullptr;
-  double *icor2 = nullptr;    // 1 / cor^2 per blob (tree order)
+  double *icor2 = nullptr;    // 1 / cor^2 per blob (tree order), formed by plain_upward
   int *perm = nullptr;        // tree position -> original blob index
   int *level = nullptr, *begin = nullptr, *end = nullptr;
   int *child = nullptr;       // 4 per cell, quadrant order, -1 = no blob there

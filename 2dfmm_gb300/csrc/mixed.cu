@@ -121,7 +121,9 @@ __global__ void __launch_bounds__(256) k_cell_info(MixedView m, unsigned *rc_bit
 // first kSetupStage blobs are kept in shared memory between the passes
 // (larger leaves form the rest again from global memory).  Each warp's leaf
 // is a chain of dependent loads, so the kernel is bounded to 32 registers:
-// 64 warps per SM (measured 16.36 -> 16.32 ms for the 512-set batch).
+// 64 warps per SM (measured 16.36 -> 16.32 ms for the 512-set batch).  FP64
+// runs at 1/64 of the FP32 rate: the leaf's constants come from k_cell_info's
+// FP32 values and core radii are compared as bits (22M blobs: 855 -> 618 us).
 constexpr int kSubCells = 64;
 constexpr int kSetupWarps = 8;
 constexpr int kSetupStage = 128;
@@ -147,7 +149,7 @@ __global__ void __launch_bounds__(32 * kSetupWarps, 8) k_leaf_setup(MixedView m,
   const int c = m.leaf_cell[wid];
   const double cx = m.cx[c], cy = m.cy[c], side = m.region[c];
   const int b = m.begin[c], e = m.end[c];
-  const float hs = (float)(0.5 * side), q = (float)(8.0 / side);
+  const float hs = 0.5f * m.h[c], q = 8.f * m.inv_h[c];  // (float)(0.5 side), (float)(8 / side): powers of two
   const unsigned lt = (1u << lane) - 1u;
   auto offset_of = [&](int i) { return make_float2((float)(x[i] - cx), (float)(y[i] - cy)); };
   auto code_of = [&](float2 lc) {
@@ -159,13 +161,14 @@ __global__ void __launch_bounds__(32 * kSetupWarps, 8) k_leaf_setup(MixedView m,
   cnt[lane] = 0;
   cnt[lane + 32] = 0;
   __syncwarp();
-  const double cor0 = cor[b];
-  bool same = true;
+  const long long cor0 = __double_as_longlong(cor[b]);
+  bool same = !nan_bits(__longlong_as_double(cor0));
   for (int i0 = b; i0 < e; i0 += 32) {
     const int i = i0 + lane, o = i - b;
     int code = kSubCells;
     if (i < e) {
-      same = same && cor[i] == cor0;
+      const long long ci = __double_as_longlong(cor[i]);
+      same = same && (ci == cor0 || ((ci | cor0) << 1) == 0);  // equal values: equal bits or two zeros
       const float2 lc = offset_of(i);
       code = code_of(lc);
       if (o < kSetupStage) {
@@ -182,9 +185,10 @@ __global__ void __launch_bounds__(32 * kSetupWarps, 8) k_leaf_setup(MixedView m,
   // stay far inside FP32 (their squares too): a core radius of 0 (the
   // mirror images are point vortices) or one far below the leaf's size
   // keeps the leaf, and so the solve, on the unscaled records.
-  const float sf0 = (float)cor0;
-  const float s0 = sqrtf(1.44269504f * __frcp_rn(sf0 * sf0));
-  const bool uniform = __all_sync(0xffffffffu, same) && s0 > 0.f && __fmul_rn(s0, (float)side) < 1e15f;
+  const float sf0 = (float)__longlong_as_double(cor0), w0 = __frcp_rn(sf0 * sf0);
+  const float s0 = sqrtf(1.44269504f * w0);
+  const bool one_core = __all_sync(0xffffffffu, same);
+  const bool uniform = one_core && s0 > 0.f && __fmul_rn(s0, (float)side) < 1e15f;
   const float sc = uniform ? s0 : 0.f;
   if (lane == 0) {
     m.lscale[c] = sc;
@@ -234,8 +238,11 @@ __global__ void __launch_bounds__(32 * kSetupWarps, 8) k_leaf_setup(MixedView m,
       // 1/sigma^2 is only kept in FP32, so it is formed in FP32 (the FP64
       // divide is slow on this GPU and buys nothing after the rounding);
       // the correctly rounded reciprocal is 1.f / (sf * sf) exactly
-      const float sf = (float)cor[i];
-      const float w = __frcp_rn(sf * sf);
+      float w = w0;
+      if (!one_core) {
+        const float sf = (float)cor[i];
+        w = __frcp_rn(sf * sf);
+      }
       m.src4[d] = make_float4(lc.x, lc.y, g, -1.44269504f * w);
       if (uniform) m.src4s[d] = make_float4(__fmul_rn(lc.x, sc), __fmul_rn(lc.y, sc), __fmul_rn(g, sc), 0.f);
       m.mperm[d] = perm[i];
@@ -926,41 +933,47 @@ __global__ void __launch_bounds__(256) k_m2m_f32(MixedView m, int lev) {
 // parent, not to c) into c's local expansion, b_l -= G w^(l+1), w = 1/z,
 // z the blob's offset from c's centre in units of c's side.  One warp per
 // cell, lanes over blobs, chunked coefficients as S2M.
+// A warp takes kP2lCells cells, most of which have no X list (a warp for each
+// cell: 420 us for the 705,779 cells of 512 sets; so 222).
+constexpr int kP2lCells = 8;
 __global__ void __launch_bounds__(256) k_p2l(MixedView m) {
   chain_wait();
   __shared__ float sh[8][32 * kCoefPitch];
-  const int c = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (c >= m.ncell) return;
-  const int *X = m.xlist + (size_t)c * 8;
-  if (X[0] < 0) return;
+  const int lane = threadIdx.x & 31, first = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kP2lCells;
   float *buf = sh[threadIdx.x >> 5];
   const int P = m.P;
-  const float ih = m.inv_h[c];
-  for (int c0 = 0; c0 < P; c0 += kCoefChunk) {
-    float acc[2 * kCoefChunk];
+  const int mine = first + lane;
+  unsigned todo = __ballot_sync(0xffffffffu, lane < kP2lCells && mine < m.ncell && m.xlist[(size_t)mine * 8] >= 0);
+  for (; todo; todo &= todo - 1) {
+    const int c = first + __ffs(todo) - 1;
+    const int *X = m.xlist + (size_t)c * 8;
+    const float ih = m.inv_h[c];
+    for (int c0 = 0; c0 < P; c0 += kCoefChunk) {
+      float acc[2 * kCoefChunk];
 #pragma unroll
-    for (int i = 0; i < 2 * kCoefChunk; i++) acc[i] = 0.f;
-    for (int e = 0; e < 8 && X[e] >= 0; e++) {
-      const int d = X[e];
-      const float ox = centre_offset(m.cxf, m.cxl, d, c), oy = centre_offset(m.cyf, m.cyl, d, c);
-      for (int j = m.begin[d] + lane; j < m.end[d]; j += 32) {
-        const float zx = (m.loc[j].x + ox) * ih, zy = (m.loc[j].y + oy) * ih;
-        const float r2 = zx * zx + zy * zy;
-        const float2 w = make_float2(zx / r2, -zy / r2);
-        const float g = m.gam[j];
-        float2 pw = w;
-        for (int k = 0; k < c0; k++) pw = fmul(pw, w);
+      for (int i = 0; i < 2 * kCoefChunk; i++) acc[i] = 0.f;
+      for (int e = 0; e < 8 && X[e] >= 0; e++) {
+        const int d = X[e];
+        const float ox = centre_offset(m.cxf, m.cxl, d, c), oy = centre_offset(m.cyf, m.cyl, d, c);
+        for (int j = m.begin[d] + lane; j < m.end[d]; j += 32) {
+          const float zx = (m.loc[j].x + ox) * ih, zy = (m.loc[j].y + oy) * ih;
+          const float r2 = zx * zx + zy * zy;
+          const float2 w = make_float2(zx / r2, -zy / r2);
+          const float g = m.gam[j];
+          float2 pw = w;
+          for (int k = 0; k < c0; k++) pw = fmul(pw, w);
 #pragma unroll
-        for (int k = 0; k < kCoefChunk; k++) {
-          acc[2 * k] = fmaf(-g, pw.x, acc[2 * k]);
-          acc[2 * k + 1] = fmaf(-g, pw.y, acc[2 * k + 1]);
-          pw = fmul(pw, w);
+          for (int k = 0; k < kCoefChunk; k++) {
+            acc[2 * k] = fmaf(-g, pw.x, acc[2 * k]);
+            acc[2 * k + 1] = fmaf(-g, pw.y, acc[2 * k + 1]);
+            pw = fmul(pw, w);
+          }
         }
       }
+      const float sum = warp_chunk_sum(acc, buf, lane);
+      const int k = c0 + (lane >> 1);
+      if (k < P) m.L[(size_t)c * 2 * P + ((lane & 1) ? P + k : k)] += sum;
     }
-    const float sum = warp_chunk_sum(acc, buf, lane);
-    const int k = c0 + (lane >> 1);
-    if (k < P) m.L[(size_t)c * 2 * P + ((lane & 1) ? P + k : k)] += sum;
   }
 }
 
@@ -2496,7 +2509,7 @@ int mixed_upward(MixedView &m, int depth, const int *lev_off, cudaStream_t s, bo
 }
 
 int mixed_downward(MixedView &m, int depth, const int *lev_off, cudaStream_t s, bool chain) {
-  chained(k_p2l, (int)(((long)m.ncell * 32 + 255) / 256), 256, 0, s)(m);
+  chained(k_p2l, (m.ncell + 8 * kP2lCells - 1) / (8 * kP2lCells), 256, 0, s)(m);
   g_launches.fetch_add(1, std::memory_order_relaxed);
   const size_t tab_bytes = 4 * sizeof(float2) * m.P * m.P;
   if (chain && m.P == 16 && depth > 3 + m.lev0 && launch_chain<false>(m, 3 + m.lev0, depth, s)) {

@@ -58,6 +58,7 @@ static_assert(sizeof(Climb) == sizeof(double2), "the climbing state replaces the
 __global__ void __launch_bounds__(256) k_climb_init(Tree t, int nt) {
   chain_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < t.n) t.icor2[c] = 1.0 / (t.cor[c] * t.cor[c]);  // here, not in the build: mixed solves do not use it
   if (c >= t.ncell) return;
   Climb *climb = reinterpret_cast<Climb *>(t.mac);
   const int4 ch = reinterpret_cast<const int4 *>(t.child)[c];
@@ -531,10 +532,10 @@ cudaError_t mac_bounds(Workspace &ws, const Tree &t, double theta, int nt, cudaS
 
 int plain_upward(Workspace &ws, const Tree &t, const Params &p, cudaStream_t s) {
   const int nt = p.nterms;
-  if (nt <= 0 || t.ncell <= 0) return TREE2D_OK;
+  if (t.ncell <= 0) return TREE2D_OK;
   ws.mac_theta = -1.0;  // the climb uses the bounds' memory
-  chained(k_climb_init, (t.ncell + 255) / 256, 256, 0, s)(t, nt);
-  if (t.nleaf > 0) chained(k_upward, (t.nleaf + 3) / 4, 128, 0, s)(t, nt);
+  chained(k_climb_init, ((t.n > t.ncell ? t.n : t.ncell) + 255) / 256, 256, 0, s)(t, nt);
+  if (t.nleaf > 0 && nt > 0) chained(k_upward, (t.nleaf + 3) / 4, 128, 0, s)(t, nt);
   ::t2d::g_launches.fetch_add(2, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;
