@@ -340,8 +340,9 @@ def _roofline(P, args, mode, b, wname, sts, sp):
         peak = P.fp64_peak_tflops(stream=sp)
         return {"bound": "fp64", "achieved": flops / (ms * 1e-3) / 1e12, "peak": peak, "unit": "TFLOP/s",
                 "frac": flops / (ms * 1e-3) / 1e12 / peak, "traffic": tr,
-                "kernel": "k_eval (traversal + M2S + P2P, FP64)",
-                "peak_source": "measured: the library's DFMA probe (8 independent chains per thread)",
+                "kernel": "k_eval (traversal + M2S + P2P, in 64-bit fixed point)",
+                "peak_source": "measured: the library's DFMA probe (8 independent chains per thread); "
+                               "the fixed-point sums run above it",
                 "algorithmic_flops_per_launch": flops, "ms_per_launch": ms}
     # mixed and learned: the evaluation kernel (direct pairs, correction
     # pairs, L2P, M2P)
