@@ -335,13 +335,15 @@ __device__ __forceinline__ unsigned axis_index(float f, int lt, uint64_t okey_po
 }
 
 // `packed` (at most 16 digits in all): one word per blob, the key in the
-// high 32 bits and the blob's index in the low 32 (vals unused).
+// high 32 bits and the blob's index in the low 32 (vals unused); the sort's
+// counters (`clears` pieces of 16 bytes) are cleared on the way.
 __global__ void __launch_bounds__(256) k_keys(const double *__restrict__ xy, int n, const RootBox *__restrict__ root,
                                               const uint64_t *__restrict__ tab, int tlev, uint64_t *__restrict__ keys,
                                               uint32_t *__restrict__ vals, int levels, const int *__restrict__ set_of,
-                                              int lev0, int packed) {
+                                              int lev0, int packed, uint4 *clear, long clears) {
   chain_wait();
   long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  for (long k = i; k < clears; k += (long)gridDim.x * blockDim.x) clear[k] = make_uint4(0u, 0u, 0u, 0u);
   if (i >= n) return;
   double x = xy[2 * i], y = xy[2 * i + 1];
   int set = 0;
@@ -697,7 +699,7 @@ __global__ void __launch_bounds__(256) k_cell_end(const uint64_t *__restrict__ k
   // first position in (b, n) whose key > hi: seven probes at a time, first 8,
   // 64, ... 2M positions on (most cells are small), then at the eighths of the
   // range.  A bisection of all keys made three times as many dependent loads
-  // (50,000 blobs: 10.4 -> 6.5 us; 22M in 512 sets: 73 -> under 58 us).
+  // (50,000 blobs: 10.4 -> 6.5 us; 22M in 512 sets: 73 -> 43 us).
   int lo = b + 1, up = n;
   for (int step = 0; lo < up; step++) {
     const int w = (up - lo + 7) >> 3, lo0 = lo, up0 = up;
@@ -962,14 +964,18 @@ retry:
   const bool packed = 2 * total_levels <= 32 && n >= 2;
   const int passes = (2 * total_levels + 7) / 8;
   uint64_t *words = packed && (passes & 1) ? keys_alt : t.keys;
-  chained(k_keys, (n + 255) / 256, 256, 0, s)(d_xy, n, t.root, ctab, tlev, words, vals, levels, set_of, lev0,
-                                         packed ? 1 : 0);
+  // a packed sort has no use for vals_alt: its scratch starts there
+  const size_t scratch = Arena::bytes_for(n, 4) + radix_sort_temp_bytes(n);
+  const bool clears = packed && n < (1 << 30);
+  chained(k_keys, (n + 255) / 256, 256, 0, s)(
+      d_xy, n, t.root, ctab, tlev, words, vals, levels, set_of, lev0, packed ? 1 : 0,
+      reinterpret_cast<uint4 *>(vals_alt),
+      clears ? (long)(radix_sort_clear_bytes(n, 64 - 2 * total_levels, scratch) / 16) : 0l);
   ::t2d::g_launches.fetch_add(2, std::memory_order_relaxed);
   // 3. sort
   if (packed)
-    // a packed sort has no use for vals_alt: its scratch starts there
     T2D_CUDA_TRY(radix_sort_packed(words, words == t.keys ? keys_alt : t.keys, n, 64 - 2 * total_levels, t.keys,
-                                   vals, vals_alt, Arena::bytes_for(n, 4) + radix_sort_temp_bytes(n), ws.status, s));
+                                   vals, vals_alt, scratch, ws.status, s, clears));
   else
     T2D_CUDA_TRY(radix_sort_pairs(t.keys, vals, keys_alt, vals_alt, n, 64 - 2 * total_levels, 64, sort_tmp, s));
   t.key_order = vals;

@@ -247,8 +247,12 @@ size_t radix_sort_temp_bytes(int n);
 // records TREE2D_ERR_TIMEOUT in st); without, the reduce-then-scan form.
 // `temp` holds temp_bytes, radix_sort_temp_bytes(n) at least; another 4 n let
 // small sorts use smaller tiles.
+// With st, the passes' counters are the first radix_sort_clear_bytes(...) of
+// temp (a multiple of 16): zero already when `cleared`, else by a memset.
 cudaError_t radix_sort_packed(uint64_t *words, uint64_t *words_alt, int n, int begin_bit, uint64_t *keys_out,
-                              uint32_t *vals_out, void *temp, size_t temp_bytes, DevStatus *st, cudaStream_t s);
+                              uint32_t *vals_out, void *temp, size_t temp_bytes, DevStatus *st, cudaStream_t s,
+                              bool cleared = false);
+size_t radix_sort_clear_bytes(int n, int begin_bit, size_t temp_bytes);
 cudaError_t radix_sort_pairs(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt, uint32_t *vals_alt,
                              int n, int begin_bit, int end_bit, void *temp, cudaStream_t s);
 

@@ -87,7 +87,12 @@ __global__ void __launch_bounds__(256) k_cell_info(MixedView m, unsigned *rc_bit
       for (int i = c; i < nsets; i += blockDim.x) rc_set_bits[i] = 0u;
   }
   if (c >= m.ncell) return;
-  m.parent[c] = -1;
+  if (c == 0) m.parent[0] = -1;
+  if (!m.leaf[c]) {
+    const int4 ch = reinterpret_cast<const int4 *>(m.child)[c];
+    for (int q = 0; q < 4; q++)
+      if ((&ch.x)[q] >= 0) m.parent[(&ch.x)[q]] = c;
+  }
   int lev = m.level[c];
   uint64_t k = m.keys[m.begin[c]];
   unsigned ix = 0, iy = 0;
@@ -467,16 +472,25 @@ __global__ void k_level_hist(MixedView m) {
     if (h[i]) atomicAdd(&m.level_off[i + 1], h[i]);
 }
 
+// One warp: lane l scans level_off[l + 1]; level_off[33] is the last level's.
 __global__ void k_level_scan(MixedView m) {
   chain_wait();
-  if (threadIdx.x != 0) return;
-  int run = 0;
-  for (int l = 0; l <= kKeyLevels; l++) {
-    run += m.level_off[l + 1];
-    m.level_off[l + 1] = run;
-    m.level_off[kKeyLevels + 2 + l] = m.level_off[l];
+  static_assert(kKeyLevels == 32, "a lane per level, and the last one apart");
+  const int lane = threadIdx.x;
+  int x = m.level_off[lane + 1], last = m.level_off[kKeyLevels + 1];
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(0xffffffffu, x, o);
+    if (lane >= o) x += y;
   }
-  for (int l = 0; l < kKeyLevels + 2; l++) m.st->level_off[l] = m.level_off[l];
+  last += __shfl_sync(0xffffffffu, x, 31);
+  const int before = __shfl_up_sync(0xffffffffu, x, 1);
+  m.level_off[lane + 1] = m.st->level_off[lane + 1] = x;
+  m.level_off[kKeyLevels + 2 + lane] = lane ? before : 0;
+  if (lane == 31) {
+    m.level_off[kKeyLevels + 1] = m.st->level_off[kKeyLevels + 1] = last;
+    m.level_off[kKeyLevels + 2 + kKeyLevels] = x;
+    m.st->level_off[0] = 0;
+  }
 }
 
 // One atomic per warp and level: lanes of equal level share a reservation.
@@ -491,16 +505,6 @@ __global__ void k_level_fill(MixedView m) {
   if (lev >= 0 && lane == leader) base = atomicAdd(&m.level_off[kKeyLevels + 2 + lev], __popc(grp));
   base = __shfl_sync(0xffffffffu, base, leader);
   if (lev >= 0) m.by_level[base + __popc(grp & ((1u << lane) - 1u))] = c;
-}
-
-__global__ void k_parent(MixedView m) {
-  chain_wait();
-  int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= m.ncell) return;
-  if (m.leaf[c]) return;
-  const int4 ch = reinterpret_cast<const int4 *>(m.child)[c];
-  for (int q = 0; q < 4; q++)
-    if ((&ch.x)[q] >= 0) m.parent[(&ch.x)[q]] = c;
 }
 
 // Distance between the boxes of cells a and b (FP32: only compared with rc).
@@ -2399,7 +2403,6 @@ int mixed_lists(MixedView &m, cudaStream_t s) {
   chained(k_level_scan, 1, 32, 0, s)(m);
   chained(k_level_fill, cb, 256, 0, s)(m);
   g_launches.fetch_add(3, std::memory_order_relaxed);
-  chained(k_parent, cb, 256, 0, s)(m);
   chained(k_colleagues, (unsigned)((9l * m.ncell + 255) / 256), 256, 0, s)(m);
   chained(k_vx_lists, (int)(((long)m.ncell * 32 + 255) / 256), 256, 0, s)(m);
   if (m.list_scratch)
@@ -2410,7 +2413,7 @@ int mixed_lists(MixedView &m, cudaStream_t s) {
   chained(k_scan3_tiles, ntiles, kScan3Threads, 0, s)(m.u_off, m.w_off, m.k_off, m.nleaf, m.scan_tmp, ntiles);
   chained(k_scan3_sums, 1, 32, 0, s)(m.scan_tmp, ntiles, m.st);
   chained(k_scan3_apply, ntiles, kScan3Threads, 0, s)(m.u_off, m.w_off, m.k_off, m.nleaf, m.scan_tmp, ntiles);
-  g_launches.fetch_add(8, std::memory_order_relaxed);
+  g_launches.fetch_add(7, std::memory_order_relaxed);
   T2D_CUDA_TRY(cudaGetLastError());
   return TREE2D_OK;
 }

@@ -389,6 +389,17 @@ static size_t onesweep_temp_bytes(int n, int tile) {
   return ((size_t)kMaxPasses * kBins + kMaxPasses + (size_t)kMaxPasses * ntiles * kBins) * sizeof(unsigned);
 }
 
+static int onesweep_tile(int n, size_t temp_bytes) {
+  constexpr int kSmallTile = kThreads * kSmallItems;
+  return n <= kSmallSort && onesweep_temp_bytes(n, kSmallTile) <= temp_bytes ? kSmallTile : kTile;
+}
+
+size_t radix_sort_clear_bytes(int n, int begin_bit, size_t temp_bytes) {
+  const int tile = onesweep_tile(n, temp_bytes);
+  const size_t passes = (64 - begin_bit + 7) / 8, ntiles = ((size_t)n + tile - 1) / tile;
+  return ((size_t)kMaxPasses * kBins + kMaxPasses + passes * ntiles * kBins) * sizeof(unsigned);
+}
+
 size_t radix_sort_temp_bytes(int n) {
   long ntiles = (n + kTile - 1) / kTile;
   const size_t classic = (size_t)kBins * (size_t)(ntiles > 0 ? ntiles : 1) * sizeof(unsigned) + kBins * sizeof(unsigned);
@@ -430,21 +441,20 @@ cudaError_t radix_sort_pairs(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt,
 }
 
 cudaError_t radix_sort_packed(uint64_t *words, uint64_t *words_alt, int n, int begin_bit, uint64_t *keys_out,
-                              uint32_t *vals_out, void *temp, size_t temp_bytes, DevStatus *st, cudaStream_t s) {
+                              uint32_t *vals_out, void *temp, size_t temp_bytes, DevStatus *st, cudaStream_t s,
+                              bool cleared) {
   if (begin_bit < 32 || begin_bit >= 64 || n < 2) return cudaErrorInvalidValue;
   const int passes = (64 - begin_bit + 7) / 8;
   uint64_t *ka = words, *kb = words_alt;
   if (n < (1 << 30) && st) {
     // single pass per digit: counts up to 2^30 - 1 fit a status word
-    constexpr int kSmallTile = kThreads * kSmallItems;
-    const bool small = n <= kSmallSort && onesweep_temp_bytes(n, kSmallTile) <= temp_bytes;
-    const int tile = small ? kSmallTile : kTile;
+    const int tile = onesweep_tile(n, temp_bytes);
+    const bool small = tile != kTile;
     const int ntiles = (n + tile - 1) / tile;
     unsigned *hist = static_cast<unsigned *>(temp);
     unsigned *ctr = hist + kMaxPasses * kBins;
     unsigned *status = ctr + kMaxPasses;
-    const size_t zero = ((size_t)kMaxPasses * kBins + kMaxPasses + (size_t)passes * ntiles * kBins) * sizeof(unsigned);
-    cudaError_t e = cudaMemsetAsync(temp, 0, zero, s);
+    cudaError_t e = cleared ? cudaSuccess : cudaMemsetAsync(temp, 0, radix_sort_clear_bytes(n, begin_bit, temp_bytes), s);
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_onesweep<kItems>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStagePackedBytes);
     if (e != cudaSuccess) return e;
