@@ -2536,8 +2536,8 @@ int mixed_downward(MixedView &m, int depth, const int *lev_off, cudaStream_t s, 
 // from global memory with 4/8 warps per block, 2/3 stage them in shared
 // memory by bulk copies with 4/8 warps per block, 4 stages them with 4
 // warps per block of up to 80 registers per thread (6 blocks per SM) and
-// the pair loops unrolled four times.  At 1M Lamb-Oseen blobs 4 is the
-// fastest, at 4M two-patch + sheet blobs 2, for the 512-set batch 0.
+// the pair loops unrolled four times.  The staged ones are within 2% of one
+// another at 1M Lamb-Oseen blobs, 4M two-patch + sheet blobs and the 512 sets.
 constexpr int kEvalVariants = kEvalVariantCount;
 
 // Blocks of a persistent near-field launch: as many as are resident on the
