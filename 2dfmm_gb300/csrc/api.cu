@@ -23,6 +23,7 @@
 #include "dev_common.cuh"
 #include "learn.h"
 #include "mixed.h"
+#include "position_hash.h"
 
 namespace t2d {
 
@@ -357,18 +358,11 @@ int solve_body(Lib &L, Solver &S, int n, const double *d_xy, const double *d_cir
   return TREE2D_OK;
 }
 
-uint64_t mix64(uint64_t x) {
-  x += 0x9e3779b97f4a7c15ull;
-  x = (x ^ (x >> 30)) * 0xbf58476d1ce4e5b9ull;
-  x = (x ^ (x >> 27)) * 0x94d049bb133111ebull;
-  return x ^ (x >> 31);
-}
-
 uint64_t pos_hash(double x, double y) {
   uint64_t a, b;
   std::memcpy(&a, &x, 8);
   std::memcpy(&b, &y, 8);
-  return mix64(a ^ mix64(b));
+  return position_hash(a, b);
 }
 
 bool same_bits(double a, double b) { return std::memcmp(&a, &b, 8) == 0; }

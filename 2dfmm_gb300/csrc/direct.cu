@@ -5,6 +5,7 @@
 // decoded once; one thread per target.
 #include "dev_common.cuh"
 #include "fix64.cuh"
+#include "position_hash.h"
 #include "tc_ptx.cuh"
 
 namespace t2d {
@@ -245,14 +246,8 @@ cudaError_t lookup_blobs(long b, long e, const double *q, long nb, const double 
 
 namespace {
 
-__device__ __forceinline__ uint64_t mix64(uint64_t x) {
-  x += 0x9e3779b97f4a7c15ull;
-  x = (x ^ (x >> 30)) * 0xbf58476d1ce4e5b9ull;
-  x = (x ^ (x >> 27)) * 0x94d049bb133111ebull;
-  return x ^ (x >> 31);
-}
 __device__ __forceinline__ unsigned position_slot(double2 p, unsigned mask) {
-  return (unsigned)mix64((uint64_t)__double_as_longlong(p.x) ^ mix64((uint64_t)__double_as_longlong(p.y))) & mask;
+  return (unsigned)position_hash((uint64_t)__double_as_longlong(p.x), (uint64_t)__double_as_longlong(p.y)) & mask;
 }
 __device__ __forceinline__ bool same_position(double2 a, double2 b) {
   return __double_as_longlong(a.x) == __double_as_longlong(b.x) && __double_as_longlong(a.y) == __double_as_longlong(b.y);
