@@ -302,7 +302,7 @@ int solve_body(Lib &L, Solver &S, int n, const double *d_xy, const double *d_cir
   T2D_CUDA_TRY(cudaEventRecord(ws.ev[1], s));
   S.plain_coef = false;
   if (L.mode == TREE2D_MODE_PLAIN) {
-    rc = plain_upward(ws, S.tree, L.params, s);
+    rc = plain_upward(ws, S.tree, s);
     if (rc) return rc;
     S.plain_coef = true;
     T2D_CUDA_TRY(cudaEventRecord(ws.ev[2], s));
@@ -318,7 +318,7 @@ int solve_body(Lib &L, Solver &S, int n, const double *d_xy, const double *d_cir
     int *kout = S.keyed.take<int>(n);
     rc = gather_targets(n, d_xy, reinterpret_cast<const int *>(S.tree.key_order), ktx, kty, kout, s);
     if (rc) return rc;
-    rc = plain_evaluate(ws, S.tree, L.params, n, ktx, kty, kout, d_uv, s);
+    rc = plain_evaluate(ws, S.tree, n, ktx, kty, kout, d_uv, s);
     if (rc) return rc;
   } else {
     T2D_CUDA_TRY(cudaEventRecord(ws.ev[2], s));
@@ -461,7 +461,7 @@ int eval_device_points(Lib &L, int m, const double *d_xy, double *d_uv) {
   // the mixed tree with its own expansions, to the mixed form's accuracy.
   const bool mixed = S.mixed_ready;
   if (!mixed && !S.plain_coef) {
-    rc = plain_upward(S.ws, S.tree, L.params, s);
+    rc = plain_upward(S.ws, S.tree, s);
     if (rc) return rc;
     S.plain_coef = true;
   }
@@ -475,7 +475,7 @@ int eval_device_points(Lib &L, int m, const double *d_xy, double *d_uv) {
   }
   if (rc) return rc;
   rc = mixed ? mixed_eval_points(S.ws, m, tx, ty, out, d_uv, s)
-             : plain_evaluate(S.ws, S.tree, L.params, m, tx, ty, out, d_uv, s);
+             : plain_evaluate(S.ws, S.tree, m, tx, ty, out, d_uv, s);
   if (rc) return rc;
   T2D_CUDA_TRY(cudaMemcpyAsync(S.ws.h_status, S.ws.status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s));
   T2D_CUDA_TRY(cudaStreamSynchronize(s));
@@ -953,7 +953,7 @@ long long tree2d_export_tree(int *perm, long long cap, int *level, int *begin, i
   long long nc = t.ncell - 1;
   if (cap <= 0) return nc;
   if (cap < nc) return -1;
-  const int nt = t.nterms;
+  const int nt = t.params.nterms;
   if (perm && cudaMemcpy(perm, t.perm, sizeof(int) * (size_t)t.n, cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
   std::vector<unsigned char> lf(nc);
   if (level) cudaMemcpy(level, t.level + 1, sizeof(int) * nc, cudaMemcpyDeviceToHost);

@@ -887,7 +887,7 @@ size_t build_cell_bytes(long long ncell, long long nleaf, int nterms, bool fixed
 int build_tree(Workspace &ws, int n, const double *d_xy, const double *d_cir, const double *d_cor, const Params &p,
                Tree &t, cudaStream_t s, const int *d_set_off, int nsets, cudaEvent_t cir_cor_ready) {
   t.n = n;
-  t.nterms = p.nterms;
+  t.params = p;
   t.leaf_cap = p.num_p - 1;
   const bool batched = nsets > 1;
   int lev0 = 0;  // levels of container cells above the set roots
@@ -1039,7 +1039,7 @@ retry:
   t.mac = ws.cell_arena.take<double2>(ncell);
   t.cf32 = ws.cell_arena.take<float4>(ncell);
   t.macf = ws.cell_arena.take<float2>(ncell);
-  ws.mac_theta = -1.0;
+  ws.mac_ready = false;
 
   // 7. cells
   EmitArgs ea{t.keys, cpl, leaf_level, part, t.root, n, cellbase, t.level, t.begin, t.leaf, t.cx, t.cy, t.region,

@@ -135,7 +135,8 @@ class Arena {
 // depth-first quadrant order, ascending original index inside a leaf);
 // cells in depth-first pre-order with the root at 0.
 struct Tree {
-  int n = 0, ncell = 0, nleaf = 0, depth = 0, nterms = 0;
+  int n = 0, ncell = 0, nleaf = 0, depth = 0;
+  Params params;              // the build's: evaluations of the tree use these, whatever is in force by then
   double *x = nullptr, *y = nullptr, *cir = nullptr, *cor = nullptr;
   double *icor2 = nullptr;    // 1 / cor^2 per blob (tree order), formed by plain_upward
   int *perm = nullptr;        // tree position -> original blob index
@@ -146,7 +147,7 @@ struct Tree {
   int *leaf_cell = nullptr;   // leaf ordinal -> cell id
   int *level_start = nullptr; // host-built cell lists per level (device copy)
   int *by_level = nullptr;    // cell ids grouped by level
-  double2 *coef = nullptr;    // ncell * nterms, FP64 Laurent coefficients
+  double2 *coef = nullptr;    // ncell * params.nterms, FP64 Laurent coefficients
   double2 *mac = nullptr;     // plain: per cell, the squared distances below / above which
                               // the opening test surely descends / accepts (k_mac_bounds)
   long long *fix = nullptr;   // plain: the coefficients in fixed point (fix64.cuh), 2 per entry, strided as coef
@@ -184,7 +185,7 @@ struct Workspace {
   std::map<uint64_t, int> eval_tuned;  // size class -> fastest near-field variant
   std::map<uint64_t, int> m2l_tuned;   // size class -> faster M2L tile rows (64 or 128)
   int last_depth = 0;  // depth of the last tree built (sizes the next keys)
-  double mac_theta = -1.0;  // theta that the tree's Tree::mac bounds were formed for (< 0: none)
+  bool mac_ready = false;  // the tree's Tree::mac bounds (and Tree::fix) are formed
   int list_cap = 256;  // entries per leaf of the one-walk list scratch (from the last solve)
   DevStatus *status = nullptr;   // device
   DevStatus *h_status = nullptr; // pinned host mirror
@@ -257,9 +258,9 @@ cudaError_t radix_sort_pairs(uint64_t *keys, uint32_t *vals, uint64_t *keys_alt,
                              int n, int begin_bit, int end_bit, void *temp, cudaStream_t s);
 
 // --- plain FP64 path (plain.cu) ---------------------------------------
-int plain_upward(Workspace &ws, const Tree &t, const Params &p, cudaStream_t s);
+int plain_upward(Workspace &ws, const Tree &t, cudaStream_t s);
 // Evaluates targets (tx,ty) in the given order, writing uv[2*out_idx[i]].
-int plain_evaluate(Workspace &ws, const Tree &t, const Params &p, int ntgt, const double *tx,
+int plain_evaluate(Workspace &ws, const Tree &t, int ntgt, const double *tx,
                    const double *ty, const int *out_idx, double *uv, cudaStream_t s);
 
 // --- direct sum (direct.cu) -------------------------------------------

@@ -519,21 +519,23 @@ __global__ void k_mac_bounds(Tree t, double theta, int nt, int fixed) {
 // grow with k (fix::cell_scale).  Above it FP64, as before.
 constexpr double kFixTheta = 2.0 * fix::kHalfTheta;
 
-cudaError_t mac_bounds(Workspace &ws, const Tree &t, double theta, int nt, cudaStream_t s) {
-  if (ws.mac_theta == theta || t.ncell <= 0) return cudaSuccess;
-  chained(k_mac_bounds, (t.ncell + 63) / 64, 64, 0, s)(t, theta, nt, theta <= kFixTheta);
+// Once per upward pass: the coefficients may be converted in place.
+cudaError_t mac_bounds(Workspace &ws, const Tree &t, cudaStream_t s) {
+  if (ws.mac_ready || t.ncell <= 0) return cudaSuccess;
+  const Params &p = t.params;
+  chained(k_mac_bounds, (t.ncell + 63) / 64, 64, 0, s)(t, p.theta, p.nterms, p.theta <= kFixTheta);
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   const cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) ws.mac_theta = theta;
+  if (e == cudaSuccess) ws.mac_ready = true;
   return e;
 }
 
 }  // namespace
 
-int plain_upward(Workspace &ws, const Tree &t, const Params &p, cudaStream_t s) {
-  const int nt = p.nterms;
+int plain_upward(Workspace &ws, const Tree &t, cudaStream_t s) {
+  const int nt = t.params.nterms;
   if (t.ncell <= 0) return TREE2D_OK;
-  ws.mac_theta = -1.0;  // the climb uses the bounds' memory
+  ws.mac_ready = false;  // the climb uses the bounds' memory
   chained(k_climb_init, ((t.n > t.ncell ? t.n : t.ncell) + 255) / 256, 256, 0, s)(t, nt);
   if (t.nleaf > 0 && nt > 0) chained(k_upward, (t.nleaf + 3) / 4, 128, 0, s)(t, nt);
   ::t2d::g_launches.fetch_add(2, std::memory_order_relaxed);
@@ -568,10 +570,11 @@ auto eval_kernel(double theta) {
                                    : k_eval<kFormHalf, kShare>;
 }
 
-int plain_evaluate(Workspace &ws, const Tree &t, const Params &p, int ntgt, const double *tx, const double *ty,
-                   const int *out_idx, double *uv, cudaStream_t s) {
+int plain_evaluate(Workspace &ws, const Tree &t, int ntgt, const double *tx, const double *ty, const int *out_idx,
+                   double *uv, cudaStream_t s) {
   if (ntgt <= 0) return TREE2D_OK;
-  T2D_CUDA_TRY(mac_bounds(ws, t, p.theta, p.nterms, s));
+  const Params &p = t.params;
+  T2D_CUDA_TRY(mac_bounds(ws, t, s));
   EvalArgs a{t, p.nterms, p.theta, ntgt, tx, ty, out_idx, uv, ws.status, fix::first_pair_term(p.theta),
              reinterpret_cast<const void *>(t.fix) != reinterpret_cast<const void *>(t.coef), fix::One()};
   const int share = eval_share(t.n, p.num_p);

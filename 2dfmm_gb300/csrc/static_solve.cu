@@ -146,9 +146,9 @@ extern "C" int tree2d_solve_device_static(int n, const double *d_xy, const doubl
     rc = TREE2D_ERR_TOO_LARGE;
   }
   if (rc) return record_error(rc);
-  rc = plain_upward(ws, t, p, s);
+  rc = plain_upward(ws, t, s);
   if (rc) return record_error(rc);
-  rc = plain_evaluate(ws, t, p, n, t.x, t.y, t.perm, d_uv, s);
+  rc = plain_evaluate(ws, t, n, t.x, t.y, t.perm, d_uv, s);
   if (rc) return record_error(rc);
   cudaError_t e = cudaMemcpyAsync(ws.h_status, ws.status, sizeof(DevStatus), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);

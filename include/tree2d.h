@@ -75,7 +75,9 @@ const char *tree2d_error_string(int code);
 
 /* Fixes the parameters (nterms = stored coefficients, num_p = leaf split
  * threshold, theta = opening angle, r_min unused as in the reference) so
- * that make_tree no longer reads the parameter file.  Returns a status. */
+ * that make_tree no longer reads the parameter file.  A tree keeps the ones
+ * it was built with: queries after a change answer by them until the next
+ * make_tree.  Returns a status. */
 int tree2d_set_params(int nterms, int num_p, double theta, double r_min);
 /* Returns make_tree to reading ../cal_cond/fmm_param.dat. */
 void tree2d_clear_params(void);
