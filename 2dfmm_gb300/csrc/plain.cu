@@ -195,7 +195,7 @@ struct EvalArgs {
   double *uv;
   DevStatus *st;
   int k0;        // first term of the sums in FP32 pairs (fix::first_pair_term)
-  bool keep64;   // t.coef still holds the FP64 coefficients (not converted in place)
+  bool keep64;   // t.coef holds every cell's FP64 coefficients (else only those left to FP64: the rest in place of them)
   fix::One one;
 };
 
@@ -499,7 +499,7 @@ __global__ void k_mac_bounds(Tree t, double theta, int nt, int fixed) {
       im = a.y;
     });
     const int k0 = fix::first_pair_term(theta);
-    for (int k = 0; k < nt - 1; k++) {
+    for (int k = 0; k < nt - 1 && sc.es != fix::kLeave; k++) {  // else the FP64 ones stay
       const double2 a = src[k];
       if (nt - 1 > k0 && k >= k0) {
         float4 v;

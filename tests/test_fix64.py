@@ -149,6 +149,60 @@ def test_cell_against_long_double(shim, kind, theta):
             assert (err <= 2.0**-50 * mag + 1e-300).all(), (R, K, float((err / np.maximum(mag, 1e-300)).max()))
 
 
+def cancelling(kind, R):
+    """Blobs whose first moments are exactly zero (dyadic offsets), or zero but
+    for what one more blob adds."""
+    if kind.startswith("line"):  # moments 0 to 2 vanish: third difference
+        p = np.array([[-0.375, 0.0], [-0.125, 0.0], [0.125, 0.0], [0.375, 0.0]])
+        g = np.array([-1.0, 3.0, -3.0, 1.0])
+    else:  # the 4 x 4 tensor product of + - - +
+        c = np.array([-0.375, -0.125, 0.125, 0.375])
+        s = np.array([1.0, -1.0, -1.0, 1.0])
+        p = np.stack(np.meshgrid(c, c), axis=-1).reshape(-1, 2)
+        g = np.outer(s, s).ravel()
+    if "+" in kind:
+        p, g = np.concatenate([p, [[0.25, -0.1875]]]), np.append(g, float(kind.split("+")[1]))
+    return p * R, g
+
+
+@pytest.mark.parametrize("kind", ["line", "square", "line+1e-12", "square+1e-30", "line+1e-200", "square+1e-280"])
+@pytest.mark.parametrize("theta", [0.3, 0.5, 0.7])
+def test_cell_whose_first_moments_cancel(shim, kind, theta):
+    """As test_cell_against_long_double, for cells whose first coefficients
+    vanish or are far below the later ones, over circulation scales and sides:
+    left to FP64, or within the a-priori bound of the FP64 Horner scheme, K
+    complex multiply-adds of 3 2^-53 each (sqrt(5) for the product, 1 for the
+    sum)."""
+    rng = np.random.default_rng(zlib.crc32(f"{kind} {theta}".encode()))
+    L = np.longdouble
+    for R in (1.0, 0.25, 2.0**-20, 3.0):
+        for scale in (1.0, 10.0, 1e-6, 1e20):
+            p, g = cancelling(kind, R)
+            g = g * scale
+            z = p[:, 0] + 1j * p[:, 1]
+            for K in (4, 5, 8, 10, 12, 20, 31):
+                a = np.zeros(K, complex)
+                pw = np.ones(len(z), complex)
+                for k in range(K):
+                    a[k] = complex(math.fsum((g * pw).real), math.fsum((g * pw).imag))
+                    pw = pw * z
+                n = 200
+                d = R / theta * np.exp(np.concatenate([rng.uniform(0, 1e-6, 50), rng.uniform(0, 1.1, n - 50)])) * (1 + 1e-14)
+                t = rng.uniform(-math.pi, math.pi, n)
+                dx, dy = d * np.cos(t), d * np.sin(t)
+                ab, out = np.ascontiguousarray(np.stack([a.real, a.imag], axis=1)), np.empty((n, 2))
+                shim.cell_terms(K, dp(ab), ctypes.c_double(R), ctypes.c_double(theta), n, dp(dx), dp(dy), dp(out))
+                w = (L(1) * dx - 1j * (L(1) * dy)) / (L(1) * dx * dx + L(1) * dy * dy)
+                s, mag, pw = np.zeros(n, np.clongdouble), np.zeros(n), w
+                for k in range(K):
+                    s = s + (L(1) * a[k].real + 1j * (L(1) * a[k].imag)) * pw
+                    mag += np.abs(a[k]) * np.abs(pw).astype(float)
+                    pw = pw * w
+                err = np.abs((out[:, 0] + 1j * out[:, 1]) - s).astype(float)
+                err[np.isnan(err)] = 0.0  # left to FP64
+                assert (err <= 3 * K * 2.0**-53 * mag + 1e-300).all(), (R, scale, K, float((err / np.maximum(mag, 1e-300)).max()))
+
+
 @pytest.mark.parametrize("span", [0, 6, 40, 200])
 def test_running_sum_is_exact_to_its_unit(shim, span):
     """Terms of exponents spread over `span` bits, in growing, falling and
@@ -200,3 +254,45 @@ def test_velocity_around_the_forms_limits(gpu_lib, theta, nterms, n, num_p):
     ref = o.biot(t)
     o.close()
     assert_parity(uv, ref, t, ext_for(b.xy, b.cir, b.cor, nterms, num_p, float(theta)), label=f"{theta} {nterms} {n}")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("theta", [0.3, 0.5, 0.7])
+def test_velocity_of_cancelling_clusters(gpu_lib, theta):
+    """A field of clusters whose first three moments vanish, so that every
+    cell's leading coefficients are rounding residues: blobs and far points
+    against the oracle, and the static solve (whose converted coefficients
+    take the place of the FP64 ones) bit for bit with the allocating one."""
+    torch = pytest.importorskip("torch")
+    from conftest import oracle
+    P = gpu_lib
+    rng = np.random.default_rng(9)
+    q, g = cancelling("line", 2.0**-8)
+    at = rng.permutation(64 * 64)[:500]
+    xy = (np.stack([at % 64, at // 64], axis=1)[:, None, :] / 64.0 + q).reshape(-1, 2)
+    cir = np.tile(g, 500)
+    cor = np.full(len(xy), 2e-3)
+    P.set_params(12, 33, theta)
+    P.set_mode(P.MODE_PLAIN)
+    try:
+        P.make_tree(xy, cir, cor)
+        pts = np.concatenate([xy, rng.uniform(-0.2, 1.2, (200, 2))])
+        uv = P.biot_tree_batch(pts)
+        d = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (xy, cir, cor)]
+        out = torch.empty_like(d[0])
+        assert P.solve_device_static(d[0].data_ptr(), d[1].data_ptr(), d[2].data_ptr(), out.data_ptr(), len(xy)) == P.OK
+        torch.cuda.synchronize()
+        assert np.array_equal(out.cpu().numpy().view(np.uint64), uv[: len(xy)].copy().view(np.uint64))
+    finally:
+        P.clear_params()
+    o = oracle().SparseOracle(12, 33, float(theta))
+    o.make_tree(xy, cir, cor)
+    ref = o.biot(pts)
+    o.close()
+    # What cancels leaves the roundings of the moments, 8 (k + 1) levels 2^-53
+    # of sum |G| (1.5 R)^k each (test_coefficients_are_the_cells_moments): at
+    # R <= 0.7 |d| and 6 levels some 2^-41 of the point vortices' speeds
+    r = np.hypot(pts[:, None, 0] - xy[:, 0], pts[:, None, 1] - xy[:, 1])
+    with np.errstate(divide="ignore"):
+        speed = np.where(r > 0, np.abs(cir) / r, 0.0).sum(axis=1) / (2 * math.pi)
+    assert (np.abs(uv - ref) <= 2.0**-41 * speed[:, None]).all()
