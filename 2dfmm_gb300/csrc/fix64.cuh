@@ -186,13 +186,17 @@ T2D_HD uint64_t recip(uint64_t m, One one) {
 
 // m 2^(e - 1075 - 10) to the nearest double (ties up), for m < 2^63 and e the
 // exponent field of a double with its leading one at m's bit 62; `sign` is
-// its sign bit.  0 on underflow, infinity on overflow.
+// its sign bit.  Infinity on overflow.
 T2D_HD double pack(uint64_t m, int e, uint64_t sign) {
   const int z = clz(m);
   e += 1 - z;
   m = m << (z & 63);  // leading one at bit 63
   uint64_t u = ((uint64_t)(uint32_t)(e - 1) << 52) + (m >> 11) + ((m >> 10) & 1);
-  if (e <= 0 || z == 64) u = 0;
+  if (e <= 0) {  // subnormal
+    const uint64_t h = shr(m, 11 - e);
+    u = (h >> 1) + (h & 1);
+  }
+  if (z == 64) u = 0;
   if (e > 0x7fe && z < 64) u = 0x7ff0000000000000ull;
   return from_bits(u | sign);
 }
@@ -554,6 +558,11 @@ T2D_HD int ilog2(double v) {
   const int e = (int)(bits(v) >> 52) & 0x7ff;
   return e ? e - 1023 : kNoLog;
 }
+// v is an infinity, a NaN or subnormal
+T2D_HD bool beyond(double v) {
+  const uint32_t e = (uint32_t)(bits(v) >> 52) & 0x7ffu;
+  return e == 0x7ffu || (e == 0 && (bits(v) << 1) != 0);
+}
 // 2^e |m| in FP32 for m = v 2^-ilog2(v), 0 below 2^-120, 2^120 above that
 T2D_HD float mag32(double v, int e) {
   if (ilog2(v) == kNoLog || e < -120) return 0.0f;
@@ -590,7 +599,9 @@ T2D_HD double scale_frac(double v) { return from_bits((bits(v) & 0x800ffffffffff
 // farther out, where the sums' measured mean error passes FP64's (2^-51.7
 // against 2^-51.7; at 2^-49: 2^-49.5 against 2^-51.6).  Ordinary cells (1 to
 // 64 random blobs of random signs) stay below 2^-50.8; moments 0 and 1
-// cancelled to about 2^-8 pass it.
+// cancelled to about 2^-8 pass it.  So is a cell with an infinity, a NaN or a
+// subnormal number among its coefficients (circulations or coordinates near
+// the ends of FP64's range).
 template <class Load>
 T2D_HD CellScale cell_scale(int K, double R, double theta, Load load) {
   const int er = ilog2(R);
@@ -600,13 +611,20 @@ T2D_HD CellScale cell_scale(int K, double R, double theta, Load load) {
     const int a = ilog2(re), b = ilog2(im);
     return a > b ? a : b;
   };
+  CellScale sc;
   int lead = kNoLog;
-  for (int k = 0; k < K && (k < 3 || lead == kNoLog); k++) {
+  for (int k = 0; k < K; k++) {
+    double re, im;
+    load(k, re, im);
+    if (beyond(re) || beyond(im)) {
+      sc.es = kLeave;
+      sc.eb = 0;
+      return sc;
+    }
     const int a = log_of(k), l = a - k * (er - 1);
-    if (a > kNoLog && l > lead) lead = l;
+    if ((k < 3 || lead == kNoLog) && a > kNoLog && l > lead) lead = l;
   }
   const int cap = theta > 0.0 ? ilog2(R / (theta <= kHalfTheta ? 2.0 * theta : theta) * (1.0 - 0x1p-20)) : er;
-  CellScale sc;
   sc.es = cap - 1;
   sc.eb = 0;
   if (lead == kNoLog) return sc;

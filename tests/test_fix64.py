@@ -203,6 +203,44 @@ def test_cell_whose_first_moments_cancel(shim, kind, theta):
                 assert (err <= 3 * K * 2.0**-53 * mag + 1e-300).all(), (R, scale, K, float((err / np.maximum(mag, 1e-300)).max()))
 
 
+@pytest.mark.parametrize("scale", [1e-290, 1e-300, 1e-306, 1e-315, 1e290, 1e300, 1e306])
+@pytest.mark.parametrize("R", [1e-3, 1.0, 1e3, 1e30])
+@pytest.mark.parametrize("theta", [0.35, 0.5, 0.7])
+def test_cell_near_the_ends_of_the_range(shim, scale, R, theta):
+    """Circulations and sides whose higher moments leave FP64's normal range:
+    such a cell is left to FP64, never summed without those moments."""
+    rng = np.random.default_rng(11)
+    p, g = rng.uniform(-0.5, 0.5, (5, 2)), rng.uniform(0.5, 1.0, 5)
+    z = (p[:, 0] + 1j * p[:, 1]) * R
+    K, n = 12, 50
+    with np.errstate(all="ignore"):
+        a = np.array([((g * scale) * z**k).sum() for k in range(K)])
+    d = R / theta * np.exp(rng.uniform(0, 1, n)) * (1 + 1e-14)
+    t = rng.uniform(-math.pi, math.pi, n)
+    dx, dy = d * np.cos(t), d * np.sin(t)
+    ab, out = np.ascontiguousarray(np.stack([a.real, a.imag], axis=1)), np.empty((n, 2))
+    shim.cell_terms(K, dp(ab), ctypes.c_double(R), ctypes.c_double(theta), n, dp(dx), dp(dy), dp(out))
+    size = np.abs(ab[ab != 0])
+    if not np.isfinite(ab).all() or (size < np.finfo(float).tiny).any():
+        assert np.isnan(out).all()
+        return
+    # the exact sum at unit scale: sum_j g_j / (z - z_j) up to order K
+    L = np.clongdouble
+    w = 1 / (L(dx) + 1j * L(dy))
+    s, pw = np.zeros(n, L), w
+    for k in range(K):
+        s, pw = s + (L(g) * L(z / R) ** k).sum() * pw * np.longdouble(R) ** k, pw * w
+    s = s * np.longdouble(scale)
+    # coefficients rounded in FP64 (k + 1 products) and the sum's own 2^-50; results
+    # beyond the largest number are infinite, those below the smallest normal
+    # one to its unit
+    for got, exact in ((out[:, 0], s.real), (out[:, 1], s.imag)):
+        large = np.abs(exact) >= np.finfo(float).max
+        assert np.isinf(got[large]).all()
+        err = np.abs(got[~large] - exact[~large])
+        assert (err <= 2.0**-47 * np.abs(s[~large]) + np.longdouble(2.0**-1074)).all()
+
+
 @pytest.mark.parametrize("span", [0, 6, 40, 200])
 def test_running_sum_is_exact_to_its_unit(shim, span):
     """Terms of exponents spread over `span` bits, in growing, falling and
@@ -296,3 +334,34 @@ def test_velocity_of_cancelling_clusters(gpu_lib, theta):
     with np.errstate(divide="ignore"):
         speed = np.where(r > 0, np.abs(cir) / r, 0.0).sum(axis=1) / (2 * math.pi)
     assert (np.abs(uv - ref) <= 2.0**-41 * speed[:, None]).all()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("size,strength", [(0.05, 3001e-290), (1.0, 1e290), (1e30, 1e-100)])
+def test_velocity_near_the_ends_of_the_range(gpu_lib, size, strength):
+    """Sets whose smaller cells' higher moments are subnormal (to 2^-35 of
+    themselves at least), or whose larger ones' are near the top of the range,
+    against the oracle; the static solve bit for bit with the allocating one."""
+    torch = pytest.importorskip("torch")
+    from conftest import oracle, workloads
+    P = gpu_lib
+    b = workloads().uniform(3001, seed=13)
+    xy, cir, cor = b.xy * size, b.cir * strength, b.cor * size
+    P.set_params(11, 33, 0.5)
+    P.set_mode(P.MODE_PLAIN)
+    try:
+        P.make_tree(xy, cir, cor)
+        uv = P.biot_tree_batch(xy)
+        d = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (xy, cir, cor)]
+        out = torch.empty_like(d[0])
+        assert P.solve_device_static(d[0].data_ptr(), d[1].data_ptr(), d[2].data_ptr(), out.data_ptr(), len(xy)) == P.OK
+        torch.cuda.synchronize()
+    finally:
+        P.clear_params()
+    assert np.array_equal(out.cpu().numpy().view(np.uint64), uv.view(np.uint64))
+    o = oracle().SparseOracle(11, 33, 0.5)
+    o.make_tree(xy, cir, cor)
+    ref = o.biot(xy)
+    o.close()
+    assert np.isfinite(uv).all()
+    assert np.abs(uv - ref).max() <= 1e-12 * np.abs(ref).max()
