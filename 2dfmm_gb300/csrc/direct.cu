@@ -56,7 +56,7 @@ __device__ __noinline__ void pair64(double rx, double ry, double g, double rc, d
 // grid.y splits the sources into chunks; each block adds its partial sums
 // into uv (zeroed by the caller) with FP64 atomics.  Bound by the dispatch of
 // integer instructions (two cycles each): 16,384 targets x 262,144 two-patch
-// sources take 32 ms, 125 ms with the pairs in FP64.
+// sources take 26.2 ms, 125 ms with the pairs in FP64.
 __global__ void __launch_bounds__(kThreads) k_direct(int ntgt, const double *__restrict__ txy, int nsrc,
                                                      const double *__restrict__ sxy, const double *__restrict__ cir,
                                                      const double *__restrict__ cor, double *__restrict__ uv, int chunk,
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(kThreads) k_direct(int ntgt, const double *__r
   const double x = valid ? txy[2 * i] : 0.0, y = valid ? txy[2 * i + 1] : 0.0;
   int odd_target = !isfinite(x) || !isfinite(y);
   asm volatile("" : "+r"(odd_target));  // once: not as two FP64 comparisons per pair
-  fix::Sum2 sum;
+  fix::SumXY sum;
   double ax = 0.0, ay = 0.0;  // the FP64 pairs
   const int s0 = blockIdx.y * chunk;
   const int s1 = min(nsrc, s0 + chunk);
@@ -110,8 +110,8 @@ __global__ void __launch_bounds__(kThreads) k_direct(int ntgt, const double *__r
     }
   }
   if (valid) {
-    ax += fix::to_double(sum.x, sum.xl, sum.e);
-    ay += fix::to_double(sum.y, sum.yl, sum.e);
+    ax += fix::to_double(sum.x.v, sum.x.l, sum.x.e);
+    ay += fix::to_double(sum.y.v, sum.y.l, sum.y.e);
     atomicAdd(&uv[2 * i], 0.5 * ax / kPi);
     atomicAdd(&uv[2 * i + 1], 0.5 * ay / kPi);
   }

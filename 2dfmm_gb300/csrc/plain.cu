@@ -222,6 +222,7 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
   __shared__ int s_cell[kEvalWarps][kStackCap];
   __shared__ unsigned s_mask[kEvalWarps][kStackCap];
   __shared__ int s_queue[kEvalWarps][kEvalTargets][kQueue];
+  __shared__ double2 s_far64[kForm == kFormFp64 ? 1 : kEvalWarps * 32];
   __shared__ uint64_t s_exp_int[fix::kExpInts], s_exp_frac[fix::kExpFracs];
   for (int j = threadIdx.x; j < fix::kExpFracs; j += kEvalWarps * 32) s_exp_frac[j] = g_exp.fracs[j];
   for (int j = threadIdx.x; j < fix::kExpInts; j += kEvalWarps * 32) s_exp_int[j] = g_exp.ints[j];
@@ -240,8 +241,13 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
   const float xh = __double2float_rn(x), yh = __double2float_rn(y);
   const float xl = __double2float_rn(x - (double)xh), yl = __double2float_rn(y - (double)yh);
   const float sxy = __fadd_rn(fabsf(xh), fabsf(yh));
-  fix::Sum2 far, near;                          // this lane's share of the target's sums
-  double2 far64 = make_double2(0.0, 0.0);       // kFormFp64, and targets far outside the blobs
+  fix::Sum2 far;                                // this lane's share of the target's sums
+  fix::SumXY near;
+  // The FP64 multipole sums: all in kFormFp64, else few (cells and targets left
+  // to FP64), in shared memory to leave the registers to the pairs.
+  double2 far64_reg = make_double2(0.0, 0.0);
+  double2 &far64 = kForm == kFormFp64 ? far64_reg : s_far64[kForm == kFormFp64 ? 0 : threadIdx.x];
+  if (kForm != kFormFp64) far64 = make_double2(0.0, 0.0);
   unsigned n_m2s = 0;
   unsigned long long n_pairs = 0;
   bool overflow = false;
@@ -433,7 +439,7 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
                                    : make_double2(0.0, 0.0);
   phi.x = __dadd_rn(phi.x, far64.x);
   phi.y = __dadd_rn(phi.y, far64.y);
-  double2 dir = make_double2(fix::to_double(near.x, near.xl, near.e), fix::to_double(near.y, near.yl, near.e));
+  double2 dir = make_double2(fix::to_double(near.x.v, near.x.l, near.x.e), fix::to_double(near.y.v, near.y.l, near.y.e));
   for (int o = 1; o < kShare; o <<= 1) {
     phi.x = __dadd_rn(phi.x, __shfl_xor_sync(0xffffffffu, phi.x, o));
     phi.y = __dadd_rn(phi.y, __shfl_xor_sync(0xffffffffu, phi.y, o));
