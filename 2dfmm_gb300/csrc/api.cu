@@ -278,10 +278,9 @@ int solve(Lib &L, Solver &S, int n, const double *d_xy, const double *d_cir, con
   return TREE2D_OK;
 }
 
-int solve_body(Lib &L, Solver &S, int n, const double *d_xy, const double *d_cir, const double *d_cor,
-               double *d_uv, cudaStream_t s, tree2d_stats_t &st, const int *d_set_off, int nsets,
-               cudaEvent_t cir_cor_ready) {
-  T2D_CUDA_TRY(workspace_init(S.ws));
+int solve_steps(Lib &L, Solver &S, int n, const double *d_xy, const double *d_cir, const double *d_cor,
+                double *d_uv, cudaStream_t s, tree2d_stats_t &st, const int *d_set_off, int nsets,
+                cudaEvent_t cir_cor_ready) {
   std::memset(&st, 0, sizeof(st));
   st.n_blobs = n;
   st.mode = L.mode;
@@ -356,6 +355,20 @@ int solve_body(Lib &L, Solver &S, int n, const double *d_xy, const double *d_cir
   st.n_launches = g_launches.load() - launches0;
   st.m2l_path = m2l_path;
   return TREE2D_OK;
+}
+
+// A solve that fails may have kernels in flight on any of its streams: it
+// returns when they are done, as a solve that succeeds does, so that the next
+// one, on another stream, finds the buffers idle.
+int solve_body(Lib &L, Solver &S, int n, const double *d_xy, const double *d_cir, const double *d_cor,
+               double *d_uv, cudaStream_t s, tree2d_stats_t &st, const int *d_set_off, int nsets,
+               cudaEvent_t cir_cor_ready) {
+  T2D_CUDA_TRY(workspace_init(S.ws));
+  const int rc = solve_steps(L, S, n, d_xy, d_cir, d_cor, d_uv, s, st, d_set_off, nsets, cir_cor_ready);
+  if (rc) {
+    for (cudaStream_t q : {s, S.ws.side, S.ws.hi}) cudaStreamSynchronize(q);
+  }
+  return rc;
 }
 
 uint64_t pos_hash(double x, double y) {

@@ -2919,24 +2919,6 @@ int mixed_solve(Workspace &ws, const Tree &t, const MixedParams &mp, double *d_u
   st.n_list_k_blobs = (long long)ws.h_status->k_blobs;
   unsigned char *u_dec = nullptr, *k_dec = nullptr, *w_dec = nullptr;
   const bool side = learned || mp.learned;
-  // after the fork, an early return first waits for the second stream, so
-  // that no kernel of this solve still runs when its buffers are reused
-  bool forked = false;
-  auto drain = [&](int code) {
-    if (forked) {
-      cudaStreamSynchronize(ws.side);
-      cudaStreamSynchronize(ws.hi);
-    }
-    return code;
-  };
-#define T2D_TRY_DRAIN(expr)                 \
-  do {                                      \
-    cudaError_t e_ = (expr);                \
-    if (e_ != cudaSuccess) {                \
-      note_cuda_error(e_, #expr);           \
-      return drain(TREE2D_ERR_CUDA);        \
-    }                                       \
-  } while (0)
   if (side) {
     // leaf statistics and u_ref (also used by sampling), then decisions
     const size_t wim = learn_weight_image_elems();
@@ -2967,25 +2949,23 @@ int mixed_solve(Workspace &ws, const Tree &t, const MixedParams &mp, double *d_u
     cudaStream_t s2 = ws.side;
     T2D_CUDA_TRY(cudaEventRecord(ws.fork_ev, s));
     T2D_CUDA_TRY(cudaStreamWaitEvent(s2, ws.fork_ev, 0));
-    forked = true;
     rc = learned_leaf_stats(m, stats, s2);
-    if (rc) return drain(rc);
+    if (rc) return rc;
     rc = t.nsets > 1 ? learned_uref_sets(m, stats, t.root, t.nsets, set_lo, set_hi, uref, s2)
                      : learned_uref(m, stats, t.root, uref, s2);
-    if (rc) return drain(rc);
+    if (rc) return rc;
     if (learned) {
       rc = learned_decide(m, stats, uref, wimg, bias, mp.lp->direct_bias, tot[0], tot[2], tot[1], u_dec, k_dec,
                           w_dec, s2);
-      if (rc) return drain(rc);
+      if (rc) return rc;
     }
-    T2D_TRY_DRAIN(schedule(s2));
-    T2D_TRY_DRAIN(cudaEventRecord(ws.join_ev, s2));
+    T2D_CUDA_TRY(schedule(s2));
+    T2D_CUDA_TRY(cudaEventRecord(ws.join_ev, s2));
   } else {
     T2D_CUDA_TRY(cudaEventRecord(ws.fork_ev, s));
     T2D_CUDA_TRY(cudaStreamWaitEvent(ws.side, ws.fork_ev, 0));
-    forked = true;
-    T2D_TRY_DRAIN(schedule(ws.side));
-    T2D_TRY_DRAIN(cudaEventRecord(ws.join_ev, ws.side));
+    T2D_CUDA_TRY(schedule(ws.side));
+    T2D_CUDA_TRY(cudaEventRecord(ws.join_ev, ws.side));
   }
   // Beside the decisions, the expansions run on the highest-priority
   // stream: their chain of short per-level kernels is the critical path,
@@ -2993,29 +2973,28 @@ int mixed_solve(Workspace &ws, const Tree &t, const MixedParams &mp, double *d_u
   // around it instead of holding them.
   cudaStream_t su = s;
   if (side) {
-    T2D_TRY_DRAIN(cudaEventRecord(ws.hi_fork, s));
-    T2D_TRY_DRAIN(cudaStreamWaitEvent(ws.hi, ws.hi_fork, 0));
+    T2D_CUDA_TRY(cudaEventRecord(ws.hi_fork, s));
+    T2D_CUDA_TRY(cudaStreamWaitEvent(ws.hi, ws.hi_fork, 0));
     su = ws.hi;
   }
   rc = mixed_upward(m, t.depth, ws.h_levels, su, mp.level_chain != 0);
-  if (rc) return drain(rc);
+  if (rc) return rc;
   rc = tc ? m2l_tc_tuned(ws, mp, m, dimg, cls_list, cls_count, su, st) : m2l_cuda_cores(m, dm2l, su);
-  if (rc) return drain(rc);
+  if (rc) return rc;
   st.m2l_path = tc ? 2 : 1;
   rc = mixed_downward(m, t.depth, ws.h_levels, su, mp.level_chain != 0);
-  if (rc) return drain(rc);
+  if (rc) return rc;
   if (side) {
-    T2D_TRY_DRAIN(cudaEventRecord(ws.hi_join, ws.hi));
-    T2D_TRY_DRAIN(cudaStreamWaitEvent(s, ws.hi_join, 0));
+    T2D_CUDA_TRY(cudaEventRecord(ws.hi_join, ws.hi));
+    T2D_CUDA_TRY(cudaStreamWaitEvent(s, ws.hi_join, 0));
   }
-  T2D_TRY_DRAIN(cudaStreamWaitEvent(s, ws.join_ev, 0));
+  T2D_CUDA_TRY(cudaStreamWaitEvent(s, ws.join_ev, 0));
   T2D_CUDA_TRY(cudaEventRecord(ws.ev[4], s));
   const Decisions dec = learned ? Decisions{u_dec, k_dec, mp.lp->order_margin, w_dec}
                                 : Decisions{nullptr, nullptr, 0, nullptr};
   rc = near_field(ws, mp, m, learned, dec, d_uv, m.mperm, s, st);
   if (rc) return rc;
   T2D_CUDA_TRY(cudaEventRecord(ws.ev[5], s));
-#undef T2D_TRY_DRAIN
   return TREE2D_OK;
 }
 
