@@ -870,14 +870,14 @@ size_t build_tmp_bytes(int n, int nsets) {
   return tneed;
 }
 
-size_t build_cell_bytes(long long ncell, long long nleaf, int nterms, bool fixed_arena) {
+size_t build_cell_bytes(long long ncell, long long nleaf, int nterms) {
   size_t cneed = 0;
   cneed += Arena::bytes_for(ncell, 4) * 3;           // level begin end
   cneed += Arena::bytes_for(ncell * 4, 4);           // child
   cneed += Arena::bytes_for(ncell, 1);               // leaf
   cneed += Arena::bytes_for(ncell, 8) * 3;           // cx cy region
   cneed += Arena::bytes_for(nleaf > 0 ? nleaf : 1, 4);  // leaf_cell
-  cneed += Arena::bytes_for(ncell * nterms, 16) * (fixed_arena ? 1 : 2);  // coef, fix
+  cneed += Arena::bytes_for(ncell * nterms, 16);     // coef
   cneed += Arena::bytes_for(ncell, 16);              // mac
   cneed += Arena::bytes_for(ncell, 16);              // cf32
   cneed += Arena::bytes_for(ncell, 8);               // macf
@@ -1023,7 +1023,7 @@ retry:
   const int nt = p.nterms;
 
   // ---- cell-sized buffers
-  T2D_CUDA_TRY(ws.cell_arena.reserve(build_cell_bytes(ncell, nleaf, nt, ws.cell_arena.fixed())));
+  T2D_CUDA_TRY(ws.cell_arena.reserve(build_cell_bytes(ncell, nleaf, nt)));
   ws.cell_arena.reset();
   t.level = ws.cell_arena.take<int>(ncell);
   t.begin = ws.cell_arena.take<int>(ncell);
@@ -1035,7 +1035,6 @@ retry:
   t.region = ws.cell_arena.take<double>(ncell);
   t.leaf_cell = ws.cell_arena.take<int>(nleaf > 0 ? nleaf : 1);
   t.coef = ws.cell_arena.take<double2>(ncell * nt);
-  t.fix = ws.cell_arena.fixed() ? reinterpret_cast<long long *>(t.coef) : ws.cell_arena.take<long long>(2 * ncell * nt);
   t.mac = ws.cell_arena.take<double2>(ncell);
   t.cf32 = ws.cell_arena.take<float4>(ncell);
   t.macf = ws.cell_arena.take<float2>(ncell);

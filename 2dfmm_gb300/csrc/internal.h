@@ -150,8 +150,6 @@ struct Tree {
   double2 *coef = nullptr;    // ncell * params.nterms, FP64 Laurent coefficients
   double2 *mac = nullptr;     // plain: per cell, the squared distances below / above which
                               // the opening test surely descends / accepts (k_mac_bounds)
-  long long *fix = nullptr;   // plain: the coefficients in fixed point (fix64.cuh), 2 per entry, strided as coef
-                              // (coef's own memory in arenas of a fixed size)
   float4 *cf32 = nullptr;     // plain: per cell, the centre as FP32 pairs (cx hi, cx lo, cy hi, cy lo)
   float2 *macf = nullptr;     // plain: mac rounded outwards to FP32 (-1 / +inf where that is unsafe)
   RootBox *root = nullptr;    // device
@@ -185,7 +183,10 @@ struct Workspace {
   std::map<uint64_t, int> eval_tuned;  // size class -> fastest near-field variant
   std::map<uint64_t, int> m2l_tuned;   // size class -> faster M2L tile rows (64 or 128)
   int last_depth = 0;  // depth of the last tree built (sizes the next keys)
-  bool mac_ready = false;  // the tree's Tree::mac bounds (and Tree::fix) are formed
+  bool mac_ready = false;  // the tree's Tree::mac bounds (and fix) are formed
+  Arena fix_arena;         // plain: the coefficients in fixed point; reserved when first needed
+  long long *fix = nullptr;  // 2 per entry (fix64.cuh), strided as Tree::coef; Tree::coef's own memory where
+                             // the arenas have a fixed size; null: FP64 sums
   int list_cap = 256;  // entries per leaf of the one-walk list scratch (from the last solve)
   DevStatus *status = nullptr;   // device
   DevStatus *h_status = nullptr; // pinned host mirror
@@ -218,9 +219,8 @@ int build_tree(Workspace &ws, int n, const double *d_xy, const double *d_cir, co
 size_t build_blob_bytes(int n, int nsets);
 size_t build_tmp_bytes(int n, int nsets);
 // Bytes build_tree reserves in ws.cell_arena for a tree of ncell cells and
-// nleaf leaves with nterms coefficients per cell (in an arena of a fixed
-// size the plain form's fixed-point coefficients replace the FP64 ones).
-size_t build_cell_bytes(long long ncell, long long nleaf, int nterms, bool fixed_arena);
+// nleaf leaves with nterms coefficients per cell.
+size_t build_cell_bytes(long long ncell, long long nleaf, int nterms);
 
 // Arbitrary points in Morton order of the root box (to about one point per
 // cell; points outside it at its edge): order[i] = index of the i-th.

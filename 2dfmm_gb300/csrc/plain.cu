@@ -194,6 +194,7 @@ struct EvalArgs {
   const int *out_idx;
   double *uv;
   DevStatus *st;
+  const longlong2 *fix;  // the coefficients in fixed point (kFormFp64: null)
   int k0;        // first term of the sums in FP32 pairs (fix::first_pair_term)
   bool keep64;   // t.coef holds every cell's FP64 coefficients (else only those left to FP64: the rest in place of them)
   fix::One one;
@@ -282,7 +283,7 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
         const double dy = fix::minus(y, t.cy[cc]);
         bool done = false;
         if constexpr (kForm != kFormFp64) {
-          const longlong2 *cf = reinterpret_cast<const longlong2 *>(t.fix) + (size_t)cc * nt;
+          const longlong2 *cf = a.fix + (size_t)cc * nt;
           const longlong2 sc = __ldg(cf + (nt - 1));
           done = fix::add_multipole<kForm == kFormHalf>(
               far, dx, dy, fix::CellScale{(int)sc.x, (int)sc.y}, nt - 1, a.k0,
@@ -480,7 +481,7 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
 // nearest float, lo = the rest, rounded) and the bounds rounded outwards to
 // FP32; a lower bound below 1e-30 becomes -1 and an upper one below 1e-30
 // +inf (no sure answer: the FP32 error bound does not cover subnormals).
-__global__ void k_mac_bounds(Tree t, double theta, int nt, int fixed) {
+__global__ void k_mac_bounds(Tree t, double theta, int nt, longlong2 *fixed) {
   chain_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= t.ncell) return;
@@ -493,12 +494,12 @@ __global__ void k_mac_bounds(Tree t, double theta, int nt, int fixed) {
   t.cf32[c] = make_float4(cxh, __double2float_rn(cx - (double)cxh), cyh, __double2float_rn(cy - (double)cyh));
   t.macf[c] = make_float2(mb.x >= 1e-30 ? __double2float_rd(mb.x) : -1.0f,
                           mb.y >= 1e-30 ? __double2float_ru(mb.y) : INFINITY);
-  if (fixed && nt >= 2) {
+  if (fixed) {
     // The coefficients in fixed point, the cell's scale in the last entry
-    // (whose a_k the sums do not use).  t.fix may be t.coef: a thread has
+    // (whose a_k the sums do not use).  `fixed` may be t.coef: a thread has
     // read what it needs of its cell before it writes entry k.
     const double2 *src = t.coef + (size_t)c * nt;
-    longlong2 *dst = reinterpret_cast<longlong2 *>(t.fix) + (size_t)c * nt;
+    longlong2 *dst = fixed + (size_t)c * nt;
     const fix::CellScale sc = fix::cell_scale(nt - 1, t.region[c], theta, [&](int k, double &re, double &im) {
       const double2 a = src[k];
       re = a.x;
@@ -529,7 +530,19 @@ constexpr double kFixTheta = 2.0 * fix::kHalfTheta;
 cudaError_t mac_bounds(Workspace &ws, const Tree &t, cudaStream_t s) {
   if (ws.mac_ready || t.ncell <= 0) return cudaSuccess;
   const Params &p = t.params;
-  chained(k_mac_bounds, (t.ncell + 63) / 64, 64, 0, s)(t, p.theta, p.nterms, p.theta <= kFixTheta);
+  ws.fix = nullptr;
+  if (p.theta <= kFixTheta && p.nterms >= 2) {
+    if (ws.cell_arena.fixed()) {
+      ws.fix = reinterpret_cast<long long *>(t.coef);
+    } else {
+      const size_t entries = 2 * (size_t)t.ncell * p.nterms;
+      const cudaError_t e = ws.fix_arena.reserve(Arena::bytes_for(entries, 8));
+      if (e != cudaSuccess) return e;
+      ws.fix_arena.reset();
+      ws.fix = ws.fix_arena.take<long long>(entries);
+    }
+  }
+  chained(k_mac_bounds, (t.ncell + 63) / 64, 64, 0, s)(t, p.theta, p.nterms, reinterpret_cast<longlong2 *>(ws.fix));
   ::t2d::g_launches.fetch_add(1, std::memory_order_relaxed);
   const cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) ws.mac_ready = true;
@@ -581,8 +594,9 @@ int plain_evaluate(Workspace &ws, const Tree &t, int ntgt, const double *tx, con
   if (ntgt <= 0) return TREE2D_OK;
   const Params &p = t.params;
   T2D_CUDA_TRY(mac_bounds(ws, t, s));
-  EvalArgs a{t, p.nterms, p.theta, ntgt, tx, ty, out_idx, uv, ws.status, fix::first_pair_term(p.theta),
-             reinterpret_cast<const void *>(t.fix) != reinterpret_cast<const void *>(t.coef), fix::One()};
+  EvalArgs a{t, p.nterms, p.theta, ntgt, tx, ty, out_idx, uv, ws.status, reinterpret_cast<const longlong2 *>(ws.fix),
+             fix::first_pair_term(p.theta),
+             reinterpret_cast<const void *>(ws.fix) != reinterpret_cast<const void *>(t.coef), fix::One()};
   const int share = eval_share(t.n, p.num_p);
   const int warps = (int)(((long)ntgt * share + 31) / 32);
   const int blocks = (warps + kEvalWarps - 1) / kEvalWarps;
