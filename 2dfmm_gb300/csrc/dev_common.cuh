@@ -66,6 +66,17 @@ __device__ __forceinline__ double2 shfl_d2(double2 v, int src) {
   return make_double2(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));
 }
 
+// 1/x for a positive normal x: the SFU's approximate reciprocal refined by
+// two Newton-Raphson steps for f(y) = 1/y - x, y <- y + y (1 - x y), each
+// with the residual 1 - x y formed by one FMA.
+__device__ __forceinline__ double rcp_nr(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  y = fma(y, fma(-x, y, 1.0), y);
+  return y;
+}
+
 // Tests on a double's bits: FP64 comparisons run at 1/64 of the integer rate.
 __device__ __forceinline__ bool finite_bits(double v) {
   return (__double2hiint(v) & 0x7ff00000) != 0x7ff00000;

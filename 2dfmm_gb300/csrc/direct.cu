@@ -14,17 +14,6 @@ namespace {
 constexpr int kThreads = 256;
 constexpr double kPi = 3.14159265358979323846;
 
-// 1/x for a positive normal x: the SFU's approximate reciprocal refined by
-// two Newton-Raphson steps y <- y + y (1 - x y) (each squares the relative
-// error), ending within an ulp or so of the correctly rounded quotient.
-__device__ __forceinline__ double rcp_nr(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = fma(y, fma(-x, y, 1.0), y);
-  y = fma(y, fma(-x, y, 1.0), y);
-  return y;
-}
-
 __device__ const fix::ExpTables g_exp = fix::make_exp_tables();
 
 // A source as the pairs need it: |G| and 1/sigma^2 as mantissas and exponent

@@ -25,17 +25,6 @@
 namespace t2d {
 namespace {
 
-// 1/x for a positive normal x: the SFU's approximate reciprocal refined by
-// two Newton-Raphson steps for f(y) = 1/y - x, y <- y + y (1 - x y), each
-// with the residual 1 - x y formed by one FMA.
-__device__ __forceinline__ double rcp_nr(double x) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  y = fma(y, fma(-x, y, 1.0), y);
-  y = fma(y, fma(-x, y, 1.0), y);
-  return y;
-}
-
 // a b + c for complex values as FMAs only: Re = a.x b.x + (c.x - a.y b.y),
 // Im = a.x b.y + (c.y + a.y b.x), each inner term one FMA and each outer one
 // another (explicit, so the rounding does not depend on how the compiler
