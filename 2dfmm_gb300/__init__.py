@@ -202,8 +202,8 @@ def set_mixed_params(pterms: int = 16, cutoff_sigmas: float = 2.5, use_tensor_co
 
 
 def set_mixed_leaf(max_blobs: int = -1):
-    """Most blobs per leaf of the mixed forms' tree: -1 by set size (64 /
-    96 / 128 from 512K / 2M blobs), 0 the parameters' num_p - 1, > 0 fixed."""
+    """Most blobs per leaf of the mixed forms' tree: -1 by set size (96, 128
+    from 2M blobs), 0 the parameters' num_p - 1, > 0 fixed."""
     _check(load().tree2d_set_mixed_leaf(max_blobs), "set_mixed_leaf")
 
 

@@ -141,8 +141,9 @@ __device__ __forceinline__ RootBox root_from_box(const Box4 &r) {
   return b;
 }
 
-// One warp: the lanes reduce strided parts, then a shuffle reduction.
-// The root box from the blocks' extremes: one block of kRootThreads.
+// The root box from the blocks' extremes: one block of kRootThreads, each
+// thread a strided part, then the warps by shuffles and their results by the
+// first thread.
 constexpr int kRootThreads = 256;
 __global__ void __launch_bounds__(kRootThreads) k_root(const Box4 *part, int nparts, RootBox *root) {
   chain_wait();
@@ -823,8 +824,8 @@ __global__ void __launch_bounds__(256) k_leaf_order(const uint32_t *__restrict__
   }
 }
 
-// Blob arrays in tree order, plus 1/sigma^2 for the direct pairs; a
-// non-finite circulation or a NaN core radius is bad input.
+// Blob arrays in tree order; a non-finite circulation or a NaN core radius is
+// bad input.
 __global__ void __launch_bounds__(256) k_gather(const double *__restrict__ xy, const double *__restrict__ cir,
                                                 const double *__restrict__ cor, const int *__restrict__ perm, int n,
                                                 double *x, double *y, double *c, double *r, DevStatus *st) {

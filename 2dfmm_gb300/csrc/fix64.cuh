@@ -5,8 +5,10 @@
 // chains, 8 warps per sub-partition).  The plain treecode's two inner terms,
 // the multipole sum and the regularised pair, are therefore formed in 64-bit
 // fixed point with explicit exponents: about 58 significant bits through
-// every step (FP64 has 53).  FP64 stays for the two coordinate differences,
-// which are exact for close pairs, and for the sums.
+// every step (FP64 has 53), and their sums held in 96.  FP64 stays for the two
+// coordinate differences, which are exact for close pairs, and for what the
+// fixed units would not hold as well: cells whose leading coefficients cancel
+// or leave FP64's normal range, targets far outside the blobs.
 //
 // A mantissa "with its leading one at bit b" lies in [2^b, 2^(b+1)); biased
 // exponents are a double's exponent field.  mulhi() leaves out the product of
@@ -63,9 +65,6 @@ T2D_HD int clz(uint64_t v) {
   return v ? __builtin_clzll(v) : 64;
 #endif
 }
-// a b and a b + c with 32-bit factors and a 64-bit result, unsigned and
-// signed: one instruction each on the device (left to itself the compiler
-// may widen the factors first and multiply 64 by 64 bits).
 T2D_HD int clz32(uint32_t v) {
 #ifdef __CUDA_ARCH__
   return __clz((int)v);
@@ -73,6 +72,9 @@ T2D_HD int clz32(uint32_t v) {
   return v ? __builtin_clz(v) : 32;
 #endif
 }
+// a b and a b + c with 32-bit factors and a 64-bit result, unsigned and
+// signed: one instruction each on the device (left to itself the compiler
+// may widen the factors first and multiply 64 by 64 bits).
 T2D_HD uint64_t wide(uint32_t a, uint32_t b) {
 #ifdef __CUDA_ARCH__
   uint64_t r;

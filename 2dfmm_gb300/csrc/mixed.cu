@@ -2591,7 +2591,7 @@ cudaError_t launch_eval(int v, const MixedView &m, double *uv, const int *perm, 
 
 // The near field with the variant the tuner chose for this size class: on
 // the first solve of a (device, form, P, leaf-count octave) class every
-// variant runs twice, in the order 0 1 2 3 3 2 1 0 (so that clocks still
+// variant runs twice, in the order 0 1 2 3 4 4 3 2 1 0 (so that clocks still
 // ramping up favour no variant), timed by CUDA events on the stream, and the
 // one with the fastest run is kept (each run writes the same velocities, so
 // the last one stands).

@@ -193,16 +193,16 @@ struct EvalArgs {
 enum EvalForm { kFormFp64, kFormFull, kFormHalf };
 
 // Bound: instruction dispatch.  Integer instructions take two dispatch cycles
-// each (ALU and multiplier pipes alike; FP32 one), and on GB300 the kernel
-// spends, at 1M Lamb-Oseen blobs, 2.4 ms in the traversal, 8.0 ms in the 250
-// M2S and 8.8 ms (some of it overlapped) in the 500 pairs per target: 18.2 ms
-// against 67.5 with both in FP64, whose pipe was 89% busy; 0.30 against
-// 0.90 ms at 20,000 uniform blobs.  Four lanes per target, not one: 8
-// targets' traversals overlap more than 32 targets', the four children of a
-// cell are tested at once, a leaf's pairs need no queue, and a small set
-// fills four times the warps (20,000 blobs: 1.43 -> 1.07 ms per solve).
-// 80 registers, 24 warps per SM: 64 registers spill (24.0 against 21.4 ms
-// per solve), 2 or 8 warps per block are slower (23.6, 22.2).
+// each (ALU and multiplier pipes alike; FP32 one): 15.0 ms for the 9.4 G of
+// them at 1M Lamb-Oseen blobs (2.4 ms' worth in the traversal, 8 in the 250
+// M2S, 9 in the 500 pairs per target), of 18.35 ms, against 67.5 with both sums
+// in FP64, whose pipe was 89% busy; 0.27 against 0.90 ms at 20,000 uniform
+// blobs.  Four lanes per target at least, not one: 8 targets' traversals
+// overlap more than 32 targets', the four children of a cell are tested at
+// once, a leaf's pairs need no queue, and a small set fills more warps (20,000
+// blobs, one lane against four: 1.43 -> 1.07 ms per solve; eval_share has 8 and
+// 16).  80 registers, 24 warps per SM: 64 registers spill (24.0 against 21.4
+// ms per solve), 2 or 8 warps per block are slower (23.6, 22.2).
 template <int kForm, int kShare>
 __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
   chain_wait();
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kEvalWarps * 32, 6) k_eval(EvalArgs a) {
     top--;
     const bool act = (m >> lane) & 1u;
     if (t.leaf[c]) {
-      // direct_evaluate, fmm.c:121-142: the leaf's blobs dealt to the four
+      // direct_evaluate, fmm.c:121-142: the leaf's blobs dealt to the kShare
       // lanes of each target that opened it
       const int b = t.begin[c], e = t.end[c];
       if (act) {
@@ -563,8 +563,11 @@ int plain_upward(Workspace &ws, const Tree &t, cudaStream_t s) {
 //   32,768   531 / 507 / 589   620 / 558 / 607  1136 / 953 / 943   2258 / 1844 / 1644
 //   65,536   963 / 985 / 1169 1122 / 1092 / 1233 2346 / 2032 / 2043 3971 / 3333 / 3205
 //  131,072  1797 / 1938 / -   2070 / 2138 / -   3608 / 3423 / 3690 6871 / 6301 / 6465
-// By the tree, not the targets' number: a point's sums do not depend on how
-// many points are asked for.
+// The lines lie where the sums of a row change hands, to within 3% (65,536
+// blobs with num_p 33 take eight lanes although four are 2% ahead), and hold
+// for other distributions as far as their targets' work is alike.  By the tree,
+// not the targets' number: a point's sums do not depend on how many points are
+// asked for.
 int eval_share(int n, int num_p) {
   if (n <= 8192 || (n <= 65536 && n <= 200l * num_p)) return 16;
   if (n <= 65536 || (n <= 131072 && n <= 1024l * num_p)) return 8;

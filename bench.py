@@ -335,14 +335,22 @@ def _roofline(P, args, mode, b, wname, sts, sp):
     st = sts[-1]
     ms = statistics.mean(s["ms_eval"] for s in sts)
     tr = roofline_traffic().get(f"{mode}:{wname}")
-    if mode == "plain":
+    if mode == "plain" and b.theta <= 0.7:
+        # 64-bit fixed point: the integer pipes' dispatch bounds it, for which
+        # there is no probe; the rate is that of the FP64 method
         flops = st["n_m2s"] * (8 * p + 10) + st["n_pairs"] * 20
+        return {"bound": "integer dispatch", "achieved": flops / (ms * 1e-3) / 1e12, "peak": None,
+                "unit": "TFLOP/s (operations of the method in FP64)", "frac": None, "traffic": tr,
+                "kernel": "k_eval (traversal + M2S + P2P, in 64-bit fixed point)", "peak_source": None,
+                "algorithmic_flops_per_launch": flops, "ms_per_launch": ms}
+    if mode == "plain":
+        # larger opening angles: the multipole sums, and only they, in FP64
+        flops = st["n_m2s"] * (8 * p + 10)
         peak = P.fp64_peak_tflops(stream=sp)
         return {"bound": "fp64", "achieved": flops / (ms * 1e-3) / 1e12, "peak": peak, "unit": "TFLOP/s",
                 "frac": flops / (ms * 1e-3) / 1e12 / peak, "traffic": tr,
-                "kernel": "k_eval (traversal + M2S + P2P, in 64-bit fixed point)",
-                "peak_source": "measured: the library's DFMA probe (8 independent chains per thread); "
-                               "the fixed-point sums run above it",
+                "kernel": "k_eval (traversal + M2S in FP64 + P2P in 64-bit fixed point)",
+                "peak_source": "measured: the library's DFMA probe (8 independent chains per thread)",
                 "algorithmic_flops_per_launch": flops, "ms_per_launch": ms}
     # mixed and learned: the evaluation kernel (direct pairs, correction
     # pairs, L2P, M2P)
@@ -350,7 +358,7 @@ def _roofline(P, args, mode, b, wname, sts, sp):
     peak = P.fp32_peak_tflops(stream=sp)
     return {"bound": "fp32", "achieved": flops / (ms * 1e-3) / 1e12, "peak": peak, "unit": "TFLOP/s",
             "frac": flops / (ms * 1e-3) / 1e12 / peak, "traffic": tr,
-            "kernel": "k_eval_mixed (P2P + correction pairs + L2P/M2P, FP32)",
+            "kernel": "k_eval_near (P2P + correction pairs + L2P/M2P, FP32)",
             "peak_source": "measured: the library's FFMA probe (8 independent chains per thread)",
             "algorithmic_flops_per_launch": flops, "ms_per_launch": ms}
 
@@ -653,7 +661,7 @@ def run_batch(args):
                     "d2h_bytes_per_step": n * 16, "api": "host->device copies + tree2d_solve_sets + device->host"},
             "roofline": {"bound": "fp32", "achieved": flops / (ms_eval * 1e-3) / 1e12, "peak": peak,
                          "unit": "TFLOP/s", "frac": flops / (ms_eval * 1e-3) / 1e12 / peak, "traffic": None,
-                         "kernel": "k_eval_mixed (P2P + correction pairs + L2P/M2P, FP32)",
+                         "kernel": "k_eval_near (P2P + correction pairs + L2P/M2P, FP32)",
                          "peak_source": "measured: the library's FFMA probe"},
             "accuracy": {"sets": len(sets), "targets_per_set": args.set_targets,
                          "relL2_max_over_sets": max(rels), "relL2_median": float(np.median(rels)),

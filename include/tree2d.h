@@ -66,7 +66,7 @@ void biot_tree(double x, double y, double *u, double *v);
 #define TREE2D_ERR_FILE 11         /* a file could not be read or has the wrong format */
 
 /* Evaluation modes (tree2d_set_mode). */
-#define TREE2D_MODE_PLAIN 0        /* FP64 treecode, reference semantics             */
+#define TREE2D_MODE_PLAIN 0        /* treecode to FP64 accuracy, reference semantics */
 #define TREE2D_MODE_MIXED 1        /* scaled FP32 FMM, tensor-core M2L, FP64 final sum */
 #define TREE2D_MODE_LEARNED 2      /* MIXED with learned per-interaction order         */
 
@@ -106,7 +106,8 @@ int tree2d_set_mixed_leaf(int max_blobs);
  * host memory) against the last make_tree.  Blob positions are answered
  * from the precomputed velocities, the rest in one GPU launch.  The points
  * are matched on the GPU (target i against blob i, bit for bit; page-locked
- * xy and uv let the copies overlap), the others through a host table.
+ * xy and uv let the copies overlap), the others through a table of the blobs
+ * by position, there too.
  * Returns a status; on error uv is filled with NaN. */
 int biot_tree_batch(int n, const double *xy, double *uv);
 
