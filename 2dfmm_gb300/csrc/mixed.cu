@@ -2536,7 +2536,8 @@ int mixed_downward(MixedView &m, int depth, const int *lev_off, cudaStream_t s, 
 // from global memory with 4/8 warps per block, 2/3 stage them in shared
 // memory by bulk copies with 4/8 warps per block, 4 stages them with 4
 // warps per block of up to 80 registers per thread (6 blocks per SM) and
-// the pair loops unrolled four times.  The staged ones are within 2% of one
+// the pair loops unrolled four times, or reads global memory so where leaves
+// can be larger than a stage buffer.  The staged ones are within 2% of one
 // another at 1M Lamb-Oseen blobs, 4M two-patch + sheet blobs and the 512 sets.
 constexpr int kEvalVariants = kEvalVariantCount;
 
@@ -2575,14 +2576,23 @@ cudaError_t launch_near(const MixedView &m, double *uv, const int *perm, Decisio
 
 template <bool kLearned, bool kScaled>
 cudaError_t launch_eval(int v, const MixedView &m, double *uv, const int *perm, Decisions d, cudaStream_t s) {
-  static int resident[kEvalVariants] = {};  // per variant (the devices here are all one model)
+  static int resident[kEvalVariants + 1] = {};  // per kernel (the devices here are all one model)
   cudaError_t e = cudaSuccess;
   switch (v) {
     case 0: e = launch_near<kLearned, kScaled, false, 4>(m, uv, perm, d, s, &resident[0]); break;
     case 1: e = launch_near<kLearned, kScaled, false, 8>(m, uv, perm, d, s, &resident[1]); break;
     case 2: e = launch_near<kLearned, kScaled, true, 4>(m, uv, perm, d, s, &resident[2]); break;
     case 3: e = launch_near<kLearned, kScaled, true, 8>(m, uv, perm, d, s, &resident[3]); break;
-    default: e = launch_near<kLearned, kScaled, true, 4, true>(m, uv, perm, d, s, &resident[4]); break;
+    default:
+      // Leaves beyond a stage buffer: the same kernel reading them from global
+      // memory, as the staged one does without unrolling (near field, ms, at
+      // 20,000 / 100,000 / 262,144 / 1M uniform blobs in leaves of up to 400 /
+      // 400 / 300 / 300: staged 1.23, 1.80, 1.04, 1.62; global with 64 registers
+      // 1.13, 1.70, 0.99, 1.44; so 0.65, 0.97, 0.60, 1.21).
+      if (m.kchunks * kChunk <= kStage)
+        e = launch_near<kLearned, kScaled, true, 4, true>(m, uv, perm, d, s, &resident[4]);
+      else
+        e = launch_near<kLearned, kScaled, false, 4, true>(m, uv, perm, d, s, &resident[5]);
   }
   if (e != cudaSuccess) return e;
   g_launches.fetch_add(1, std::memory_order_relaxed);

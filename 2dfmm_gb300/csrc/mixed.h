@@ -44,7 +44,7 @@ struct MixedView {
                          // Morton order, tree order inside one), not in the tree's order
   float4 *cbox;          // per leaf cell, kchunks entries: bounding box {xmin, ymin, xmax, ymax}
                          // of each kChunk-blob chunk of the leaf (from its first blob), leaf-local
-  int kchunks;           // chunk boxes per cell: ceil(most blobs per leaf / 32)
+  int kchunks;           // chunk boxes per cell: ceil(most blobs per leaf / kChunk)
   float *cxf, *cyf;      // per cell, FP32 centre (rounded)
   float *cxl, *cyl;      // per cell, the rest: centre - (double)cxf, in FP32
   int *coll, *coarse;    // 9 per cell
